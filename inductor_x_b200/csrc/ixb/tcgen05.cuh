@@ -76,6 +76,72 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// ---- one 128 x 128 x 128 product, issued by a whole converged warp -----------------------
+// Every lane runs the issuing loop and one elected lane executes the instructions: the
+// operands then stay warp-uniform.  In a loop that a single lane runs (`if (lane == 0)`) the
+// compiler has to move each operand of each MMA from a per-lane register first, which costs
+// issue slots that the arithmetic warps beside it win.
+// D = A B^T, both operands K-major tiles (two boxes of 64 columns, `kBox` bytes apart): 8 steps
+// of 16 along the reduced axis, 32 bytes a step inside the 128-byte swizzled row.
+template <int kBox>
+__device__ __forceinline__ void product_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e, f, t;\n\t"
+      ".reg .b64 a1, a2, a3, a4, a5, a6, a7, b1, b2, b3, b4, b5, b6, b7;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 f, 0, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a1, %1, 2;\n\tadd.s64 b1, %2, 2;\n\t"
+      "add.s64 a2, %1, 4;\n\tadd.s64 b2, %2, 4;\n\t"
+      "add.s64 a3, %1, 6;\n\tadd.s64 b3, %2, 6;\n\t"
+      "add.s64 a4, %1, %4;\n\tadd.s64 b4, %2, %4;\n\t"
+      "add.s64 a5, a4, 2;\n\tadd.s64 b5, b4, 2;\n\t"
+      "add.s64 a6, a4, 4;\n\tadd.s64 b6, b4, 4;\n\t"
+      "add.s64 a7, a4, 6;\n\tadd.s64 b7, b4, 6;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, f;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a4, b4, %3, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a5, b5, %3, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a6, b6, %3, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a7, b7, %3, t;\n\t"
+      "}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(kBox >> 4)
+      : "memory");
+}
+// D (+)= A B over N steps of 16 of the reduced index: A in TMEM as 16-bit pairs (8 columns a
+// step), B a tile in MN-major form (16 rows = 2048 bytes a step)
+template <int N> __device__ __forceinline__ void product_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                            uint32_t idesc, uint32_t accumulate) {
+  static_assert(N == 2 || N == 4 || N == 6 || N == 8, "whole pairs of steps");
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e, f, t;\n\t"
+      ".reg .b32 a;\n\t"
+      ".reg .b64 b;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 f, %4, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 a, %1, 8;\n\tadd.s64 b, %2, 128;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, f;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      "}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+  if constexpr (N > 2) product_ts<N - 2>(d_tmem, a_tmem + 16, b_desc + 256, idesc, 1u);
+}
+// mma_commit by the elected lane of a converged warp (the one that issued the products)
+__device__ __forceinline__ void commit_elected(uint64_t* bar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}" ::"r"(smem_u32(bar))
+      : "memory");
+}
 // The mbarrier gets one arrival when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -123,6 +189,46 @@ __device__ __forceinline__ void tmem_wait_ld() {
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// ---- register split between warpgroups (whole warpgroup) -------------------------------
+template <int N> __device__ __forceinline__ void regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N> __device__ __forceinline__ void regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
+// ---- work of blocks that have not started yet (one thread) -----------------------------------
+// Asks for the index of a block of this grid that the hardware has not launched; the answer
+// (16 bytes) lands in shared memory and completes 16 bytes on `bar`.  A running block that
+// takes over a pending one keeps its tensor memory, barriers and pipelines.
+__device__ __forceinline__ void request_next_block(void* answer, uint64_t* bar) {
+  mbar_arrive_expect_tx(bar, 16);
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+          smem_u32(answer)),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+// blockIdx.x of the block taken over, or -1 when none was left
+__device__ __forceinline__ int next_block(const void* answer) {
+  int taken, x = 0;
+  asm volatile(
+      "{\n\t"
+      ".reg .b128 h;\n\t"
+      ".reg .pred p;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.s32 %0, 1, 0, p;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t"
+      "}"
+      : "=r"(taken), "+r"(x)
+      : "r"(smem_u32(answer))
+      : "memory");
+  // the copy engine may write the next answer over this one once the reader says so
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  return taken ? x : -1;
 }
 
 // ---- tiled TMA load, rank 4, this CTA only --------------------------------------------
