@@ -23,13 +23,17 @@
 // here - lse and delta come in precomputed - so the split costs nothing).  Every wait is
 // bounded; a wait that gives up raises a flag in `status` and lets the CTA drain and exit.
 //
-// Measured on B200 (4096 keys, causal): per 128 x 128 tile pair the tensor core needs about
-// 2050 cycles for the four products (one 128x128x16 MMA per 64 cycles, SS or TS form, one or
-// two issuing threads alike) and the element-wise warps about 2300 (the exponentials alone
-// fill the ex2 unit for 1024); with one tile in flight the two add up (4330 cycles per tile
-// pair).  A variant with 64-query sub-tiles, double-buffered score columns and a four-stage
-// ring overlapped them but ran 30 % slower: an SS-form MMA with N = 64 takes 48 cycles, not 32
-// (both operands come from shared memory at 128 bytes per cycle), and the hand-offs double.
+// Bound: the tensor core, at the rate the power limit leaves it.  Measured at 8 x 32 heads, 4096
+// keys, causal, bf16: delta 0.11 ms, dK/dV 2.12 ms, dQ 1.51 ms in a short run; with the
+// element-wise warps only passing the barriers on, the products of the two kernels alone take
+// 1.64 and 1.43 ms, without the exponentials 2.07 and 1.50.  The products are issued by a whole
+// warp through an elected lane (4426 us a call before, one lane issuing; 4200 after, both in a
+// run long enough to sit at the power limit).  Two ways to overlap more were built and dropped:
+// dS in tensor-memory columns of its own, so that the next scores never wait for the product
+// behind them (dQ 1.51 -> 1.83 ms), and P^T as a shared-memory operand, which frees the score
+// columns earlier but reads another 32 KB of shared memory a step (dK/dV 2.12 -> 2.36 ms).  A
+// variant with 64-query sub-tiles and double-buffered score columns ran 30 % slower: an SS-form
+// MMA with N = 64 takes 48 cycles, not 32, and the hand-offs double.
 #include <atomic>
 #include "fa_maps.h"
 #include "ixb/tcgen05.cuh"
@@ -134,13 +138,10 @@ __device__ __forceinline__ void load_tile(unsigned char* dst, const CUtensorMap*
   tc::tma_load_4d(dst + kHalfBytes, map, bar, 64, row0, h, b);
 }
 
+// The products are issued by a whole warp through an elected lane (see tc::product_ss).
 // D = A B^T, both operands K-major tiles of 128 x 128 (8 steps of 16 along the head dimension)
 __device__ __forceinline__ void issue_ss(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-#pragma unroll
-  for (int ks = 0; ks < HD / 16; ++ks) {
-    const uint32_t off = ((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4;
-    tc::mma_ss(d, a_desc + off, b_desc + off, idesc, ks > 0);
-  }
+  tc::product_ss<kHalfBytes>(d, a_desc, b_desc, idesc);
 }
 // D (+)= A B with A in TMEM as 16-bit pairs (group g wrote its GC values of the reduced index
 // as GC / 2 columns starting at column a + GC * g) and B a tile in MN-major form (16 rows =
@@ -148,11 +149,8 @@ __device__ __forceinline__ void issue_ss(uint32_t d, uint64_t a_desc, uint64_t b
 __device__ __forceinline__ void issue_ts(uint32_t d, uint32_t a, uint64_t b_desc_mn, uint32_t idesc,
                                          bool accumulate) {
 #pragma unroll
-  for (int ks = 0; ks < 128 / 16; ++ks) {
-    constexpr int kStepsPerGroup = GC / 16;
-    const uint32_t col = a + (ks / kStepsPerGroup) * GC + (ks % kStepsPerGroup) * 8;
-    tc::mma_ts(d, col, b_desc_mn + (uint32_t)(ks * 2048 >> 4), idesc, (accumulate || ks > 0) ? 1u : 0u);
-  }
+  for (int g = 0; g < NG; ++g)
+    tc::product_ts<GC / 16>(d, a + g * GC, b_desc_mn + (uint32_t)(g * GC * 128 >> 4), idesc, (accumulate || g > 0) ? 1u : 0u);
 }
 
 // GC accumulator columns of this thread's row -> 16-bit values in global memory
@@ -198,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0);  // known uniform to the compiler
   const int lane = threadIdx.x & 31;
 
   const int n_kv_tiles = (p.Sk + BN - 1) / BN;
@@ -273,59 +271,55 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0) {
       constexpr uint32_t idesc_kk = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 0);
       constexpr uint32_t idesc_mn = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 1);
       const uint64_t k_desc = tc::smem_desc(smem_u32(k_smem), 16, 1024);
       const uint64_t v_desc = tc::smem_desc(smem_u32(v_smem), 16, 1024);
-      uint64_t q_desc[kStages], do_desc[kStages], q_desc_mn[kStages], do_desc_mn[kStages];
-#pragma unroll
-      for (int s = 0; s < kStages; ++s) {
-        const uint32_t qa = smem_u32(q_smem + (size_t)s * kTileBytes);
-        const uint32_t da = smem_u32(do_smem + (size_t)s * kTileBytes);
-        q_desc[s] = tc::smem_desc(qa, 16, 1024);
-        do_desc[s] = tc::smem_desc(da, 16, 1024);
-        q_desc_mn[s] = tc::smem_desc(qa, kHalfBytes, 1024);
-        do_desc_mn[s] = tc::smem_desc(da, kHalfBytes, 1024);
-      }
-      const uint32_t t_s = tmem_base + kColS, t_dp = tmem_base + kColDP;
-      const uint32_t t_dv = tmem_base + kColAcc0, t_dk = tmem_base + kColAcc1;
-      bool ok = mbar_wait(&kv_full, 0, &failed);
-      ok = ok && mbar_wait(&qdo_full[0], 0, &failed);
+      const uint64_t q_desc = tc::smem_desc(smem_u32(q_smem), 16, 1024);
+      const uint64_t do_desc = tc::smem_desc(smem_u32(do_smem), 16, 1024);
+      const uint64_t q_desc_mn = tc::smem_desc(smem_u32(q_smem), kHalfBytes, 1024);
+      const uint64_t do_desc_mn = tc::smem_desc(smem_u32(do_smem), kHalfBytes, 1024);
+      constexpr uint32_t kStep = kTileBytes >> 4;  // one stage further, in descriptor units
+      const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
+      const uint32_t t_s = tmem + kColS, t_dp = tmem + kColDP;
+      const uint32_t t_dv = tmem + kColAcc0, t_dk = tmem + kColAcc1;
+      bool ok = __all_sync(kFull, mbar_wait(&kv_full, 0, &failed));
+      ok = ok && __all_sync(kFull, mbar_wait(&qdo_full[0], 0, &failed));
       if (ok) {
         tc::fence_after_sync();
-        issue_ss(t_s, k_desc, q_desc[0], idesc_kk);  // S^T = K Q^T
-        tc::mma_commit(&s_full);
-        issue_ss(t_dp, v_desc, do_desc[0], idesc_kk);  // dP^T = V dO^T
-        tc::mma_commit(&dp_full);
+        issue_ss(t_s, k_desc, q_desc, idesc_kk);  // S^T = K Q^T
+        tc::commit_elected(&s_full);
+        issue_ss(t_dp, v_desc, do_desc, idesc_kk);  // dP^T = V dO^T
+        tc::commit_elected(&dp_full);
       }
       for (int it = 0; it < n_it && ok; ++it) {
         const int s = it & 1, s1 = (it + 1) & 1;
         const bool next = it + 1 < n_it;
-        ok = mbar_wait(&p_full, it & 1, &failed);
+        ok = __all_sync(kFull, mbar_wait(&p_full, it & 1, &failed));
         if (!ok) break;
         tc::fence_after_sync();
-        issue_ts(t_dv, t_s, (s ? do_desc_mn[1] : do_desc_mn[0]), idesc_mn, it > 0);  // dV += P^T dO
+        issue_ts(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, it > 0);  // dV += P^T dO
         if (next) {
-          ok = mbar_wait(&qdo_full[s1], ((it + 1) >> 1) & 1, &failed);
+          ok = __all_sync(kFull, mbar_wait(&qdo_full[s1], ((it + 1) >> 1) & 1, &failed));
           if (!ok) break;
           tc::fence_after_sync();
           // the tensor core runs its MMAs in order: P^T has been consumed when this one starts
-          issue_ss(t_s, k_desc, (s1 ? q_desc[1] : q_desc[0]), idesc_kk);
-          tc::mma_commit(&s_full);
+          issue_ss(t_s, k_desc, q_desc + s1 * kStep, idesc_kk);
+          tc::commit_elected(&s_full);
         }
-        ok = mbar_wait(&ds_full, it & 1, &failed);
+        ok = __all_sync(kFull, mbar_wait(&ds_full, it & 1, &failed));
         if (!ok) break;
         tc::fence_after_sync();
-        issue_ts(t_dk, t_dp, (s ? q_desc_mn[1] : q_desc_mn[0]), idesc_mn, it > 0);  // dK += dS^T Q
-        tc::mma_commit(&qdo_empty[s]);
+        issue_ts(t_dk, t_dp, q_desc_mn + s * kStep, idesc_mn, it > 0);  // dK += dS^T Q
+        tc::commit_elected(&qdo_empty[s]);
         if (next) {
-          issue_ss(t_dp, v_desc, (s1 ? do_desc[1] : do_desc[0]), idesc_kk);
-          tc::mma_commit(&dp_full);
+          issue_ss(t_dp, v_desc, do_desc + s1 * kStep, idesc_kk);
+          tc::commit_elected(&dp_full);
         }
       }
-      if (ok) tc::mma_commit(&acc_done);
-      if (!ok) failed = 1;
+      if (ok) tc::commit_elected(&acc_done);
+      if (!ok && lane == 0) failed = 1;
     }
     __syncwarp();
   } else {
@@ -479,7 +473,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0);  // known uniform to the compiler
   const int lane = threadIdx.x & 31;
 
   const int n_q_tiles = (p.Sq + BM - 1) / BM;
@@ -541,59 +535,56 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_kk = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 0);
       constexpr uint32_t idesc_mn = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 1);
       const uint64_t q_desc = tc::smem_desc(smem_u32(q_smem), 16, 1024);
       const uint64_t do_desc = tc::smem_desc(smem_u32(do_smem), 16, 1024);
-      uint64_t k_desc[kStages], v_desc[kStages], k_desc_mn[kStages];
-#pragma unroll
-      for (int s = 0; s < kStages; ++s) {
-        const uint32_t ka = smem_u32(k_smem + (size_t)s * kTileBytes);
-        k_desc[s] = tc::smem_desc(ka, 16, 1024);
-        k_desc_mn[s] = tc::smem_desc(ka, kHalfBytes, 1024);
-        v_desc[s] = tc::smem_desc(smem_u32(v_smem + (size_t)s * kTileBytes), 16, 1024);
-      }
-      const uint32_t t_s = tmem_base + kColS, t_dp = tmem_base + kColDP, t_dq = tmem_base + kColAcc0;
-      bool ok = mbar_wait(&qdo_full, 0, &failed);
-      ok = ok && mbar_wait(&k_full[0], 0, &failed);
-      ok = ok && mbar_wait(&v_full[0], 0, &failed);
+      const uint64_t k_desc = tc::smem_desc(smem_u32(k_smem), 16, 1024);
+      const uint64_t v_desc = tc::smem_desc(smem_u32(v_smem), 16, 1024);
+      const uint64_t k_desc_mn = tc::smem_desc(smem_u32(k_smem), kHalfBytes, 1024);
+      constexpr uint32_t kStep = kTileBytes >> 4;  // one stage further, in descriptor units
+      const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
+      const uint32_t t_s = tmem + kColS, t_dp = tmem + kColDP, t_dq = tmem + kColAcc0;
+      bool ok = __all_sync(kFull, mbar_wait(&qdo_full, 0, &failed));
+      ok = ok && __all_sync(kFull, mbar_wait(&k_full[0], 0, &failed));
+      ok = ok && __all_sync(kFull, mbar_wait(&v_full[0], 0, &failed));
       if (ok) {
         tc::fence_after_sync();
-        issue_ss(t_s, q_desc, k_desc[0], idesc_kk);  // S = Q K^T
-        tc::mma_commit(&s_full);
-        issue_ss(t_dp, do_desc, v_desc[0], idesc_kk);  // dP = dO V^T
-        tc::mma_commit(&dp_full);
-        tc::mma_commit(&v_empty[0]);
+        issue_ss(t_s, q_desc, k_desc, idesc_kk);  // S = Q K^T
+        tc::commit_elected(&s_full);
+        issue_ss(t_dp, do_desc, v_desc, idesc_kk);  // dP = dO V^T
+        tc::commit_elected(&dp_full);
+        tc::commit_elected(&v_empty[0]);
       }
       for (int j = 0; j < n_kv && ok; ++j) {
         const int s = j & 1, s1 = (j + 1) & 1, n1 = (j + 1) >> 1;
         const bool next = j + 1 < n_kv;
         if (next) {
           // S(j) is in registers of the element-wise warps: its columns can take S(j+1)
-          ok = mbar_wait(&s_read, j & 1, &failed);
-          ok = ok && mbar_wait(&k_full[s1], n1 & 1, &failed);
+          ok = __all_sync(kFull, mbar_wait(&s_read, j & 1, &failed));
+          ok = ok && __all_sync(kFull, mbar_wait(&k_full[s1], n1 & 1, &failed));
           if (!ok) break;
           tc::fence_after_sync();
-          issue_ss(t_s, q_desc, (s1 ? k_desc[1] : k_desc[0]), idesc_kk);
-          tc::mma_commit(&s_full);
+          issue_ss(t_s, q_desc, k_desc + s1 * kStep, idesc_kk);
+          tc::commit_elected(&s_full);
         }
-        ok = mbar_wait(&ds_full, j & 1, &failed);
+        ok = __all_sync(kFull, mbar_wait(&ds_full, j & 1, &failed));
         if (!ok) break;
         tc::fence_after_sync();
-        issue_ts(t_dq, t_dp, (s ? k_desc_mn[1] : k_desc_mn[0]), idesc_mn, j > 0);  // dQ += dS K
-        tc::mma_commit(&k_empty[s]);
+        issue_ts(t_dq, t_dp, k_desc_mn + s * kStep, idesc_mn, j > 0);  // dQ += dS K
+        tc::commit_elected(&k_empty[s]);
         if (next) {
-          ok = mbar_wait(&v_full[s1], n1 & 1, &failed);
+          ok = __all_sync(kFull, mbar_wait(&v_full[s1], n1 & 1, &failed));
           if (!ok) break;
           tc::fence_after_sync();
-          issue_ss(t_dp, do_desc, (s1 ? v_desc[1] : v_desc[0]), idesc_kk);  // after dQ(j): dS(j) has been consumed
-          tc::mma_commit(&dp_full);
-          tc::mma_commit(&v_empty[s1]);
+          issue_ss(t_dp, do_desc, v_desc + s1 * kStep, idesc_kk);  // after dQ(j): dS(j) has been consumed
+          tc::commit_elected(&dp_full);
+          tc::commit_elected(&v_empty[s1]);
         }
       }
-      if (ok) tc::mma_commit(&acc_done);
-      if (!ok) failed = 1;
+      if (ok) tc::commit_elected(&acc_done);
+      if (!ok && lane == 0) failed = 1;
     }
     __syncwarp();
   } else {
