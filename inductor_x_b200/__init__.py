@@ -24,7 +24,10 @@ from . import ops  # noqa: F401
 
 
 def get_current_raw_stream(device=None) -> int:
-    """Raw handle of the current CUDA stream (``inductor_x/__init__.py:26-27``)."""
+    """Raw handle of the current CUDA stream (``inductor_x/__init__.py:26-27``).  Wrapper code asks
+    once per call with the device's index: the handle itself then, without a Stream object (2 us)."""
+    if type(device) is int and device >= 0:
+        return torch._C._cuda_getCurrentRawStream(device)
     return torch.cuda.current_stream(device).cuda_stream
 
 

@@ -31,6 +31,15 @@ _lock = threading.Lock()
 _loaded: dict = {}
 
 
+def _native_launcher():
+    """``_ixb_host.Launcher`` (``csrc/host_launch.cpp``); raises if the extension is not built."""
+    try:
+        from .. import _ixb_host
+    except ImportError as e:
+        raise ImportError(f"{e}: build the launch extension with `make -C {_CSRC}` (or __graft_entry__.build())") from e
+    return _ixb_host.Launcher
+
+
 class GeneratedKernel:
     """Callable handle of one compiled functor module."""
 
@@ -39,14 +48,21 @@ class GeneratedKernel:
         self.path = path
         self.meta = dict(meta)
         self.src = src
-        self.launches = 0
+        self._launches = 0           # those of the general route
         self.shape = None            # launch shape in use, once a measurement picked one
         self.tuning = None           # [(shape, us)] of the last measurement
-        self._bind(path)
+        # what wrapper code calls: native, falling back to the general route below for whatever
+        # is not a plain launch; it reads the configuration's switches on every call
+        self.run = _native_launcher()(self._run_general, vars(config))
         tune = self.meta.get("tune")
         self._tune_pending = bool(
             tune and tune.get("candidates") and tune.get("idempotent") and config.autotune
             and tune.get("rows", 0) * tune.get("row_bytes", 0) >= config.autotune_min_bytes)
+        self._bind(path)
+
+    @property
+    def launches(self) -> int:
+        return self._launches + self.run.launches
 
     def _bind(self, path: str) -> None:
         self.lib = ctypes.CDLL(path)
@@ -55,8 +71,15 @@ class GeneratedKernel:
         self.fn.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_longlong),
                             ctypes.c_void_p]
         self.path = path
+        self._arm()
 
-    def run(self, *args, stream=None):
+    def _arm(self) -> None:
+        """Plain launches go straight to the module; a pending measurement and the bounds report
+        of debug builds need the general route on every call."""
+        direct = not self._tune_pending and not self.meta.get("bounds")
+        self.run.bind(ctypes.cast(self.fn, ctypes.c_void_p).value if direct else 0)
+
+    def _run_general(self, *args, stream=None):
         ptrs, ints, keep = [], [], []
         for a in args:
             if isinstance(a, torch.Tensor):
@@ -81,10 +104,11 @@ class GeneratedKernel:
         if self._tune_pending and not torch.cuda.is_current_stream_capturing():
             self._tune_pending = False
             self._autotune(pa, ia, stream)
+            self._arm()
         if config.profile_bandwidth:
             return self._run_profiled(pa, ia, stream, args)
         rc = self.fn(pa, ia, stream)
-        self.launches += 1
+        self._launches += 1
         if rc != 0:
             hint = (" (a run-time reduced extent beyond the capacity the module was compiled for?)"
                     if rc == 1 and self.meta.get("family") == "row" else "")

@@ -191,9 +191,12 @@ def index_select_rows(table: torch.Tensor, idx: torch.Tensor, *, wrap_negative: 
     return out
 
 
+_I64x3 = ctypes.c_int64 * 3
+
+
 def _bhs_strides(t: torch.Tensor):
-    arr = (ctypes.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
-    return arr
+    b, h, s, _ = t.stride()
+    return _I64x3(b, h, s)
 
 
 def fused_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float, *,

@@ -157,6 +157,9 @@ def check(fn: str, status: int) -> None:
 def raw_stream(device=None) -> int:
     """Handle of the current CUDA stream of ``device`` (the reference's
     ``get_current_raw_stream``, ``inductor_x/__init__.py:26-27``)."""
+    index = getattr(device, "index", None)
+    if index is not None:      # a tensor's device: the handle itself, without a Stream object around it
+        return torch._C._cuda_getCurrentRawStream(index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
