@@ -510,6 +510,9 @@ class B200Kernel(SIMDKernel):
             if x_contig:
                 al = self._fast_flag(exp, self._outer_vec)
                 outer_text = f"{G}ldvec<{ctype}, kVec, {al}>(({var}) + {G}lane0({idx}), nvalid)"
+        elif not indirect and not masked and has_r:
+            # the same for every kept position (a per-row statistic): one load a reduced step
+            outer_text = f"{G}ld_uniform({var}, {G}lane0({idx}), nvalid > 0, {other})"
         tag = self._placeholder("L", (name, idx, str(self._load_mask), other), row_text, outer_text,
                                 stride=stride, has_r=has_r, x_contig=x_contig, indirect=indirect, exp=exp,
                                 in_reduction=self.inside_reduction)
@@ -958,16 +961,21 @@ class B200Kernel(SIMDKernel):
     # ------------------------------------------------------------------ mapping choice
     def _choose_outer(self, body_text: str) -> bool:
         """Outer mapping iff the group is one ordinary reduction whose reduced axis is not
-        stride-1 in any load, at least one load is contiguous along the kept axis, nothing
-        r-dependent is stored, and nothing computed inside the reduction loop is used after
-        it except the reduction result."""
+        stride-1 in any load that depends on the kept axis, at least one load is contiguous
+        along the kept axis, nothing r-dependent is stored, and nothing computed inside the
+        reduction loop is used after it except the reduction result.  A load that does not
+        depend on the kept axis (the per-row statistic in a weight gradient, sum over the
+        tokens of ``dy * x * rstd[token]``) is stride-1 along the reduced axis without being a
+        row operand: it is one scalar a step.  Taken as a row, the group read its other operands
+        one element per 8 KB (32768 tokens x 4096 columns bf16: 1.0 ms against 0.09 ms here)."""
         import re
 
         reds = [v for v in self._ph.values() if v["kind"] == "R"]
         if len(reds) != 1 or not reds[0].get("outer_ok"):
             return False
         loads = [v for v in self._ph.values() if v["kind"] == "L" and v["has_r"]]
-        if not loads or any(v["indirect"] or v["stride"] in (None, 1) for v in loads):
+        xsym = self._root("x").symbol()
+        if not loads or any(v["indirect"] or (v["stride"] in (None, 1) and xsym in v["exp"].free_symbols) for v in loads):
             return False
         if not any(v["x_contig"] for v in loads):
             return False
