@@ -496,11 +496,12 @@ class B200Kernel(SIMDKernel):
                     self._row_prefetch.append(row_ptr)     # streamed once per row: worth prefetching
                 aligned = index_ir.row_starts_aligned(exp, xr.symbol(), rr.symbol(), cfg.vec) and \
                     not self._is_dynamic("r0_") and self._numel_hint("r0_") % cfg.vec == 0
-                if narrow_ok and aligned and not self.looped:
-                    member = next((m for m, _, ptr in self.staged if ptr == row_ptr), None)
+                if narrow_ok and not self.looped:
+                    member = next((m for m, _, ptr, _ in self.staged if ptr == row_ptr), None)
                     if member is None and len(self.staged) < MAX_STAGED:
                         member = f"raw.s{len(self.staged)}"
-                        self.staged.append((member, ctype, row_ptr))
+                        # rows that may start off a 16-byte boundary are staged as covering words
+                        self.staged.append((member, ctype, row_ptr, "RawRow" if aligned else "RawRowU"))
                     if member is not None:
                         row_text = f"c.template operand<STAGED, {ctype}>({member}, {row_ptr})"
         outer_text = gather.replace("@M@", "xmask")
@@ -569,11 +570,12 @@ class B200Kernel(SIMDKernel):
                 row_ptr = f"({var}) + ({G}lane0({idx}) - {G}lane0(r0_index))"
                 row_text = f"c.store_row({row_ptr}, {value});"
                 cfg = self._row_cfg
-                if not self.looped and index_ir.row_starts_aligned(exp, xr.symbol(), rr.symbol(), cfg.vec) and \
-                        not self._is_dynamic("r0_") and self._numel_hint("r0_") % cfg.vec == 0 and \
-                        dtype in FLOAT_DTYPES and \
+                if not self.looped and dtype in FLOAT_DTYPES and \
                         config_bytes(dtype) >= config_bytes(self._narrowest_node_dtype()):
-                    row_text = f"c.template put_row<STAGED>({row_ptr}, {value});"
+                    aligned = index_ir.row_starts_aligned(exp, xr.symbol(), rr.symbol(), cfg.vec) and \
+                        not self._is_dynamic("r0_") and self._numel_hint("r0_") % cfg.vec == 0
+                    put = "c.template put_row<STAGED>" if aligned else "c.put_row_any"
+                    row_text = f"{put}({row_ptr}, {value});"
         outer_text = f"{G}scatter({var}, {idx}, ixb::gen::op::logical_and(xmask, c.writer()), {value});"
         if not indirect and not has_r and self._outer_x_contiguous(exp):
             outer_text = (f"{G}stvec<{ctype}, kVec>(({var}) + {G}lane0({idx}), c.writer() ? nvalid : 0, "
@@ -1287,8 +1289,8 @@ class B200Kernel(SIMDKernel):
                 src.writeline("};")
                 src.writeline("struct Raw {")
                 with src.indent():
-                    for member, ctype, _ in self.staged:
-                        src.writeline(f"{G}RawRow<{ctype}, IXB_ROW_VPT, {cfg.vec}> {member[4:]};")
+                    for member, ctype, _, raw in self.staged:
+                        src.writeline(f"{G}{raw}<{ctype}, IXB_ROW_VPT, {cfg.vec}> {member[4:]};")
                 src.writeline("};")
                 # operands that are the same for every row: once per thread
                 src.writeline("template <class Ctx>")
@@ -1311,7 +1313,7 @@ class B200Kernel(SIMDKernel):
                         src.writeline("const auto r0_index = c.rindex();")
                         src.splice(x_idx)
                         src.splice(r_idx)
-                        for member, _, ptr in self.staged:
+                        for member, _, ptr, _ in self.staged:
                             src.writeline(f"c.fetch_row({ptr}, {member});")
                 src.writeline("}")
                 src.writeline("template <bool STAGED, class Ctx>")
@@ -1432,11 +1434,11 @@ class B200Kernel(SIMDKernel):
                 rt = {torch.float32: "float", torch.bfloat16: "ixb::bf16", torch.float16: "ixb::f16"}.get(
                     narrow, f"ixb::Lanes<{cfg.vec}>")
                 nptr = len([a for a in assigns if 'ptrs[' in a])
-                # FULL: the row fills every vector of the team, no ragged tail to test for
-                full = "false" if dyn_r or self.looped else f"IXB_ROW_TEAM * IXB_ROW_VPT * {cfg.vec} == {rnumel}"
-                src.writeline(f"constexpr bool kFull = {full};")
+                # a row length known here lets the template leave out the tests of vectors that lie
+                # inside the row in every thread
+                src.writeline(f"constexpr int kCols = {0 if dyn_r or self.looped else rnumel};")
                 src.writeline(f"return {G}launch_row_gen<Body, {rt}, IXB_ROW_TEAM, IXB_ROW_TEAMS, IXB_ROW_VPT, "
-                              f"IXB_GEN_MIN_CTAS, IXB_ROW_PF, kFull>(b, xnumel, {rnumel}, stream, "
+                              f"IXB_GEN_MIN_CTAS, IXB_ROW_PF, kCols>(b, xnumel, {rnumel}, stream, "
                               f"{G}pointers_aligned(ptrs, {nptr}));")
             else:
                 launcher = "launch_pointwise_tile" if self._register_tile(self._transposing_order()) else "launch_pointwise"

@@ -54,6 +54,7 @@ def narrowest_dtype(dtypes: Iterable[torch.dtype]) -> torch.dtype:
 
 MAX_TEAM = 1024
 MIN_TEAM = 8          # teams narrower than a warp serve rows of a few vectors
+MAX_EXACT_VPT = 5    # vectors per thread up to which a row may be cut to fit its length
 MAX_VPT = 32         # beyond 8 the row no longer fits the register file and spills: slow but correct
 MAX_PERSISTENT_VPT = 8   # static rows longer than MAX_TEAM x this many vectors are walked in chunks
 
@@ -84,8 +85,16 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
         vpt *= 2
     while vpt > 1 and team * (vpt // 2) >= nvec:   # short rows: no idle vectors
         vpt //= 2
+    if MIN_TEAM * 4 <= team <= MAX_TEAM and vpt <= MAX_EXACT_VPT:
+        # rows of no power-of-two number of vectors: of this team, half and a quarter of it, the
+        # one that leaves the fewest vectors idle (softmax -> LayerNorm, 5000 x 5003 bf16: 512
+        # threads x 2 vectors 85 us, 256 x 3 62 us, 128 x 5 48 us; 60000 x 331 fp32: 64 x 2 95 us,
+        # 32 x 3 52 us); lengths that are a power of two of vectors keep their shape
+        team = min((t for t in (team, team // 2, team // 4) if t >= 32 and -(-nvec // t) <= MAX_EXACT_VPT),
+                   key=lambda t: t * -(-nvec // t), default=team)
+        vpt = -(-nvec // team)
     teams = max(1, 128 // team)
-    min_ctas = max(1, 1024 // (team * teams))
+    min_ctas = max(1, (1024 if vpt <= 2 else 512) // (team * teams))
     row_bytes = rnumel * config.byte_per_numel(dtype) if dtype in config.BYTES_PER_ELEMENT else rnumel * 4
     streamed = rows is None or rows * row_bytes >= (64 << 20)
     return RowConfig(team=team, teams=teams, vpt=vpt, vec=vec, min_ctas=min_ctas,
@@ -125,12 +134,10 @@ def row_candidates(rnumel: int, chosen: RowConfig, rows: Optional[int] = None, n
                 out.append(shape)
         return out
     ranked = []
-    for vpt in (1, 2, 4):
-        team = 32
-        while team < MAX_TEAM and team * vpt < nvec:
-            team *= 2
-        if team * vpt < nvec or (vpt > 1 and team * (vpt // 2) >= nvec):
-            continue                      # does not cover the row / leaves idle vectors
+    for team in (32, 64, 128, 256, 512, 1024):
+        vpt = -(-nvec // team)
+        if vpt > MAX_EXACT_VPT or (vpt == 1 and nvec <= team // 2 and team > 32):
+            continue                      # too thick / half the team idle
         for teams in sorted({max(1, 128 // team), max(1, 256 // team), max(1, 384 // team)}):
             threads = team * teams
             if threads > 1024:

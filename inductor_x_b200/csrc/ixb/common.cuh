@@ -117,6 +117,52 @@ template <> __device__ __forceinline__ uint4 pack<f16>(const float* in) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// ---- 128-bit access to data that starts off a 16-byte boundary ------------------------
+// 128 bits starting `s` elements into the 256 bits (lo, hi), 0 <= s < elements of a word: what
+// an unaligned 128-bit access is made of
+template <class U> __device__ __forceinline__ uint4 shift_words(const uint4& lo, const uint4& hi, int s) {
+  static_assert(sizeof(U) == 2 || sizeof(U) == 4, "16- and 32-bit elements");
+  const int words = sizeof(U) == 4 ? s : s >> 1;
+  const uint32_t x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  uint32_t y[7], z[5];
+#pragma unroll
+  for (int k = 0; k < 7; ++k) y[k] = (words & 1) ? x[k + 1] : x[k];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) z[k] = (words & 2) ? y[k + 2] : y[k];
+  if constexpr (sizeof(U) == 4) return make_uint4(z[0], z[1], z[2], z[3]);
+  const int bits = (s & 1) * 16;
+  return make_uint4(__funnelshift_r(z[0], z[1], bits), __funnelshift_r(z[1], z[2], bits),
+                    __funnelshift_r(z[2], z[3], bits), __funnelshift_r(z[3], z[4], bits));
+}
+// elements between the 16-byte boundary at or before p, and p
+template <class U> __device__ __forceinline__ int off_boundary(const U* p) {
+  return (int)(reinterpret_cast<uintptr_t>(p) & 15u) / (int)sizeof(U);
+}
+
+  // the first n elements of a word, zeros behind them
+template <class U> __device__ __forceinline__ uint4 keep_elements(const uint4& v, int n) {
+  uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  constexpr int kPerWord = 4 / (int)sizeof(U);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int left = n - k * kPerWord;
+    w[k] = left >= kPerWord ? w[k] : (kPerWord == 2 && left == 1 ? w[k] & 0xffffu : 0u);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// elements [first, end) of a word
+  template <class U> __device__ __forceinline__ void put_elements(U* p, const uint4& v, int first, int end) {
+    constexpr int kPer = 16 / (int)sizeof(U);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      if (e >= first && e < end) {
+        if constexpr (sizeof(U) == 4) reinterpret_cast<uint32_t*>(p)[e] = w[e];
+        else reinterpret_cast<unsigned short*>(p)[e] = (unsigned short)((e & 1) ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
+      }
+    }
+  }
+
 // ---------------------------------------------------------------------------------
 // Reduction operators.  `combine` must be associative and commutative.
 // ---------------------------------------------------------------------------------

@@ -164,7 +164,9 @@ __device__ __forceinline__ void scatter_add(T* p, const I& idx, const M& mask, c
   }
 }
 
-// contiguous run of N elements starting at p: 128-bit accesses when the address allows.
+// contiguous run of N elements starting at p: 128-bit accesses when the address allows.  A
+// complete run that starts off a 16-byte boundary is cut out of the aligned words that cover it
+// (each of them holds at least one element of the run, so nothing beyond its 16 bytes is read).
 // FAST: the caller knows the run is complete and 16-byte aligned (full tile, aligned base
 // pointer checked on the host, index proven a multiple of the vector), so the access is
 // unconditional - no branch separates the loads of an unrolled loop and they overlap.
@@ -180,6 +182,18 @@ __device__ __forceinline__ typename vec_of<typename Mem<T>::val, N>::type ldvec(
       for (int c = 0; c < N / kPer; ++c) {
         if constexpr (STREAM) unpack<T>(ldg_stream(p + c * kPer), &r.v[c * kPer]);
         else unpack<T>(ldg_keep(p + c * kPer), &r.v[c * kPer]);  // may be re-read: keep in L1
+      }
+      return r;
+    }
+    if (nvalid >= N && !STREAM) {
+      const int s = off_boundary(p);
+      const T* a = p - s;
+      uint4 lo = ldg_keep(a);
+#pragma unroll
+      for (int c = 0; c < N / kPer; ++c) {
+        const uint4 hi = ldg_keep(a + (c + 1) * kPer);
+        unpack<T>(shift_words<T>(lo, hi, s), &r.v[c * kPer]);
+        lo = hi;
       }
       return r;
     }
@@ -404,8 +418,10 @@ template <class Body> int launch_pointwise(const Body& body, long long xnumel, v
 // ---- persistent row family ---------------------------------------------------------------
 // The generated body sees a context that maps vector element e = i * kVec + j of this
 // thread to column vec_col(i) + j of the row, exactly as RowCtx does for the prebuilt bodies.
-// FULL: the row fills every vector of the team exactly (length == TEAM * VPT * kVec), so no
-// element needs a validity test.
+// COLS is the row length when it is known at compile time (0: at run time, or walked in chunks).
+// Vectors that every thread of the team has inside the row - all of them when the length is
+// TEAM * VPT * kVec (FULL), all but the last one or two of an odd length - then need no validity
+// test and fold in packed pairs; without it every element of an odd row paid one per fold.
 //
 // A generated row body has four parts:
 //   Consts / init(c, k)            operands that do not change from row to row (per-column
@@ -421,6 +437,14 @@ template <class U, int VPT, int KVEC> struct RawRow {
   static constexpr int kChunks = KVEC * (int)sizeof(U) / 16;  // 128-bit words per vector
   static_assert(kChunks >= 1, "staged operands are at least as wide as the row's vector type");
   uint4 q[VPT][kChunks];
+};
+
+// the same for rows that may start anywhere: the aligned words that cover the thread's vectors,
+// one more than the vectors themselves fill
+template <class U, int VPT, int KVEC> struct RawRowU {
+  static constexpr int kChunks = KVEC * (int)sizeof(U) / 16;
+  static_assert(kChunks >= 1, "staged operands are at least as wide as the row's vector type");
+  uint4 q[VPT][kChunks + 1];
 };
 
 // exact 64-bit integer reduction operators
@@ -475,10 +499,14 @@ template <class Op> __device__ __forceinline__ float warp_all(float v) {
   else return warp_reduce<Op>(v);
 }
 
-template <typename T, int TEAM, int TEAMS, int VPT, bool FULL = false>
+template <typename T, int TEAM, int TEAMS, int VPT, int COLS = 0>
 struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   using Base = RowCtx<T, TEAM, TEAMS, VPT, false>;
   static constexpr int kE = VPT * Base::kVec;
+  static constexpr bool FULL = COLS == TEAM * VPT * Base::kVec;
+  // vector i of every thread lies inside the row
+  static __device__ __forceinline__ constexpr bool full(int i) { return COLS >= (i + 1) * TEAM * Base::kVec; }
+  __device__ __forceinline__ int ncols() const { return COLS > 0 ? COLS : this->cols; }
   static constexpr int kGroup = TEAM < 32 ? TEAM : 32;  // lanes of one warp that share a row
   static constexpr int kW = Base::kWarpsPerTeam;        // warps per team (0 for sub-warp teams)
   static constexpr int kChains = (kE / 2) >= 4 ? 4 : ((kE / 2) >= 2 ? 2 : 1);  // accumulator chains
@@ -533,7 +561,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   __device__ __forceinline__ bool leader() const { return this->lane == 0 && live; }
   // element j of vector i lies inside the row
   __device__ __forceinline__ bool inside(int i, int j) const {
-    return FULL ? true : (this->vec_col(i) + j < this->cols);
+    return full(i) || this->vec_col(i) + j < ncols();
   }
   __device__ __forceinline__ vi<kE> rindex() const {
     vi<kE> r;
@@ -558,7 +586,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int c0 = this->vec_col(i);
-      const int left = FULL ? Base::kVec : this->cols - c0;
+      const int left = full(i) ? Base::kVec : ncols() - c0;
       auto part = ldvec<U, Base::kVec>(rowp + c0, left > 0 ? left : 0);
 #pragma unroll
       for (int j = 0; j < Base::kVec; ++j) r.v[i * Base::kVec + j] = part.v[j];
@@ -574,7 +602,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       const int c0 = this->vec_col(i);
 #pragma unroll
       for (int k = 0; k < kC; ++k)
-        raw.q[i][k] = (FULL || c0 < this->cols) ? ldg_stream(reinterpret_cast<const uint4*>(rowp + c0) + k)
+        raw.q[i][k] = (full(i) || c0 < ncols()) ? ldg_stream(reinterpret_cast<const uint4*>(rowp + c0) + k)
                                                : make_uint4(0, 0, 0, 0);
     }
   }
@@ -587,6 +615,89 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
       for (int k = 0; k < kC; ++k) unpack<U>(raw.q[i][k], &r.v[i * Base::kVec + k * kPer]);
     return r;
+  }
+  // Rows that start off a 16-byte boundary (an odd row length moves every row): the words that
+  // cover a thread's vectors are fetched aligned - the one it shares with the next lane comes
+  // out of L1 - and shifted into place when the row is worked on.  Only words that hold an
+  // element of the row are read.  Element-wise loads of such rows touch every line eight times
+  // and cannot be requested a row ahead: softmax -> LayerNorm of 20011 x 1537 fp16 took 103 us
+  // with them, 90 us this way, 73 us with the length known at compile time (COLS), 59 us in the
+  // launch shape that measures best (six teams of 64 threads with four vectors each).
+  template <class U> __device__ __forceinline__ void fetch_row(const U* rowp, RawRowU<U, VPT, Base::kVec>& raw) const {
+    constexpr int kC = RawRowU<U, VPT, Base::kVec>::kChunks;
+    constexpr int kPer = 16 / (int)sizeof(U);
+    const int off = off_boundary(rowp);     // whole vectors lie between the row start and any other vector
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int c0 = this->vec_col(i) - off;   // column of the first element of the first word
+#pragma unroll
+      for (int k = 0; k <= kC; ++k) {
+        const bool need = (full(i) || (c0 + off < ncols() && c0 + k * kPer < ncols())) && (k < kC || off > 0);
+        raw.q[i][k] = need ? ldg_keep(rowp + (c0 + k * kPer)) : make_uint4(0, 0, 0, 0);
+      }
+    }
+  }
+  template <class U> __device__ __forceinline__ vf<kE> widen(const RawRowU<U, VPT, Base::kVec>& raw, const U* rowp) const {
+    constexpr int kC = RawRowU<U, VPT, Base::kVec>::kChunks;
+    constexpr int kPer = 16 / (int)sizeof(U);
+    const int off = off_boundary(rowp);
+    vf<kE> r;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+#pragma unroll
+      for (int k = 0; k < kC; ++k)
+        unpack<U>(shift_words<U>(raw.q[i][k], raw.q[i][k + 1], off), &r.v[i * Base::kVec + k * kPer]);
+      if (!full(i) && this->vec_col(i) + Base::kVec > ncols()) {     // what follows the row is not its business
+#pragma unroll
+        for (int j = 0; j < Base::kVec; ++j)
+          if (!inside(i, j)) r.v[i * Base::kVec + j] = 0.f;
+      }
+    }
+    return r;
+  }
+  template <bool STAGED, class U>
+  __device__ __forceinline__ vf<kE> operand(const RawRowU<U, VPT, Base::kVec>& raw, const U* rowp) const {
+    if constexpr (STAGED) return widen<U>(raw, rowp);
+    else return load_row(rowp);
+  }
+  // Store to such a row: a lane owns the aligned word that ends in its vector, i.e. the last
+  // elements of the vector before it (from the lane before it) and the first of its own.  The
+  // ends of a warp's run and of the row are written element by element.
+  template <class U, class A> __device__ __forceinline__ void put_row_any(U* rowp, const A& val) const {
+    if constexpr (std::is_same<typename Mem<U>::val, float>::value && (sizeof(U) == 2 || sizeof(U) == 4) &&
+                  std::is_same<A, vf<kE>>::value) {
+      constexpr int kPer = 16 / (int)sizeof(U);
+      constexpr int kC = Base::kVec / kPer;
+      const int off = off_boundary(rowp);
+      const int wl = this->lane & (kGroup - 1);
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        uint4 w[kC + 1];       // the vector's words behind the last word of the lane before
+#pragma unroll
+        for (int k = 0; k < kC; ++k) w[k + 1] = pack<U>(&val.v[i * Base::kVec + k * kPer]);
+        w[0].x = __shfl_up_sync(kFull, w[kC].x, 1, kGroup);
+        w[0].y = __shfl_up_sync(kFull, w[kC].y, 1, kGroup);
+        w[0].z = __shfl_up_sync(kFull, w[kC].z, 1, kGroup);
+        w[0].w = __shfl_up_sync(kFull, w[kC].w, 1, kGroup);
+        if (!live) continue;
+#pragma unroll
+        for (int k = 0; k < kC; ++k) {
+          const int col = this->vec_col(i) + k * kPer - off;
+          const uint4 v = off == 0 ? w[k + 1] : shift_words<U>(w[k], w[k + 1], kPer - off);
+          const int first = (k > 0 || wl > 0) ? 0 : off;
+          if (first == 0 && (full(i) || col + kPer <= ncols())) stg_stream(rowp + col, v);
+          else put_elements(rowp + col, v, first, ncols() - col);
+        }
+        // the last lane of a run has nobody behind it to write the end of its vector
+        if (off > 0 && wl == kGroup - 1) {
+          const int col = this->vec_col(i) + Base::kVec - off;
+          const int left = ncols() - col;
+          put_elements(rowp + col, shift_words<U>(w[kC], w[kC], kPer - off), 0, left < off ? left : off);
+        }
+      }
+    } else {
+      store_row(rowp, val);
+    }
   }
   // a streamed operand inside row(): from the fetched vectors, or loaded on the spot
   template <bool STAGED, class U>
@@ -611,7 +722,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int c0 = this->vec_col(i);
-      const int left = FULL ? Base::kVec : this->cols - c0;
+      const int left = full(i) ? Base::kVec : ncols() - c0;
       typename vec_of<V, Base::kVec>::type part;
 #pragma unroll
       for (int j = 0; j < Base::kVec; ++j) part.v[j] = Cast<V>::from(at(val, i * Base::kVec + j));
@@ -627,7 +738,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
         const int c0 = this->vec_col(i);
-        if (FULL || c0 < this->cols) {
+        if (full(i) || c0 < ncols()) {
 #pragma unroll
           for (int k = 0; k < Base::kVec / kPer; ++k)
             stg_stream(rowp + c0 + k * kPer, pack<U>(&val.v[i * Base::kVec + k * kPer]));
@@ -788,6 +899,23 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   }
 
   // ---- thread-local folds -------------------------------------------------------------------
+  // sum of pairs of elements (pair p = elements 2p, 2p + 1) in independent chains of packed adds;
+  // only the vectors that may reach past the end of the row are tested
+  template <class F> __device__ __forceinline__ float fold_pairs(const F& pair) const {
+    float2 acc[kChains];
+#pragma unroll
+    for (int c = 0; c < kChains; ++c) acc[c] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < kE / 2; ++p) {
+      float2 v = pair(p);
+      if (!inside((2 * p) / Base::kVec, (2 * p) % Base::kVec)) v.x = 0.f;
+      if (!inside((2 * p + 1) / Base::kVec, (2 * p + 1) % Base::kVec)) v.y = 0.f;
+      acc[p % kChains] = add2(acc[p % kChains], v);
+    }
+#pragma unroll
+    for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
+    return acc[0].x + acc[0].y;
+  }
   template <class A> __device__ __forceinline__ float local_sum(const A& val) const {
     if constexpr (FULL && op::is_fvec<A>::value) {
       // kChains independent chains of packed adds: a single chain would serialise on the
@@ -800,6 +928,8 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
       for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
       return acc[0].x + acc[0].y;
+    } else if constexpr (COLS > 0 && op::is_fvec<A>::value) {
+      return fold_pairs([&](int p) { return op::pr(val, p); });
     } else {
       float acc = 0.f;
 #pragma unroll
@@ -821,6 +951,8 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
       for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
       return acc[0].x + acc[0].y;
+    } else if constexpr (COLS > 0 && op::packable2<A, B>::value) {
+      return fold_pairs([&](int p) { return mul2(op::pr(a, p), op::pr(b, p)); });
     } else {
       float acc = 0.f;
 #pragma unroll
@@ -1238,10 +1370,10 @@ template <class K> inline int row_resident(K kern, int threads, size_t smem = 0)
   return n;
 }
 
-template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS, int PF, bool FULL, bool STAGED>
+template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS, int PF, int COLS, bool STAGED>
 __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     row_gen_kernel(const Body body, const long long rows, const int cols) {
-  using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, FULL>;
+  using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS>;
   constexpr int kSlots = TEAM > 32 ? 2 * (TEAM / 32) * 4 : 1;  // exchange floats per team
   __shared__ __align__(16) float exchange[TEAMS * kSlots];
   extern __shared__ __align__(16) unsigned char operand_table[];   // Body::kSmemConsts slots
@@ -1309,10 +1441,10 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     }
   }
 }
-template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS = 1, int PF = 0, bool FULL = false>
+template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS = 1, int PF = 0, int COLS = 0>
 int launch_row_gen(const Body& body, long long rows, int cols, void* stream, bool aligned = false) {
   if (rows <= 0) return 0;
-  if (FULL && cols != TEAM * VPT * Elem<T>::kVec) return (int)cudaErrorInvalidValue;
+  if (COLS > 0 && cols != COLS) return (int)cudaErrorInvalidValue;
   // a row longer than the team can hold (a run-time extent beyond the compiled capacity);
   // looped bodies walk any length in chunks
   if (cols < 0 || (!Body::kLooped && cols > TEAM * VPT * Elem<T>::kVec)) return (int)cudaErrorInvalidValue;
@@ -1320,17 +1452,17 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long groups = (rows + TEAMS - 1) / TEAMS;
-  using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, FULL>;
+  using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS>;
   const size_t smem = (size_t)Body::kSmemConsts * Ctx::kQuads * Ctx::kTabVecs * sizeof(float4);
   if (aligned) {
-    auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, FULL, true>;
+    auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, COLS, true>;
     const int resident = row_resident(kern, TEAM * TEAMS, smem);
     if (resident < 1) return (int)cudaErrorInvalidConfiguration;
     long long grid = (long long)sms * resident;
     if (grid > groups) grid = groups;
     return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
   }
-  auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, FULL, false>;
+  auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, COLS, false>;
   const int resident = row_resident(kern, TEAM * TEAMS, smem);
   if (resident < 1) return (int)cudaErrorInvalidConfiguration;
   long long grid = (long long)sms * resident;

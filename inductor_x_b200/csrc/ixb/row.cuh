@@ -56,24 +56,43 @@ template <typename T, int TEAM, int TEAMS, int VPT, bool ALIGNED> struct RowCtx 
       if (!valid(i)) return make_uint4(0, 0, 0, 0);
       return STREAM ? ldg_stream(base + vec_col(i)) : ldg_keep(base + vec_col(i));
     } else {
-      union {
-        uint4 u;
-        T e[kVec];
-      } v;
-      v.u = make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < kVec; ++j)
-        if (vec_col(i) + j < cols) v.e[j] = base[vec_col(i) + j];
-      return v.u;
+      uint4 words[2];
+      fetch(base, i, words);
+      return settle(base, i, words);
     }
   }
+  // Rows that start off a 16-byte boundary: the two aligned words that cover vector i (only
+  // those that hold an element of the row are read) ...
+  __device__ __forceinline__ void fetch(const T* base, int i, uint4 (&words)[2]) const {
+    const int off = off_boundary(base), c0 = vec_col(i) - off;
+    words[0] = valid(i) ? ldg_keep(base + c0) : make_uint4(0, 0, 0, 0);
+    words[1] = valid(i) && off > 0 && c0 + kVec < cols ? ldg_keep(base + c0 + kVec) : make_uint4(0, 0, 0, 0);
+  }
+  // ... and the vector cut out of them, zero past the end of the row
+  __device__ __forceinline__ uint4 settle(const T* base, int i, const uint4 (&words)[2]) const {
+    const uint4 v = shift_words<T>(words[0], words[1], off_boundary(base));
+    return vec_col(i) + kVec <= cols ? v : keep_elements<T>(v, cols - vec_col(i));
+  }
+  // Every lane of the warp calls this together.  Off a boundary a lane writes the aligned word
+  // that ends in its vector: the last elements of the lane before it and the first of its own;
+  // the ends of the warp's run and of the row go element by element.
   __device__ __forceinline__ void store(T* base, int i, const float* vals) const {
     if constexpr (ALIGNED) {
       if (valid(i)) stg_stream(base + vec_col(i), pack<T>(vals));
     } else {
-#pragma unroll
-      for (int j = 0; j < kVec; ++j)
-        if (vec_col(i) + j < cols) base[vec_col(i) + j] = Elem<T>::from_f(vals[j]);
+      const int off = off_boundary(base), wl = lane & 31;
+      const uint4 own = pack<T>(vals);
+      const uint4 prev = make_uint4(__shfl_up_sync(kFull, own.x, 1), __shfl_up_sync(kFull, own.y, 1),
+                                    __shfl_up_sync(kFull, own.z, 1), __shfl_up_sync(kFull, own.w, 1));
+      const int col = vec_col(i) - off;
+      const uint4 v = off == 0 ? own : shift_words<T>(prev, own, kVec - off);
+      const int first = wl > 0 ? 0 : off;
+      if (first == 0 && col + kVec <= cols) stg_stream(base + col, v);
+      else put_elements(base + col, v, first, cols - col);
+      if (off > 0 && wl == 31) {
+        const int left = cols - (col + kVec);
+        put_elements(base + col + kVec, shift_words<T>(own, own, kVec - off), 0, left < off ? left : off);
+      }
     }
   }
 
@@ -223,24 +242,37 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
   const long long stride = (long long)gridDim.x * TEAMS;
   long long r = (long long)blockIdx.x * TEAMS + c.team;
 
-  uint4 nxt[NIN][VPT];
+  constexpr int kWords = ALIGNED ? 1 : 2;  // 128-bit words that cover a vector
+  // Two words per vector are requested a row ahead only where registers allow: thicker threads
+  // spill (up to 2 KB a thread at eight vectors) and load their unaligned row on the spot.
+  constexpr bool kAhead = ALIGNED || VPT * NIN <= 2;
+  uint4 nxt[NIN][VPT][kWords];
   auto fetch = [&](long long row) {
 #pragma unroll
     for (int k = 0; k < NIN; ++k) {
       const T* base = Body::row_ptr(p, k) + row * (long long)cols;
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) nxt[k][i] = c.load(base, i);
+      for (int i = 0; i < VPT; ++i) {
+        if constexpr (ALIGNED) nxt[k][i][0] = c.load(base, i);
+        else c.fetch(base, i, nxt[k][i]);
+      }
     }
   };
-  if (r < rows) fetch(r);
+  if (kAhead && r < rows) fetch(r);
   while (r < rows) {
     uint4 cur[NIN][VPT];
 #pragma unroll
-    for (int k = 0; k < NIN; ++k)
+    for (int k = 0; k < NIN; ++k) {
+      const T* base = Body::row_ptr(p, k) + r * (long long)cols;
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) cur[k][i] = nxt[k][i];
+      for (int i = 0; i < VPT; ++i) {
+        if constexpr (ALIGNED) cur[k][i] = nxt[k][i][0];
+        else if constexpr (kAhead) cur[k][i] = c.settle(base, i, nxt[k][i]);
+        else cur[k][i] = c.load(base, i);
+      }
+    }
     const long long rn = r + stride;
-    if (rn < rows) fetch(rn);
+    if (kAhead && rn < rows) fetch(rn);
     body.row(p, c, r, cur);
     r = rn;
   }

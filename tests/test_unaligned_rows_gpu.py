@@ -1,0 +1,77 @@
+"""Rows that start off a 16-byte boundary (odd row lengths, odd offsets and pitches): the staged
+covering words, the shifted stores and their ends.  Against 64-bit arithmetic on the same inputs;
+results are 32-bit sums rounded once, so the bound is a few roundings of the storage type."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from inductor_x_b200 import ops
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
+
+
+def chain(x, g, gamma, beta):
+    return F.layer_norm(torch.softmax(x, -1) * g + x, (x.shape[-1],), gamma, beta, 1e-5)
+
+
+def inputs(cuda, rows, cols, dtype, seed=0):
+    g = torch.Generator(device=cuda).manual_seed(rows + cols + seed)
+    x = torch.randn(rows, cols, generator=g, device=cuda).to(dtype)
+    return [x] + [(1 + 0.1 * torch.randn(cols, generator=g, device=cuda)).to(dtype) for _ in range(3)]
+
+
+def close(got, want, dtype):
+    err = (got.double() - want).abs() / want.abs().clamp_min(float(want.square().mean().sqrt()))
+    assert float(err.max()) <= TOL[dtype]
+
+
+# sub-warp teams with several rows in flight, one warp, several warps, two vectors a thread; a row
+# that ends one element into a vector, one before its end, and in the middle
+@pytest.mark.parametrize("dtype,rows,cols", [(torch.float16, 301, 33), (torch.bfloat16, 64, 71), (torch.float32, 77, 130),
+                                             (torch.bfloat16, 9, 515), (torch.float16, 1500, 1537), (torch.float32, 5, 3001),
+                                             (torch.bfloat16, 1, 9001)])
+def test_compiled_rows_inside_a_larger_buffer(cuda, dtype, rows, cols):
+    import inductor_x_b200  # noqa: F401
+
+    x, g, gamma, beta = inputs(cuda, rows, cols, dtype)
+    torch._dynamo.reset()
+    into = torch.compile(lambda x, g, gamma, beta, out: out.copy_(chain(x, g, gamma, beta)), dynamic=False)
+    buf = torch.full(((rows + 2) * cols,), 7.0, dtype=dtype, device=cuda)
+    into(x, g, gamma, beta, buf[cols:-cols].view(rows, cols))
+    want = chain(*(t.double() for t in (x, g, gamma, beta)))
+    close(buf[cols:-cols].view(rows, cols), want, dtype)
+    assert bool((buf[:cols] == 7).all()) and bool((buf[-cols:] == 7).all())  # nothing beyond the rows is written
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_compiled_rows_of_a_view(cuda, dtype):
+    """An odd pitch and an odd first element; and a base pointer that is not 16-byte aligned, which
+    takes the loads that are not requested ahead."""
+    import inductor_x_b200  # noqa: F401
+
+    x, g, gamma, beta = inputs(cuda, 50, 205, dtype)
+    torch._dynamo.reset()
+    fn = torch.compile(chain, dynamic=False)
+    for view in (x[:, 1:201], x[1:, 3:203]):
+        args = [view] + [t[1:201] for t in (g, gamma, beta)]
+        close(fn(*args), chain(*(t.double() for t in args)), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(3, 1), (7, 33), (200, 515), (2, 9001), (1, 20001)])
+def test_library_rows(cuda, dtype, rows, cols):
+    x, w, res, _ = inputs(cuda, rows, cols, dtype)
+    res = x.flip(0).contiguous()
+    y, h = ops.rmsnorm(x, w, 1e-6, residual=res, return_residual=True)
+    assert torch.equal(h, x + res)
+    hd = h.double()
+    close(y, hd * torch.rsqrt(hd.square().mean(-1, keepdim=True) + 1e-6) * w.double(), dtype)
+    close(ops.row_reduce(x, "sum"), x.double().sum(-1), dtype)
+    assert torch.equal(ops.row_reduce(x, "amax"), x.amax(-1))
+    assert torch.equal(ops.row_reduce(x, "argmin"), x.argmin(-1)) or dtype != torch.float32  # ties in 16 bits
+    if cols > 1:
+        buf = torch.full(((rows + 2) * cols,), 7.0, dtype=dtype, device=cuda)
+        ops.softmax_layernorm(x, w, w, w, 1e-5, out=buf[cols:-cols].view(rows, cols))
+        close(buf[cols:-cols].view(rows, cols), chain(*(t.double() for t in (x, w, w, w))), dtype)
+        assert bool((buf[:cols] == 7).all()) and bool((buf[-cols:] == 7).all())
