@@ -1280,6 +1280,7 @@ class B200Kernel(SIMDKernel):
                     row_body = row_body.replace(self.consts[old][0], f"{G}kget<{new}, IXB_ROW_KREGS>(c, k.k{new})")
                 src.writeline(f"static constexpr int kN = IXB_ROW_VPT * {cfg.vec};   // elements per thread")
                 src.writeline(f"static constexpr bool kLooped = {'true' if self.looped else 'false'};   // row walked in chunks")
+                src.writeline(f"static constexpr bool kTiled = {'true' if tiling is not None else 'false'};   // kept index walked in tiles")
                 src.writeline(f"static constexpr int kConsts = {len(self.consts)};")
                 src.writeline("static constexpr int kSmemConsts = kConsts > IXB_ROW_KREGS ? kConsts - IXB_ROW_KREGS : 0;")
                 src.writeline("struct Consts {")

@@ -1405,17 +1405,24 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     // worked on: kBatch independent loads in flight per thread instead of one.
     constexpr int kBatch = STAGED ? 4 : 1;
     typename Body::Raw raw[kBatch];
-    for (long long base = (long long)blockIdx.x * TEAMS; base < rows; base += stride * kBatch) {
+    // Rows walked in tiles (tile_order), with enough of them to go round: the rows of a batch
+    // follow each other, so that a CTA reads a whole 16 x 16 tile at a time - 2 KB from each of 16
+    // places instead of 512 bytes - and DRAM pages are used up while they are open (sum over the
+    // last axis of a permuted 64 x 128 x 256 x 64 fp16: 54.6 -> 52.4 us).  Rows in memory order
+    // gain nothing from it (43.3 against 44.8 us) and keep the strided batches.
+    const bool blocked = Body::kTiled && rows >= stride * kBatch;
+    const long long ustep = blocked ? TEAMS : stride;
+    for (long long base = (long long)blockIdx.x * TEAMS * (blocked ? kBatch : 1); base < rows; base += stride * kBatch) {
       if constexpr (STAGED) {
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
-          const long long r = base + u * stride + c.team;
+          const long long r = base + u * ustep + c.team;
           body.fetch(c, r < rows ? r : rows - 1, raw[u]);
         }
       }
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const long long b = base + u * stride;
+        const long long b = base + u * ustep;
         if (b >= rows) break;            // uniform over the CTA
         const long long r = b + c.team;
         c.live = r < rows;
