@@ -186,12 +186,14 @@ __device__ __forceinline__ typename vec_of<typename Mem<T>::val, N>::type ldvec(
       return r;
     }
     if (nvalid >= N && !STREAM) {
+      // (plain loads, as the element-wise ones they replace: a later pass of a looped row may read
+      // what an earlier one stored)
       const int s = off_boundary(p);
-      const T* a = p - s;
-      uint4 lo = ldg_keep(a);
+      const uint4* a = reinterpret_cast<const uint4*>(p - s);
+      uint4 lo = a[0];
 #pragma unroll
       for (int c = 0; c < N / kPer; ++c) {
-        const uint4 hi = ldg_keep(a + (c + 1) * kPer);
+        const uint4 hi = a[c + 1];
         unpack<T>(shift_words<T>(lo, hi, s), &r.v[c * kPer]);
         lo = hi;
       }
