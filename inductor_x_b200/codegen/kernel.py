@@ -135,13 +135,15 @@ class B200Kernel(SIMDKernel):
         self.is_row = self.features.is_reduction()
         if self.is_row:
             # a symbolic reduced extent is served up to the capacity of the launch shape chosen
-            # for the extent seen at trace time (the launcher refuses longer rows)
+            # for the extent seen at trace time (the launcher refuses longer rows), so that shape
+            # is not cut to fit the one extent
             rnumel = self._numel_hint("r0_")
             dt = self._narrowest_node_dtype()
             if self.looped:
                 self._row_cfg = split_tiling.choose_loop_config(dt)
             else:
-                self._row_cfg = split_tiling.choose_row_config(rnumel, dt, rows=self._numel_hint("x"))
+                self._row_cfg = split_tiling.choose_row_config(rnumel, dt, rows=self._numel_hint("x"),
+                                                                exact=not self._is_dynamic("r0_"))
                 if self._row_cfg is None and self._reads_are_strided():
                     # an outer reduction of any length: the outer mapping loops over the reduced
                     # axis itself; the row text is never used

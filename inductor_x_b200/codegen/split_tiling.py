@@ -60,7 +60,7 @@ MAX_PERSISTENT_VPT = 8   # static rows longer than MAX_TEAM x this many vectors 
 
 
 def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = None,
-                      target_vpt: int = 2) -> Optional[RowConfig]:
+                      target_vpt: int = 2, exact: bool = True) -> Optional[RowConfig]:
     """Launch shape of a generated persistent-row kernel.
 
     A generated body keeps several fp32 copies of its part of the row live, so the row is
@@ -68,11 +68,16 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
     that covers it (measured on the softmax->LayerNorm chain at 4096 bf16 columns: 256
     threads x 2 vectors ran 1.2-2x faster than 128 x 4).  Only rows longer than 1024
     threads x ``target_vpt`` vectors take more per thread, and rows of a few vectors get
-    teams of 8 or 16 lanes so that a warp works on several rows at once.  CTAs hold 128 threads or one
-    team, whichever is larger, and the register allocation is bounded for 1024 resident
-    threads per SM (the module loader relaxes the bound if that makes the body spill).
-    Rows that are streamed long enough get an L2 prefetch two rows ahead.  None if the
-    row does not fit on chip."""
+    teams of 8 or 16 lanes so that a warp works on several rows at once.  A row of no
+    power-of-two number of vectors is cut to fit: up to ``MAX_EXACT_VPT`` vectors per thread
+    over that team, half or a quarter of it, whichever leaves the fewest vectors idle.
+    ``exact=False`` leaves that cut out: the extent is only the first one seen of a run-time
+    size, the module serves every row up to the shape's capacity, and the slack of the
+    power-of-two cover is what longer ones run in.  CTAs hold 128 threads or one team,
+    whichever is larger, and the register allocation is bounded for 1024 resident threads per
+    SM, 512 where a thread holds more than two vectors (the module loader relaxes the bound if
+    that makes the body spill).  Rows that are streamed long enough get an L2 prefetch two rows
+    ahead.  None if the row does not fit on chip."""
     vec = min(max(config.get_aligned_numel(dtype), 1), 8)
     nvec = -(-rnumel // vec)
     if nvec > MAX_TEAM * MAX_VPT:
@@ -85,7 +90,7 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
         vpt *= 2
     while vpt > 1 and team * (vpt // 2) >= nvec:   # short rows: no idle vectors
         vpt //= 2
-    if MIN_TEAM * 4 <= team <= MAX_TEAM and vpt <= MAX_EXACT_VPT:
+    if exact and MIN_TEAM * 4 <= team <= MAX_TEAM and vpt <= MAX_EXACT_VPT:
         # rows of no power-of-two number of vectors: of this team, half and a quarter of it, the
         # one that leaves the fewest vectors idle (softmax -> LayerNorm, 5000 x 5003 bf16: 512
         # threads x 2 vectors 85 us, 256 x 3 62 us, 128 x 5 48 us; 60000 x 331 fp32: 64 x 2 95 us,
@@ -111,9 +116,10 @@ def choose_loop_config(dtype: torch.dtype) -> RowConfig:
 def row_candidates(rnumel: int, chosen: RowConfig, rows: Optional[int] = None, n_consts: int = 0,
                    kregs: int = 0):
     """Launch shapes worth measuring for a generated row kernel besides the chosen one:
-    ``(team, teams, vpt, min_ctas, prefetch, kregs)`` tuples.  One, two and four vectors per
-    thread over the matching power-of-two team; one, two or three teams per CTA; registers
-    bounded for 256 to 1024 resident threads per SM; and, where the body has per-column
+    ``(team, teams, vpt, min_ctas, prefetch, kregs)`` tuples.  Every power-of-two team from a
+    warp to 1024 threads that covers the row with at most ``MAX_EXACT_VPT`` vectors per thread;
+    about 128, 256 or 384 threads of whole teams per CTA; registers bounded for 256 to 1024
+    resident threads per SM; and, where the body has per-column
     operands, how many of them stay in registers (``kregs``; the rest are read from the
     shared-memory table, which frees registers for more resident warps).  The module loader
     builds the first few and keeps the one with the highest measured bandwidth
