@@ -79,7 +79,9 @@ class GeneratedKernel:
         direct = not self._tune_pending and not self.meta.get("bounds")
         self.run.bind(ctypes.cast(self.fn, ctypes.c_void_p).value if direct else 0)
 
-    def _run_general(self, *args, stream=None):
+    def _run_general(self, *args, stream=None, status=None):
+        if status is not None:       # what a native launch returned: to be worded, not launched again
+            self._raise_on_status(status)
         ptrs, ints, keep = [], [], []
         for a in args:
             if isinstance(a, torch.Tensor):
@@ -110,12 +112,14 @@ class GeneratedKernel:
         rc = self.fn(pa, ia, stream)
         self._launches += 1
         if rc != 0:
-            hint = (" (a run-time reduced extent beyond the capacity the module was compiled for?)"
-                    if rc == 1 and self.meta.get("family") == "row" else "")
-            raise RuntimeError(f"generated kernel {self.meta.get('name', self.key)} failed to launch: "
-                               f"cudaError {rc}{hint}")
+            self._raise_on_status(rc)
         if self.meta.get("bounds"):
             self._raise_on_bad_index()
+
+    def _raise_on_status(self, rc: int) -> None:
+        hint = (" (a run-time reduced extent beyond the capacity the module was compiled for?)"
+                if rc == 1 and self.meta.get("family") == "row" else "")
+        raise RuntimeError(f"generated kernel {self.meta.get('name', self.key)} failed to launch: cudaError {rc}{hint}")
 
     def _raise_on_bad_index(self) -> None:
         """Debug builds: read the module's status words (this synchronises) and report an

@@ -7,8 +7,9 @@
 // ctypes call) this took 5.3 us; here it takes 0.2.  A compiled call of one small kernel (gelu row
 // sum, 64 x 1024) went from 30.2 to 23.8 us, the rest being Dynamo's guards and the wrapper.
 // Anything out of the ordinary - a host tensor, a tensor subclass, a size that is not an int, no
-// stream, a non-zero status - goes to the Python method given as `general`, which also words the
-// errors.  It stands for the launcher closure of the reference
+// stream - goes to the Python method given as `general`.  A launch that returns a non-zero status is
+// not tried again (the status may be an earlier call's, and the kernel may have run): the method is
+// called with `status` and words the error.  It stands for the launcher closure of the reference
 // (inductor_x/npu_triton_heuristics.py:239-253).
 #include <Python.h>
 #include <structmember.h>
@@ -30,6 +31,7 @@ struct Launcher {
 };
 
 PyObject *name_profile, *name_dry_run;  // interned: "profile_bandwidth", "dry_run"
+PyObject* name_status;                  // ("status",): the keyword of a failed launch
 
 // neither of the two switches that the general route serves is set
 bool switches_off(PyObject* flags) {
@@ -74,7 +76,11 @@ PyObject* launch(PyObject* self_, PyObject* const* args, size_t nargsf, PyObject
       ++self->launches;
       Py_RETURN_NONE;
     }
-    // the general route launches again and words the error if there still is one
+    PyObject* status = PyLong_FromLong(rc);
+    if (status == nullptr) return nullptr;
+    PyObject* raised = PyObject_Vectorcall(self->general, &status, 0, name_status);
+    Py_DECREF(status);
+    return raised;
   }
   return PyObject_Vectorcall(self->general, args, nargsf & ~PY_VECTORCALL_ARGUMENTS_OFFSET, kwnames);
 }
@@ -141,7 +147,8 @@ PyMODINIT_FUNC PyInit__ixb_host(void) {
   LauncherType.tp_members = members;
   name_profile = PyUnicode_InternFromString("profile_bandwidth");
   name_dry_run = PyUnicode_InternFromString("dry_run");
-  if (name_profile == nullptr || name_dry_run == nullptr || PyType_Ready(&LauncherType) < 0) return nullptr;
+  name_status = Py_BuildValue("(s)", "status");
+  if (name_profile == nullptr || name_dry_run == nullptr || name_status == nullptr || PyType_Ready(&LauncherType) < 0) return nullptr;
   PyObject* m = PyModule_Create(&module_def);
   if (m == nullptr) return nullptr;
   Py_INCREF(&LauncherType);

@@ -64,6 +64,20 @@ def test_failure_is_raised(kernel):
         kernel.run(1, 2, stream=0)
 
 
+def test_failed_launch_is_not_tried_again(kernel):
+    """Its status may be an earlier call's and the kernel may have run: an update in place would be
+    applied twice."""
+    kernel.lib.set_status(1)
+    with pytest.raises(RuntimeError, match="cudaError 1"):
+        kernel.run(1, 2, stream=0)
+    assert kernel.lib.get(-1) == 1 and kernel.launches == 0
+    seen = []
+    k = jit._native_launcher()(lambda *a, **kw: seen.append((a, kw)), vars(config))
+    k.bind(ctypes.cast(kernel.fn, ctypes.c_void_p).value)
+    k(1, 2, stream=0)
+    assert kernel.lib.get(-1) == 2 and seen == [((), {"status": 1})]
+
+
 def test_pending_measurement_and_bounds_reports_are_not_passed_by(kernel):
     tuned = jit.GeneratedKernel("t", kernel.path, {"tune": dict(candidates=[(1,) * 6], idempotent=True, default=[1] * 6,
                                                                 rows=1 << 20, row_bytes=1 << 10)})
