@@ -60,6 +60,15 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 __device__ __forceinline__ uint4 ldg_keep(const void* p) {
   return __ldg(reinterpret_cast<const uint4*>(p));
 }
+// Ordinary load that stays in L1 (a neighbour reads part of the same word).  Rows that generated
+// kernels may write in place are read with it: __ldg promises data that nobody writes while the
+// kernel runs, and a kernel launched as a dependent starts before its producer has ended.  A
+// volatile statement keeps its place behind the wait for the producer.
+__device__ __forceinline__ uint4 ldg_shared_word(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
 __device__ __forceinline__ void stg_stream(void* p, uint4 v) {
   asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
                "r"(v.w)

@@ -635,7 +635,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
       for (int k = 0; k <= kC; ++k) {
         const bool need = (full(i) || (c0 + off < ncols() && c0 + k * kPer < ncols())) && (k < kC || off > 0);
-        raw.q[i][k] = need ? ldg_keep(rowp + (c0 + k * kPer)) : make_uint4(0, 0, 0, 0);
+        raw.q[i][k] = need ? ldg_shared_word(rowp + (c0 + k * kPer)) : make_uint4(0, 0, 0, 0);
       }
     }
   }

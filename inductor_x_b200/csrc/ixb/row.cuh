@@ -65,8 +65,8 @@ template <typename T, int TEAM, int TEAMS, int VPT, bool ALIGNED> struct RowCtx 
   // those that hold an element of the row are read) ...
   __device__ __forceinline__ void fetch(const T* base, int i, uint4 (&words)[2]) const {
     const int off = off_boundary(base), c0 = vec_col(i) - off;
-    words[0] = valid(i) ? ldg_keep(base + c0) : make_uint4(0, 0, 0, 0);
-    words[1] = valid(i) && off > 0 && c0 + kVec < cols ? ldg_keep(base + c0 + kVec) : make_uint4(0, 0, 0, 0);
+    words[0] = valid(i) ? ldg_shared_word(base + c0) : make_uint4(0, 0, 0, 0);
+    words[1] = valid(i) && off > 0 && c0 + kVec < cols ? ldg_shared_word(base + c0 + kVec) : make_uint4(0, 0, 0, 0);
   }
   // ... and the vector cut out of them, zero past the end of the row
   __device__ __forceinline__ uint4 settle(const T* base, int i, const uint4 (&words)[2]) const {
