@@ -904,18 +904,19 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   }
 
   // ---- thread-local folds -------------------------------------------------------------------
-  // sum of pairs of elements (pair p = elements 2p, 2p + 1) in independent chains of packed adds;
-  // only the vectors that may reach past the end of the row are tested
-  template <class F> __device__ __forceinline__ float fold_pairs(const F& pair) const {
+  // sum over pairs of elements (pair p = elements 2p, 2p + 1) in independent chains: step(p, acc) is
+  // the accumulator with pair p added; only the vectors that may reach past the end of the row are
+  // tested, and what lies there leaves the accumulator as it was
+  template <class F> __device__ __forceinline__ float fold_pairs(const F& step) const {
     float2 acc[kChains];
 #pragma unroll
     for (int c = 0; c < kChains; ++c) acc[c] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int p = 0; p < kE / 2; ++p) {
-      float2 v = pair(p);
-      if (!inside((2 * p) / Base::kVec, (2 * p) % Base::kVec)) v.x = 0.f;
-      if (!inside((2 * p + 1) / Base::kVec, (2 * p + 1) % Base::kVec)) v.y = 0.f;
-      acc[p % kChains] = add2(acc[p % kChains], v);
+      float2& a = acc[p % kChains];
+      const float2 v = step(p, a);
+      if (inside((2 * p) / Base::kVec, (2 * p) % Base::kVec)) a.x = v.x;
+      if (inside((2 * p + 1) / Base::kVec, (2 * p + 1) % Base::kVec)) a.y = v.y;
     }
 #pragma unroll
     for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
@@ -934,7 +935,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
       return acc[0].x + acc[0].y;
     } else if constexpr (COLS > 0 && op::is_fvec<A>::value) {
-      return fold_pairs([&](int p) { return op::pr(val, p); });
+      return fold_pairs([&](int p, const float2& acc) { return add2(acc, op::pr(val, p)); });
     } else {
       float acc = 0.f;
 #pragma unroll
@@ -957,7 +958,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
       return acc[0].x + acc[0].y;
     } else if constexpr (COLS > 0 && op::packable2<A, B>::value) {
-      return fold_pairs([&](int p) { return mul2(op::pr(a, p), op::pr(b, p)); });
+      return fold_pairs([&](int p, const float2& acc) { return fma2(op::pr(a, p), op::pr(b, p), acc); });
     } else {
       float acc = 0.f;
 #pragma unroll

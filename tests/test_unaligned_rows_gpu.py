@@ -77,3 +77,21 @@ def test_library_rows(cuda, dtype, rows, cols):
         ops.softmax_layernorm(x, w, w, w, 1e-5, out=buf[cols:-cols].view(rows, cols))
         close(buf[cols:-cols].view(rows, cols), chain(*(t.double() for t in (x, w, w, w))), dtype)
         assert bool((buf[:cols] == 7).all()) and bool((buf[-cols:] == 7).all())
+
+
+def test_products_are_not_rounded_before_they_are_added(cuda):
+    """A thread's products meet in one fma, in the vector that the row ends in as in the others:
+    -(1 + 2^-11) and (1 + 2^-12)^2 leave 2^-24, which a rounded product would have lost.  Of 64
+    threads with five vectors of four, columns 0-3 and 1024-1027 are the first one's, column 4 and
+    1028, the last, the second one's."""
+    import inductor_x_b200  # noqa: F401
+    from torch._inductor.utils import run_and_get_code
+
+    a, b = (torch.zeros(3, 1029, device=cuda) for _ in range(2))
+    a[:, :5], b[:, :5] = -(1 + 2.0 ** -11), 1
+    a[:, 1024:], b[:, 1024:] = 1 + 2.0 ** -12, 1 + 2.0 ** -12
+    torch._dynamo.reset()
+    out, code = run_and_get_code(torch.compile(lambda a, b: (a * b).sum(-1), dynamic=False), a, b)
+    code = "\n".join(code)
+    assert "reduce_dot(" in code and "#define IXB_ROW_TEAM 64" in code and "#define IXB_ROW_VPT 5" in code
+    assert torch.equal(out, torch.full_like(out, 5 * 2.0 ** -24))
