@@ -1157,15 +1157,22 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       const float2 x = make_float2(Cast<float>::from(at(val, 2 * p)), Cast<float>::from(at(val, 2 * p + 1)));
       const float2 t = fma2(x, make_float2(kLog2e, kLog2e), make_float2(shift, shift));
       float2 ex = make_float2(fast_exp2(t.x), fast_exp2(t.y));
-      if constexpr (!FULL) {
-        if (!inside((2 * p) / Base::kVec, (2 * p) % Base::kVec)) ex.x = 0.f;
-        if (!inside((2 * p + 1) / Base::kVec, (2 * p + 1) % Base::kVec)) ex.y = 0.f;
-      }
+      const bool in0 = inside((2 * p) / Base::kVec, (2 * p) % Base::kVec);
+      const bool in1 = inside((2 * p + 1) / Base::kVec, (2 * p + 1) % Base::kVec);
+      if (!in0) ex.x = 0.f;
+      if (!in1) ex.y = 0.f;
       o.e.v[2 * p] = ex.x;
       o.e.v[2 * p + 1] = ex.y;
       acc[0][p % kChains] = add2(acc[0][p % kChains], ex);
 #pragma unroll
-      for (int k = 0; k < NS; ++k) acc[1 + k][p % kChains] = fma2(ex, op::pr(*w.p[k], p), acc[1 + k][p % kChains]);
+      for (int k = 0; k < NS; ++k) {
+        // a weight past the end of the row was computed from zeros and may be infinite or NaN,
+        // which no zero exponential removes
+        float2 weight = op::pr(*w.p[k], p);
+        if (!in0) weight.x = 0.f;
+        if (!in1) weight.y = 0.f;
+        acc[1 + k][p % kChains] = fma2(ex, weight, acc[1 + k][p % kChains]);
+      }
     }
 #pragma unroll
     for (int k = 0; k < 1 + NS; ++k) {
