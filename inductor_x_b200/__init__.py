@@ -101,6 +101,16 @@ def _route_random_ops_to_aten():
     inductor_config.fallback_random = True
 
 
+def _keep_reduction_orders_apart():
+    """A kernel of these templates reduces along one axis.  Inductor's fusion of a sum over rows with
+    the column sum of a weight's gradient - a normalisation layer's backward from 8192 x 2048 on -
+    asks the backend for a kernel that does both, which ended the compilation."""
+    from torch._inductor import config as inductor_config
+
+    if hasattr(inductor_config.triton, "mix_order_reduction"):
+        inductor_config.triton.mix_order_reduction = False
+
+
 def _specialize_python_floats():
     """Python ``float`` arguments of a compiled function are baked into the graph as constants
     (Dynamo's ``specialize_float``; a new value recompiles).  Left symbolic, such a float enters
@@ -125,6 +135,7 @@ def register():
     _register_device_interface()
     _enable_online_softmax_pattern()
     _route_random_ops_to_aten()
+    _keep_reduction_orders_apart()
     _specialize_python_floats()
     from .codegen.ir import install_num_splits
 
