@@ -515,7 +515,8 @@ extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return ixb_host::cuda_status(e);
     // the softmax warps' setmaxnreg waits for registers the block owns: never launch a build
-    // that was given fewer at launch than the split adds up to
+    // that was given fewer at launch than the split adds up to (the Makefile fails on one; this
+    // is for objects built without it)
     cudaFuncAttributes at;
     e = cudaFuncGetAttributes(&at, kern);
     if (e != cudaSuccess) return ixb_host::cuda_status(e);
