@@ -21,7 +21,8 @@
 // element-wise work in NG groups of four warps that split the 128 columns of a tile between
 // them (a warp may only touch the 32 TMEM lanes of its quadrant; no row reduction is needed
 // here - lse and delta come in precomputed - so the split costs nothing).  Every wait is
-// bounded; a wait that gives up raises a flag in `status` and lets the CTA drain and exit.
+// bounded; a wait that gives up raises a flag in `status`, and the CTA exits when the copies
+// and products under way have ended.
 //
 // Bound: the tensor core, at the rate the power limit leaves it.  Measured at 8 x 32 heads, 4096
 // keys, causal, bf16: delta 0.11 ms, dK/dV 2.12 ms, dQ 1.51 ms in a short run; with the
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* do_smem = smem + 4 * kTileBytes;  // kStages tiles
 
   __shared__ __align__(8) uint64_t kv_full, qdo_full[kStages], qdo_empty[kStages], s_full, dp_full, p_full,
-      ds_full, acc_done;
+      ds_full, acc_done, drained;
   __shared__ __align__(16) float lse_s[kStages][BM], delta_s[kStages][BM];
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(&p_full, kWorkers / 32);
     mbar_init(&ds_full, kWorkers / 32);
     mbar_init(&acc_done, 1);
+    mbar_init(&drained, 1);
     failed = 0;
     mbar_init_fence();
   }
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
 
+  int loads = 0;  // producer: query tiles it has asked for
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0 && n_it > 0) {
@@ -266,6 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         load_tile(q_smem + (size_t)s * kTileBytes, &map_q, &qdo_full[s], qt0, h, b);
         load_tile(do_smem + (size_t)s * kTileBytes, &map_do, &qdo_full[s], qt0, h, b);
       }
+      loads = it + 1;
     }
     if (!ok && lane == 0) failed = 1;
     __syncwarp();
@@ -445,6 +449,15 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   tc::fence_before_sync();
   __syncthreads();
+  if (failed && n_it > 0) {  // (uniform: nobody writes it any more)
+    // a role gave up: what the others have under way has to end before the block does
+    if (threadIdx.x == 0) {
+      tc::await_copies<1>(&kv_full, 1);
+      tc::await_copies<kStages>(qdo_full, loads);
+    }
+    if (warp == 1) tc::await_products(&drained);
+    __syncthreads();
+  }
   if (threadIdx.x == 0 && failed && p.status != nullptr) atomicExch(p.status, 1);
   if (warp == 1) {
     tc::fence_after_sync();
@@ -469,7 +482,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* v_smem = smem + 4 * kTileBytes;  // kStages tiles
 
   __shared__ __align__(8) uint64_t qdo_full, k_full[kStages], k_empty[kStages], v_full[kStages],
-      v_empty[kStages], s_full, dp_full, s_read, ds_full, acc_done;
+      v_empty[kStages], s_full, dp_full, s_read, ds_full, acc_done, drained;
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
@@ -503,6 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(&s_read, kWorkers / 32);
     mbar_init(&ds_full, kWorkers / 32);
     mbar_init(&acc_done, 1);
+    mbar_init(&drained, 1);
     failed = 0;
     mbar_init_fence();
   }
@@ -512,6 +526,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
 
+  int k_loads = 0, v_loads = 0;  // producer: key and value tiles it has asked for
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
@@ -525,10 +540,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!ok) break;
         mbar_arrive_expect_tx(&k_full[s], kTileBytes);
         load_tile(k_smem + (size_t)s * kTileBytes, &map_k, &k_full[s], j * BN, h, b);
+        k_loads = j + 1;
         if (n > 0) ok = mbar_wait(&v_empty[s], (n - 1) & 1, &failed);
         if (!ok) break;
         mbar_arrive_expect_tx(&v_full[s], kTileBytes);
         load_tile(v_smem + (size_t)s * kTileBytes, &map_v, &v_full[s], j * BN, h, b);
+        v_loads = j + 1;
       }
       if (!ok) failed = 1;
     }
@@ -674,6 +691,15 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   tc::fence_before_sync();
   __syncthreads();
+  if (failed) {  // (as above)
+    if (threadIdx.x == 0) {
+      tc::await_copies<1>(&qdo_full, 1);
+      tc::await_copies<kStages>(k_full, k_loads);
+      tc::await_copies<kStages>(v_full, v_loads);
+    }
+    if (warp == 1) tc::await_products(&drained);
+    __syncthreads();
+  }
   if (threadIdx.x == 0 && failed && p.status != nullptr) atomicExch(p.status, 1);
   if (warp == 1) {
     tc::fence_after_sync();

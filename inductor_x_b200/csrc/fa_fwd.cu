@@ -21,7 +21,7 @@
 //              maximum has grown by more than 2^8 since the last rescale (the final division
 //              by the running sum makes a stale reference exact).
 // Hand-offs are mbarriers; every wait is bounded and a wait that gives up raises a flag in
-// `status` and lets the CTA drain and exit.
+// `status`; the CTA exits when the copies and products under way have ended.
 //
 // TMEM columns: [0,128) S/P of A, [128,256) S/P of B, [256,384) O of A, [384,512) O of B.
 //
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   __shared__ __align__(16) uint4 next_answer[2];
   __shared__ __align__(8) uint64_t q_full, q_empty, next_full[2], next_taken[2], k_full[kStages], k_empty[kStages], v_full[kStages],
-      v_empty[kStages], s_full[NQ], p_full[NQ], p_rest[NQ], pv_done[NQ];
+      v_empty[kStages], s_full[NQ], p_full[NQ], p_rest[NQ], pv_done[NQ], drained;
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&p_rest[t], 128);
       mbar_init(&pv_done[t], 1);
     }
+    mbar_init(&drained, 1);
     failed = 0;
     mbar_init_fence();
   }
@@ -176,6 +177,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     return index;
   };
 
+  int q_loads = 0, k_loads = 0, v_loads = 0;  // producer, lane 0: what it has asked for
+  int asked = 0;                              // scheduler: the same
   if (warp < 4) {
     tc::regs_dec<kRegsIssue>();
     if (warp == 0) {
@@ -188,6 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) {
           bool good = n == 0 || mbar_wait(&q_empty, (n - 1) & 1, &failed);
           if (good) {
+            ++q_loads;
             mbar_arrive_expect_tx(&q_full, kTileBytes * NQ);
 #pragma unroll
             for (int t = 0; t < NQ; ++t) {
@@ -204,12 +208,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_arrive_expect_tx(&k_full[s], kTileBytes);
             tc::tma_load_4d(kd, &map_k, &k_full[s], 0, j * BN, w.h, w.b);
             tc::tma_load_4d(kd + kHalfBytes, &map_k, &k_full[s], 64, j * BN, w.h, w.b);
+            k_loads = step + j + 1;
             good = u == 0 || mbar_wait(&v_empty[s], (u - 1) & 1, &failed);
             if (!good) break;
             unsigned char* vd = v_smem + (size_t)s * kTileBytes;
             mbar_arrive_expect_tx(&v_full[s], kTileBytes);
             tc::tma_load_4d(vd, &map_v, &v_full[s], 0, j * BN, w.h, w.b);
             tc::tma_load_4d(vd + kHalfBytes, &map_v, &v_full[s], 64, j * BN, w.h, w.b);
+            v_loads = step + j + 1;
           }
           mine = good ? 1 : 0;
         }
@@ -298,6 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (n > 0) ok = __all_sync(kFull, mbar_wait(&next_taken[(n - 1) & 1], ((n - 1) >> 1) & 1, &failed));
         if (!ok) break;
         if (lane == 0) tc::request_next_block(&next_answer[n & 1], &next_full[n & 1]);
+        asked = n + 1;
         ok = __all_sync(kFull, mbar_wait(&next_full[n & 1], (n >> 1) & 1, &failed));
         if (!ok || __shfl_sync(kFull, tc::next_block(&next_answer[n & 1]), 0) < 0) break;
       }
@@ -450,6 +457,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   tc::fence_before_sync();
   __syncthreads();
+  if (failed) {  // (uniform: nobody writes it any more)
+    // a role gave up: what the others have under way has to end before the block does
+    if (threadIdx.x == 0) {
+      tc::await_copies<1>(&q_full, q_loads);
+      tc::await_copies<kStages>(k_full, k_loads);
+      tc::await_copies<kStages>(v_full, v_loads);
+    }
+    if (warp == 1) tc::await_products(&drained);
+    if (warp == 2 && lane == 0) tc::await_copies<2>(next_full, asked);
+    __syncthreads();
+  }
   if (threadIdx.x == 0 && failed && p.status != nullptr) atomicExch(p.status, 1);
   if (warp == 1) {
     tc::fence_after_sync();

@@ -191,6 +191,24 @@ __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// ---- leaving after a wait that gave up --------------------------------------------------------
+// A block must not leave while copies into its shared memory or MMAs on its operands are under way.
+// Bounded like every wait, and without a look at the abort flag, which is up by then.
+// The last copies into a ring of STAGES tiles, `issued` of them so far (one thread).
+template <int STAGES> __device__ __forceinline__ void await_copies(uint64_t* full, int issued) {
+#pragma unroll
+  for (int s = 1; s <= STAGES; ++s) {
+    const int last = issued - s;
+    if (last >= 0) mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+  }
+}
+// Every product this warp has issued; `bar` (one arrival) is used for nothing else (whole warp).
+__device__ __forceinline__ void await_products(uint64_t* bar) {
+  __syncwarp();
+  commit_elected(bar);
+  __all_sync(kFull, mbar_wait(bar, 0));
+}
+
 // ---- register split between warpgroups (whole warpgroup) -------------------------------
 template <int N> __device__ __forceinline__ void regs_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
