@@ -148,7 +148,7 @@ template <class U> __device__ __forceinline__ int off_boundary(const U* p) {
   return (int)(reinterpret_cast<uintptr_t>(p) & 15u) / (int)sizeof(U);
 }
 
-  // the first n elements of a word, zeros behind them
+// the first n elements of a word, zeros behind them
 template <class U> __device__ __forceinline__ uint4 keep_elements(const uint4& v, int n) {
   uint32_t w[4] = {v.x, v.y, v.z, v.w};
   constexpr int kPerWord = 4 / (int)sizeof(U);
@@ -160,17 +160,17 @@ template <class U> __device__ __forceinline__ uint4 keep_elements(const uint4& v
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 // elements [first, end) of a word
-  template <class U> __device__ __forceinline__ void put_elements(U* p, const uint4& v, int first, int end) {
-    constexpr int kPer = 16 / (int)sizeof(U);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+template <class U> __device__ __forceinline__ void put_elements(U* p, const uint4& v, int first, int end) {
+  constexpr int kPer = 16 / (int)sizeof(U);
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-      if (e >= first && e < end) {
-        if constexpr (sizeof(U) == 4) reinterpret_cast<uint32_t*>(p)[e] = w[e];
-        else reinterpret_cast<unsigned short*>(p)[e] = (unsigned short)((e & 1) ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
-      }
+  for (int e = 0; e < kPer; ++e) {
+    if (e >= first && e < end) {
+      if constexpr (sizeof(U) == 4) reinterpret_cast<uint32_t*>(p)[e] = w[e];
+      else reinterpret_cast<unsigned short*>(p)[e] = (unsigned short)((e & 1) ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
     }
   }
+}
 
 // ---------------------------------------------------------------------------------
 // Reduction operators.  `combine` must be associative and commutative.

@@ -51,31 +51,6 @@ __device__ __forceinline__ void fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// ---- MMA issue (one thread) -----------------------------------------------------------
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // ---- one 128 x 128 x 128 product, issued by a whole converged warp -----------------------
 // Every lane runs the issuing loop and one elected lane executes the instructions: the
 // operands then stay warp-uniform.  In a loop that a single lane runs (`if (lane == 0)`) the
@@ -132,7 +107,8 @@ template <int N> __device__ __forceinline__ void product_ts(uint32_t d_tmem, uin
       : "memory");
   if constexpr (N > 2) product_ts<N - 2>(d_tmem, a_tmem + 16, b_desc + 256, idesc, 1u);
 }
-// mma_commit by the elected lane of a converged warp (the one that issued the products)
+// By the elected lane of a converged warp, the one that issued the products: the mbarrier gets one
+// arrival when every MMA issued so far by this lane has finished.
 __device__ __forceinline__ void commit_elected(uint64_t* bar) {
   asm volatile(
       "{\n\t"
@@ -141,12 +117,6 @@ __device__ __forceinline__ void commit_elected(uint64_t* bar) {
       "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
       "}" ::"r"(smem_u32(bar))
       : "memory");
-}
-// The mbarrier gets one arrival when every MMA issued so far by this thread has finished.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
 }
 
 // ---- TMEM <-> registers: 32 lanes x 32 columns of 32 bits, thread i <-> lane base+i ---
