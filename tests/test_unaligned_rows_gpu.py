@@ -1,6 +1,7 @@
 """Rows that start off a 16-byte boundary (odd row lengths, odd offsets and pitches): the staged
-covering words, the shifted stores and their ends.  Against 64-bit arithmetic on the same inputs;
-results are 32-bit sums rounded once, so the bound is a few roundings of the storage type."""
+covering words, the loads on the spot, the shifted stores and their ends.  Against 64-bit arithmetic
+on the same inputs; results are 32-bit sums rounded once, so the bound is a few roundings of the
+storage type."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -28,10 +29,37 @@ def close(got, want, dtype):
 
 # sub-warp teams with several rows in flight, one warp, several warps, two vectors a thread; a row
 # that ends one element into a vector, one before its end, and in the middle
-@pytest.mark.parametrize("dtype,rows,cols", [(torch.float16, 301, 33), (torch.bfloat16, 64, 71), (torch.float32, 77, 130),
-                                             (torch.bfloat16, 9, 515), (torch.float16, 1500, 1537), (torch.float32, 5, 3001),
-                                             (torch.bfloat16, 1, 9001)])
+SHAPES = [(torch.float16, 301, 33), (torch.bfloat16, 64, 71), (torch.float32, 77, 130), (torch.bfloat16, 9, 515),
+          (torch.float16, 1500, 1537), (torch.float32, 5, 3001), (torch.bfloat16, 1, 9001)]
+
+
+@pytest.mark.parametrize("dtype,rows,cols", SHAPES)
+def test_compiled_rows_requested_ahead(cuda, dtype, rows, cols):
+    """Every base pointer is 16-byte aligned, so the covering words of a row are fetched while the one
+    before it is worked on; an odd length or pitch moves the rows off the boundary.  NaN in the gap
+    between rows and behind the last one is not to reach a result."""
+    import inductor_x_b200  # noqa: F401
+
+    x, g, gamma, beta = inputs(cuda, rows, cols, dtype)
+    want = chain(*(t.double() for t in (x, g, gamma, beta)))
+    for pitch in (cols, cols + 4 if cols % 2 else cols + 3):
+        torch._dynamo.reset()
+        into = torch.compile(lambda x, g, gamma, beta, out: out.copy_(chain(x, g, gamma, beta)), dynamic=False)
+        store = torch.full((rows * pitch + 64,), float("nan"), dtype=dtype, device=cuda)
+        src = store[:rows * pitch].view(rows, pitch)[:, :cols]
+        src.copy_(x)
+        buf = torch.full((rows * pitch + 128,), 7.0, dtype=dtype, device=cuda)
+        dst = buf[64:64 + rows * pitch].view(rows, pitch)[:, :cols]
+        assert all(t.data_ptr() % 16 == 0 for t in (src, g, gamma, beta, dst))
+        into(src, g, gamma, beta, dst)
+        close(dst, want, dtype)
+        dst.fill_(7)  # nothing beyond the rows is written
+        assert bool((buf == 7).all())
+
+
+@pytest.mark.parametrize("dtype,rows,cols", SHAPES)
 def test_compiled_rows_inside_a_larger_buffer(cuda, dtype, rows, cols):
+    """An output whose base pointer is not 16-byte aligned: rows are loaded when they are worked on."""
     import inductor_x_b200  # noqa: F401
 
     x, g, gamma, beta = inputs(cuda, rows, cols, dtype)
@@ -46,8 +74,8 @@ def test_compiled_rows_inside_a_larger_buffer(cuda, dtype, rows, cols):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 def test_compiled_rows_of_a_view(cuda, dtype):
-    """An odd pitch and an odd first element; and a base pointer that is not 16-byte aligned, which
-    takes the loads that are not requested ahead."""
+    """An odd pitch, an odd first element and per-column operands off a boundary: base pointers that are
+    not 16-byte aligned take the loads that are not requested ahead."""
     import inductor_x_b200  # noqa: F401
 
     x, g, gamma, beta = inputs(cuda, 50, 205, dtype)
@@ -71,7 +99,9 @@ def test_library_rows(cuda, dtype, rows, cols):
     close(y, hd * torch.rsqrt(hd.square().mean(-1, keepdim=True) + 1e-6) * w.double(), dtype)
     close(ops.row_reduce(x, "sum"), x.double().sum(-1), dtype)
     assert torch.equal(ops.row_reduce(x, "amax"), x.amax(-1))
-    assert torch.equal(ops.row_reduce(x, "argmin"), x.argmin(-1)) or dtype != torch.float32  # ties in 16 bits
+    at = ops.row_reduce(x, "argmin")
+    assert bool(((at >= 0) & (at < cols)).all()) and torch.equal(x.gather(-1, at[:, None]), x.amin(-1, keepdim=True))
+    assert dtype != torch.float32 or torch.equal(at, x.argmin(-1))  # 16-bit rows have ties
     if cols > 1:
         buf = torch.full(((rows + 2) * cols,), 7.0, dtype=dtype, device=cuda)
         ops.softmax_layernorm(x, w, w, w, 1e-5, out=buf[cols:-cols].view(rows, cols))
