@@ -123,6 +123,7 @@ class B200Kernel(SIMDKernel):
         self.const_of: dict = {}     # value name -> Consts member text
         self.online: dict = {}       # name of a softmax input -> its online-softmax exchange
         self.online_exp: dict = {}   # name of exp(input - max) -> exchange
+        self.zero_past_end: set = set()    # operands that are zero past the end of a row (plain loads)
         self.checked_indices = 0     # data-dependent indices checked on the device (debug builds)
         self.x_indexing = IndentedBuffer()
         self.r_indexing = IndentedBuffer()
@@ -525,6 +526,8 @@ class B200Kernel(SIMDKernel):
             self.scalars.add(out.name)
         if const_member is not None:
             self.const_of[out.name] = const_member
+        if not masked:
+            self.zero_past_end.update({out.name, const_member} - {None})
         return out
 
     # ------------------------------------------------------------------ stores
@@ -851,7 +854,13 @@ class B200Kernel(SIMDKernel):
                     wt = self._early_text(b, ex)
                     if wt is None:
                         return None
-                    return [(coef, kind, wt if w is None else f"{OPN}mul({w}, {wt})") for coef, kind, w in fa]
+                    out = []
+                    for coef, kind, w in fa:
+                        both = wt if w is None else f"{OPN}mul({w}, {wt})"
+                        if wt in self.zero_past_end and w in self.zero_past_end:
+                            self.zero_past_end.add(both)
+                        out.append((coef, kind, both))
+                    return out
             return None
         if opn == "truediv" and len(args) == 2 and self.is_scalar(args[1]):
             fa = self._linear_form(args[0], ex, depth + 1)
@@ -1128,7 +1137,8 @@ class B200Kernel(SIMDKernel):
         for tag, v in self._ph.items():
             if v.get("online") and not outer:
                 rs, rp = v["riders_s"], v["riders_p"]
-                v["row"] = (f"c.template online_softmax<{len(rs)}, {len(rp)}>({v['value']}, "
+                computed = "" if self.zero_past_end.issuperset(rs) else ", true"
+                v["row"] = (f"c.template online_softmax<{len(rs)}, {len(rp)}{computed}>({v['value']}, "
                             f"{G}refs<kN>({', '.join(rs)}), {G}refs<kN>({', '.join(rp)}))")
             text = text.replace(tag, v["outer"] if outer else v["row"])
         return text

@@ -1122,7 +1122,9 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     vf<kE> e;
     float scaled[NS > 0 ? NS : 1], plain[NP > 0 ? NP : 1];
   };
-  template <int NS, int NP, class A>
+  // COMPUTED: some w is not a plain operand, which is zero past the end of the row, but computed from
+  // such zeros, and may be infinite or NaN there; no zero exponential removes that, so it is masked.
+  template <int NS, int NP, bool COMPUTED = false, class A>
   __device__ __forceinline__ Online<NS, NP> online_softmax(const A& val, const VecRefs<kE, NS>& w,
                                                             const VecRefs<kE, NP>& pl) {
     static_assert(NS + NP <= 2, "a slot holds the maximum, the sum and two riders");
@@ -1166,11 +1168,9 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       acc[0][p % kChains] = add2(acc[0][p % kChains], ex);
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
-        // a weight past the end of the row was computed from zeros and may be infinite or NaN,
-        // which no zero exponential removes
         float2 weight = op::pr(*w.p[k], p);
-        if (!in0) weight.x = 0.f;
-        if (!in1) weight.y = 0.f;
+        if (COMPUTED && !in0) weight.x = 0.f;
+        if (COMPUTED && !in1) weight.y = 0.f;
         acc[1 + k][p % kChains] = fma2(ex, weight, acc[1 + k][p % kChains]);
       }
     }

@@ -22,5 +22,5 @@ def test_weights_past_the_end_of_the_row(cuda, cols):
     x, y = torch.randn(64, cols, generator=g, device=cuda), 1 + torch.rand(64, cols, generator=g, device=cuda)
     torch._dynamo.reset()
     out, code = run_and_get_code(torch.compile(weighted, dynamic=False), x, y)
-    assert "online_softmax<1, 0>" in "\n".join(code)
+    assert "online_softmax<1, 0, true>" in "\n".join(code)
     torch.testing.assert_close(out.double(), weighted(x.double(), y.double()), rtol=1e-5, atol=0)
