@@ -172,8 +172,10 @@ __device__ __forceinline__ void scatter_add(T* p, const I& idx, const M& mask, c
 // unconditional - no branch separates the loads of an unrolled loop and they overlap.
 // STREAM: the run is read once and nothing near it is (a gathered table row): no L1 allocation.
 // CUT = false leaves out the form for runs off a boundary (element by element then): for loads that
-// are made once per thread, where the extra code costs the rows that follow more than it gives - the
-// per-column operands of softmax -> LayerNorm, 16384 x 4096 bf16: 59.4 us with it, 58.7 without.
+// are made once per thread, where the extra code costs the rows that follow more than it gives.
+// softmax -> LayerNorm with it in all, in none, in the shared-memory table of rows that do not fill
+// their team only, as it is used: 16384 x 4096 bf16 60.1, 59.4, 59.4 us; 20011 x 1537 fp16 59.4,
+// 58.3, 58.3; 9000 x 3001 fp32 78.0, 76.7, 76.7; 5000 x 5003 bf16 47.5, 48.2, 47.5.
 template <class T, int N, bool FAST = false, bool STREAM = false, bool CUT = true>
 __device__ __forceinline__ typename vec_of<typename Mem<T>::val, N>::type ldvec(const T* p, int nvalid) {
   using V = typename Mem<T>::val;
@@ -539,7 +541,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     for (int v = threadIdx.x; v < kTabVecs; v += blockDim.x) {
       const int c0 = v * Base::kVec;
       const int left = this->cols - c0;
-      const auto part = ldvec<U, Base::kVec, false, false, false>(rowp + (left > 0 ? c0 : 0), left > 0 ? left : 0);
+      const auto part = ldvec<U, Base::kVec, false, false, !FULL>(rowp + (left > 0 ? c0 : 0), left > 0 ? left : 0);
 #pragma unroll
       for (int q = 0; q < kQuads; ++q)
         tab[q * kTabVecs + v] = make_float4(part.v[4 * q], part.v[4 * q + 1], part.v[4 * q + 2], part.v[4 * q + 3]);
