@@ -92,9 +92,10 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
         vpt //= 2
     if exact and MIN_TEAM * 4 <= team <= MAX_TEAM and vpt <= MAX_EXACT_VPT:
         # rows of no power-of-two number of vectors: of this team, half and a quarter of it, the
-        # one that leaves the fewest vectors idle (softmax -> LayerNorm, 5000 x 5003 bf16: 512
-        # threads x 2 vectors 85 us, 256 x 3 62 us, 128 x 5 48 us; 60000 x 331 fp32: 64 x 2 95 us,
-        # 32 x 3 52 us); lengths that are a power of two of vectors keep their shape
+        # one that leaves the fewest vectors idle.  softmax -> LayerNorm, the row's length known to
+        # the template: 5000 x 5003 bf16 512 threads x 2 vectors 85 us, 256 x 3 62 us, 128 x 5 48 us
+        # (135 us before, element-wise); 60000 x 331 fp32 64 x 2 95 us, 32 x 3 50 us (50 us before).
+        # Lengths that are a power of two of vectors keep their shape
         team = min((t for t in (team, team // 2, team // 4) if t >= 32 and -(-nvec // t) <= MAX_EXACT_VPT),
                    key=lambda t: t * -(-nvec // t), default=team)
         vpt = -(-nvec // team)

@@ -24,17 +24,20 @@
 // bounded; a wait that gives up raises a flag in `status`, and the CTA exits when the copies
 // and products under way have ended.
 //
-// Bound: the tensor core, at the rate the power limit leaves it.  Measured at 8 x 32 heads, 4096
-// keys, causal, bf16: delta 0.11 ms, dK/dV 2.12 ms, dQ 1.51 ms in a short run; with the
-// element-wise warps only passing the barriers on, the products of the two kernels alone take
-// 1.64 and 1.43 ms, without the exponentials 2.07 and 1.50.  The products are issued by a whole
-// warp through an elected lane (4426 us a call before, one lane issuing; 4200 after, both in a
-// run long enough to sit at the power limit).  Two ways to overlap more were built and dropped:
-// dS in tensor-memory columns of its own, so that the next scores never wait for the product
-// behind them (dQ 1.51 -> 1.83 ms), and P^T as a shared-memory operand, which frees the score
-// columns earlier but reads another 32 KB of shared memory a step (dK/dV 2.12 -> 2.36 ms).  A
-// variant with 64-query sub-tiles and double-buffered score columns ran 30 % slower: an SS-form
-// MMA with N = 64 takes 48 cycles, not 32, and the hand-offs double.
+// Bound.  Measured at 8 x 32 heads, 4096 keys, causal, bf16: delta 0.11 ms, dK/dV 2.12 ms, dQ 1.51 ms
+// in a short run; with the element-wise warps only passing the barriers on, the products of the two
+// kernels alone take 1.64 and 1.43 ms, without the exponentials 2.07 and 1.50.  dQ is near the tensor
+// core's time at the power limit.  In dK/dV the element-wise work does not hide behind the products:
+// with one tile in flight the chain scores -> P -> product is serial, and 128-wide double buffering
+// would need more tensor memory than one SM has at this head dimension (two SMs to a tile,
+// cta_group::2, not built).  The products are issued by a whole warp through an elected lane (4426 us
+// a call with one lane issuing, 4200 so, both in a run long enough to sit at the power limit).  Two
+// other ways to overlap more were built and dropped: dS in tensor-memory columns of its own, so that
+// the next scores never wait for the product behind them (dQ 1.51 -> 1.83 ms), and P^T as a
+// shared-memory operand, which frees the score columns earlier but reads another 32 KB of shared
+// memory a step (dK/dV 2.12 -> 2.36 ms).  A variant with 64-query sub-tiles and double-buffered score
+// columns ran 30 % slower: an SS-form MMA with N = 64 takes 48 cycles, not 32, and the hand-offs
+// double.
 #include <atomic>
 #include "fa_maps.h"
 #include "ixb/tcgen05.cuh"

@@ -627,9 +627,10 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   // cover a thread's vectors are fetched aligned - the one it shares with the next lane comes
   // out of L1 - and shifted into place when the row is worked on.  Only words that hold an
   // element of the row are read.  Element-wise loads of such rows touch every line eight times
-  // and cannot be requested a row ahead: softmax -> LayerNorm of 20011 x 1537 fp16 took 103 us
+  // and cannot be requested a row ahead: softmax -> LayerNorm of 20011 x 1537 fp16 took 104 us
   // with them, 90 us this way, 73 us with the length known at compile time (COLS), 59 us in the
-  // launch shape that measures best (six teams of 64 threads with four vectors each).
+  // launch shape that measures best (six teams of 64 threads with four vectors each), 57 us with
+  // plain loads of the per-column operands.
   template <class U> __device__ __forceinline__ void fetch_row(const U* rowp, RawRowU<U, VPT, Base::kVec>& raw) const {
     constexpr int kC = RawRowU<U, VPT, Base::kVec>::kChunks;
     constexpr int kPer = 16 / (int)sizeof(U);
