@@ -638,8 +638,8 @@ class B200AttentionPass(CustomGraphModulePass):
     def uuid(self):
         # Part of Inductor's FX-graph cache key.  Everything that changes the text this backend
         # generates for a given graph has to be in it, or a cached wrapper from an earlier
-        # setting would be served: the code generator's sources, the template headers and the
-        # configuration flags.
+        # setting would be served: the code generator's sources, the template headers, the
+        # configuration flags, and how large the run-time sizes are that the graph is compiled at.
         import glob
         import hashlib
         import os
@@ -654,4 +654,17 @@ class B200AttentionPass(CustomGraphModulePass):
         h = hashlib.sha256(get_hash_for_files(files))
         h.update(jit._template_digest())
         h.update(repr(flags).encode())
+        h.update(repr(_run_time_size_classes()).encode())
         return h.digest()
+
+
+def _run_time_size_classes():
+    """The power-of-two class of each run-time size of the graph being compiled.  A row whose length
+    is such a size is served up to the capacity of the shape compiled for the first length seen, the
+    power of two of vectors that covers it; Inductor keys the size by its symbol alone, so the module
+    of a first length of 384 would be found for one of 600, and refuse it.  (The class of a sum or
+    product of two sizes is not told by theirs: such a length can still meet a smaller module.)"""
+    context = torch._guards.TracingContext.try_get()
+    shape_env = getattr(getattr(context, "fake_mode", None), "shape_env", None)
+    values = getattr(shape_env, "backed_var_to_val", None) or getattr(shape_env, "var_to_val", None) or {}
+    return sorted((str(symbol), (int(value) - 1).bit_length()) for symbol, value in values.items())
