@@ -247,6 +247,23 @@ int ixb_fa_bwd(int dtype, const void* q, const void* k, const void* v, const voi
                const int64_t* dv_strides, float scale, int causal, int32_t* status,
                ixb_stream stream);
 
+/* The same with room for dS, which spares the second computation of the probabilities: dS is
+ * kept as 16-bit values (what its product takes) for as many heads at a time as `scratch`
+ * (16-byte aligned, `scratch_bytes` long, contents lost) holds; with room for less than one
+ * head, or a NULL scratch, the call is ixb_fa_bwd.  ixb_fa_bwd_scratch_bytes says how much of
+ * at most `limit` bytes is of use (0: less than one head fits). */
+size_t ixb_fa_bwd_scratch_bytes(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal,
+                                size_t limit);
+int ixb_fa_bwd_scratch(int dtype, const void* q, const void* k, const void* v, const void* o,
+                       const void* dout, const float* lse, void* dq, void* dk, void* dv,
+                       float* delta, void* scratch, size_t scratch_bytes, int32_t B, int32_t H,
+                       int32_t Sq, int32_t Sk, int32_t D, const int64_t* q_strides,
+                       const int64_t* k_strides, const int64_t* v_strides,
+                       const int64_t* o_strides, const int64_t* do_strides,
+                       const int64_t* dq_strides, const int64_t* dk_strides,
+                       const int64_t* dv_strides, float scale, int causal, int32_t* status,
+                       ixb_stream stream);
+
 /* ---- context-parallel attention merge ---------------------------------------------------- */
 
 /* Fold the partial attention result of one ring step into the running one, (max, sum) form:

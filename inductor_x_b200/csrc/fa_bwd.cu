@@ -5,39 +5,42 @@
 //
 // With P = exp(S * scale - lse), dP = dO V^T, delta = rowsum(dO * O) and
 // dS = P * (dP - delta):   dV = P^T dO,   dK = scale * dS^T Q,   dQ = scale * dS K.
-// Three launches, no atomics, no scratch besides `delta`:
-//   fa_bwd_delta_kernel  delta[b, h, i] (one warp per row)
+// No atomics, one owner for every output, so the bits are the same from run to run:
+//   fa_bwd_delta_kernel  delta[b, h, i] (half a warp per row)
 //   fa_bwd_dkv_kernel    one CTA owns a 128-key tile and walks the query tiles that see it;
 //                        it forms S^T = K Q^T and dP^T = V dO^T (thread <-> key, columns <->
 //                        queries), so that P^T and dS^T - written back over S^T and dP^T as
 //                        16-bit values - are the TMEM operands of dV += P^T dO and
-//                        dK += dS^T Q, which stay in TMEM until the tile is finished
-//   fa_bwd_dq_kernel     one CTA owns a 128-row query tile and walks its key tiles;
-//                        S = Q K^T, dP = dO V^T (thread <-> query), dS over dP, dQ += dS K
-// The probabilities are recomputed in both kernels (7 products instead of 5) - that is what
-// keeps each output with a single owner.
+//                        dK += dS^T Q, which stay in TMEM until the tile is finished.  With
+//                        scratch, four warps copy the 16-bit dS^T to memory
+//   fa_bwd_dq_ds_kernel  one CTA owns two query tiles: dQ += dS K, with dS from memory
+//   fa_bwd_dq_kernel     the same without scratch: S = Q K^T, dP = dO V^T (thread <-> query),
+//                        dS over dP, dQ += dS K - the probabilities are computed once more, seven
+//                        products instead of five
 //
-// Warp 0 is the TMA producer, warp 1 the MMA issuer, the other 4 * NG warps do the
-// element-wise work in NG groups of four warps that split the 128 columns of a tile between
-// them (a warp may only touch the 32 TMEM lanes of its quadrant; no row reduction is needed
-// here - lse and delta come in precomputed - so the split costs nothing).  Every wait is
-// bounded; a wait that gives up raises a flag in `status`, and the CTA exits when the copies
-// and products under way have ended.
+// Warp 0 is the TMA producer, warp 1 the MMA issuer; 4 * NG warps do the element-wise work in NG
+// groups of four warps that split the 128 columns of a tile between them (a warp may only touch the
+// 32 TMEM lanes of its quadrant; no row reduction is needed here - lse and delta come in
+// precomputed - so the split costs nothing).  Every wait is bounded; a wait that gives up raises a
+// flag in `status`, and the CTA exits when the copies and products under way have ended.
 //
-// Bound.  Measured at 8 x 32 heads, 4096 keys, causal, bf16: delta 0.11 ms, dK/dV 2.12 ms, dQ 1.51 ms
-// in a short run; with the element-wise warps only passing the barriers on, the products of the two
-// kernels alone take 1.64 and 1.43 ms, without the exponentials 2.07 and 1.50.  dQ is near the tensor
-// core's time at the power limit.  In dK/dV the element-wise work does not hide behind the products:
-// with one tile in flight the chain scores -> P -> product is serial, and 128-wide double buffering
-// would need more tensor memory than one SM has at this head dimension (two SMs to a tile,
-// cta_group::2, not built).  The products are issued by a whole warp through an elected lane (4426 us
-// a call with one lane issuing, 4200 so, both in a run long enough to sit at the power limit).  Two
-// other ways to overlap more were built and dropped: dS in tensor-memory columns of its own, so that
-// the next scores never wait for the product behind them (dQ 1.51 -> 1.83 ms), and P^T as a
-// shared-memory operand, which frees the score columns earlier but reads another 32 KB of shared
-// memory a step (dK/dV 2.12 -> 2.36 ms).  A variant with 64-query sub-tiles and double-buffered score
-// columns ran 30 % slower: an SS-form MMA with N = 64 takes 48 cycles, not 32, and the hand-offs
-// double.
+// Bound.  In a run of calls the power limit (1000 W, clocks down to 1.5 - 1.7 GHz): at 4 x 32 heads,
+// 4096 keys, causal, bf16 a call took 1865 us (delta 60, dK/dV 1165 - 1190, dQ 825), 1800 with the
+// reworked dK/dV (1000), 1625 with dS kept (dK/dV 1240, dQ 400); 8 heads without a mask, short enough
+// for the full clock: 229, 226, 214; 8 x 16 heads of 1000, no mask: 315, 291, 265.  Keeping dS
+// spares two of seven products and costs 4.4 GB to and from memory at the first of these sizes; what
+// dK/dV loses to its stores (240 us) dQ gains nearly twice.
+// Inside a step of dK/dV the chain is S -> P -> dV, next S: at the full clock 3100 cycles, of which the
+// tensor core works 2048.  What shortened it: P handed over group by group, Q and dO in rings of
+// their own whose copies are asked for before anything else, the statistics of a tile read ahead into
+// registers (with both operands in shared memory a product takes all 128 bytes a cycle of it, and
+// reads beside it are slow).  Two tiles in flight would need more tensor memory than one SM has.
+// Built, measured and dropped: a share of the exponentials on the fma pipe (1049 - 1070 against 1000:
+// the ex2 unit is not the limit, power is); sixteen element-wise warps (the same); dS to memory by way
+// of shared memory and bulk copies (171 against 162 for the 8 heads) or stored by the element-wise
+// warps themselves (184); dS in tensor-memory columns of its own (dQ 1.51 -> 1.83 ms); P^T as a
+// shared-memory operand (dK/dV 2.12 -> 2.36 ms); 64-query sub-tiles (30 % slower: an SS-form MMA with
+// N = 64 takes 48 cycles, not 32).
 #include <atomic>
 #include "fa_maps.h"
 #include "ixb/tcgen05.cuh"
@@ -56,6 +59,11 @@ constexpr int NG = 2;             // groups of element-wise warps; each takes 12
 constexpr int GC = 128 / NG;      // columns per group
 constexpr int kWorkers = 128 * NG;
 constexpr int kThreads = 64 + kWorkers;
+constexpr int kDkvThreads = 128 * (2 + NG);  // dK/dV: issuers, element-wise groups, dS stores: a warpgroup each
+// Registers of the dK/dV kernel: launched with what 16 warps can have; the element-wise warps hold a
+// tile's statistics besides its scores.
+constexpr int kRegsLaunch = 128, kRegsIssue = 80, kRegsWork = 168, kRegsStore = 96;
+static_assert(kRegsIssue + NG * kRegsWork + kRegsStore <= (2 + NG) * kRegsLaunch, "setmaxnreg draws on the block's own registers");
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColS = 0, kColDP = 128, kColAcc0 = 256, kColAcc1 = 384;
 constexpr size_t kSmemBytes = (size_t)kTileBytes * 6 + 1024;
@@ -73,7 +81,24 @@ struct BwdParams {
   float scale, scale_log2;
   int causal;
   int head_group;
+  unsigned char* ds;   // tiles of dS^T of the heads of this launch (see ds_tile), or null
+  int bh0, n_bh;       // first head of this launch and how many (all of them where dS is not kept)
+  int tiles_per_head;  // tiles of dS^T a head has
 };
+
+// dS^T goes to memory in tiles of 128 keys x 128 queries of 16-bit values, every tile in the form in
+// which it is read back as a shared-memory operand: 16-byte pieces of 8 queries of one key, piece
+// ((key / 32) * 16 + query / 8) * 32 + key % 32.  A warp (32 keys) stores 512 contiguous bytes an
+// instruction, a tile is one 32 KB bulk copy.  Only tiles that some query of the tile sees are kept,
+// key tile by key tile.
+// Tile (kv, i) of a head: key tile kv sees query tiles from kv - hide on.
+__host__ __device__ __forceinline__ int hidden_tiles(int causal, int Sq, int Sk, int n_kv_tiles) {
+  return causal ? (Sk - Sq + 127) / 128 : n_kv_tiles;  // kv <= hide: every query tile
+}
+__host__ __device__ __forceinline__ long long ds_tile(int kv, int i, int n_q_tiles, int hide) {
+  const long long u = kv > hide + 1 ? kv - 1 - hide : 0;  // query tiles that key tiles before kv do not see
+  return (long long)kv * n_q_tiles - u * (u + 1) / 2 + i - (kv > hide ? kv - hide : 0);
+}
 
 __device__ __forceinline__ uint32_t pack_pair(float lo, float hi, bool is_bf16) {
   if (is_bf16) {
@@ -157,6 +182,12 @@ __device__ __forceinline__ void issue_ts(uint32_t d, uint32_t a, uint64_t b_desc
     tc::product_ts<GC / 16>(d, a + g * GC, b_desc_mn + (uint32_t)(g * GC * 128 >> 4), idesc, (accumulate || g > 0) ? 1u : 0u);
 }
 
+// The part of it that group G's values make.
+template <int G>
+__device__ __forceinline__ void issue_ts_group(uint32_t d, uint32_t a, uint64_t b_desc_mn, uint32_t idesc, bool accumulate) {
+  tc::product_ts<GC / 16>(d, a + G * GC, b_desc_mn + (uint32_t)(G * GC * 128 >> 4), idesc, accumulate ? 1u : 0u);
+}
+
 // GC accumulator columns of this thread's row -> 16-bit values in global memory
 template <bool IS_BF16>
 __device__ __forceinline__ void store_cols(uint32_t taddr, unsigned char* dst, float mult, bool live) {
@@ -182,7 +213,7 @@ __device__ __forceinline__ void store_cols(uint32_t taddr, unsigned char* dst, f
 // ------------------------------------------------------------------------------ dK, dV
 // TMEM columns: [0,128) S^T then P^T, [128,256) dP^T then dS^T, [256,384) dV, [384,512) dK.
 template <bool IS_BF16>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kDkvThreads, 1)
     fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                       const BwdParams p) {
@@ -194,9 +225,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* q_smem = smem + 2 * kTileBytes;   // kStages tiles
   unsigned char* do_smem = smem + 4 * kTileBytes;  // kStages tiles
 
-  __shared__ __align__(8) uint64_t kv_full, qdo_full[kStages], qdo_empty[kStages], s_full, dp_full, p_full,
-      ds_full, acc_done, drained;
-  __shared__ __align__(16) float lse_s[kStages][BM], delta_s[kStages][BM];
+  __shared__ __align__(8) uint64_t kv_full, q_full[kStages], q_empty[kStages], do_full[kStages], do_empty[kStages],
+      s_full, dp_full, p_full[NG], ds_full, ds_read, acc_done, drained;
+  // of a query tile: -lse in log2 units (-inf past the end: P = 0) and -delta
+  __shared__ __align__(16) float nlse_s[kStages][BM], ndelta_s[kStages][BM];
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
@@ -206,7 +238,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int n_kv_tiles = (p.Sk + BN - 1) / BN;
   const int n_q_tiles = (p.Sq + BM - 1) / BM;
   int kv_tile, bh;
-  cta_order(n_kv_tiles, p.B * p.H, p.head_group, &kv_tile, &bh);  // early key tiles see the most queries
+  cta_order(n_kv_tiles, p.n_bh, p.head_group, &kv_tile, &bh);  // early key tiles see the most queries
+  const int hide = hidden_tiles(p.causal, p.Sq, p.Sk, n_kv_tiles);
+  unsigned char* ds_head = p.ds + (long long)bh * p.tiles_per_head * kTileBytes;
+  const bool keep_ds = p.ds != nullptr;
+  bh += p.bh0;
   const int b = bh / p.H, h = bh % p.H;
   const int kt0 = kv_tile * BN;
   const int diag = p.Sk - p.Sq;  // key j is visible to query i when j <= i + diag
@@ -220,13 +256,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (threadIdx.x == 0) {
     mbar_init(&kv_full, 1);
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&qdo_full[s], 1);
-      mbar_init(&qdo_empty[s], 1);
+      mbar_init(&q_full[s], 2);  // the copy and the statistics
+      mbar_init(&q_empty[s], 1);
+      mbar_init(&do_full[s], 1);
+      mbar_init(&do_empty[s], 1);
     }
     mbar_init(&s_full, 1);
     mbar_init(&dp_full, 1);
-    mbar_init(&p_full, kWorkers / 32);
+    for (int g = 0; g < NG; ++g) mbar_init(&p_full[g], 4);
     mbar_init(&ds_full, kWorkers / 32);
+    mbar_init(&ds_read, 4);
     mbar_init(&acc_done, 1);
     mbar_init(&drained, 1);
     failed = 0;
@@ -238,7 +277,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
 
-  int loads = 0;  // producer: query tiles it has asked for
+  int q_loads = 0, do_loads = 0;  // producer: query tiles it has asked for
+  if (warp < 4) tc::regs_dec<kRegsIssue>();
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0 && n_it > 0) {
@@ -246,33 +286,44 @@ __global__ void __launch_bounds__(kThreads, 1)
       load_tile(k_smem, &map_k, &kv_full, kt0, h, b);
       load_tile(v_smem, &map_v, &kv_full, kt0, h, b);
     }
+    // the statistics of a tile are read a tile ahead, so that nothing waits for that read
+    float lse_r[4], delta_r[4];
+    auto read_stats = [&](int qt0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int qi = qt0 + e * 32 + lane;
+        const long long at = (long long)bh * p.Sq + qi;
+        lse_r[e] = qi < p.Sq ? p.lse[at] * -kLog2e : -INFINITY;
+        delta_r[e] = qi < p.Sq ? -p.delta[at] : 0.f;
+      }
+    };
+    read_stats(i0 * BM);
     bool ok = true;
     for (int it = 0; it < n_it && ok; ++it) {
       const int s = it % kStages, n = it / kStages;
       const int qt0 = (i0 + it) * BM;
-      if (n > 0) {
-        int mine = 1;
-        if (lane == 0) mine = mbar_wait(&qdo_empty[s], (n - 1) & 1, &failed) ? 1 : 0;
-        ok = __shfl_sync(kFull, mine, 0) != 0;
-        if (!ok) break;
+      if (n > 0) ok = __all_sync(kFull, mbar_wait(&q_empty[s], (n - 1) & 1, &failed));
+      if (!ok) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&q_full[s], kTileBytes);
+        load_tile(q_smem + (size_t)s * kTileBytes, &map_q, &q_full[s], qt0, h, b);
       }
-      // per-query statistics of the tile: lse in log2 units (+inf past the end: P = 0), delta
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int r = lane * 4 + e;
-        const int qi = qt0 + r;
-        const bool live = qi < p.Sq;
-        const long long at = (long long)bh * p.Sq + qi;
-        lse_s[s][r] = live ? p.lse[at] * kLog2e : INFINITY;
-        delta_s[s][r] = live ? p.delta[at] : 0.f;
+        nlse_s[s][e * 32 + lane] = lse_r[e];
+        ndelta_s[s][e * 32 + lane] = delta_r[e];
       }
       __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&q_full[s]);
+      q_loads = it + 1;
+      if (it + 1 < n_it) read_stats(qt0 + BM);
+      if (n > 0) ok = __all_sync(kFull, mbar_wait(&do_empty[s], (n - 1) & 1, &failed));
+      if (!ok) break;
       if (lane == 0) {
-        mbar_arrive_expect_tx(&qdo_full[s], 2 * kTileBytes);
-        load_tile(q_smem + (size_t)s * kTileBytes, &map_q, &qdo_full[s], qt0, h, b);
-        load_tile(do_smem + (size_t)s * kTileBytes, &map_do, &qdo_full[s], qt0, h, b);
+        mbar_arrive_expect_tx(&do_full[s], kTileBytes);
+        load_tile(do_smem + (size_t)s * kTileBytes, &map_do, &do_full[s], qt0, h, b);
       }
-      loads = it + 1;
+      do_loads = it + 1;
     }
     if (!ok && lane == 0) failed = 1;
     __syncwarp();
@@ -291,36 +342,46 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
       const uint32_t t_s = tmem + kColS, t_dp = tmem + kColDP;
       const uint32_t t_dv = tmem + kColAcc0, t_dk = tmem + kColAcc1;
-      bool ok = __all_sync(kFull, mbar_wait(&kv_full, 0, &failed));
-      ok = ok && __all_sync(kFull, mbar_wait(&qdo_full[0], 0, &failed));
-      if (ok) {
+      auto wait = [&](uint64_t* bar, int parity) {
+        const bool up = __all_sync(kFull, mbar_wait(bar, parity, &failed));
         tc::fence_after_sync();
+        return up;
+      };
+      bool ok = wait(&kv_full, 0) && wait(&q_full[0], 0);
+      if (ok) {
         issue_ss(t_s, k_desc, q_desc, idesc_kk);  // S^T = K Q^T
         tc::commit_elected(&s_full);
+        ok = wait(&do_full[0], 0);
+      }
+      if (ok) {
         issue_ss(t_dp, v_desc, do_desc, idesc_kk);  // dP^T = V dO^T
         tc::commit_elected(&dp_full);
       }
       for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it & 1, s1 = (it + 1) & 1;
+        const int s = it & 1, s1 = (it + 1) & 1, n1 = (it + 1) >> 1;
         const bool next = it + 1 < n_it;
-        ok = __all_sync(kFull, mbar_wait(&p_full, it & 1, &failed));
+        // dV += P^T dO in two parts: of the two groups, which share the ex2 unit, one is ahead
+        ok = wait(&p_full[0], it & 1);
         if (!ok) break;
-        tc::fence_after_sync();
-        issue_ts(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, it > 0);  // dV += P^T dO
+        issue_ts_group<0>(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, it > 0);
+        ok = wait(&p_full[1], it & 1);
+        if (!ok) break;
+        issue_ts_group<1>(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, true);
+        tc::commit_elected(&do_empty[s]);
         if (next) {
-          ok = __all_sync(kFull, mbar_wait(&qdo_full[s1], ((it + 1) >> 1) & 1, &failed));
+          ok = wait(&q_full[s1], n1 & 1);
           if (!ok) break;
-          tc::fence_after_sync();
           // the tensor core runs its MMAs in order: P^T has been consumed when this one starts
           issue_ss(t_s, k_desc, q_desc + s1 * kStep, idesc_kk);
           tc::commit_elected(&s_full);
         }
-        ok = __all_sync(kFull, mbar_wait(&ds_full, it & 1, &failed));
+        ok = wait(&ds_full, it & 1);
         if (!ok) break;
-        tc::fence_after_sync();
         issue_ts(t_dk, t_dp, q_desc_mn + s * kStep, idesc_mn, it > 0);  // dK += dS^T Q
-        tc::commit_elected(&qdo_empty[s]);
+        tc::commit_elected(&q_empty[s]);
         if (next) {
+          ok = wait(&do_full[s1], n1 & 1) && (!keep_ds || wait(&ds_read, it & 1));
+          if (!ok) break;
           issue_ss(t_dp, v_desc, do_desc + s1 * kStep, idesc_kk);
           tc::commit_elected(&dp_full);
         }
@@ -329,9 +390,38 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok && lane == 0) failed = 1;
     }
     __syncwarp();
-  } else {
+  } else if (warp >= 4 + 4 * NG) {
+    tc::regs_dec<kRegsStore>();
+    // ------------------------------------------------------------------ dS to memory
+    // Warps of their own read the 16-bit dS^T once more from tensor memory: the element-wise warps
+    // are what a step waits for, and shared memory, by way of which a bulk copy would go, is the
+    // products' (see the head of this file).
+    const int quad = warp & 3;
+    const uint32_t dp_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + kColDP;
+    bool ok = true;
+    for (int it = 0; it < n_it && keep_ds; ++it) {
+      ok = __all_sync(kFull, mbar_wait(&ds_full, it & 1, &failed));
+      if (!ok) break;
+      tc::fence_after_sync();
+      uint32_t d[NG][GC / 2];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) tc::tmem_ld32(dp_addr + GC * g, d[g]);
+      tc::tmem_wait_ld();
+      tc::fence_before_sync();
+      warp_arrive(&ds_read, lane);
+      uint4* dst = reinterpret_cast<uint4*>(ds_head + ds_tile(kv_tile, i0 + it, n_q_tiles, hide) * kTileBytes) +
+                   quad * (BM / 8) * 32 + lane;
+#pragma unroll
+      for (int u = 0; u < BM / 8; ++u) {
+        const uint32_t* w = &d[u * 8 / GC][(u * 4) % (GC / 2)];
+        __stcs(dst + u * 32, make_uint4(w[0], w[1], w[2], w[3]));
+      }
+    }
+    if (!ok) failed = 1;
+  } else if (warp >= 4) {
     // ------------------------------------------------------------------ element-wise work
-    const int g = (warp - 2) >> 2;  // group: query columns [GC g, GC g + GC) of a tile
+    tc::regs_inc<kRegsWork>();
+    const int g = (warp - 4) >> 2;  // group: query columns [GC g, GC g + GC) of a tile
     const int quad = warp & 3;
     const int row = quad * 32 + lane;  // key inside the tile
     const int kj = kt0 + row;
@@ -344,77 +434,81 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int it = 0; it < n_it; ++it) {
       const int s = it & 1;
       const int qt0 = (i0 + it) * BM;
-      bool w = mbar_wait(&qdo_full[s], (it >> 1) & 1, &failed);
-      w = w && mbar_wait(&s_full, it & 1, &failed);
-      if (!__all_sync(kFull, w)) {
+      // the tile's statistics come into registers ahead of its scores: shared memory is busy with
+      // the products' operands, and every read of it is slow
+      float4 stat[GC / 4];
+      bool w = __all_sync(kFull, mbar_wait(&q_full[s], (it >> 1) & 1, &failed));
+      if (w) {
+#pragma unroll
+        for (int e = 0; e < GC / 4; ++e) stat[e] = *reinterpret_cast<const float4*>(&nlse_s[s][GC * g + 4 * e]);
+        w = __all_sync(kFull, mbar_wait(&s_full, it & 1, &failed));
+      }
+      if (!w) {
         ok = false;
         break;
       }
       tc::fence_after_sync();
-      // query column e of this group is visible to key kj when qt0 + GC g + e >= kj - diag
-      const bool edge = p.causal && (kt0 + BN - 1 > qt0 + diag);
-      const int lo = edge ? kj - diag - (qt0 + GC * g) : 0;
-      const float* lse_row = &lse_s[s][GC * g];
-      float pr[GC];
+      // query column e of this group is visible to key kj when qt0 + GC g + e >= kj - diag; a row
+      // past the last key has no gradients of its own, but its dS would meet zeros of K in dQ
+      // (and need not be finite)
+      const bool edge = (kt0 + BN > p.Sk) || (p.causal && (kt0 + BN - 1 > qt0 + diag));
+      const int lo = !edge ? 0 : kj >= p.Sk ? GC : p.causal ? kj - diag - (qt0 + GC * g) : 0;
+      uint32_t raw[GC];
 #pragma unroll
-      for (int c = 0; c < GC / 32; ++c) {
-        uint32_t raw[32];
-        tc::tmem_ld32(s_addr + c * 32, raw);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(lse_row + c * 32 + e);
-          const float2 a0 = fma2(make_float2(__uint_as_float(raw[e]), __uint_as_float(raw[e + 1])), sc2,
-                                 make_float2(-l4.x, -l4.y));
-          const float2 a1 = fma2(make_float2(__uint_as_float(raw[e + 2]), __uint_as_float(raw[e + 3])), sc2,
-                                 make_float2(-l4.z, -l4.w));
-          float* o = &pr[c * 32 + e];
-          o[0] = fast_exp2(a0.x);
-          o[1] = fast_exp2(a0.y);
-          o[2] = fast_exp2(a1.x);
-          o[3] = fast_exp2(a1.y);
-          if (edge) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (c * 32 + e + u < lo) o[u] = 0.f;
-          }
-        }
-      }
-      // all of this group's S columns are in registers: P^T goes over their first half
+      for (int c = 0; c < GC / 32; ++c) tc::tmem_ld32(s_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
+      tc::tmem_wait_ld();
+      float2 pr[GC / 2];
 #pragma unroll
       for (int c = 0; c < GC / 32; ++c) {
         uint32_t pk[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) pk[e] = pack_pair(pr[c * 32 + 2 * e], pr[c * 32 + 2 * e + 1], IS_BF16);
+        for (int e = 0; e < 32; e += 4) {
+          const float4 l4 = stat[c * 8 + e / 4];
+          const float2 l2[2] = {make_float2(l4.x, l4.y), make_float2(l4.z, l4.w)};
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int at = c * 32 + e + 2 * u;
+            const float2 a = fma2(make_float2(__uint_as_float(raw[at]), __uint_as_float(raw[at + 1])), sc2, l2[u]);
+            float2 x = make_float2(fast_exp2(a.x), fast_exp2(a.y));
+            if (edge) {
+              if (at < lo) x.x = 0.f;
+              if (at + 1 < lo) x.y = 0.f;
+            }
+            pr[at / 2] = x;
+            pk[e / 2 + u] = pack_pair(x.x, x.y, IS_BF16);
+          }
+        }
+        // all of this group's S columns are in registers: P^T goes over their first half
         tc::tmem_st16(s_addr + c * 16, pk);
       }
       tc::tmem_wait_st();
       tc::fence_before_sync();
-      warp_arrive(&p_full, lane);
+      warp_arrive(&p_full[g], lane);
+#pragma unroll
+      for (int e = 0; e < GC / 4; ++e) stat[e] = *reinterpret_cast<const float4*>(&ndelta_s[s][GC * g + 4 * e]);
 
       if (!__all_sync(kFull, mbar_wait(&dp_full, it & 1, &failed))) {
         ok = false;
         break;
       }
       tc::fence_after_sync();
-      const float* delta_row = &delta_s[s][GC * g];
+#pragma unroll
+      for (int c = 0; c < GC / 32; ++c) tc::tmem_ld32(dp_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
+      tc::tmem_wait_ld();
 #pragma unroll
       for (int c = 0; c < GC / 32; ++c) {
-        uint32_t d[32];
-        tc::tmem_ld32(dp_addr + c * 32, d);
-        tc::tmem_wait_ld();
         uint32_t pk[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
-          const float4 d4 = *reinterpret_cast<const float4*>(delta_row + c * 32 + e);
-          const float x0 = pr[c * 32 + e] * (__uint_as_float(d[e]) - d4.x);
-          const float x1 = pr[c * 32 + e + 1] * (__uint_as_float(d[e + 1]) - d4.y);
-          const float x2 = pr[c * 32 + e + 2] * (__uint_as_float(d[e + 2]) - d4.z);
-          const float x3 = pr[c * 32 + e + 3] * (__uint_as_float(d[e + 3]) - d4.w);
-          pk[e / 2] = pack_pair(x0, x1, IS_BF16);
-          pk[e / 2 + 1] = pack_pair(x2, x3, IS_BF16);
+          const float4 d4 = stat[c * 8 + e / 4];
+          const float2 d2[2] = {make_float2(d4.x, d4.y), make_float2(d4.z, d4.w)};
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int at = c * 32 + e + 2 * u;
+            const float2 x = mul2(pr[at / 2], add2(make_float2(__uint_as_float(raw[at]), __uint_as_float(raw[at + 1])), d2[u]));
+            pk[e / 2 + u] = pack_pair(x.x, x.y, IS_BF16);
+          }
         }
-        // columns [16c, 16c+16) of this group: their dP values are already in registers
         tc::tmem_st16(dp_addr + c * 16, pk);
       }
       tc::tmem_wait_st();
@@ -456,7 +550,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     // a role gave up: what the others have under way has to end before the block does
     if (threadIdx.x == 0) {
       tc::await_copies<1>(&kv_full, 1);
-      tc::await_copies<kStages>(qdo_full, loads);
+      tc::await_copies<kStages>(q_full, q_loads);
+      tc::await_copies<kStages>(do_full, do_loads);
     }
     if (warp == 1) tc::await_products(&drained);
     __syncthreads();
@@ -494,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const int n_q_tiles = (p.Sq + BM - 1) / BM;
   int slot, bh;
-  cta_order(n_q_tiles, p.B * p.H, p.head_group, &slot, &bh);
+  cta_order(n_q_tiles, p.n_bh, p.head_group, &slot, &bh);
   const int q_tile = n_q_tiles - 1 - slot;  // late query tiles see the most keys: first
   const int b = bh / p.H, h = bh % p.H;
   const int qt0 = q_tile * BM;
@@ -710,9 +805,170 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// ------------------------------------------------------------------ dQ from kept dS
+// One CTA owns two query tiles of a head and walks the key tiles they see: dQ += dS K, with the
+// tiles of dS^T as the first operand (MN-major, no swizzle) and K in MN-major form.  Bound: the 32 KB
+// of dS a product reads; two query tiles share a K tile, which comes from L2.  2.2 GB of dS (4 x 32
+// heads of 4096, causal) in 400 us, 5500 GB/s.  TMEM: 2 x 128 columns.
+constexpr int kQT = 2;        // query tiles a CTA
+constexpr int kDsStages = 4;  // tiles of dS^T in flight
+constexpr int kDsThreads = 64 + 128;
+template <bool IS_BF16>
+__global__ void __launch_bounds__(kDsThreads, 1)
+    fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap map_k, const BwdParams p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* k_smem = smem;                    // kStages tiles
+  unsigned char* ds_smem = smem + 2 * kTileBytes;  // kDsStages tiles
+
+  __shared__ __align__(8) uint64_t k_full[kStages], k_empty[kStages], ds_full[kDsStages], ds_empty[kDsStages],
+      acc_done, drained;
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ volatile int failed;
+
+  const int warp = __shfl_sync(kFull, (int)threadIdx.x >> 5, 0);  // known uniform to the compiler
+  const int lane = threadIdx.x & 31;
+
+  const int n_q_tiles = (p.Sq + BM - 1) / BM;
+  const int n_kv_tiles = (p.Sk + BN - 1) / BN;
+  const int n_slots = (n_q_tiles + kQT - 1) / kQT;
+  int slot, bh;
+  cta_order(n_slots, p.n_bh, p.head_group, &slot, &bh);
+  bh = p.n_bh - 1 - bh;  // the last heads first: some of their dS is still in L2
+  const int first = (n_slots - 1 - slot) * kQT;  // late query tiles see the most keys: first
+  const int tiles = min(kQT, n_q_tiles - first);
+  const int hide = hidden_tiles(p.causal, p.Sq, p.Sk, n_kv_tiles);
+  const unsigned char* ds_head = p.ds + (long long)bh * p.tiles_per_head * kTileBytes;
+  bh += p.bh0;
+  const int b = bh / p.H, h = bh % p.H;
+  // key tiles that the first query tile sees, and that either sees
+  const int n_kv0 = p.causal ? min(n_kv_tiles, first + hide + 1) : n_kv_tiles;
+  const int n_kv = p.causal ? min(n_kv_tiles, first + tiles + hide) : n_kv_tiles;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
+    }
+    for (int s = 0; s < kDsStages; ++s) {
+      mbar_init(&ds_full[s], 1);
+      mbar_init(&ds_empty[s], 1);
+    }
+    mbar_init(&acc_done, 1);
+    mbar_init(&drained, 1);
+    failed = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) tc::tmem_alloc(&tmem_base_slot, kQT * 128);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem_base = tmem_base_slot;
+
+  int k_loads = 0, ds_loads = 0;  // producer: key and dS tiles it has asked for
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (lane == 0) {
+      bool ok = true;
+      for (int j = 0; j < n_kv && ok; ++j) {
+        const int s = j % kStages, n = j / kStages;
+        if (n > 0) ok = mbar_wait(&k_empty[s], (n - 1) & 1, &failed);
+        if (!ok) break;
+        mbar_arrive_expect_tx(&k_full[s], kTileBytes);
+        load_tile(k_smem + (size_t)s * kTileBytes, &map_k, &k_full[s], j * BN, h, b);
+        k_loads = j + 1;
+        for (int t = j < n_kv0 ? 0 : 1; t < tiles; ++t) {
+          const int u = ds_loads % kDsStages, m = ds_loads / kDsStages;
+          if (m > 0) ok = mbar_wait(&ds_empty[u], (m - 1) & 1, &failed);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&ds_full[u], kTileBytes);
+          bulk_g2s(ds_smem + (size_t)u * kTileBytes, ds_head + ds_tile(j, first + t, n_q_tiles, hide) * kTileBytes,
+                   kTileBytes, &ds_full[u]);
+          ++ds_loads;
+        }
+      }
+      if (!ok) failed = 1;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    constexpr uint32_t idesc = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 1, 1);
+    const uint64_t k_desc = tc::smem_desc(smem_u32(k_smem), kHalfBytes, 1024);
+    // 8 keys to the next 8: 128 bytes; 8 queries to the next 8: 32 pieces
+    const uint64_t ds_desc = tc::smem_desc_plain(smem_u32(ds_smem), 128, 32 * 16);
+    constexpr uint32_t kStep = kTileBytes >> 4;
+    const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
+    bool ok = true;
+    int n = 0;  // tiles of dS consumed
+    for (int j = 0; j < n_kv && ok; ++j) {
+      const int s = j % kStages;
+      ok = __all_sync(kFull, mbar_wait(&k_full[s], (j / kStages) & 1, &failed));
+      for (int t = j < n_kv0 ? 0 : 1; t < tiles && ok; ++t, ++n) {
+        const int u = n % kDsStages;
+        ok = __all_sync(kFull, mbar_wait(&ds_full[u], (n / kDsStages) & 1, &failed));
+        if (!ok) break;
+        tc::fence_after_sync();
+        // 16 keys a step: 256 bytes inside 32 keys of a dS tile, 16 rows (2048 bytes) of K
+#pragma unroll
+        for (int kq = 0; kq < 4; ++kq)
+          tc::product_ss_steps<2, 256, 2048>(tmem + 128 * t, ds_desc + u * kStep + kq * (kTileBytes / 4 >> 4),
+                                             k_desc + s * kStep + kq * (2 * 2048 >> 4), idesc, j > 0 || kq > 0 ? 1u : 0u);
+        tc::commit_elected(&ds_empty[u]);
+      }
+      if (ok) tc::commit_elected(&k_empty[s]);
+    }
+    if (ok) tc::commit_elected(&acc_done);
+    if (!ok && lane == 0) failed = 1;
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ results
+    const int quad = warp & 3;
+    bool ok = mbar_wait(&acc_done, 0, &failed);
+    ok = __all_sync(kFull, ok);
+    if (ok) {
+      tc::fence_after_sync();
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+      for (int t = 0; t < tiles; ++t) {
+        const int qi = (first + t) * BM + quad * 32 + lane;
+        unsigned char* dq_row = reinterpret_cast<unsigned char*>(p.dq.ptr) +
+                                2 * ((long long)b * p.dq.sb + (long long)h * p.dq.sh + (long long)qi * p.dq.ss);
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+          store_cols<IS_BF16>(lane_addr + 128 * t + GC * g, dq_row + 2 * GC * g, p.scale, qi < p.Sq);
+      }
+    } else {
+      failed = 1;
+    }
+  }
+
+  tc::fence_before_sync();
+  __syncthreads();
+  if (failed) {  // (as above)
+    if (threadIdx.x == 0) {
+      tc::await_copies<kStages>(k_full, k_loads);
+      tc::await_copies<kDsStages>(ds_full, ds_loads);
+    }
+    if (warp == 1) tc::await_products(&drained);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && failed && p.status != nullptr) atomicExch(p.status, 1);
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem_base, kQT * 128);
+  }
+}
+
+// `regs`: the registers a thread that a kernel with a register split has to be launched with, or 0.
 template <class K>
-int opt_in_smem(K kern, std::atomic<bool>& done) {
+int opt_in_smem(K kern, std::atomic<bool>& done, int regs = 0) {
   if (!done.load(std::memory_order_acquire)) {
+    if (regs != 0) {
+      cudaFuncAttributes at;
+      cudaError_t e = cudaFuncGetAttributes(&at, kern);
+      if (e != cudaSuccess) return ixb_host::cuda_status(e);
+      if (at.numRegs != regs) return IXB_ERR_UNSUPPORTED;
+    }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return ixb_host::cuda_status(e);
     done.store(true, std::memory_order_release);
@@ -720,18 +976,34 @@ int opt_in_smem(K kern, std::atomic<bool>& done) {
   return IXB_OK;
 }
 
+// Tiles of dS^T one head has.
+long long tiles_of_head(int Sq, int Sk, int causal) {
+  const int n_q = (int)((Sq + (long long)BM - 1) / BM), n_kv = (int)((Sk + (long long)BN - 1) / BN);
+  return ds_tile(n_kv - 1, n_q - 1, n_q, hidden_tiles(causal, Sq, Sk, n_kv)) + 1;
+}
+
 }  // namespace
 
-extern "C" int ixb_fa_bwd(int dtype, const void* q, const void* k, const void* v, const void* o,
-                          const void* dout, const float* lse, void* dq, void* dk, void* dv, float* delta,
-                          int32_t B, int32_t H, int32_t Sq, int32_t Sk, int32_t D, const int64_t* q_strides,
-                          const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides,
-                          const int64_t* do_strides, const int64_t* dq_strides, const int64_t* dk_strides,
-                          const int64_t* dv_strides, float scale, int causal, int32_t* status,
-                          ixb_stream stream) {
+extern "C" size_t ixb_fa_bwd_scratch_bytes(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, size_t limit) {
+  if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0 || (causal && Sk < Sq)) return 0;
+  const long long n_bh = (long long)B * H, tiles = tiles_of_head(Sq, Sk, causal != 0);
+  const long long fit = (long long)(limit / kTileBytes) / tiles;  // heads within the limit
+  if (fit <= 0 || tiles > 0x7fffffffLL) return 0;
+  const long long launches = (n_bh + fit - 1) / fit;
+  return (size_t)((n_bh + launches - 1) / launches * tiles) * kTileBytes;
+}
+
+extern "C" int ixb_fa_bwd_scratch(int dtype, const void* q, const void* k, const void* v, const void* o,
+                                  const void* dout, const float* lse, void* dq, void* dk, void* dv, float* delta,
+                                  void* scratch, size_t scratch_bytes, int32_t B, int32_t H, int32_t Sq, int32_t Sk,
+                                  int32_t D, const int64_t* q_strides, const int64_t* k_strides,
+                                  const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
+                                  const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides,
+                                  float scale, int causal, int32_t* status, ixb_stream stream) {
   if (B < 0 || H < 0 || Sq < 0 || Sk < 0) return IXB_ERR_ARG;
   if (B == 0 || H == 0 || Sq == 0 || Sk == 0) return IXB_OK;
   if (!q || !k || !v || !o || !dout || !lse || !dq || !dk || !dv || !delta) return IXB_ERR_ARG;
+  if (!ixb_host::aligned16(scratch)) return IXB_ERR_ALIGN;
   if (dtype != IXB_BF16 && dtype != IXB_F16) return IXB_ERR_DTYPE;
   if (D != HD) return IXB_ERR_SHAPE;
   if (causal && Sk < Sq) return IXB_ERR_SHAPE;
@@ -775,18 +1047,48 @@ extern "C" int ixb_fa_bwd(int dtype, const void* q, const void* k, const void* v
   auto kern_delta = is_bf16 ? fa_bwd_delta_kernel<true> : fa_bwd_delta_kernel<false>;
   auto kern_dkv = is_bf16 ? fa_bwd_dkv_kernel<true> : fa_bwd_dkv_kernel<false>;
   auto kern_dq = is_bf16 ? fa_bwd_dq_kernel<true> : fa_bwd_dq_kernel<false>;
-  static std::atomic<bool> configured[2][2][64];
+  auto kern_dq_ds = is_bf16 ? fa_bwd_dq_ds_kernel<true> : fa_bwd_dq_ds_kernel<false>;
+  static std::atomic<bool> configured[3][2][64];
   int devid = 0;
   cudaGetDevice(&devid);
-  if (int st = opt_in_smem(kern_dkv, configured[0][is_bf16][devid & 63])) return st;
+  if (int st = opt_in_smem(kern_dkv, configured[0][is_bf16][devid & 63], kRegsLaunch)) return st;
   if (int st = opt_in_smem(kern_dq, configured[1][is_bf16][devid & 63])) return st;
+  if (int st = opt_in_smem(kern_dq_ds, configured[2][is_bf16][devid & 63])) return st;
+
+  // The heads go in as many equal launches as the scratch asks for; without room for one head's dS the
+  // probabilities are recomputed for dQ.
+  const long long tiles = tiles_of_head(Sq, Sk, p.causal);
+  const long long fit = scratch != nullptr && tiles <= 0x7fffffffLL ? (long long)(scratch_bytes / kTileBytes) / tiles : 0;
+  const long long launches = fit > 0 ? (n_bh + fit - 1) / fit : 1;
+  const long long heads = (n_bh + launches - 1) / launches;
+  p.ds = fit > 0 ? static_cast<unsigned char*>(scratch) : nullptr;
+  p.tiles_per_head = fit > 0 ? (int)tiles : 0;
 
   cudaStream_t cs = (cudaStream_t)stream;
   const long long rows = n_bh * Sq;
   kern_delta<<<(unsigned)((rows + 15) / 16), 256, 0, cs>>>(
       static_cast<const unsigned char*>(o), static_cast<const unsigned char*>(dout), delta, H, Sq, rows,
       o_strides[0], o_strides[1], o_strides[2], do_strides[0], do_strides[1], do_strides[2]);
-  kern_dkv<<<(unsigned)(n_kv_tiles * n_bh), kThreads, kSmemBytes, cs>>>(mq, mk, mv, mdo, p);
-  kern_dq<<<(unsigned)(n_q_tiles * n_bh), kThreads, kSmemBytes, cs>>>(mq, mk, mv, mdo, p);
+  for (long long at = 0; at < n_bh; at += heads) {
+    p.bh0 = (int)at;
+    p.n_bh = (int)(heads < n_bh - at ? heads : n_bh - at);
+    kern_dkv<<<(unsigned)(n_kv_tiles * p.n_bh), kDkvThreads, kSmemBytes, cs>>>(mq, mk, mv, mdo, p);
+    if (fit > 0)
+      kern_dq_ds<<<(unsigned)((n_q_tiles + kQT - 1) / kQT * p.n_bh), kDsThreads, kSmemBytes, cs>>>(mk, p);
+    else
+      kern_dq<<<(unsigned)(n_q_tiles * p.n_bh), kThreads, kSmemBytes, cs>>>(mq, mk, mv, mdo, p);
+  }
   return ixb_host::cuda_status(cudaGetLastError());
+}
+
+extern "C" int ixb_fa_bwd(int dtype, const void* q, const void* k, const void* v, const void* o,
+                          const void* dout, const float* lse, void* dq, void* dk, void* dv, float* delta,
+                          int32_t B, int32_t H, int32_t Sq, int32_t Sk, int32_t D, const int64_t* q_strides,
+                          const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides,
+                          const int64_t* do_strides, const int64_t* dq_strides, const int64_t* dk_strides,
+                          const int64_t* dv_strides, float scale, int causal, int32_t* status,
+                          ixb_stream stream) {
+  return ixb_fa_bwd_scratch(dtype, q, k, v, o, dout, lse, dq, dk, dv, delta, nullptr, 0, B, H, Sq, Sk, D, q_strides,
+                            k_strides, v_strides, o_strides, do_strides, dq_strides, dk_strides, dv_strides, scale,
+                            causal, status, stream);
 }

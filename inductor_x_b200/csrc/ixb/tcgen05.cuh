@@ -23,6 +23,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t lbo_b
   return d;
 }
 
+// the same without a swizzle: 8 x 8 blocks of 128 contiguous bytes
+__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return smem_desc(smem_addr, lbo_bytes, sbo_bytes) & ~((uint64_t)7 << 61);
+}
+
 // ---- instruction descriptor for kind::f16 (fp32 accumulate) ---------------------------
 // is_bf16: operand format (0 = f16, 1 = bf16); *_mn_major: 0 = K-major, 1 = MN-major.
 __host__ __device__ constexpr uint32_t instr_desc(int m, int n, int is_bf16, int a_mn_major,
@@ -106,6 +111,26 @@ template <int N> __device__ __forceinline__ void product_ts(uint32_t d_tmem, uin
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
   if constexpr (N > 2) product_ts<N - 2>(d_tmem, a_tmem + 16, b_desc + 256, idesc, 1u);
+}
+// D (+)= A B over N steps of 16 of the reduced index, both operands in shared memory, kA and kB bytes a step
+template <int N, int kA, int kB>
+__device__ __forceinline__ void product_ss_steps(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  static_assert(N % 2 == 0, "whole pairs of steps");
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e, f, t;\n\t"
+      ".reg .b64 a, b;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 f, %4, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, f;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(kA >> 4), "n"(kB >> 4)
+      : "memory");
+  if constexpr (N > 2) product_ss_steps<N - 2, kA, kB>(d_tmem, a_desc + 2 * (kA >> 4), b_desc + 2 * (kB >> 4), idesc, 1u);
 }
 // By the elected lane of a converged warp, the one that issued the products: the mbarrier gets one
 // arrival when every MMA issued so far by this lane has finished.

@@ -8,6 +8,7 @@ there is no host path.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -229,6 +230,29 @@ def fused_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: fl
     return (out, lse) if return_lse else out
 
 
+#: bytes of dS the attention backward keeps at most between its two products (see ixb_fa_bwd_scratch):
+#: what 4 x 32 heads of 4096 causal keys need in one go, 1/70 of the memory of a B200.  The same heads
+#: in three launches with 1 GiB: 1700 us a call against 1625, the GPU drains after each
+SCORE_GRADIENT_BYTES = 5 << 29
+
+
+@functools.lru_cache(maxsize=1024)
+def _score_gradient_room(B, H, Sq, Sk, causal, limit):
+    return rt.load().ixb_fa_bwd_scratch_bytes(B, H, Sq, Sk, int(causal), limit)
+
+
+def _backward_scratch(B, H, Sq, Sk, causal, device):
+    """(one allocation, its bytes for dS ahead of the B * H * Sq floats of delta).  Where the memory
+    is not to be had the backward does without dS: it then computes the probabilities twice."""
+    room = _score_gradient_room(B, H, Sq, Sk, causal, SCORE_GRADIENT_BYTES)
+    if room:
+        try:
+            return torch.empty(room + 4 * B * H * Sq, dtype=torch.uint8, device=device), room
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return torch.empty(4 * B * H * Sq, dtype=torch.uint8, device=device), 0
+
+
 def fused_attention_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor,
                              lse: torch.Tensor, dout: torch.Tensor, scale: float, *, causal: bool = False,
                              check: bool = False):
@@ -255,14 +279,16 @@ def fused_attention_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     dq = torch.empty((B, H, Sq, D), dtype=q.dtype, device=q.device)
     dk = torch.empty((B, H, Sk, D), dtype=q.dtype, device=q.device)
     dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=q.device)
-    delta = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
+    scratch, room = _backward_scratch(B, H, Sq, Sk, causal, q.device)
     status = torch.zeros(1, dtype=torch.int32, device=q.device) if check else None
-    rt.check("ixb_fa_bwd", rt.load().ixb_fa_bwd(
+    q_like, kv_like = _bhs_strides(dq), _bhs_strides(dk)
+    rt.check("ixb_fa_bwd", rt.load().ixb_fa_bwd_scratch(
         rt.DTYPE_CODE[q.dtype], q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
-        lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), B, H, Sq, Sk, D,
+        lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), scratch.data_ptr() + room,
+        scratch.data_ptr() if room else None, room,
+        B, H, Sq, Sk, D,
         _bhs_strides(q), _bhs_strides(k), _bhs_strides(v), _bhs_strides(out), _bhs_strides(dout),
-        _bhs_strides(dq), _bhs_strides(dk), _bhs_strides(dv), float(scale), int(causal), rt.ptr(status),
-        rt.raw_stream(q.device)))
+        q_like, kv_like, kv_like, float(scale), int(causal), rt.ptr(status), rt.raw_stream(q.device)))
     if status is not None and int(status.item()) != 0:
         raise RuntimeError("ixb_fa_bwd: an internal pipeline wait gave up; gradients are undefined")
     return dq, dk, dv

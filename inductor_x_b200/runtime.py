@@ -105,6 +105,9 @@ _SIGNATURES = {
                            POINTER(c_int64), POINTER(c_int64), c_float, c_int, c_void_p, c_void_p]),
     "ixb_fa_bwd": (c_int, [c_int] + [c_void_p] * 10 + [c_int32] * 5 + [POINTER(c_int64)] * 8 +
                    [c_float, c_int, c_void_p, c_void_p]),
+    "ixb_fa_bwd_scratch_bytes": (c_size_t, [c_int32] * 4 + [c_int, c_size_t]),
+    "ixb_fa_bwd_scratch": (c_int, [c_int] + [c_void_p] * 11 + [c_size_t] + [c_int32] * 5 + [POINTER(c_int64)] * 8 +
+                           [c_float, c_int, c_void_p, c_void_p]),
     "ixb_index_select_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                       c_int, c_int, c_void_p, c_void_p]),
     "ixb_cp_forward_update": (c_int, [c_int] + [c_void_p] * 9 + [c_int32] * 4 + [c_int64] * 3 + [c_void_p]),

@@ -1,0 +1,88 @@
+"""The attention backward with dS kept in scratch (ixb_fa_bwd_scratch)."""
+import math
+
+import pytest
+import torch
+
+from inductor_x_b200 import ops
+from inductor_x_b200 import runtime as rt
+from oracle import graphs
+
+TILE = 128 * 128 * 2
+
+
+def _tiles(Sq, Sk, causal):
+    """Tiles of 128 keys x 128 queries in which some query sees some key."""
+    return sum(not causal or kv <= q + 127 + (Sk - Sq) for kv in range(0, Sk, 128) for q in range(0, Sq, 128))
+
+
+@pytest.mark.parametrize("causal", [0, 1])
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (128, 128), (129, 129), (1000, 1000), (130, 450), (1, 4096), (200, 263), (384, 640)])
+def test_scratch_size(Sq, Sk, causal):
+    per_head = _tiles(Sq, Sk, causal) * TILE
+    size = lambda heads, limit: rt.load().ixb_fa_bwd_scratch_bytes(1, heads, Sq, Sk, causal, limit)
+    assert size(3, 1 << 40) == 3 * per_head
+    assert size(3, 3 * per_head - 1) == 2 * per_head       # two launches of two heads and one
+    assert size(7, 4 * per_head) == 4 * per_head
+    assert size(9, 4 * per_head) == 3 * per_head           # three equal launches instead of 4 + 4 + 1
+    assert size(3, per_head - 1) == 0 and size(0, 1 << 40) == 0
+
+
+def test_scratch_arguments():
+    assert rt.load().ixb_fa_bwd_scratch_bytes(1, 1, 256, 128, 1, 1 << 40) == 0   # refused by the kernels as well
+    assert rt.load().ixb_fa_bwd_scratch_bytes(-1, 1, 128, 128, 0, 1 << 40) == 0
+
+
+# Tolerance as for the backward without scratch: probabilities and their gradients are 16-bit operands.
+TOL = {torch.bfloat16: 4e-2, torch.float16: 8e-3}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Sq,Sk,causal,dtype", [
+    (128, 128, True, torch.bfloat16), (129, 129, True, torch.float16), (77, 77, False, torch.float16), (640, 640, True, torch.float16),
+    (130, 450, True, torch.float16), (257, 384, True, torch.bfloat16), (300, 130, False, torch.float16), (1, 300, True, torch.float16)])
+def test_backward_with_room_for_some_heads(cuda, monkeypatch, Sq, Sk, causal, dtype):
+    """Odd numbers of query tiles, ragged ends of both lengths, tiles past the diagonal; five heads in one
+    launch, in two of three and two (the scratch holds three), and without room for one."""
+    g = torch.Generator().manual_seed(Sq + Sk)
+    q, dy = (torch.randn(1, 5, Sq, 128, generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(1, 5, Sk, 128, generator=g).to(dtype) for _ in range(2))
+    scale = 1 / math.sqrt(128)
+    want = graphs.attention_backward(q, k, v, dy, scale, causal=causal)
+    qd, kd, vd, dyd = (t.to(cuda) for t in (q, k, v, dy))
+    out, lse = ops.fused_attention(qd, kd, vd, scale, causal=causal, return_lse=True, check=True)
+    per_head = _tiles(Sq, Sk, causal) * TILE
+    for room in (5 * per_head, 3 * per_head, per_head - 1):
+        monkeypatch.setattr(ops, "SCORE_GRADIENT_BYTES", room)
+        got = ops.fused_attention_backward(qd, kd, vd, out, lse, dyd, scale, causal=causal, check=True)
+        for name, a, e in zip(("dq", "dk", "dv"), got, want):
+            assert graphs.max_rel_err(a.float().cpu(), e) <= TOL[dtype], (name, room)
+
+
+@pytest.mark.gpu
+def test_keys_past_the_end_do_not_reach_dq(cuda, monkeypatch):
+    """All scores far below zero: exp(0 - lse), what the zeros past the last key would give, overflows.
+    Both ways round dS to 16 bits before the same product, so they are as close as its roundings."""
+    g = torch.Generator().manual_seed(9)
+    q, dy = (torch.randn(1, 2, 130, 128, generator=g).to(torch.bfloat16).to(cuda) for _ in range(2))
+    k, v = (torch.randn(1, 2, 130, 128, generator=g).to(torch.bfloat16).to(cuda) for _ in range(2))
+    q, k = q + 3.25, k - 3.25
+    scale = 1 / math.sqrt(128)
+    out, lse = ops.fused_attention(q, k, v, scale, return_lse=True, check=True)
+    assert float(lse.max()) < -89                              # exp(89) is past the largest float
+    got = ops.fused_attention_backward(q, k, v, out, lse, dy, scale, check=True)
+    monkeypatch.setattr(ops, "SCORE_GRADIENT_BYTES", 0)
+    want = ops.fused_attention_backward(q, k, v, out, lse, dy, scale, check=True)
+    for a, e in zip(got, want):
+        assert bool(a.isfinite().all()) and graphs.max_rel_err(a.float().cpu(), e.float().cpu()) <= TOL[torch.bfloat16]
+
+
+@pytest.mark.gpu
+def test_scratch_must_be_aligned(cuda):
+    q = torch.zeros(1, 1, 8, 128, dtype=torch.bfloat16, device=cuda)
+    st = ops._bhs_strides(q)
+    f = torch.zeros(64, device=cuda)
+    scratch = torch.zeros(2 * TILE, dtype=torch.uint8, device=cuda)
+    assert rt.load().ixb_fa_bwd_scratch(rt.IXB_BF16, *[q.data_ptr()] * 5, f.data_ptr(), *[q.data_ptr()] * 3, f.data_ptr(),
+                                        scratch.data_ptr() + 8, TILE, 1, 1, 8, 8, 128, *[st] * 8, 1.0, 0, None,
+                                        rt.raw_stream(q.device)) == rt.IXB_ERR_ALIGN
