@@ -124,6 +124,7 @@ class B200Kernel(SIMDKernel):
         self.online: dict = {}       # name of a softmax input -> its online-softmax exchange
         self.online_exp: dict = {}   # name of exp(input - max) -> exchange
         self.zero_past_end: set = set()    # operands that are zero past the end of a row (plain loads)
+        self.row_exps: list = []     # index expressions of the accesses that walk a row of their own
         self.checked_indices = 0     # data-dependent indices checked on the device (debug builds)
         self.x_indexing = IndentedBuffer()
         self.r_indexing = IndentedBuffer()
@@ -143,7 +144,7 @@ class B200Kernel(SIMDKernel):
             if self.looped:
                 self._row_cfg = split_tiling.choose_loop_config(dt)
             else:
-                self._row_cfg = split_tiling.choose_row_config(rnumel, dt, rows=self._numel_hint("x"),
+                self._row_cfg = split_tiling.choose_row_config(self._covering(rnumel, dt), dt, rows=self._numel_hint("x"),
                                                                 exact=not self._is_dynamic("r0_"))
                 if self._row_cfg is None and self._reads_are_strided():
                     # an outer reduction of any length: the outer mapping loops over the reduced
@@ -160,6 +161,37 @@ class B200Kernel(SIMDKernel):
 
     def create_cse_var(self, *args, **kwargs):
         return B200CSEVariable(*args, **kwargs)
+
+    def _covering(self, rnumel: int, dt: torch.dtype) -> int:
+        """Elements of the aligned vectors that a row of ``rnumel`` may touch: one vector's worth
+        less one more where its length moves the rows off a boundary (see _row_shift)."""
+        vec = min(max(ixb_config.get_aligned_numel(dt), 1), 8)
+        return rnumel if rnumel % vec == 0 or self._is_dynamic("r0_") else rnumel + vec - 1
+
+    def _row_shift(self, tiling):
+        """(pitch, first element, period) when every access of the group that walks a row of its own
+        reads or writes element ``pitch * x + first + r`` of its buffer, with the same pitch and first
+        element modulo the vector width: the rows that are ``period`` apart then lie alike against
+        the 16-byte boundaries, and a block of the row template keeps to those (``kShiftPeriod`` in
+        gen.cuh).  None where the words have to be shifted row by row: run-time lengths, several
+        pitches, scans, index expressions of any other form, rows short enough for sub-warp teams."""
+        cfg = self._row_cfg
+        if self.looped or self._is_dynamic("r0_") or tiling is not None or getattr(self, "_has_scan", False) or \
+                cfg.team < 32 or not self.row_exps or self._static_numel("r0_") % cfg.vec == 0:
+            return None
+        xr, rr = self._xr_roots()
+        found = set()
+        for exp in self.row_exps:
+            rest = sympy.expand(exp - rr.symbol())
+            pitch = rest.coeff(xr.symbol(), 1)
+            first = sympy.expand(rest - pitch * xr.symbol())
+            if not (pitch.is_Integer and first.is_Integer):
+                return None
+            found.add((int(pitch) % cfg.vec, int(first) % cfg.vec))
+        if len(found) != 1:
+            return None
+        pitch, first = found.pop()
+        return pitch, first, cfg.vec // math.gcd(pitch, cfg.vec)
 
     # ------------------------------------------------------------------ value table
     def note_op(self, var, name, args, kwargs=None) -> None:
@@ -495,6 +527,7 @@ class B200Kernel(SIMDKernel):
                 if const_member is not None:
                     row_text = const_member
             else:
+                self.row_exps.append(exp)
                 if row_ptr not in self._row_prefetch:
                     self._row_prefetch.append(row_ptr)     # streamed once per row: worth prefetching
                 aligned = index_ir.row_starts_aligned(exp, xr.symbol(), rr.symbol(), cfg.vec) and \
@@ -575,6 +608,7 @@ class B200Kernel(SIMDKernel):
                 row_ptr = f"({var}) + ({G}lane0({idx}) - {G}lane0(r0_index))"
                 row_text = f"c.store_row({row_ptr}, {value});"
                 cfg = self._row_cfg
+                self.row_exps.append(exp)
                 if not self.looped and dtype in FLOAT_DTYPES and \
                         config_bytes(dtype) >= config_bytes(self._narrowest_node_dtype()):
                     aligned = index_ir.row_starts_aligned(exp, xr.symbol(), rr.symbol(), cfg.vec) and \
@@ -1285,6 +1319,9 @@ class B200Kernel(SIMDKernel):
                              f"const long long xindex = {G}tile_order<{tiling[0]}, {tiling[1]}, 16, 16, "
                              f"{'true' if b_first else 'false'}>(xslot);")
                 row_body = re.sub(r"@B\d+@\n?", "", self._substitute(body_text, False))
+                shift = self._row_shift(tiling)
+                if shift is not None:
+                    row_body = row_body.replace("c.put_row_any(", "c.template put_row_shifted<STAGED>(")
                 # per-column operands, most used first: the first IXB_ROW_KREGS of them are
                 # registers, the others are read from the shared-memory table
                 order = sorted(range(len(self.consts)), key=lambda j: -row_body.count(self.consts[j][0]))
@@ -1293,6 +1330,11 @@ class B200Kernel(SIMDKernel):
                 src.writeline(f"static constexpr int kN = IXB_ROW_VPT * {cfg.vec};   // elements per thread")
                 src.writeline(f"static constexpr bool kLooped = {'true' if self.looped else 'false'};   // row walked in chunks")
                 src.writeline(f"static constexpr bool kTiled = {'true' if tiling is not None else 'false'};   // kept index walked in tiles")
+                pitch, first, period = shift or (0, 0, 0)
+                src.writeline(f"static constexpr int kShiftPeriod = {period};   // rows after which the offset from a "
+                              "16-byte boundary repeats, 0: not made use of")
+                src.writeline("__device__ __forceinline__ int row_offset(int x) const { "
+                              f"return (int)(((long long)x * {pitch} + {first}) % {cfg.vec}); }}")
                 src.writeline(f"static constexpr int kConsts = {len(self.consts)};")
                 src.writeline("static constexpr int kSmemConsts = kConsts > IXB_ROW_KREGS ? kConsts - IXB_ROW_KREGS : 0;")
                 src.writeline("struct Consts {")
@@ -1303,6 +1345,7 @@ class B200Kernel(SIMDKernel):
                 src.writeline("struct Raw {")
                 with src.indent():
                     for member, ctype, _, raw in self.staged:
+                        raw = "RawRow" if shift is not None else raw
                         src.writeline(f"{G}{raw}<{ctype}, IXB_ROW_VPT, {cfg.vec}> {member[4:]};")
                 src.writeline("};")
                 # operands that are the same for every row: once per thread
@@ -1469,7 +1512,7 @@ class B200Kernel(SIMDKernel):
             cfg = self._row_cfg
             inplace = bool(self.args.inplace_buffers)
             kregs = min(len(self.consts), MAX_CONST_REGS // max(cfg.elems_per_thread, 1))
-            shapes = split_tiling.row_candidates(self._static_numel("r0_"), cfg, rows=xnumel_hint,
+            shapes = split_tiling.row_candidates(self._covering(self._static_numel("r0_"), self._narrowest_node_dtype()), cfg, rows=xnumel_hint,
                                                  n_consts=len(self.consts), kregs=kregs)
             meta += (f", tune=dict(default={(cfg.team, cfg.teams, cfg.vpt, cfg.min_ctas, cfg.prefetch, kregs)!r}, "
                      f"candidates={shapes!r}, rows={xnumel_hint}, row_bytes={self._static_numel('r0_') * config_bytes(self._narrowest_node_dtype())}, "

@@ -506,13 +506,18 @@ template <class Op> __device__ __forceinline__ float warp_all(float v) {
   else return warp_reduce<Op>(v);
 }
 
-template <typename T, int TEAM, int TEAMS, int VPT, int COLS = 0>
+// SHIFT: the thread's vectors are those of memory, not of the row: vector 0 of lane 0 is the aligned one
+// that holds the row's first element, `off` elements into it, and column vec_col(0) is -off there.
+template <typename T, int TEAM, int TEAMS, int VPT, int COLS = 0, bool SHIFT = false>
 struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   using Base = RowCtx<T, TEAM, TEAMS, VPT, false>;
   static constexpr int kE = VPT * Base::kVec;
-  static constexpr bool FULL = COLS == TEAM * VPT * Base::kVec;
+  static constexpr bool FULL = !SHIFT && COLS == TEAM * VPT * Base::kVec;
+  static constexpr bool kShift = SHIFT;
   // vector i of every thread lies inside the row
-  static __device__ __forceinline__ constexpr bool full(int i) { return COLS >= (i + 1) * TEAM * Base::kVec; }
+  static __device__ __forceinline__ constexpr bool full(int i) {
+    return COLS >= (i + 1) * TEAM * Base::kVec && !(SHIFT && i == 0);
+  }
   __device__ __forceinline__ int ncols() const { return COLS > 0 ? COLS : this->cols; }
   static constexpr int kGroup = TEAM < 32 ? TEAM : 32;  // lanes of one warp that share a row
   static constexpr int kW = Base::kWarpsPerTeam;        // warps per team (0 for sub-warp teams)
@@ -525,7 +530,10 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   // so every access below is relative to the chunk.
   int chunk0 = 0;
   static constexpr int kCap = TEAM * VPT * Base::kVec;
-  __device__ __forceinline__ int vec_col(int i) const { return chunk0 + (this->lane + i * TEAM) * Base::kVec; }
+  int off = 0;
+  __device__ __forceinline__ int vec_col(int i) const {
+    return chunk0 + (this->lane + i * TEAM) * Base::kVec - (SHIFT ? off : 0);
+  }
   __device__ __forceinline__ int nchunks() const { return (this->cols + kCap - 1) / kCap; }
   __device__ __forceinline__ void set_chunk(int chunk) { chunk0 = chunk * kCap; }
   // Per-column operands that are not kept in registers live in a CTA-wide shared-memory
@@ -538,6 +546,20 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   template <int SLOT, class U> __device__ __forceinline__ void fill_sconst(const U* rowp) const {
     static_assert(Base::kVec % 4 == 0, "shared-memory operands need whole quads per vector");
     float4* tab = const_cast<float4*>(ktab) + SLOT * kQuads * kTabVecs;
+    if constexpr (SHIFT) {
+      for (int v = threadIdx.x; v < kTabVecs; v += blockDim.x)
+#pragma unroll
+        for (int q = 0; q < kQuads; ++q) {
+          float part[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int col = v * Base::kVec + 4 * q + j - off;
+            part[j] = (unsigned)col < (unsigned)ncols() ? Cast<float>::from(Mem<U>::ld(rowp + col)) : 0.f;
+          }
+          tab[q * kTabVecs + v] = make_float4(part[0], part[1], part[2], part[3]);
+        }
+      return;
+    }
     for (int v = threadIdx.x; v < kTabVecs; v += blockDim.x) {
       const int c0 = v * Base::kVec;
       const int left = this->cols - c0;
@@ -568,7 +590,12 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   __device__ __forceinline__ bool leader() const { return this->lane == 0 && live; }
   // element j of vector i lies inside the row
   __device__ __forceinline__ bool inside(int i, int j) const {
+    if constexpr (SHIFT) return full(i) || (unsigned)(this->vec_col(i) + j) < (unsigned)ncols();
     return full(i) || this->vec_col(i) + j < ncols();
+  }
+  // vector i may hold elements that are not the row's
+  __device__ __forceinline__ bool cut(int i) const {
+    return !full(i) && ((SHIFT && this->vec_col(i) < 0) || this->vec_col(i) + Base::kVec > ncols());
   }
   __device__ __forceinline__ vi<kE> rindex() const {
     vi<kE> r;
@@ -593,6 +620,12 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int c0 = this->vec_col(i);
+      if (SHIFT && cut(i)) {
+#pragma unroll
+        for (int j = 0; j < Base::kVec; ++j)
+          r.v[i * Base::kVec + j] = inside(i, j) ? Mem<U>::ld(rowp + c0 + j) : V();
+        continue;
+      }
       const int left = full(i) ? Base::kVec : ncols() - c0;
       auto part = ldvec<U, Base::kVec, false, false, CUT>(rowp + c0, left > 0 ? left : 0);
 #pragma unroll
@@ -608,9 +641,18 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     for (int i = 0; i < VPT; ++i) {
       const int c0 = this->vec_col(i);
 #pragma unroll
-      for (int k = 0; k < kC; ++k)
-        raw.q[i][k] = (full(i) || c0 < ncols()) ? ldg_stream(reinterpret_cast<const uint4*>(rowp + c0) + k)
-                                               : make_uint4(0, 0, 0, 0);
+      for (int k = 0; k < kC; ++k) {
+        if constexpr (SHIFT) {
+          // (the words at the two ends are written by the blocks of the neighbouring rows as well, in
+          // place as it may be: no __ldg)
+          constexpr int kPer = 16 / (int)sizeof(U);
+          const int w0 = c0 + k * kPer;
+          raw.q[i][k] = (full(i) || (w0 + kPer > 0 && w0 < ncols())) ? ldg_word_stream(rowp + w0) : make_uint4(0, 0, 0, 0);
+        } else {
+          raw.q[i][k] = (full(i) || c0 < ncols()) ? ldg_stream(reinterpret_cast<const uint4*>(rowp + c0) + k)
+                                                 : make_uint4(0, 0, 0, 0);
+        }
+      }
     }
   }
   template <class U> __device__ __forceinline__ vf<kE> widen(const RawRow<U, VPT, Base::kVec>& raw) const {
@@ -621,9 +663,19 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     for (int i = 0; i < VPT; ++i)
 #pragma unroll
       for (int k = 0; k < kC; ++k) unpack<U>(raw.q[i][k], &r.v[i * Base::kVec + k * kPer]);
+    if constexpr (SHIFT) {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i)
+        if (cut(i)) {
+#pragma unroll
+          for (int j = 0; j < Base::kVec; ++j)
+            if (!inside(i, j)) r.v[i * Base::kVec + j] = 0.f;
+        }
+    }
     return r;
   }
-  // Rows that start off a 16-byte boundary (an odd row length moves every row): the words that
+  // Rows that start off a 16-byte boundary (an odd row length moves every row) where the block cannot
+  // keep to one offset (SHIFT) - run-time lengths, operands of several pitches: the words that
   // cover a thread's vectors are fetched aligned - the one it shares with the next lane comes
   // out of L1 - and shifted into place when the row is worked on.  Only words that hold an
   // element of the row are read.  Element-wise loads of such rows touch every line eight times
@@ -720,7 +772,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     for (int i = 0; i < VPT; ++i) {
       const int c0 = this->vec_col(i);
       const U* p = rowp + c0;
-      const bool opens = (reinterpret_cast<unsigned long long>(p) & 127ull) < Base::kVec * sizeof(U) || c0 == 0;
+      const bool opens = (reinterpret_cast<unsigned long long>(p) & 127ull) < Base::kVec * sizeof(U) || c0 <= 0;
       if (c0 < this->cols && opens) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
     }
   }
@@ -730,6 +782,12 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int c0 = this->vec_col(i);
+      if (SHIFT && cut(i)) {
+#pragma unroll
+        for (int j = 0; j < Base::kVec; ++j)
+          if (inside(i, j)) Mem<U>::st(rowp + c0 + j, Cast<V>::from(at(val, i * Base::kVec + j)));
+        continue;
+      }
       const int left = full(i) ? Base::kVec : ncols() - c0;
       typename vec_of<V, Base::kVec>::type part;
 #pragma unroll
@@ -746,6 +804,12 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
         const int c0 = this->vec_col(i);
+        if (SHIFT && cut(i)) {
+#pragma unroll
+          for (int j = 0; j < Base::kVec; ++j)
+            if (inside(i, j)) Mem<U>::st(rowp + c0 + j, val.v[i * Base::kVec + j]);
+          continue;
+        }
         if (full(i) || c0 < ncols()) {
 #pragma unroll
           for (int k = 0; k < Base::kVec / kPer; ++k)
@@ -755,6 +819,12 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     } else {
       store_row(rowp, val);
     }
+  }
+
+  // rows that may start off a boundary: whole vectors of memory where the block works in those
+  template <bool STAGED, class U, class A> __device__ __forceinline__ void put_row_shifted(U* rowp, const A& val) const {
+    if constexpr (SHIFT) put_row<STAGED>(rowp, val);
+    else put_row_any(rowp, val);
   }
 
   // ---- team exchange --------------------------------------------------------------------
@@ -1389,7 +1459,12 @@ template <class K> inline int row_resident(K kern, int threads, size_t smem = 0)
 template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS, int PF, int COLS, bool STAGED>
 __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     row_gen_kernel(const Body body, const long long rows, const int cols) {
-  using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS>;
+  // Rows off a 16-byte boundary repeat their offset every kShiftPeriod rows.  Block b works on rows b,
+  // b + period, ... only: its offset stays what it is, and the row is worked on in the aligned
+  // vectors of memory as if it began there (`off` elements that are masked), per-column operands
+  // shifted once to match - nothing is shifted per row.
+  constexpr int kPeriod = STAGED && TEAM >= 32 ? Body::kShiftPeriod : 0;
+  using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS, (kPeriod > 0)>;
   constexpr int kSlots = TEAM > 32 ? 2 * (TEAM / 32) * 4 : 1;  // exchange floats per team
   __shared__ __align__(16) float exchange[TEAMS * kSlots];
   extern __shared__ __align__(16) unsigned char operand_table[];   // Body::kSmemConsts slots
@@ -1405,12 +1480,17 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
   pdl_launch_dependents();
   pdl_wait();
   const long long stride = (long long)gridDim.x * TEAMS;
+  long long row0 = (long long)blockIdx.x * TEAMS + c.team;
+  if constexpr (kPeriod > 0) {
+    const int cls = (int)(blockIdx.x % kPeriod);
+    row0 = cls + kPeriod * ((long long)(blockIdx.x / kPeriod) * TEAMS + c.team);
+    c.off = body.row_offset(cls);
+  }
   // the first row's vectors are requested before the per-column operands are loaded and
   // widened, so that both latencies overlap (it matters for kernels of a few microseconds)
   typename Body::Raw nxt;
   if constexpr (TEAM >= 32 && STAGED) {
-    const long long r0 = (long long)blockIdx.x * TEAMS + c.team;
-    if (r0 < rows) body.fetch(c, r0, nxt);
+    if (row0 < rows) body.fetch(c, row0, nxt);
   }
   typename Body::Consts k;
   body.init(c, k);
@@ -1447,7 +1527,7 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     }
     return;
   } else {
-    long long r = (long long)blockIdx.x * TEAMS + c.team;
+    long long r = row0;
     while (r < rows) {
       const typename Body::Raw cur = nxt;
       const long long rn = r + stride;
@@ -1477,12 +1557,21 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   const long long groups = (rows + TEAMS - 1) / TEAMS;
   using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS>;
   const size_t smem = (size_t)Body::kSmemConsts * Ctx::kQuads * Ctx::kTabVecs * sizeof(float4);
+  constexpr int kPeriod = TEAM >= 32 ? Body::kShiftPeriod : 0;
+  // (a row in the vectors of memory may need one vector more than its own length)
+  if (kPeriod > 0 && cols + Elem<T>::kVec - 1 > TEAM * VPT * Elem<T>::kVec) aligned = false;
   if (aligned) {
     auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, COLS, true>;
     const int resident = row_resident(kern, TEAM * TEAMS, smem);
     if (resident < 1) return (int)cudaErrorInvalidConfiguration;
     long long grid = (long long)sms * resident;
-    if (grid > groups) grid = groups;
+    if constexpr (kPeriod > 0) {      // as many blocks for each offset
+      const long long most = grid < kPeriod ? kPeriod : grid / kPeriod * kPeriod;
+      grid = (groups + kPeriod - 1) / kPeriod * kPeriod;
+      if (grid > most) grid = most;
+    } else if (grid > groups) {
+      grid = groups;
+    }
     return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
   }
   auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, COLS, false>;
