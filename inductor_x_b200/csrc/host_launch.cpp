@@ -1,7 +1,9 @@
-// Native launch path of generated kernels: what the wrapper code Inductor prints calls once per
-// fused kernel, `kernel.run(tensor, ..., size, ..., stream=handle)`.
+// Native launch paths: of generated kernels - what the wrapper code Inductor prints calls once per
+// fused kernel, `kernel.run(tensor, ..., size, ..., stream=handle)` - and of three library entry points
+// whose calls are short enough for the host to count (rms_norm, fused_attention and its backward, at the
+// end of this file).
 //
-// The call turns its arguments into the two arrays of the generated module's C entry
+// The call of a generated kernel turns its arguments into the two arrays of the generated module's C entry
 // (`ixb_gen_launch(ptrs, ints, stream)`) and calls it with the interpreter lock released.  In
 // Python (an isinstance test, data_ptr() and a list append per argument, two ctypes arrays, the
 // ctypes call) this took 5.3 us; here it takes 0.2.  A compiled call of one small kernel (gelu row
@@ -14,7 +16,11 @@
 #include <Python.h>
 #include <structmember.h>
 
+#include <ATen/Functions.h>
+#include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/ixb.h"
 
 namespace {
 
@@ -131,6 +137,186 @@ PyMemberDef members[] = {{"launches", T_LONGLONG, offsetof(Launcher, launches), 
 PyTypeObject LauncherType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_ixb_host", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
 
+// ---- library entry points ------------------------------------------------------------------------
+// Each takes the arguments of the Python function of the same purpose (ops.py), does what it does for a
+// plain call - checks, allocations, strides, the C entry on the current stream - and returns the
+// result; a status other than 0 comes back as an int, which the caller words.  Anything else (a tensor
+// subclass or a wrapper without storage, a host tensor, a shape, dtype or layout that Python would
+// refuse or copy, an exception) gives None: the Python function then goes its own way, errors included.
+// A call of rms_norm (16 x 4096 bf16 with residual) took 9.5 us in Python, launch and two
+// allocations included.
+decltype(&ixb_rmsnorm) entry_rmsnorm;
+decltype(&ixb_fa_fwd) entry_fa_fwd;
+decltype(&ixb_fa_bwd_scratch_bytes) entry_fa_bwd_room;
+decltype(&ixb_fa_bwd_scratch) entry_fa_bwd;
+
+// bind_library(rmsnorm, fa_fwd, fa_bwd_scratch_bytes, fa_bwd_scratch): addresses of the C entries
+PyObject* bind_library(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  void* p[4];
+  if (n != 4) {
+    PyErr_SetString(PyExc_TypeError, "bind_library takes four addresses");
+    return nullptr;
+  }
+  for (int i = 0; i < 4; ++i) {
+    p[i] = PyLong_AsVoidPtr(args[i]);
+    if (p[i] == nullptr && PyErr_Occurred()) return nullptr;
+  }
+  entry_rmsnorm = reinterpret_cast<decltype(entry_rmsnorm)>(p[0]);
+  entry_fa_fwd = reinterpret_cast<decltype(entry_fa_fwd)>(p[1]);
+  entry_fa_bwd_room = reinterpret_cast<decltype(entry_fa_bwd_room)>(p[2]);
+  entry_fa_bwd = reinterpret_cast<decltype(entry_fa_bwd)>(p[3]);
+  Py_RETURN_NONE;
+}
+
+// a CUDA tensor with memory of its own kind behind it
+const at::Tensor* plain_tensor(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && t.has_storage() ? &t : nullptr;
+}
+int dtype_code(const at::Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return IXB_F32;
+    case at::kHalf: return IXB_F16;
+    case at::kBFloat16: return IXB_BF16;
+    default: return -1;
+  }
+}
+bool alike(const at::Tensor& a, const at::Tensor& b) {
+  return a.scalar_type() == b.scalar_type() && a.device() == b.device();
+}
+ixb_stream stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+PyObject* pair(at::Tensor a, at::Tensor b) {
+  PyObject *x = THPVariable_Wrap(std::move(a)), *y = x ? THPVariable_Wrap(std::move(b)) : nullptr;
+  PyObject* out = y ? PyTuple_Pack(2, x, y) : nullptr;
+  Py_XDECREF(x);
+  Py_XDECREF(y);
+  return out;
+}
+
+// rms_norm(x, w, eps, residual or None, return_residual)
+PyObject* rms_norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 5 || entry_rmsnorm == nullptr || !PyFloat_CheckExact(args[2]) || !PyBool_Check(args[4])) Py_RETURN_NONE;
+  try {
+    const at::Tensor *x = plain_tensor(args[0]), *w = plain_tensor(args[1]);
+    if (x == nullptr || w == nullptr || x->dim() < 1 || !x->is_contiguous() || dtype_code(*x) < 0) Py_RETURN_NONE;
+    const int64_t cols = x->size(-1), rows = cols ? x->numel() / cols : 0;
+    if (!alike(*x, *w) || w->dim() != 1 || w->size(0) != cols || !w->is_contiguous()) Py_RETURN_NONE;
+    const at::Tensor* r = nullptr;
+    if (args[3] != Py_None) {
+      r = plain_tensor(args[3]);
+      if (r == nullptr || !alike(*x, *r) || r->sizes() != x->sizes() || !r->is_contiguous()) Py_RETURN_NONE;
+    }
+    at::Tensor y = at::empty_like(*x), h;
+    if (r != nullptr && args[4] == Py_True) h = at::empty_like(*x);
+    const ixb_stream stream = stream_of(*x);
+    const float eps = (float)PyFloat_AS_DOUBLE(args[2]);
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = entry_rmsnorm(dtype_code(*x), x->data_ptr(), r ? r->data_ptr() : nullptr, w->data_ptr(), y.data_ptr(),
+                       h.defined() ? h.data_ptr() : nullptr, rows, cols, eps, nullptr, stream);
+    Py_END_ALLOW_THREADS
+    if (st != 0) return PyLong_FromLong(st);
+    return h.defined() ? pair(std::move(y), std::move(h)) : THPVariable_Wrap(std::move(y));
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+}
+
+struct Strides {
+  int64_t v[3];
+  explicit Strides(const at::Tensor& t) : v{t.stride(0), t.stride(1), t.stride(2)} {}
+};
+// q[B, H, Sq, D], k and v [B, H, Sk, D], 16-bit, D contiguous
+bool attention_operands(const at::Tensor* q, const at::Tensor* k, const at::Tensor* v) {
+  return q && k && v && q->dim() == 4 && k->dim() == 4 && k->sizes() == v->sizes() && q->size(0) == k->size(0) &&
+         q->size(1) == k->size(1) && q->size(3) == k->size(3) && dtype_code(*q) > IXB_F32 && alike(*q, *k) && alike(*q, *v) &&
+         q->stride(3) == 1 && k->stride(3) == 1 && v->stride(3) == 1 && q->numel() <= INT32_MAX * (int64_t)128 &&
+         k->numel() <= INT32_MAX * (int64_t)128;
+}
+
+// fused_attention(q, k, v, scale, causal, return_lse)
+PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 6 || entry_fa_fwd == nullptr || !PyFloat_CheckExact(args[3]) || !PyBool_Check(args[4]) || !PyBool_Check(args[5]))
+    Py_RETURN_NONE;
+  try {
+    const at::Tensor *q = plain_tensor(args[0]), *k = plain_tensor(args[1]), *v = plain_tensor(args[2]);
+    if (!attention_operands(q, k, v)) Py_RETURN_NONE;
+    const int64_t B = q->size(0), H = q->size(1), Sq = q->size(2), D = q->size(3), Sk = k->size(2);
+    at::Tensor out = at::empty({B, H, Sq, D}, q->options()), lse;
+    if (args[5] == Py_True) lse = at::empty({B, H, Sq}, q->options().dtype(at::kFloat));
+    const Strides qs(*q), ks(*k), vs(*v), os(out);
+    const ixb_stream stream = stream_of(*q);
+    const float scale = (float)PyFloat_AS_DOUBLE(args[3]);
+    const int causal = args[4] == Py_True;
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = entry_fa_fwd(dtype_code(*q), q->data_ptr(), k->data_ptr(), v->data_ptr(), out.data_ptr(),
+                      lse.defined() ? static_cast<float*>(lse.data_ptr()) : nullptr, (int32_t)B, (int32_t)H, (int32_t)Sq,
+                      (int32_t)Sk, (int32_t)D, qs.v, ks.v, vs.v, os.v, scale, causal, nullptr, stream);
+    Py_END_ALLOW_THREADS
+    if (st != 0) return PyLong_FromLong(st);
+    return lse.defined() ? pair(std::move(out), std::move(lse)) : THPVariable_Wrap(std::move(out));
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+}
+
+// fused_attention_backward(q, k, v, out, lse, dout, scale, causal, bytes of dS at most)
+PyObject* fused_attention_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 9 || entry_fa_bwd == nullptr || !PyFloat_CheckExact(args[6]) || !PyBool_Check(args[7]) || !PyLong_CheckExact(args[8]))
+    Py_RETURN_NONE;
+  try {
+    const at::Tensor *q = plain_tensor(args[0]), *k = plain_tensor(args[1]), *v = plain_tensor(args[2]),
+                     *o = plain_tensor(args[3]), *lse = plain_tensor(args[4]), *go = plain_tensor(args[5]);
+    const long long limit = PyLong_AsLongLong(args[8]);
+    if (limit < 0) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    if (!attention_operands(q, k, v) || !o || !lse || !go || o->sizes() != q->sizes() || go->sizes() != q->sizes() ||
+        !alike(*q, *o) || !alike(*q, *go) || o->stride(3) != 1 || go->stride(3) != 1)
+      Py_RETURN_NONE;
+    const int64_t B = q->size(0), H = q->size(1), Sq = q->size(2), D = q->size(3), Sk = k->size(2);
+    for (int i = 0; i < 3; ++i)
+      if (go->stride(i) % 8 != 0) Py_RETURN_NONE;
+    if (lse->dim() != 3 || lse->size(0) != B || lse->size(1) != H || lse->size(2) != Sq ||
+        lse->scalar_type() != at::kFloat || lse->device() != q->device() || !lse->is_contiguous())
+      Py_RETURN_NONE;
+    at::Tensor dq = at::empty({B, H, Sq, D}, q->options()), dk = at::empty({B, H, Sk, D}, q->options()),
+               dv = at::empty({B, H, Sk, D}, q->options());
+    const int causal = args[7] == Py_True;
+    // (where the memory for dS is not to be had, the Python function sees to it)
+    const size_t room = entry_fa_bwd_room((int32_t)B, (int32_t)H, (int32_t)Sq, (int32_t)Sk, causal, (size_t)limit);
+    at::Tensor scratch = at::empty({(int64_t)room + 4 * B * H * Sq}, q->options().dtype(at::kByte));
+    unsigned char* base = static_cast<unsigned char*>(scratch.data_ptr());
+    const Strides qs(*q), ks(*k), vs(*v), os(*o), gs(*go), dqs(dq), dks(dk), dvs(dv);
+    const ixb_stream stream = stream_of(*q);
+    const float scale = (float)PyFloat_AS_DOUBLE(args[6]);
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = entry_fa_bwd(dtype_code(*q), q->data_ptr(), k->data_ptr(), v->data_ptr(), o->data_ptr(), go->data_ptr(),
+                      static_cast<const float*>(lse->data_ptr()), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                      reinterpret_cast<float*>(base + room), room ? base : nullptr, room, (int32_t)B, (int32_t)H,
+                      (int32_t)Sq, (int32_t)Sk, (int32_t)D, qs.v, ks.v, vs.v, os.v, gs.v, dqs.v, dks.v, dvs.v, scale, causal,
+                      nullptr, stream);
+    Py_END_ALLOW_THREADS
+    if (st != 0) return PyLong_FromLong(st);
+    PyObject* rest = pair(std::move(dk), std::move(dv));
+    PyObject* first = rest ? THPVariable_Wrap(std::move(dq)) : nullptr;
+    PyObject* all = first ? PyTuple_Pack(3, first, PyTuple_GET_ITEM(rest, 0), PyTuple_GET_ITEM(rest, 1)) : nullptr;
+    Py_XDECREF(first);
+    Py_XDECREF(rest);
+    return all;
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+}
+
+#define IXB_FASTCALL(fn) {#fn, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef functions[] = {IXB_FASTCALL(bind_library), IXB_FASTCALL(rms_norm), IXB_FASTCALL(fused_attention),
+                           IXB_FASTCALL(fused_attention_backward), {nullptr, nullptr, 0, nullptr}};
+
 }  // namespace
 
 PyMODINIT_FUNC PyInit__ixb_host(void) {
@@ -149,6 +335,7 @@ PyMODINIT_FUNC PyInit__ixb_host(void) {
   name_dry_run = PyUnicode_InternFromString("dry_run");
   name_status = Py_BuildValue("(s)", "status");
   if (name_profile == nullptr || name_dry_run == nullptr || name_status == nullptr || PyType_Ready(&LauncherType) < 0) return nullptr;
+  module_def.m_methods = functions;
   PyObject* m = PyModule_Create(&module_def);
   if (m == nullptr) return nullptr;
   Py_INCREF(&LauncherType);

@@ -13,6 +13,7 @@ from typing import Optional, Sequence, Tuple
 
 import torch
 
+from . import _ixb_host
 from . import runtime as rt
 
 
@@ -20,6 +21,17 @@ def launch_count() -> int:
     """Calls made into the kernel library's launching entry points so far (each enqueues one
     kernel; a split outer reduction two)."""
     return rt.native_calls
+
+
+def _native(fn: str, done):
+    """What a native entry point (``csrc/host_launch.cpp``) returned: None for a call it leaves to
+    Python, the status of one that failed, else the result."""
+    if done is None:
+        return None
+    if type(done) is int:
+        rt.check(fn, done)
+    rt.native_calls += 1
+    return done
 
 
 def _need_cuda(*ts: Optional[torch.Tensor]) -> None:
@@ -77,6 +89,10 @@ def rmsnorm(x, w, eps: float = 1e-6, *, residual=None, return_residual: bool = F
     """RMSNorm over the last axis with an optional fused residual add.
 
     Returns ``y`` or ``(y, h)`` where ``h = x + residual`` (rounded to the storage dtype)."""
+    if cfg is None:
+        done = _native("ixb_rmsnorm", _ixb_host.rms_norm(x, w, eps, residual, return_residual))
+        if done is not None:
+            return done
     _need_cuda(x, w, residual)
     if not x.is_contiguous():
         raise ValueError("x must be contiguous")
@@ -208,6 +224,10 @@ def fused_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: fl
     Returns ``out`` (contiguous ``[B, H, Sq, D]``) or ``(out, lse)`` with ``lse`` the fp32
     log-sum-exp of the scaled scores ``[B, H, Sq]``.  ``check=True`` reads the kernel's
     status word back (synchronises) and raises if an internal wait gave up."""
+    if not check:
+        done = _native("ixb_fa_fwd", _ixb_host.fused_attention(q, k, v, scale, causal, return_lse))
+        if done is not None:
+            return done
     _need_cuda(q, k, v)
     if q.dim() != 4 or k.shape != v.shape or q.shape[:2] != k.shape[:2] or q.shape[3] != k.shape[3]:
         raise ValueError("expected q[B,H,Sq,D], k[B,H,Sk,D], v[B,H,Sk,D]")
@@ -259,6 +279,11 @@ def fused_attention_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     """Gradients ``(dq, dk, dv)`` of :func:`fused_attention` from its inputs, its output
     ``out``, its log-sum-exp ``lse`` (``return_lse=True``) and the incoming gradient ``dout``
     (tcgen05 kernels behind ``ixb_fa_bwd``; deterministic, no atomics)."""
+    if not check:
+        done = _native("ixb_fa_bwd", _ixb_host.fused_attention_backward(q, k, v, out, lse, dout, scale, causal,
+                                                                        SCORE_GRADIENT_BYTES))
+        if done is not None:
+            return done
     _need_cuda(q, k, v, out, dout, lse)
     if q.dim() != 4 or k.shape != v.shape or q.shape[:2] != k.shape[:2] or q.shape[3] != k.shape[3]:
         raise ValueError("expected q[B,H,Sq,D], k[B,H,Sk,D], v[B,H,Sk,D]")

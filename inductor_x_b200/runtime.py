@@ -134,6 +134,10 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     if lib.ixb_abi_version() != 1:
         raise ImportError(f"{LIB_PATH}: ABI version {lib.ixb_abi_version()} != 1")
+    from . import _ixb_host
+
+    _ixb_host.bind_library(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in (
+        "ixb_rmsnorm", "ixb_fa_fwd", "ixb_fa_bwd_scratch_bytes", "ixb_fa_bwd_scratch")))
     _lib = lib
     return lib
 
