@@ -57,6 +57,8 @@ MAX_CONST_REGS = 64
 MAX_CONSTS = 6
 #: streamed operands fetched one row ahead as raw 128-bit vectors
 MAX_STAGED = 2
+#: rows of partial sums that a column sum beside a row kernel may have (kMaxPartials in gen.cuh)
+MAX_PARTIALS = 592
 
 
 class UnsupportedByTemplates(NotImplementedError):
@@ -125,6 +127,9 @@ class B200Kernel(SIMDKernel):
         self.online_exp: dict = {}   # name of exp(input - max) -> exchange
         self.zero_past_end: set = set()    # operands that are zero past the end of a row (plain loads)
         self.row_exps: list = []     # index expressions of the accesses that walk a row of their own
+        self.columns: list = []      # sums over the rows beside the row's work: (output pointer, ctype)
+        self.column_casts: dict = {}  # buffers of column sums -> the buffers of their converted values
+        self.column_mode = False     # the node being emitted sums over the rows (see scheduling.py)
         self.checked_indices = 0     # data-dependent indices checked on the device (debug builds)
         self.x_indexing = IndentedBuffer()
         self.r_indexing = IndentedBuffer()
@@ -311,6 +316,8 @@ class B200Kernel(SIMDKernel):
                 rvars = [v for v in rvars if v in dep.index.free_symbols]
                 if not rvars:
                     continue             # broadcast along the reduced axis
+                if len(rvars) < len(dep.var_names) and not any(v in dep.index.free_symbols for v in dep.var_names if v not in rvars):
+                    continue             # the same for every kept position: a per-row statistic, not a row
                 saw = True
                 strides = V.graph.sizevars.stride_vars(dep.index, rvars)
                 if any(st == 1 for st in strides):
@@ -625,6 +632,11 @@ class B200Kernel(SIMDKernel):
         self.compute.writeline(DeferredLine(name, tag))
 
     def store_reduction(self, name: str, index: sympy.Expr, value: CSEVariable) -> None:
+        if self.column_mode:
+            into = self.column_casts.get(name, name)     # converted where it is stored
+            self.store_buffer_names.add(into)
+            self.columns.append((self.args.output(into), self.dtype_to_str(V.graph.get_dtype(into))))
+            return
         prior = self.inside_reduction
         self.inside_reduction = False
         compute = self.compute
@@ -682,6 +694,14 @@ class B200Kernel(SIMDKernel):
 
     def reduction(self, dtype, src_dtype, reduction_type, value):
         assert self.inside_reduction and self.is_row
+        if self.column_mode:
+            # into this thread's sum for its columns; stored when the block has no rows left
+            factors = self.op_of(value, "mul")
+            acc = f"cols.a{len(self.columns)}"
+            step = (f"op::fma({factors[0]}, {factors[1]}, {acc})" if factors is not None and
+                    all(self.is_float(f) for f in factors) else f"op::add({acc}, {value})")
+            self.compute.writeline(f"{acc} = {G}{step};")
+            return self.cse.newvar(dtype=torch.float32)
         key = (src_dtype, reduction_type, value)
         if key in self.cse.reduction_cache:
             return self.cse.reduction_cache[key]
@@ -1342,6 +1362,27 @@ class B200Kernel(SIMDKernel):
                     for new in range(len(order)):
                         src.writeline(f"{G}vf<kN> k{new};")
                 src.writeline("};")
+                src.writeline(f"static constexpr int kColumns = {len(self.columns)};   // sums over the rows")
+                src.writeline("struct Cols {")
+                with src.indent():
+                    for n in range(len(self.columns)):
+                        src.writeline(f"{G}vf<kN> a{n};")
+                src.writeline("};")
+                src.writeline("__device__ __forceinline__ void clear(Cols& cols) const {")
+                with src.indent():
+                    for n in range(len(self.columns)):
+                        src.writeline("#pragma unroll")
+                        src.writeline(f"for (int e = 0; e < kN; ++e) cols.a{n}.v[e] = 0.f;")
+                src.writeline("}")
+                if self.columns:
+                    src.writeline("float* partial;   // [kColumns][kMaxPartials][columns]")
+                    src.writeline("template <class Ctx>")
+                    src.writeline("__device__ __forceinline__ void flush(const Ctx& c, const Cols& cols, float4* tab) const {")
+                    with src.indent():
+                        for n in range(len(self.columns)):
+                            src.writeline(f"c.flush_column(cols.a{n}, tab, partial + ({n}LL * {G}kMaxPartials + blockIdx.x) * "
+                                          f"{G}partial_pitch({self._static_numel('r0_')}));")
+                    src.writeline("}")
                 src.writeline("struct Raw {")
                 with src.indent():
                     for member, ctype, _, raw in self.staged:
@@ -1374,7 +1415,7 @@ class B200Kernel(SIMDKernel):
                 src.writeline("}")
                 src.writeline("template <bool STAGED, class Ctx>")
                 src.writeline("__device__ __forceinline__ void row(Ctx& c, const Consts& k, const long long xslot, "
-                              "const Raw& raw) const {")
+                              "const Raw& raw, Cols& cols) const {")
                 with src.indent():
                     src.writeline(slot_line)
                     if self.looped:
@@ -1493,9 +1534,19 @@ class B200Kernel(SIMDKernel):
                 # a row length known here lets the template leave out the tests of vectors that lie
                 # inside the row in every thread
                 src.writeline(f"constexpr int kCols = {0 if dyn_r or self.looped else rnumel};")
-                src.writeline(f"return {G}launch_row_gen<Body, {rt}, IXB_ROW_TEAM, IXB_ROW_TEAMS, IXB_ROW_VPT, "
-                              f"IXB_GEN_MIN_CTAS, IXB_ROW_PF, kCols>(b, xnumel, {rnumel}, stream, "
-                              f"{G}pointers_aligned(ptrs, {nptr}));")
+                launch = (f"{G}launch_row_gen<Body, {rt}, IXB_ROW_TEAM, IXB_ROW_TEAMS, IXB_ROW_VPT, "
+                          f"IXB_GEN_MIN_CTAS, IXB_ROW_PF, kCols>(b, xnumel, {rnumel}, stream, "
+                          f"{G}pointers_aligned(ptrs, {nptr})")
+                if not self.columns:
+                    src.writeline(f"return {launch});")
+                else:
+                    src.writeline(f"b.partial = (float*)ptrs[{nptr}];")
+                    src.writeline("long long blocks = 0;")
+                    src.writeline(f"int rc = {launch}, &blocks);")
+                    for n, (ptr, ctype) in enumerate(self.columns):
+                        src.writeline(f"if (rc == 0) rc = {G}finish_columns<{ctype}>(b.partial + {n}LL * {G}kMaxPartials * "
+                                      f"{G}partial_pitch(kCols), blocks, kCols, b.{ptr}, stream);")
+                    src.writeline("return rc;")
             else:
                 launcher = "launch_pointwise_tile" if self._register_tile(self._transposing_order()) else "launch_pointwise"
                 src.writeline(f"return {G}{launcher}<Body>(b, xnumel, stream, "
@@ -1534,11 +1585,19 @@ class B200Kernel(SIMDKernel):
                 wrapper.ensure_size_computed(sym)
             call_args.append(self.pexpr(rn))
         device = V.graph.get_current_device_or_throw()
+        if self.columns:
+            # the blocks' partial sums, behind the tensors of the group
+            pitch = -(-self._static_numel("r0_") // 4) * 4
+            ws = f"ixb_partials_{wrapper.next_kernel_suffix()}"
+            wrapper.writeline(f"{ws} = empty_strided_{device.type}(({len(self.columns) * MAX_PARTIALS * pitch},), (1,), torch.float32)")
+            call_args.append(ws)
         if device.type == "cuda":
             stream = wrapper.write_get_raw_stream(device.index, V.graph.name)
             wrapper.writeline(f"{name}.run({', '.join(map(str, call_args))}, stream={stream})")
         else:
             wrapper.writeline(f"{name}.run({', '.join(map(str, call_args))}, stream=None)")
+        if self.columns:
+            wrapper.writeline(f"del {ws}")
 
     def codegen_nan_check(self) -> None:
         return

@@ -435,8 +435,9 @@ template <class Body> int launch_pointwise(const Body& body, long long xnumel, v
 //                                  scales and shifts): loaded and widened once per thread
 //   Raw / fetch(c, x, raw)         the 128-bit vectors of the operands streamed once per row,
 //                                  requested one row ahead of the arithmetic
-//   row<STAGED>(c, k, x, raw)      the math of row x; STAGED says whether `raw` was fetched
-//                                  (aligned operands) or the body loads for itself
+//   row<STAGED>(c, k, x, raw, cols) the math of row x; STAGED says whether `raw` was fetched
+//                                  (aligned operands) or the body loads for itself; `cols` holds
+//                                  the thread's part of sums over the rows (Cols, clear, flush)
 //   prefetch(c, x)                 L2 prefetch of the streamed operands of a later row
 
 // raw 128-bit vectors of one row-shaped operand of storage type U, as one thread holds them
@@ -825,6 +826,42 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   template <bool STAGED, class U, class A> __device__ __forceinline__ void put_row_shifted(U* rowp, const A& val) const {
     if constexpr (SHIFT) put_row<STAGED>(rowp, val);
     else put_row_any(rowp, val);
+  }
+
+  // ---- sums over the rows -----------------------------------------------------------------
+  // What this thread has summed for its columns, over the teams of the block (team after team, through
+  // `tab`, which nothing else uses any more) and into the block's row of partial sums.
+  __device__ __forceinline__ void flush_column(const vf<kE>& sum, float4* tab, float* partial) const {
+    vf<kE> a = sum;
+#pragma unroll 1
+    for (int t = 0; t < TEAMS; ++t) {
+      if (TEAMS > 1) __syncthreads();
+      if (this->team != t) continue;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i)
+#pragma unroll
+        for (int q = 0; q < kQuads; ++q) {
+          float4& mine = tab[q * kTabVecs + this->lane + i * TEAM];
+          float* v = &a.v[i * Base::kVec + 4 * q];
+          if (t > 0) {
+            const float4 p = mine;
+            v[0] += p.x;
+            v[1] += p.y;
+            v[2] += p.z;
+            v[3] += p.w;
+          }
+          if (t < TEAMS - 1) {
+            mine = make_float4(v[0], v[1], v[2], v[3]);
+          } else if (!SHIFT && !cut(i)) {
+            *reinterpret_cast<float4*>(partial + this->vec_col(i) + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (inside(i, 4 * q + j)) partial[this->vec_col(i) + 4 * q + j] = v[j];
+          }
+        }
+    }
+    if (TEAMS > 1) __syncthreads();
   }
 
   // ---- team exchange --------------------------------------------------------------------
@@ -1456,6 +1493,47 @@ template <class K> inline int row_resident(K kern, int threads, size_t smem = 0)
   return n;
 }
 
+// Sums over the rows beside the row's own work (the gradient of a norm's weight beside that of its input):
+// every thread sums its columns over the rows of its team in fp32, a block folds its teams and stores one
+// row of partial sums, and finish_columns adds those.  A kernel of its own reads both operands a second
+// time: 32768 x 4096 bf16, gradient of the input 121 us and of the weight 88,
+// both together 127.
+constexpr int kMaxPartials = 592;   // rows of partial sums of one column sum: blocks of the row kernel at most
+__host__ __device__ constexpr long long partial_pitch(long long cols) { return (cols + 3) / 4 * 4; }
+// 32 columns a block, a warp for every 32nd partial row: there are few of them to go round (eight warps
+// a block took 4 us longer on 1024 columns)
+constexpr int kFinishSlices = 32;
+template <class U>
+__global__ void __launch_bounds__(32 * kFinishSlices) finish_columns_kernel(const float* partial, int rows, int cols, U* out) {
+  __shared__ float fold[kFinishSlices][33];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int col = (int)blockIdx.x * 32 + lane;
+  pdl_launch_dependents();
+  pdl_wait();
+  float s[2] = {0.f, 0.f};
+  if (col < cols) {
+    const float* p = partial + col;
+    const long long pitch = partial_pitch(cols);
+    int r = slice;
+#pragma unroll 2
+    for (; r + kFinishSlices < rows; r += 2 * kFinishSlices) {
+      s[0] += p[r * pitch];
+      s[1] += p[(r + kFinishSlices) * pitch];
+    }
+    if (r < rows) s[0] += p[r * pitch];
+  }
+  fold[slice][lane] = s[0] + s[1];
+  __syncthreads();
+  // a warp for each column
+  const float t = warp_reduce<SumOp>(fold[lane][slice]);
+  const int mine = (int)blockIdx.x * 32 + slice;
+  if (lane == 0 && mine < cols) Mem<U>::st(out + mine, t);
+}
+template <class U> int finish_columns(const float* partial, long long rows, int cols, U* out, void* stream) {
+  return (int)launch_pdl(finish_columns_kernel<U>, (unsigned)((cols + 31) / 32), 32 * kFinishSlices, 0, (cudaStream_t)stream, partial,
+                         (int)rows, cols, out);
+}
+
 template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS, int PF, int COLS, bool STAGED>
 __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     row_gen_kernel(const Body body, const long long rows, const int cols) {
@@ -1463,6 +1541,7 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
   // b + period, ... only: its offset stays what it is, and the row is worked on in the aligned
   // vectors of memory as if it began there (`off` elements that are masked), per-column operands
   // shifted once to match - nothing is shifted per row.
+  static_assert(Body::kColumns == 0 || TEAM >= 32, "sums over the rows want whole warps to a row");
   constexpr int kPeriod = STAGED && TEAM >= 32 ? Body::kShiftPeriod : 0;
   using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS, (kPeriod > 0)>;
   constexpr int kSlots = TEAM > 32 ? 2 * (TEAM / 32) * 4 : 1;  // exchange floats per team
@@ -1492,6 +1571,8 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
   if constexpr (TEAM >= 32 && STAGED) {
     if (row0 < rows) body.fetch(c, row0, nxt);
   }
+  typename Body::Cols sums;
+  body.clear(sums);
   typename Body::Consts k;
   body.init(c, k);
   if constexpr (Body::kSmemConsts > 0) __syncthreads();   // the operand table is complete
@@ -1522,7 +1603,7 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
         if (b >= rows) break;            // uniform over the CTA
         const long long r = b + c.team;
         c.live = r < rows;
-        body.template row<STAGED>(c, k, c.live ? r : rows - 1, raw[u]);
+        body.template row<STAGED>(c, k, c.live ? r : rows - 1, raw[u], sums);
       }
     }
     return;
@@ -1539,13 +1620,18 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
         const long long ahead = r + (PF + (STAGED ? 1 : 0)) * stride;
         if (ahead < rows) body.prefetch(c, ahead);
       }
-      body.template row<STAGED>(c, k, r, cur);
+      body.template row<STAGED>(c, k, r, cur, sums);
       r = rn;
+    }
+    if constexpr (Body::kColumns > 0) {
+      __syncthreads();    // the operand table is done with
+      body.flush(c, sums, reinterpret_cast<float4*>(operand_table));
     }
   }
 }
 template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS = 1, int PF = 0, int COLS = 0>
-int launch_row_gen(const Body& body, long long rows, int cols, void* stream, bool aligned = false) {
+int launch_row_gen(const Body& body, long long rows, int cols, void* stream, bool aligned = false,
+                   long long* blocks = nullptr) {
   if (rows <= 0) return 0;
   if (COLS > 0 && cols != COLS) return (int)cudaErrorInvalidValue;
   // a row longer than the team can hold (a run-time extent beyond the compiled capacity);
@@ -1556,7 +1642,9 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long groups = (rows + TEAMS - 1) / TEAMS;
   using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS>;
-  const size_t smem = (size_t)Body::kSmemConsts * Ctx::kQuads * Ctx::kTabVecs * sizeof(float4);
+  // (the table also takes one column sum of the block's teams)
+  constexpr int kSlots = Body::kSmemConsts > 0 ? Body::kSmemConsts : (Body::kColumns > 0 && TEAMS > 1 ? 1 : 0);
+  const size_t smem = (size_t)kSlots * Ctx::kQuads * Ctx::kTabVecs * sizeof(float4);
   constexpr int kPeriod = TEAM >= 32 ? Body::kShiftPeriod : 0;
   // (a row in the vectors of memory may need one vector more than its own length)
   if (kPeriod > 0 && cols + Elem<T>::kVec - 1 > TEAM * VPT * Elem<T>::kVec) aligned = false;
@@ -1565,6 +1653,7 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
     const int resident = row_resident(kern, TEAM * TEAMS, smem);
     if (resident < 1) return (int)cudaErrorInvalidConfiguration;
     long long grid = (long long)sms * resident;
+    if (Body::kColumns > 0 && grid > kMaxPartials) grid = kMaxPartials;
     if constexpr (kPeriod > 0) {      // as many blocks for each offset
       const long long most = grid < kPeriod ? kPeriod : grid / kPeriod * kPeriod;
       grid = (groups + kPeriod - 1) / kPeriod * kPeriod;
@@ -1572,13 +1661,16 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
     } else if (grid > groups) {
       grid = groups;
     }
+    if (blocks != nullptr) *blocks = grid;
     return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
   }
   auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, COLS, false>;
   const int resident = row_resident(kern, TEAM * TEAMS, smem);
   if (resident < 1) return (int)cudaErrorInvalidConfiguration;
   long long grid = (long long)sms * resident;
+  if (Body::kColumns > 0 && grid > kMaxPartials) grid = kMaxPartials;
   if (grid > groups) grid = groups;
+  if (blocks != nullptr) *blocks = grid;
   return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
 }
 

@@ -65,3 +65,15 @@ def test_against_64_bits(cuda, fn, dtype, rows, cols):
     tol = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}[dtype]
     err = (got.double() - want.double()).abs() / want.double().abs().clamp_min(float(want.double().square().mean().sqrt()))
     assert float(err.max()) <= tol
+
+
+def test_sum_over_many_rows_with_a_statistic_is_an_outer_reduction(dry_backend):
+    """More rows than one block could hold as a row: the statistic's stride of 1 along them does not make
+    the group a row walked in chunks (100000 x 1024: 870 us that way against 90)."""
+    from torch._inductor.utils import run_and_get_code
+
+    torch._dynamo.reset()
+    x, dy = (torch.empty(70000, 64, dtype=torch.bfloat16) for _ in range(2))
+    fn = lambda x, dy, rstd: (dy.float() * x.float() * rstd).sum(0)
+    code = "\n".join(run_and_get_code(torch.compile(fn, dynamic=False), x, dy, torch.empty(70000, 1))[1])
+    assert "launch_outer" in code and "launch_row_gen" not in code
