@@ -71,6 +71,7 @@ constexpr size_t kSmemBytes = (size_t)kTileBytes * 6 + 1024;
 struct Out {
   void* ptr;
   long long sb, sh, ss;  // strides in elements
+  bool wide;             // every row is a multiple of 32 bytes
 };
 struct BwdParams {
   const float* lse;    // [B, H, Sq] natural-log sum of exponentials of the forward
@@ -190,23 +191,13 @@ __device__ __forceinline__ void issue_ts_group(uint32_t d, uint32_t a, uint64_t 
 
 // GC accumulator columns of this thread's row -> 16-bit values in global memory
 template <bool IS_BF16>
-__device__ __forceinline__ void store_cols(uint32_t taddr, unsigned char* dst, float mult, bool live) {
+__device__ __forceinline__ void store_cols(uint32_t taddr, unsigned char* dst, float mult, bool live, bool wide) {
 #pragma unroll
   for (int c = 0; c < GC / 32; ++c) {
     uint32_t acc[32];
     tc::tmem_ld32(taddr + c * 32, acc);
     tc::tmem_wait_ld();
-    if (live) {
-#pragma unroll
-      for (int e = 0; e < 32; e += 8) {
-        uint4 w;
-        w.x = pack_pair(__uint_as_float(acc[e]) * mult, __uint_as_float(acc[e + 1]) * mult, IS_BF16);
-        w.y = pack_pair(__uint_as_float(acc[e + 2]) * mult, __uint_as_float(acc[e + 3]) * mult, IS_BF16);
-        w.z = pack_pair(__uint_as_float(acc[e + 4]) * mult, __uint_as_float(acc[e + 5]) * mult, IS_BF16);
-        w.w = pack_pair(__uint_as_float(acc[e + 6]) * mult, __uint_as_float(acc[e + 7]) * mult, IS_BF16);
-        *reinterpret_cast<uint4*>(dst + (c * 32 + e) * 2) = w;
-      }
-    }
+    if (live) tc::store_row32<IS_BF16>(dst + c * 64, acc, mult, wide);
   }
 }
 
@@ -528,8 +519,8 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
                               2 * ((long long)b * p.dk.sb + (long long)h * p.dk.sh + (long long)kj * p.dk.ss) +
                               2 * GC * g;
       if (n_it > 0) {
-        store_cols<IS_BF16>(lane_addr + kColAcc0 + GC * g, dv_row, 1.f, live);
-        store_cols<IS_BF16>(lane_addr + kColAcc1 + GC * g, dk_row, p.scale, live);
+        store_cols<IS_BF16>(lane_addr + kColAcc0 + GC * g, dv_row, 1.f, live, p.dv.wide);
+        store_cols<IS_BF16>(lane_addr + kColAcc1 + GC * g, dk_row, p.scale, live, p.dk.wide);
       } else if (live) {
         // no query sees this key tile: the gradients are zero
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
@@ -781,7 +772,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       unsigned char* dq_row = reinterpret_cast<unsigned char*>(p.dq.ptr) +
                               2 * ((long long)b * p.dq.sb + (long long)h * p.dq.sh + (long long)qi * p.dq.ss) +
                               2 * GC * g;
-      store_cols<IS_BF16>(lane_addr + kColAcc0 + GC * g, dq_row, p.scale, live);
+      store_cols<IS_BF16>(lane_addr + kColAcc0 + GC * g, dq_row, p.scale, live, p.dq.wide);
     } else {
       failed = 1;
     }
@@ -935,7 +926,7 @@ __global__ void __launch_bounds__(kDsThreads, 1)
                                 2 * ((long long)b * p.dq.sb + (long long)h * p.dq.sh + (long long)qi * p.dq.ss);
 #pragma unroll
         for (int g = 0; g < NG; ++g)
-          store_cols<IS_BF16>(lane_addr + 128 * t + GC * g, dq_row + 2 * GC * g, p.scale, qi < p.Sq);
+          store_cols<IS_BF16>(lane_addr + 128 * t + GC * g, dq_row + 2 * GC * g, p.scale, qi < p.Sq, p.dq.wide);
       }
     } else {
       failed = 1;
@@ -1030,9 +1021,9 @@ extern "C" int ixb_fa_bwd_scratch(int dtype, const void* q, const void* k, const
   BwdParams p;
   p.lse = lse;
   p.delta = delta;
-  p.dq = Out{dq, dq_strides[0], dq_strides[1], dq_strides[2]};
-  p.dk = Out{dk, dk_strides[0], dk_strides[1], dk_strides[2]};
-  p.dv = Out{dv, dv_strides[0], dv_strides[1], dv_strides[2]};
+  p.dq = Out{dq, dq_strides[0], dq_strides[1], dq_strides[2], ixb_host::rows_aligned32(dq, dq_strides)};
+  p.dk = Out{dk, dk_strides[0], dk_strides[1], dk_strides[2], ixb_host::rows_aligned32(dk, dk_strides)};
+  p.dv = Out{dv, dv_strides[0], dv_strides[1], dv_strides[2], ixb_host::rows_aligned32(dv, dv_strides)};
   p.status = status;
   p.B = B;
   p.H = H;

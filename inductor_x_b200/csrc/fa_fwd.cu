@@ -32,7 +32,15 @@
 // per item; 963 us with the warp-wide issue, the row in registers and P handed over in two parts
 // (at 64 keys instead of 96: 945 against 933 below); 933 us with items taken over by running
 // blocks - 966, 1142, 1179 TFLOP/s.  The products alone take 803 us, everything but the
-// exponentials 858 us.  16 x 16 heads of 1000 keys, fp16: 177, 156, 138 us.
+// exponentials 858 us.  16 x 16 heads of 1000 keys, fp16: 177, 156, 138 us; 127 - 133 with whole sectors
+// stored and only those columns of an edge tile looked at that some row does not see (512 keys: 52 and
+// 50).  An item of eight key tiles takes 29400 cycles there, 2870 a step, of which the tensor core works
+// 2048, and 6500 between the last scores of one item and the first of the next: all SMs store and load at
+// once.  Built, measured and dropped: O by way of shared memory, a line a store (512 keys 48, but 128
+// keys 19.5 against 18.7 and 300 keys 38.3 against 36.3); the next item's first scores behind the
+// last product of the first tile (no difference); one, two, three of eight exponentials on the fma pipe
+// (1000 keys 130, 131, 134 against 129, 4096 causal keys 973 - 1009, 1020 - 1038, 1093 against 985 - 1006:
+// power, not the ex2 unit, is the limit there).
 #include <atomic>
 #include "host.h"
 #include "fa_maps.h"
@@ -68,6 +76,7 @@ struct FaParams {
   int B, H, Sq, Sk;
   float scale_log2;      // softmax scale * log2(e), > 0
   int causal;
+  int wide;        // the rows of o are multiples of 32 bytes
   int head_group;  // heads whose CTAs are dispatched together (see the CTA order in the kernel)
 };
 
@@ -352,8 +361,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc::tmem_wait_ld();
         if (edge) {
 #pragma unroll
-          for (int e = 0; e < BN; ++e)
-            if (e > lim) raw[e] = 0xff800000u;  // -inf
+          for (int c = 0; c < BN / 32; ++c) {
+            if (__all_sync(kFull, lim >= c * 32 + 31)) continue;  // (what every row of the warp sees stays)
+#pragma unroll
+            for (int e = c * 32; e < c * 32 + 32; ++e)
+              if (e > lim) raw[e] = 0xff800000u;  // -inf
+          }
         }
         // four independent chains: one chain of 64 dependent max3 would cost its latency 64 times
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -429,17 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t o[32];
             tc::tmem_ld32(o_addr + c * 32, o);
             tc::tmem_wait_ld();
-            if (live) {
-#pragma unroll
-              for (int e = 0; e < 32; e += 8) {
-                uint4 w;
-                w.x = pack_pair(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv, IS_BF16);
-                w.y = pack_pair(__uint_as_float(o[e + 2]) * inv, __uint_as_float(o[e + 3]) * inv, IS_BF16);
-                w.z = pack_pair(__uint_as_float(o[e + 4]) * inv, __uint_as_float(o[e + 5]) * inv, IS_BF16);
-                w.w = pack_pair(__uint_as_float(o[e + 6]) * inv, __uint_as_float(o[e + 7]) * inv, IS_BF16);
-                *reinterpret_cast<uint4*>(orow + (c * 32 + e) * 2) = w;
-              }
-            }
+            if (live) tc::store_row32<IS_BF16>(orow + c * 64, o, inv, p.wide != 0);
           }
           if (live && p.lse != nullptr) {
             const float lse = (l > 0.f) ? (m_used + log2f(l)) * 0.69314718055994530942f : -INFINITY;
@@ -515,6 +518,7 @@ extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v
   p.Sk = Sk;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.causal = causal ? 1 : 0;
+  p.wide = ixb_host::rows_aligned32(o, o_strides) ? 1 : 0;
   // Without a mask every query block of a head reads all of its K and V, so the heads go one
   // after the other (group of 1: blockIdx order = head-major, as a 2-D grid would give).
   // Under a causal mask 8 heads run together (measured at 4096 keys: 1, 8, 16 heads within 1 %

@@ -14,6 +14,10 @@ int cuda_status(cudaError_t e);
 const ixb_devinfo* current_device();
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+// rows of 16-bit values, (batch, head, sequence) strides in elements: every row a multiple of 32 bytes
+inline bool rows_aligned32(const void* p, const int64_t* strides) {
+  return (reinterpret_cast<uintptr_t>(p) & 31u) == 0 && strides[0] % 16 == 0 && strides[1] % 16 == 0 && strides[2] % 16 == 0;
+}
 inline int elem_size(int dtype) {
   switch (dtype) {
     case IXB_F32: return 4;

@@ -186,6 +186,38 @@ __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// ---- 32 accumulators of one row to memory as 16-bit values ----------------------------------------
+// A lane stores its own row, so the lanes of a warp touch 32 lines an instruction, and the waits of the
+// other roles queue behind in the load/store unit: a store moves a whole 32-byte sector where the
+// rows allow it (`wide`: `dst` is a multiple of 32 bytes), half of one otherwise.
+template <bool IS_BF16> __device__ __forceinline__ uint32_t round_pair(float lo, float hi) {
+  if constexpr (IS_BF16) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+template <bool IS_BF16>
+__device__ __forceinline__ void store_row32(unsigned char* dst, const uint32_t (&acc)[32], float mult, bool wide) {
+  uint32_t w[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k)
+    w[k] = round_pair<IS_BF16>(__uint_as_float(acc[2 * k]) * mult, __uint_as_float(acc[2 * k + 1]) * mult);
+  if (wide) {
+#pragma unroll
+    for (int k = 0; k < 16; k += 8)
+      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 4 * k), "r"(w[k]), "r"(w[k + 1]),
+                   "r"(w[k + 2]), "r"(w[k + 3]), "r"(w[k + 4]), "r"(w[k + 5]), "r"(w[k + 6]), "r"(w[k + 7])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int k = 0; k < 16; k += 4)
+      *reinterpret_cast<uint4*>(dst + 4 * k) = make_uint4(w[k], w[k + 1], w[k + 2], w[k + 3]);
+  }
+}
+
 // ---- leaving after a wait that gave up --------------------------------------------------------
 // A block must not leave while copies into its shared memory or MMAs on its operands are under way.
 // Bounded like every wait, and without a look at the abort flag, which is up by then.
