@@ -14,6 +14,7 @@ import copy
 
 import sympy
 import torch
+from torch._inductor import config as inductor_config
 from torch._inductor.codegen.common import BackendFeature
 from torch._inductor.codegen.simd import SIMDScheduling
 from torch._inductor.dependencies import MemoryDep
@@ -107,8 +108,8 @@ class ColumnGroup:
             if n in sums:
                 continue
             reads, writes = list(n.read_writes.reads), list(n.get_buffer_names())
-            if n._body.op_counts != {"load": 1, "to_dtype": 1, "store": 1, "output": 1} or len(reads) != 1 or len(writes) != 1 or \
-                    reads[0].name not in made or reads[0].name in casts or V.graph.get_dtype(reads[0].name) != torch.float32:
+            if getattr(n._body, "op_counts", None) != {"load": 1, "to_dtype": 1, "store": 1, "output": 1} or len(reads) != 1 or len(writes) != 1 or \
+                    reads[0].name not in made or reads[0].name in casts or _dtype(reads[0].name) != torch.float32:
                 return None
             users = {u.node.get_name() for out in made[reads[0].name].get_outputs() for u in out.users}
             index = reads[0].index
@@ -126,7 +127,7 @@ class ColumnGroup:
         """``group`` is one of row reductions over the same rows, worked on by the row template, that
         reads all that the sums read (so that none of it is given back or written over before)
         and has nothing to do with their results, and its threads can hold their part of the sums."""
-        if type(group).__name__ not in ("SchedulerNode", "FusedSchedulerNode") or not group.is_reduction() or \
+        if not _is_generated(group) or not group.is_reduction() or \
                 [_static(v) for v in group.group[1]] != [self.rows, self.cols]:
             return False
         reads, writes = {d.name for d in _reads(group)}, set(group.get_buffer_names())
@@ -149,9 +150,9 @@ class ColumnGroup:
                 return False
             seen.add(d.name)
         for n in [*group.get_nodes(), *self.nodes]:
-            dtypes += [V.graph.get_dtype(d.name) for d in [*n.read_writes.reads, *n.read_writes.writes]]
+            dtypes += [_dtype(d.name) for d in [*n.read_writes.reads, *n.read_writes.writes]]
         floats = [d for d in dtypes if d in (torch.float32, torch.float16, torch.bfloat16)]
-        if seen != self.matrices or len(floats) != len([d for d in dtypes if d.is_floating_point]):
+        if None in dtypes or seen != self.matrices or len(floats) != len([d for d in dtypes if d.is_floating_point]):
             return False
         # whole warps to a row, and at most 64 registers of sums in the default launch shape
         cfg = split_tiling.choose_row_config(self.cols, split_tiling.narrowest_dtype(floats), rows=self.rows)
@@ -165,6 +166,17 @@ class ColumnGroup:
 
 def _static(numel):
     return int(numel) if isinstance(numel, int) or getattr(numel, "is_Integer", False) else None
+
+
+def _dtype(name):
+    try:
+        return V.graph.get_dtype(name)
+    except Exception:
+        return None
+
+
+def _is_generated(node) -> bool:
+    return type(node).__name__ in ("SchedulerNode", "FusedSchedulerNode")
 
 
 def _reads(node):
@@ -213,7 +225,8 @@ class B200Scheduling(SIMDScheduling):
     def codegen_node(self, node):
         if self._done.pop(id(node), None) is not None:
             return None
-        if config.merged_column_sums and id(node) not in self._put_off:
+        # (combo kernels are emitted past this function)
+        if config.merged_column_sums and not inductor_config.combo_kernels and id(node) not in self._put_off:
             sums = ColumnGroup.of(node)
             partner = self._partner(node, lambda later: sums.fits(later), lambda between: sums) if sums else None
             if partner is not None:
@@ -259,9 +272,11 @@ class B200Scheduling(SIMDScheduling):
         if at is None:
             return None
         for later in order[at + 1:at + 1 + self.COLUMN_SUM_WINDOW]:
-            if type(later).__name__ in ("SchedulerNode", "FusedSchedulerNode") and id(later) not in self._put_off and \
+            if _is_generated(later) and id(later) not in self._put_off and \
                     id(later) not in self._done and later.get_device() == node.get_device() and wanted(later):
                 return later
+            if inductor_config.graph_partition and not (_is_generated(later) and later.get_device() == node.get_device()):
+                return None      # what follows may belong to another partition of the graph
             if sums is not None and sums(later).is_touched_by(later):
                 return None
         return None

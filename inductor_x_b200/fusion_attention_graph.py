@@ -650,7 +650,8 @@ class B200AttentionPass(CustomGraphModulePass):
         here = os.path.dirname(os.path.abspath(__file__))
         files = tuple(sorted(glob.glob(os.path.join(here, "*.py")) + glob.glob(os.path.join(here, "codegen", "*.py"))))
         flags = (config.merged_welford, config.merged_online_softmax, config.debug_bounds, config.fp64_as_fp32,
-                 config.attention_fp32_as_fp16)
+                 config.attention_fp32_as_fp16, config.merged_column_sums, config.column_sum_elements,
+                 config.column_sum_elements_odd)
         h = hashlib.sha256(get_hash_for_files(files))
         h.update(jit._template_digest())
         h.update(repr(flags).encode())

@@ -61,7 +61,7 @@ def test_sums_behind_the_row_kernel_and_their_conversions(dry_backend):
 @needs_nvcc
 @pytest.mark.parametrize("why", ["off", "few rows", "small", "wide", "other order", "used between", "short rows"])
 def test_what_stays_a_kernel_of_its_own(dry_backend, monkeypatch, why):
-    rows, cols = {"few rows": (100, 65536), "small": (2048, 4096), "wide": (2048, 32768 * 4), "short rows": (1 << 18, 128)}.get(why, (4096, 4096))
+    rows, cols = {"few rows": (100, 65536), "small": (1024, 4096), "wide": (2048, 32768 * 4), "short rows": (1 << 18, 128)}.get(why, (4096, 4096))
     monkeypatch.setattr(config, "merged_column_sums", why != "off")
     x, dy = (torch.empty(rows, cols, dtype=torch.bfloat16) for _ in range(2))
     w, rstd = torch.empty(cols, dtype=torch.bfloat16), torch.empty(rows, 1)
