@@ -1497,7 +1497,7 @@ template <class K> inline int row_resident(K kern, int threads, size_t smem = 0)
 // every thread sums its columns over the rows of its team in fp32, a block folds its teams and stores one
 // row of partial sums, and finish_columns adds those.  A kernel of its own reads both operands a second
 // time: 32768 x 4096 bf16, gradient of the input 121 us and of the weight 88,
-// both together 127.
+// both together 123.
 constexpr int kMaxPartials = 592;   // rows of partial sums of one column sum: blocks of the row kernel at most
 __host__ __device__ constexpr long long partial_pitch(long long cols) { return (cols + 3) / 4 * 4; }
 // 32 columns a block, a warp for every 32nd partial row: there are few of them to go round (eight warps
