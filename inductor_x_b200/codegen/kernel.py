@@ -263,7 +263,8 @@ class B200Kernel(SIMDKernel):
         always use the outer mapping, whose body loops over the reduced axis anyway."""
         if not self.features.is_reduction():
             return True
-        vec = min(max(ixb_config.get_aligned_numel(self._narrowest_node_dtype()), 1), 8)
+        dt = self._narrowest_node_dtype()
+        vec = min(max(ixb_config.get_aligned_numel(dt), 1), 8)
         try:
             rnumel = int(self.features.reduction_numel)
         except TypeError:
@@ -273,8 +274,7 @@ class B200Kernel(SIMDKernel):
             hint = int(V.graph.sizevars.size_hint(self.features.reduction_numel))
             self.looped = -(-hint // vec) > split_tiling.MAX_TEAM * split_tiling.MAX_VPT
             return not self.looped
-        nvec = -(-rnumel // vec)
-        long_row = nvec > split_tiling.MAX_TEAM * split_tiling.MAX_PERSISTENT_VPT
+        long_row = split_tiling.walked_in_chunks(rnumel, dt)
         try:
             kept = int(self.features.numel)
         except TypeError:
@@ -695,6 +695,8 @@ class B200Kernel(SIMDKernel):
     def reduction(self, dtype, src_dtype, reduction_type, value):
         assert self.inside_reduction and self.is_row
         if self.column_mode:
+            if self.looped:         # (one set of sums a thread: every chunk would go into it)
+                raise UnsupportedByTemplates("sums over the rows beside rows walked in chunks")
             # into this thread's sum for its columns; stored when the block has no rows left
             factors = self.op_of(value, "mul")
             acc = f"cols.a{len(self.columns)}"

@@ -149,13 +149,17 @@ class ColumnGroup:
             if stride != self.rows * self.cols or sympy.expand(d.index - expected) != 0:
                 return False
             seen.add(d.name)
-        for n in [*group.get_nodes(), *self.nodes]:
+        # (what the kernel will see: a conversion is not a node of it)
+        for n in [*group.get_nodes(), *self.sums]:
             dtypes += [_dtype(d.name) for d in [*n.read_writes.reads, *n.read_writes.writes]]
         floats = [d for d in dtypes if d in (torch.float32, torch.float16, torch.bfloat16)]
         if None in dtypes or seen != self.matrices or len(floats) != len([d for d in dtypes if d.is_floating_point]):
             return False
+        narrowest = split_tiling.narrowest_dtype(floats)
+        if split_tiling.walked_in_chunks(self.cols, narrowest):
+            return False          # a thread's sums are those of one chunk
         # whole warps to a row, and at most 64 registers of sums in the default launch shape
-        cfg = split_tiling.choose_row_config(self.cols, split_tiling.narrowest_dtype(floats), rows=self.rows)
+        cfg = split_tiling.choose_row_config(self.cols, narrowest, rows=self.rows)
         return cfg is not None and cfg.team >= 32 and cfg.vec % 4 == 0 and cfg.elems_per_thread * len(self.sums) <= 64
 
     def is_touched_by(self, group) -> bool:

@@ -107,6 +107,12 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
                      prefetch=2 if streamed and row_bytes >= 2048 else 0)
 
 
+def walked_in_chunks(rnumel: int, dtype: torch.dtype) -> bool:
+    """A stride-1 row of this length is walked in chunks instead of being held on chip."""
+    vec = min(max(config.get_aligned_numel(dtype), 1), 8)
+    return -(-rnumel // vec) > MAX_TEAM * MAX_PERSISTENT_VPT
+
+
 def choose_loop_config(dtype: torch.dtype) -> RowConfig:
     """Launch shape of a row kernel that walks its rows in chunks: one team of 512 threads
     per CTA, two vectors per thread and chunk, registers bounded for two resident CTAs."""

@@ -1541,7 +1541,7 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
   // b + period, ... only: its offset stays what it is, and the row is worked on in the aligned
   // vectors of memory as if it began there (`off` elements that are masked), per-column operands
   // shifted once to match - nothing is shifted per row.
-  static_assert(Body::kColumns == 0 || TEAM >= 32, "sums over the rows want whole warps to a row");
+  static_assert(Body::kColumns == 0 || (TEAM >= 32 && !Body::kLooped), "sums over the rows want whole warps to a row, and the row on chip");
   constexpr int kPeriod = STAGED && TEAM >= 32 ? Body::kShiftPeriod : 0;
   using Ctx = GenRowCtx<T, TEAM, TEAMS, VPT, COLS, (kPeriod > 0)>;
   constexpr int kSlots = TEAM > 32 ? 2 * (TEAM / 32) * 4 : 1;  // exchange floats per team

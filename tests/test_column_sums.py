@@ -76,6 +76,22 @@ def test_what_stays_a_kernel_of_its_own(dry_backend, monkeypatch, why):
     assert not re.search(r"kColumns = [1-9]", code) and "ixb_partials" not in code
 
 
+@needs_nvcc
+@pytest.mark.parametrize("cols,into", [(32769, torch.float32), (40960, torch.float32), (40960, torch.bfloat16), (65536, torch.float32)])
+def test_rows_walked_in_chunks_leave_the_sums_to_a_kernel_of_their_own(dry_backend, cols, into):
+    """fp32 rows of more than 8192 vectors; a sum that is converted to 16 bits does not make them shorter."""
+    x, dy = (torch.empty(256, cols) for _ in range(2))
+    w, rstd = torch.empty(cols), torch.empty(256, 1)
+
+    def fn(x, w, dy, rstd):
+        dw, dx = _dx_dw(x, w, dy, rstd)
+        return dw.to(into), dx
+
+    code = _code(fn, x, w, dy, rstd)
+    assert code.count("kLooped = true;") == 1 and code.count("ixb_load_kernel('''") >= 2
+    assert not re.search(r"kColumns = [1-9]", code) and "ixb_partials" not in code
+
+
 TOL = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
 
 
@@ -113,6 +129,25 @@ def test_training_step_of_a_norm(cuda, monkeypatch, dtype, rows, cols):
     _close(y.detach(), yd.detach(), dtype)
     _close(dx, ex, dtype)
     _close(dw, ew, dtype)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(256, 32769), (203, 50257)])
+def test_training_step_of_rows_walked_in_chunks(cuda, rows, cols):
+    """fp32 rows longer than a block holds, of a size whose sums would otherwise come out of the row kernel."""
+    import inductor_x_b200  # noqa: F401
+
+    g = torch.Generator(device=cuda).manual_seed(rows)
+    x, dy = (torch.randn(rows, cols, generator=g, device=cuda) for _ in range(2))
+    w = 1 + 0.1 * torch.randn(cols, generator=g, device=cuda)
+    a, b = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+    torch._dynamo.reset()
+    dx, dw = torch.autograd.grad(torch.compile(_norm, dynamic=False)(a, b), (a, b), dy)
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    yd = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * wd
+    ex, ew = torch.autograd.grad(yd, (xd, wd), dy.double())
+    _close(dx, ex, torch.float32)
+    _close(dw, ew, torch.float32)
 
 
 @pytest.mark.gpu
