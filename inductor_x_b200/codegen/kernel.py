@@ -50,9 +50,6 @@ REDUCTION_OPS = {
 
 INT_REDUCTION_OPS = {"sum": "ISum", "prod": "IProd", "max": "IMax", "min": "IMin"}
 
-#: registers a thread may spend on operands that are the same for every row; operands beyond
-#: that budget (the least used ones) live in a shared-memory table
-MAX_CONST_REGS = 64
 #: per-column operands hoisted out of the row loop at most (registers + shared memory)
 MAX_CONSTS = 6
 #: streamed operands fetched one row ahead as raw 128-bit vectors
@@ -149,7 +146,7 @@ class B200Kernel(SIMDKernel):
             if self.looped:
                 self._row_cfg = split_tiling.choose_loop_config(dt)
             else:
-                self._row_cfg = split_tiling.choose_row_config(self._covering(rnumel, dt), dt, rows=self._numel_hint("x"),
+                self._row_cfg = split_tiling.choose_row_config(rnumel, dt, rows=self._numel_hint("x"),
                                                                 exact=not self._is_dynamic("r0_"))
                 if self._row_cfg is None and self._reads_are_strided():
                     # an outer reduction of any length: the outer mapping loops over the reduced
@@ -166,12 +163,6 @@ class B200Kernel(SIMDKernel):
 
     def create_cse_var(self, *args, **kwargs):
         return B200CSEVariable(*args, **kwargs)
-
-    def _covering(self, rnumel: int, dt: torch.dtype) -> int:
-        """Elements of the aligned vectors that a row of ``rnumel`` may touch: one vector's worth
-        less one more where its length moves the rows off a boundary (see _row_shift)."""
-        vec = min(max(ixb_config.get_aligned_numel(dt), 1), 8)
-        return rnumel if rnumel % vec == 0 or self._is_dynamic("r0_") else rnumel + vec - 1
 
     def _row_shift(self, tiling):
         """(pitch, first element, period) when every access of the group that walks a row of its own
@@ -197,6 +188,19 @@ class B200Kernel(SIMDKernel):
             return None
         pitch, first = found.pop()
         return pitch, first, cfg.vec // math.gcd(pitch, cfg.vec)
+
+    def _settle_row_shape(self, tiling):
+        """What _row_shift says, with a launch shape that has a place for every vector a row may touch;
+        None where there is no such shape."""
+        shift = self._row_shift(tiling)
+        if shift is None:
+            return None
+        cfg = split_tiling.covering_config(self._static_numel("r0_"), self._narrowest_node_dtype(), self._row_cfg,
+                                           len(self.consts), rows=self._numel_hint("x"))
+        if cfg is None:
+            return None
+        self._row_cfg = cfg
+        return shift
 
     # ------------------------------------------------------------------ value table
     def note_op(self, var, name, args, kwargs=None) -> None:
@@ -527,8 +531,10 @@ class B200Kernel(SIMDKernel):
                 # the same for every row (a per-column scale or shift): loaded and widened
                 # once per thread while registers allow
                 const_member = next((m for m, ptr, _ in self.consts if ptr == row_ptr), None)
-                if const_member is None and narrow_ok and len(self.consts) < MAX_CONSTS and \
-                        cfg.team >= 32 and cfg.vec % 4 == 0 and not self.looped:
+                n_consts = len(self.consts) + 1
+                if const_member is None and narrow_ok and n_consts <= MAX_CONSTS and \
+                        cfg.team >= 32 and cfg.vec % 4 == 0 and not self.looped and \
+                        split_tiling.table_fits(n_consts, split_tiling.const_regs(n_consts, n), cfg.capacity):
                     const_member = f"@K{len(self.consts)}@"      # final slot and home decided at print time
                     self.consts.append((const_member, row_ptr, n))
                 if const_member is not None:
@@ -1213,6 +1219,8 @@ class B200Kernel(SIMDKernel):
                 f"a strided reduction over {self._static_numel('r0_')} elements that the outer template cannot "
                 "take (several reductions or values shared across the reduction loop)")
 
+        tiling = self._short_row_tiling() if self.mapping == "row" else None
+        shift = self._settle_row_shape(tiling) if self.mapping == "row" else None
         src = IndentedBuffer()
         if self.checked_indices:
             src.writeline("#define IXB_DEBUG_BOUNDS 1")
@@ -1222,7 +1230,7 @@ class B200Kernel(SIMDKernel):
             # same body in other shapes (-D...) and keep the one that measures fastest;
             # IXB_GEN_MIN_CTAS bounds the registers and is relaxed by the loader on spills.
             cfg = self._row_cfg
-            kregs = min(len(self.consts), MAX_CONST_REGS // max(cfg.elems_per_thread, 1))
+            kregs = split_tiling.const_regs(len(self.consts), cfg.elems_per_thread)
             for macro, val in (("IXB_GEN_MIN_CTAS", cfg.min_ctas), ("IXB_ROW_TEAM", cfg.team),
                                ("IXB_ROW_TEAMS", cfg.teams), ("IXB_ROW_VPT", cfg.vpt),
                                ("IXB_ROW_PF", cfg.prefetch), ("IXB_ROW_KREGS", kregs)):
@@ -1333,7 +1341,6 @@ class B200Kernel(SIMDKernel):
                 import re
 
                 cfg = self._row_cfg
-                tiling = self._short_row_tiling()
                 # rows of a whole 128-byte line or more: the output digit runs fastest inside a tile
                 b_first = tiling is not None and \
                     self._static_numel("r0_") * config_bytes(self._narrowest_node_dtype()) >= 128
@@ -1341,7 +1348,6 @@ class B200Kernel(SIMDKernel):
                              f"const long long xindex = {G}tile_order<{tiling[0]}, {tiling[1]}, 16, 16, "
                              f"{'true' if b_first else 'false'}>(xslot);")
                 row_body = re.sub(r"@B\d+@\n?", "", self._substitute(body_text, False))
-                shift = self._row_shift(tiling)
                 if shift is not None:
                     row_body = row_body.replace("c.put_row_any(", "c.template put_row_shifted<STAGED>(")
                 # per-column operands, most used first: the first IXB_ROW_KREGS of them are
@@ -1564,9 +1570,9 @@ class B200Kernel(SIMDKernel):
         if self.mapping == "row" and not self._is_dynamic("r0_") and not self.looped:
             cfg = self._row_cfg
             inplace = bool(self.args.inplace_buffers)
-            kregs = min(len(self.consts), MAX_CONST_REGS // max(cfg.elems_per_thread, 1))
-            shapes = split_tiling.row_candidates(self._covering(self._static_numel("r0_"), self._narrowest_node_dtype()), cfg, rows=xnumel_hint,
-                                                 n_consts=len(self.consts), kregs=kregs)
+            kregs = split_tiling.const_regs(len(self.consts), cfg.elems_per_thread)
+            touched = self._static_numel("r0_") + (cfg.vec - 1 if shift is not None else 0)
+            shapes = split_tiling.row_candidates(touched, cfg, rows=xnumel_hint, n_consts=len(self.consts), kregs=kregs)
             meta += (f", tune=dict(default={(cfg.team, cfg.teams, cfg.vpt, cfg.min_ctas, cfg.prefetch, kregs)!r}, "
                      f"candidates={shapes!r}, rows={xnumel_hint}, row_bytes={self._static_numel('r0_') * config_bytes(self._narrowest_node_dtype())}, "
                      f"idempotent={not inplace!r})")

@@ -57,6 +57,21 @@ MIN_TEAM = 8          # teams narrower than a warp serve rows of a few vectors
 MAX_EXACT_VPT = 5    # vectors per thread up to which a row may be cut to fit its length
 MAX_VPT = 32         # beyond 8 the row no longer fits the register file and spills: slow but correct
 MAX_PERSISTENT_VPT = 8   # static rows longer than MAX_TEAM x this many vectors are walked in chunks
+#: registers a thread may spend on operands that are the same for every row; operands beyond
+#: that budget (the least used ones) live in a shared-memory table
+MAX_CONST_REGS = 64
+#: shared memory of a block that the table may take: 227 KiB less what the exchanges use
+MAX_TABLE_BYTES = 224 * 1024
+
+
+def const_regs(n_consts: int, elems_per_thread: int) -> int:
+    """Per-column operands that stay in registers."""
+    return min(n_consts, MAX_CONST_REGS // max(elems_per_thread, 1))
+
+
+def table_fits(n_consts: int, kregs: int, capacity: int) -> bool:
+    """The other per-column operands, as fp32 rows of the launch shape's capacity, fit in the table."""
+    return (n_consts - kregs) * capacity * 4 <= MAX_TABLE_BYTES
 
 
 def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = None,
@@ -105,6 +120,23 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
     streamed = rows is None or rows * row_bytes >= (64 << 20)
     return RowConfig(team=team, teams=teams, vpt=vpt, vec=vec, min_ctas=min_ctas,
                      prefetch=2 if streamed and row_bytes >= 2048 else 0)
+
+
+def covering_config(rnumel: int, dtype: torch.dtype, base: RowConfig, n_consts: int,
+                    rows: Optional[int] = None) -> Optional[RowConfig]:
+    """The shape for rows that are worked on in the aligned vectors of memory and so may touch one
+    vector more than their length fills: ``base`` where it has that place, the next one up where
+    every vector of it is taken - 16-bit rows of 1017 to 1023 elements, say - or None where that
+    shape is twice as thick as the row needs (past ``MAX_EXACT_VPT``, 16-bit rows of 32761 to 32767
+    and 65529 to 65535) or has no room for the table of per-column operands."""
+    cover = rnumel + base.vec - 1
+    if cover <= base.capacity:
+        return base
+    wide = choose_row_config(cover, dtype, rows=rows)
+    if wide is None or wide.vpt > MAX_EXACT_VPT or \
+            not table_fits(n_consts, const_regs(n_consts, wide.elems_per_thread), wide.capacity):
+        return None
+    return wide
 
 
 def walked_in_chunks(rnumel: int, dtype: torch.dtype) -> bool:
@@ -159,7 +191,7 @@ def row_candidates(rnumel: int, chosen: RowConfig, rows: Optional[int] = None, n
                 if threads * min_ctas > 1024 or (min_ctas > 1 and threads * min_ctas < 256):
                     continue
                 for kr in sorted({kregs, min(n_consts, 1), 0}, reverse=True):
-                    if kr > n_consts:
+                    if kr > n_consts or not table_fits(n_consts, kr, team * vpt * vec):
                         continue
                     shape = (team, teams, vpt, min_ctas, chosen.prefetch, kr)
                     if shape == default or shape in [s for _, s in ranked]:

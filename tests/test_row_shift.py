@@ -53,6 +53,49 @@ def test_rows_of_several_pitches_are_shifted_one_by_one(dry_backend):
     assert period == 0                                     # teams narrower than a warp
 
 
+def _shape(code):
+    return tuple(int(re.search(rf"#define IXB_ROW_{m} (\d+)", code).group(1)) for m in ("TEAM", "VPT", "KREGS")) + \
+        tuple(int(re.search(rf"constexpr int {m} = (\d+);", code).group(1)) for m in ("kConsts", "kShiftPeriod"))
+
+
+@needs_nvcc
+@pytest.mark.parametrize("dtype,cols,kind,shape", [
+    # nothing is shifted: the shape is that of the length itself
+    (torch.float16, 61, "sum", (8, 1, 0, 0, 0)), (torch.bfloat16, 127, "sum", (8, 2, 0, 0, 0)), (torch.float32, 63, "sum", (8, 2, 0, 0, 0)),
+    (torch.float16, 511, "scan", (32, 2, 0, 0, 0)), (torch.float16, 511, "pitches", (32, 2, 1, 1, 0)),
+    # a row of whole warps whose every place is taken, in the next shape
+    (torch.float16, 511, "affine", (32, 3, 2, 2, 8)), (torch.float32, 16379, "affine", (1024, 4, 2, 2, 4)),
+    # ... or, where that would be twice as thick as the row, in its own
+    (torch.float32, 16383, "affine", (1024, 4, 2, 2, 0)), (torch.float32, 32767, "affine", (1024, 8, 2, 2, 0)),
+    (torch.bfloat16, 32767, "affine", (1024, 4, 2, 2, 0)), (torch.bfloat16, 65535, "sum", (1024, 8, 0, 0, 0))])
+def test_shape_of_odd_rows(dry_backend, dtype, cols, kind, shape):
+    x = torch.empty(40, cols + 9).to(dtype)[:, :cols] if kind == "pitches" else torch.empty(40, cols).to(dtype)
+    w, b = (torch.empty(cols).to(dtype) for _ in range(2))
+    fn, args = {"sum": (lambda x: x.float().sum(-1), (x,)), "scan": (lambda x: x.cumsum(-1), (x,)),
+                "pitches": (lambda x, w: (x * w).softmax(-1), (x, w)),
+                "affine": (lambda x, w, b: F.layer_norm(x, (cols,), w, b), (x, w, b))}[kind]
+    assert _shape(_period(fn, *args)[2]) == shape
+
+
+def test_shared_memory_of_every_shape():
+    """What the emitter gives a row and what is measured beside it stay within a block's shared memory."""
+    from inductor_x_b200.codegen import split_tiling as st
+
+    for dtype, vec in ((torch.float32, 4), (torch.float16, 8)):
+        for nvec in sorted({n for k in range(5, 14) for n in (2 ** k - 1, 2 ** k, 2 ** k + 1, 3 * 2 ** k // 2, 5 * 2 ** k // 4)} | {2500}):
+            for cols in (nvec * vec, nvec * vec - 1):
+                if st.walked_in_chunks(cols, dtype):
+                    continue
+                base = st.choose_row_config(cols, dtype, rows=1 << 20)
+                for n in range(7):
+                    cfg = st.covering_config(cols, dtype, base, n, rows=1 << 20)
+                    assert cfg is None or cfg is base or st.table_fits(n, st.const_regs(n, cfg.elems_per_thread), cfg.capacity)
+                    for team, teams, vpt, _, _, kregs in st.row_candidates(cols, base, n_consts=n, kregs=st.const_regs(n, base.elems_per_thread)):
+                        table = max(0, n - kregs) * team * vpt * vec * 4
+                        # 32 bytes a warp of exchange, beside 227 KiB a block may have
+                        assert team < 32 or table + team * teams <= 227 * 1024
+
+
 TOL = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
 
 
@@ -79,6 +122,30 @@ def test_chain_of_odd_rows(cuda, dtype, rows, cols):
     into(x, *p, out)
     _close(out, chain(*(t.double() for t in (x, *p))), dtype)
     assert bool((buf[rows * cols:] == 7).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,cols", [(torch.float32, 32767), (torch.bfloat16, 32767), (torch.float16, 32761), (torch.float32, 16383),
+                                        (torch.float16, 65535), (torch.bfloat16, 32768)])
+@pytest.mark.parametrize("operands", [1, 2, 3, 5])
+def test_long_rows_with_per_column_operands(cuda, dtype, cols, operands):
+    """Rows that fill their team, with more per-column operands than registers and shared memory hold."""
+    import inductor_x_b200  # noqa: F401
+
+    g = torch.Generator(device=cuda).manual_seed(cols)
+    rows = 67
+    x = torch.randn(rows, cols, generator=g, device=cuda).to(dtype)
+    p = [(1 + 0.1 * torch.randn(cols, generator=g, device=cuda)).to(dtype) for _ in range(operands)]
+
+    def fn(x, *p):
+        y = (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6)) * p[0]
+        for n, w in enumerate(p[1:]):
+            y = y + w if n % 2 == 0 else y * w
+        return y
+
+    torch._dynamo.reset()
+    got = torch.compile(lambda x, *p: fn(x.float(), *(w.float() for w in p)).to(dtype), dynamic=False)(x, *p)
+    _close(got, fn(x.double(), *(w.double() for w in p)), dtype)
 
 
 @pytest.mark.gpu
