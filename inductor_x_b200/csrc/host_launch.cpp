@@ -17,6 +17,7 @@
 #include <structmember.h>
 
 #include <ATen/Functions.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -142,7 +143,8 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_ixb_host", nullptr, -1, nullp
 // plain call - checks, allocations, strides, the C entry on the current stream - and returns the
 // result; a status other than 0 comes back as an int, which the caller words.  Anything else (a tensor
 // subclass or a wrapper without storage, a host tensor, a shape, dtype or layout that Python would
-// refuse or copy, an exception) gives None: the Python function then goes its own way, errors included.
+// refuse or copy, a dispatch mode that wants to see the allocations, an exception) gives None: the
+// Python function then goes its own way, errors included.
 // A call of rms_norm (16 x 4096 bf16 with residual) took 9.5 us in Python, launch and two
 // allocations included.
 decltype(&ixb_rmsnorm) entry_rmsnorm;
@@ -167,6 +169,12 @@ PyObject* bind_library(PyObject*, PyObject* const* args, Py_ssize_t n) {
   entry_fa_bwd = reinterpret_cast<decltype(entry_fa_bwd)>(p[3]);
   Py_RETURN_NONE;
 }
+
+PyObject* left_to_python() {
+  PyErr_Clear();   // (an exception that came out of Python code leaves its error set)
+  Py_RETURN_NONE;
+}
+bool observed() { return c10::impl::TorchDispatchModeTLS::any_modes_set(); }
 
 // a CUDA tensor with memory of its own kind behind it
 const at::Tensor* plain_tensor(PyObject* o) {
@@ -196,7 +204,7 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
 
 // rms_norm(x, w, eps, residual or None, return_residual)
 PyObject* rms_norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 5 || entry_rmsnorm == nullptr || !PyFloat_CheckExact(args[2]) || !PyBool_Check(args[4])) Py_RETURN_NONE;
+  if (n != 5 || entry_rmsnorm == nullptr || observed() || !PyFloat_CheckExact(args[2]) || !PyBool_Check(args[4])) Py_RETURN_NONE;
   try {
     const at::Tensor *x = plain_tensor(args[0]), *w = plain_tensor(args[1]);
     if (x == nullptr || w == nullptr || x->dim() < 1 || !x->is_contiguous() || dtype_code(*x) < 0) Py_RETURN_NONE;
@@ -219,7 +227,7 @@ PyObject* rms_norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (st != 0) return PyLong_FromLong(st);
     return h.defined() ? pair(std::move(y), std::move(h)) : THPVariable_Wrap(std::move(y));
   } catch (...) {
-    Py_RETURN_NONE;
+    return left_to_python();
   }
 }
 
@@ -237,7 +245,7 @@ bool attention_operands(const at::Tensor* q, const at::Tensor* k, const at::Tens
 
 // fused_attention(q, k, v, scale, causal, return_lse)
 PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 6 || entry_fa_fwd == nullptr || !PyFloat_CheckExact(args[3]) || !PyBool_Check(args[4]) || !PyBool_Check(args[5]))
+  if (n != 6 || entry_fa_fwd == nullptr || observed() || !PyFloat_CheckExact(args[3]) || !PyBool_Check(args[4]) || !PyBool_Check(args[5]))
     Py_RETURN_NONE;
   try {
     const at::Tensor *q = plain_tensor(args[0]), *k = plain_tensor(args[1]), *v = plain_tensor(args[2]);
@@ -258,13 +266,13 @@ PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (st != 0) return PyLong_FromLong(st);
     return lse.defined() ? pair(std::move(out), std::move(lse)) : THPVariable_Wrap(std::move(out));
   } catch (...) {
-    Py_RETURN_NONE;
+    return left_to_python();
   }
 }
 
 // fused_attention_backward(q, k, v, out, lse, dout, scale, causal, bytes of dS at most)
 PyObject* fused_attention_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 9 || entry_fa_bwd == nullptr || !PyFloat_CheckExact(args[6]) || !PyBool_Check(args[7]) || !PyLong_CheckExact(args[8]))
+  if (n != 9 || entry_fa_bwd == nullptr || observed() || !PyFloat_CheckExact(args[6]) || !PyBool_Check(args[7]) || !PyLong_CheckExact(args[8]))
     Py_RETURN_NONE;
   try {
     const at::Tensor *q = plain_tensor(args[0]), *k = plain_tensor(args[1]), *v = plain_tensor(args[2]),
@@ -309,7 +317,7 @@ PyObject* fused_attention_backward(PyObject*, PyObject* const* args, Py_ssize_t 
     Py_XDECREF(rest);
     return all;
   } catch (...) {
-    Py_RETURN_NONE;
+    return left_to_python();
   }
 }
 

@@ -99,3 +99,48 @@ def test_errors_are_what_they_were(cuda):
         ops.fused_attention(q, q[..., :64], q, 1.0)
     with pytest.raises(RuntimeError):      # a batched tensor has no memory of its own
         torch.vmap(lambda t: ops.rmsnorm(t, w))(x.unsqueeze(0).repeat(2, 1, 1))
+
+
+@pytest.mark.gpu
+def test_dispatch_modes_see_what_python_would_show_them(cuda, monkeypatch):
+    """A mode that raises, one that counts the operations, a fake-tensor mode with real operands: the same
+    error or the same operations with and without the native entries."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchDispatchMode):
+        def __init__(self, raises=False):
+            super().__init__()
+            self.ops, self.raises = [], raises
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.ops.append(str(func))
+            if self.raises:
+                raise KeyError("not here")
+            return func(*args, **(kwargs or {}))
+
+    rt.load()
+    x, w = torch.ones(4, 8, device=cuda), torch.ones(8, device=cuda)
+    q = torch.ones(1, 1, 8, 128, dtype=torch.bfloat16, device=cuda)
+    lse = torch.ones(1, 1, 8, device=cuda)
+    calls = (lambda: ops.rmsnorm(x, w, residual=x, return_residual=True), lambda: ops.fused_attention(q, q, q, 1.0, return_lse=True),
+             lambda: ops.fused_attention_backward(q, q, q, q, lse, q, 1.0))
+
+    def outcome(make, call):
+        mode = make()
+        with mode:
+            try:
+                call()
+                out = None
+            except Exception as e:
+                out = type(e)
+        return out, getattr(mode, "ops", None)
+
+    for call in calls:
+        for make in (Seen, lambda: Seen(True), lambda: FakeTensorMode(allow_non_fake_inputs=True)):
+            with_native = outcome(make, call)
+            with monkeypatch.context() as m:
+                m.setattr(ops, "_ixb_host", types.SimpleNamespace(**{n: lambda *a: None for n in NAMES}))
+                assert outcome(make, call) == with_native
+        assert outcome(lambda: Seen(True), call)[0] is KeyError and outcome(Seen, call)[1]
+    torch.cuda.synchronize()
