@@ -270,7 +270,8 @@ PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
 }
 
-// fused_attention_backward(q, k, v, out, lse, dout, scale, causal, bytes of dS at most)
+// fused_attention_backward(q, k, v, out, lse, dout, scale, causal, bytes of dS at most); False where all
+// but the memory for dS was to be had, so that the caller does not ask for the same again
 PyObject* fused_attention_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 9 || entry_fa_bwd == nullptr || observed() || !PyFloat_CheckExact(args[6]) || !PyBool_Check(args[7]) || !PyLong_CheckExact(args[8]))
     Py_RETURN_NONE;
@@ -294,9 +295,14 @@ PyObject* fused_attention_backward(PyObject*, PyObject* const* args, Py_ssize_t 
     at::Tensor dq = at::empty({B, H, Sq, D}, q->options()), dk = at::empty({B, H, Sk, D}, q->options()),
                dv = at::empty({B, H, Sk, D}, q->options());
     const int causal = args[7] == Py_True;
-    // (where the memory for dS is not to be had, the Python function sees to it)
     const size_t room = entry_fa_bwd_room((int32_t)B, (int32_t)H, (int32_t)Sq, (int32_t)Sk, causal, (size_t)limit);
-    at::Tensor scratch = at::empty({(int64_t)room + 4 * B * H * Sq}, q->options().dtype(at::kByte));
+    at::Tensor scratch;
+    try {
+      scratch = at::empty({(int64_t)room + 4 * B * H * Sq}, q->options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+      if (room > 0) Py_RETURN_FALSE;
+      throw;
+    }
     unsigned char* base = static_cast<unsigned char*>(scratch.data_ptr());
     const Strides qs(*q), ks(*k), vs(*v), os(*o), gs(*go), dqs(dq), dks(dk), dvs(dv);
     const ixb_stream stream = stream_of(*q);

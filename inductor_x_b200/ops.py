@@ -256,20 +256,40 @@ def fused_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: fl
 SCORE_GRADIENT_BYTES = 5 << 29
 
 
+#: a request that fails makes the caching allocator give back all it holds, so a device that could not
+#: give what was asked for is asked for less in this many calls
+SCORE_GRADIENT_RETRY = 1000
+_score_gradient_limits: dict = {}      # device index -> (bytes at most, calls left)
+
+
 @functools.lru_cache(maxsize=1024)
 def _score_gradient_room(B, H, Sq, Sk, causal, limit):
     return rt.load().ixb_fa_bwd_scratch_bytes(B, H, Sq, Sk, int(causal), limit)
 
 
-def _backward_scratch(B, H, Sq, Sk, causal, device):
+def _score_gradient_limit(device: int) -> int:
+    limit, left = _score_gradient_limits.get(device, (SCORE_GRADIENT_BYTES, 0))
+    if left > 1:
+        _score_gradient_limits[device] = (limit, left - 1)
+    else:
+        _score_gradient_limits.pop(device, None)
+    return min(limit, SCORE_GRADIENT_BYTES)
+
+
+def _backward_scratch(B, H, Sq, Sk, causal, device, limit, refused=False):
     """(one allocation, its bytes for dS ahead of the B * H * Sq floats of delta).  Where the memory
-    is not to be had the backward does without dS: it then computes the probabilities twice."""
-    room = _score_gradient_room(B, H, Sq, Sk, causal, SCORE_GRADIENT_BYTES)
-    if room:
-        try:
-            return torch.empty(room + 4 * B * H * Sq, dtype=torch.uint8, device=device), room
-        except torch.cuda.OutOfMemoryError:
-            pass
+    is not to be had (``refused``: it was asked for already) the backward does with half of it, in more
+    launches, and so on down to one head; without dS it computes the probabilities twice."""
+    room = _score_gradient_room(B, H, Sq, Sk, causal, limit)
+    while room:
+        if not refused:
+            try:
+                return torch.empty(room + 4 * B * H * Sq, dtype=torch.uint8, device=device), room
+            except torch.cuda.OutOfMemoryError:
+                pass
+        refused, less = False, room // 2
+        _score_gradient_limits[device.index] = (less, SCORE_GRADIENT_RETRY)
+        room = _score_gradient_room(B, H, Sq, Sk, causal, less)
     return torch.empty(4 * B * H * Sq, dtype=torch.uint8, device=device), 0
 
 
@@ -279,9 +299,12 @@ def fused_attention_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     """Gradients ``(dq, dk, dv)`` of :func:`fused_attention` from its inputs, its output
     ``out``, its log-sum-exp ``lse`` (``return_lse=True``) and the incoming gradient ``dout``
     (tcgen05 kernels behind ``ixb_fa_bwd``; deterministic, no atomics)."""
+    limit = SCORE_GRADIENT_BYTES if not _score_gradient_limits else _score_gradient_limit(q.device.index)
+    refused = False
     if not check:
-        done = _native("ixb_fa_bwd", _ixb_host.fused_attention_backward(q, k, v, out, lse, dout, scale, causal,
-                                                                        SCORE_GRADIENT_BYTES))
+        done = _ixb_host.fused_attention_backward(q, k, v, out, lse, dout, scale, causal, limit)
+        refused = done is False
+        done = None if refused else _native("ixb_fa_bwd", done)
         if done is not None:
             return done
     _need_cuda(q, k, v, out, dout, lse)
@@ -304,7 +327,7 @@ def fused_attention_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     dq = torch.empty((B, H, Sq, D), dtype=q.dtype, device=q.device)
     dk = torch.empty((B, H, Sk, D), dtype=q.dtype, device=q.device)
     dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=q.device)
-    scratch, room = _backward_scratch(B, H, Sq, Sk, causal, q.device)
+    scratch, room = _backward_scratch(B, H, Sq, Sk, causal, q.device, limit, refused)
     status = torch.zeros(1, dtype=torch.int32, device=q.device) if check else None
     q_like, kv_like = _bhs_strides(dq), _bhs_strides(dk)
     rt.check("ixb_fa_bwd", rt.load().ixb_fa_bwd_scratch(

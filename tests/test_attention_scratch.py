@@ -86,3 +86,59 @@ def test_scratch_must_be_aligned(cuda):
     assert rt.load().ixb_fa_bwd_scratch(rt.IXB_BF16, *[q.data_ptr()] * 5, f.data_ptr(), *[q.data_ptr()] * 3, f.data_ptr(),
                                         scratch.data_ptr() + 8, TILE, 1, 1, 8, 8, 128, *[st] * 8, 1.0, 0, None,
                                         rt.raw_stream(q.device)) == rt.IXB_ERR_ALIGN
+
+
+def test_what_is_not_to_be_had_is_asked_for_once(monkeypatch):
+    """The device has room for less than was asked for: every size is tried once, the next calls begin
+    with the one that was to be had, and the whole is asked for again after a while."""
+    device = torch.device("cpu", 0)
+    per_head = _tiles(1000, 1000, 1) * TILE
+    asked, room = [], 3 * per_head + 8 * 4 * 1000
+
+    def empty(size, **kw):
+        asked.append(size)
+        if size > room:
+            raise torch.cuda.OutOfMemoryError("no")
+        return size
+
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    monkeypatch.setattr(ops, "_score_gradient_limits", {})
+    monkeypatch.setattr(ops, "SCORE_GRADIENT_RETRY", 3)
+    get = lambda **kw: ops._backward_scratch(1, 8, 1000, 1000, True, device, ops._score_gradient_limit(0), **kw)[1] // per_head
+    assert get() == 2 and [a // per_head for a in asked] == [8, 4, 2]
+    asked.clear()
+    assert [get() for _ in range(3)] == [2, 2, 2] and [a // per_head for a in asked] == [2, 2, 2]
+    asked.clear()
+    assert get(refused=True) == 2 and [a // per_head for a in asked] == [4, 2]     # (the native entry asked for all)
+    room = 0
+    with pytest.raises(torch.cuda.OutOfMemoryError):       # not even delta
+        get()
+    assert ops._score_gradient_limit(1) == ops.SCORE_GRADIENT_BYTES                # another device
+
+
+@pytest.mark.gpu
+def test_backward_on_a_full_device(cuda, monkeypatch):
+    """The allocator may not grow by what dS takes, and refuses it once: the same gradients, in launches of
+    fewer heads."""
+    g = torch.Generator(device=cuda).manual_seed(2)
+    q, k, v, dy = (torch.randn(1, 32, 2048, 128, generator=g, device=cuda).bfloat16() for _ in range(4))
+    out, lse = ops.fused_attention(q, k, v, 0.1, causal=True, return_lse=True)
+    want = ops.fused_attention_backward(q, k, v, out, lse, dy, 0.1, causal=True)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    monkeypatch.setattr(ops, "_score_gradient_limits", {}, raising=False)
+    whole = rt.load().ixb_fa_bwd_scratch_bytes(1, 32, 2048, 2048, 1, 1 << 40)
+    total = torch.cuda.get_device_properties(0).total_memory
+    refusals = lambda: torch.cuda.memory_stats()["num_ooms"]
+    before = refusals()
+    # room for the three gradients and two thirds of dS
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 3 * q.numel() * 2 + whole * 2 // 3 + (8 << 20)) / total)
+    try:
+        for calls in (1, 2):
+            got = ops.fused_attention_backward(q, k, v, out, lse, dy, 0.1, causal=True)
+            assert refusals() == before + 1
+            assert all(torch.equal(a, e) for a, e in zip(got, want))
+            del got
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert ops._score_gradient_limits[0][0] == whole // 2
