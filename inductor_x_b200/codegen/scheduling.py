@@ -158,9 +158,40 @@ class ColumnGroup:
         narrowest = split_tiling.narrowest_dtype(floats)
         if split_tiling.walked_in_chunks(self.cols, narrowest):
             return False          # a thread's sums are those of one chunk
+        shape = split_tiling.choose_row_config(self.cols, narrowest, rows=self.rows)
         # whole warps to a row, and at most 64 registers of sums in the default launch shape
-        cfg = split_tiling.choose_row_config(self.cols, narrowest, rows=self.rows)
-        return cfg is not None and cfg.team >= 32 and cfg.vec % 4 == 0 and cfg.elems_per_thread * len(self.sums) <= 64
+        return shape is not None and shape.team >= 32 and shape.vec % 4 == 0 and \
+            shape.elems_per_thread * len(self.sums) <= 64 and self._pays(shape, narrowest)
+
+    def _pays(self, shape, dtype) -> bool:
+        """One kernel is quicker than two.  A kernel of its own reads the matrices a second time, and is
+        slow where it is two sums (two passes) or where the last 32 vectors of a row are not whole (they
+        are read one load at a time, and the rest waits for them).  Beside the row the sums take registers,
+        of which a thread of a 1024-thread team has 64, and where there are few rows to a block its partial
+        sums are as much as what they spare.  Backward of a norm, two kernels / one, us:
+          one sum, whole vectors, 1024 threads: bf16 448 x 16384 17.6 / 22.9, 4096 x 16384 109 / 125,
+            1024 x 24576 66 / 78, 1024 x 32768 103 / 156; fp32 700 x 16384 57.9 / 57.0, 4096 x 16384 293 / 269,
+            1024 x 24576 159 / 205.  Fewer threads: bf16 1024 x 12288 23.4 / 18.7, 400 x 8192 10.7 / 8.5,
+            256 x 12288 9.6 / 10.6
+          one sum, ragged: bf16 220 x 16000 21.3 / 16.6, 200 x 16383 31.7 / 27.7, 1024 x 24571 173 / 101,
+            512 x 32767 178 / 162, 150 x 32767 64 / 73, 300 x 50257 146 / 200, 512 x 65535 528 / 540
+          two sums: bf16 400 x 16384 62 / 41, 256 x 16384 28 / 34, 1024 x 32768 339 / 323, 512 x 32767 197 / 226;
+            fp32 1024 x 20000 251 / 198, 512 x 16383 129 / 156
+        (512 x 32767 and 512 x 16383 fill their team, so the words of their rows are shifted one by one.)
+        With equal thresholds the kernel of its own counts as slow everywhere."""
+        full = False
+        if self.cols % shape.vec:
+            shifted = split_tiling.covering_config(self.cols, dtype, shape, 0, rows=self.rows)
+            full, shape = shifted is None, shifted or shape
+        quick = len(self.sums) == 1 and self.cols % (32 * shape.vec) == 0 and \
+            config.column_sum_elements > config.column_sum_elements_odd
+        few = self.rows < 400
+        if shape.team < split_tiling.MAX_TEAM:
+            return not (quick and few)
+        elems = shape.elems_per_thread
+        if quick:
+            return not few and shape.vec == 4 and elems <= 16
+        return elems <= 32 and not (few and elems * len(self.sums) > 16) and not (full and len(self.sums) > 1)
 
     def is_touched_by(self, group) -> bool:
         """A group between the two wants the sums, or writes what they are made of."""

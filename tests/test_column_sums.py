@@ -92,6 +92,39 @@ def test_rows_walked_in_chunks_leave_the_sums_to_a_kernel_of_their_own(dry_backe
     assert not re.search(r"kColumns = [1-9]", code) and "ixb_partials" not in code
 
 
+@pytest.mark.parametrize("dtype,rows,cols,sums,pays", [
+    # one sum over whole vectors beside a team of 1024 threads
+    (torch.bfloat16, 4096, 16384, 1, False), (torch.bfloat16, 1024, 24576, 1, False), (torch.float32, 4096, 16384, 1, True),
+    (torch.float32, 1024, 24576, 1, False), (torch.float32, 256, 16384, 1, False), (torch.float32, 400, 8192, 1, True),
+    # beside fewer threads
+    (torch.bfloat16, 1024, 12288, 1, True), (torch.bfloat16, 400, 8192, 1, True), (torch.bfloat16, 256, 12288, 1, False),
+    # rows of other lengths
+    (torch.bfloat16, 220, 16000, 1, True), (torch.bfloat16, 200, 16383, 1, True), (torch.bfloat16, 1024, 24571, 1, True),
+    (torch.bfloat16, 512, 32767, 1, True), (torch.bfloat16, 150, 32767, 1, False), (torch.bfloat16, 300, 50257, 1, False),
+    (torch.bfloat16, 512, 65535, 1, False), (torch.bfloat16, 512, 65529, 1, False),
+    # two sums
+    (torch.bfloat16, 400, 16384, 2, True), (torch.bfloat16, 256, 16384, 2, False), (torch.bfloat16, 1024, 32768, 2, True),
+    (torch.bfloat16, 512, 32767, 2, False), (torch.float32, 1024, 20000, 2, True), (torch.float32, 512, 16383, 2, False)])
+def test_where_one_kernel_is_quicker(dtype, rows, cols, sums, pays):
+    from inductor_x_b200.codegen import scheduling, split_tiling
+
+    group = scheduling.ColumnGroup([], [], [], set(), rows, cols)
+    group.sums = [None] * sums
+    shape = split_tiling.choose_row_config(cols, dtype, rows=rows)
+    assert group._pays(shape, dtype) == pays
+    # whatever pays leaves a thread of the shape in use no more sums than it has registers
+    used = shape if cols % shape.vec == 0 else split_tiling.covering_config(cols, dtype, shape, 0, rows=rows) or shape
+    assert not pays or used.elems_per_thread * sums <= 65536 // (used.team * used.teams)
+
+
+@needs_nvcc
+@pytest.mark.parametrize("dtype,rows,cols", [(torch.bfloat16, 300, 65535), (torch.bfloat16, 1024, 16384), (torch.float32, 300, 32768)])
+def test_long_rows_keep_their_registers(dry_backend, dtype, rows, cols):
+    x, dy = (torch.empty(rows, cols, dtype=dtype) for _ in range(2))
+    code = _code(_dx_dw, x, torch.empty(cols, dtype=dtype), dy, torch.empty(rows, 1))
+    assert not re.search(r"kColumns = [1-9]", code) and "ixb_partials" not in code
+
+
 TOL = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
 
 
