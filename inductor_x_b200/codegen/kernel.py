@@ -54,8 +54,9 @@ INT_REDUCTION_OPS = {"sum": "ISum", "prod": "IProd", "max": "IMax", "min": "IMin
 MAX_CONSTS = 6
 #: streamed operands fetched one row ahead as raw 128-bit vectors
 MAX_STAGED = 2
-#: rows of partial sums that a column sum beside a row kernel may have (kMaxPartials in gen.cuh)
-MAX_PARTIALS = 592
+#: rows of partial sums of a column sum beside a row kernel at most: one for each of its blocks, four blocks
+#: an SM
+MAX_PARTIALS = 4 * ixb_config.num_sms
 
 
 class UnsupportedByTemplates(NotImplementedError):
@@ -163,6 +164,11 @@ class B200Kernel(SIMDKernel):
 
     def create_cse_var(self, *args, **kwargs):
         return B200CSEVariable(*args, **kwargs)
+
+    def _partials(self) -> int:
+        """Rows of partial sums the blocks may need: there are no more blocks than rows, but as many for
+        each offset from a boundary (kShiftPeriod, 8 at most)."""
+        return min(MAX_PARTIALS, -(-self._static_numel("x") // 8) * 8)
 
     def _row_shift(self, tiling):
         """(pitch, first element, period) when every access of the group that walks a row of its own
@@ -1371,6 +1377,7 @@ class B200Kernel(SIMDKernel):
                         src.writeline(f"{G}vf<kN> k{new};")
                 src.writeline("};")
                 src.writeline(f"static constexpr int kColumns = {len(self.columns)};   // sums over the rows")
+                src.writeline(f"static constexpr int kPartials = {self._partials() if self.columns else 0};   // blocks at most, with sums")
                 src.writeline("struct Cols {")
                 with src.indent():
                     for n in range(len(self.columns)):
@@ -1383,12 +1390,12 @@ class B200Kernel(SIMDKernel):
                         src.writeline(f"for (int e = 0; e < kN; ++e) cols.a{n}.v[e] = 0.f;")
                 src.writeline("}")
                 if self.columns:
-                    src.writeline("float* partial;   // [kColumns][kMaxPartials][columns]")
+                    src.writeline("float* partial;   // [kColumns][kPartials][columns]")
                     src.writeline("template <class Ctx>")
                     src.writeline("__device__ __forceinline__ void flush(const Ctx& c, const Cols& cols, float4* tab) const {")
                     with src.indent():
                         for n in range(len(self.columns)):
-                            src.writeline(f"c.flush_column(cols.a{n}, tab, partial + ({n}LL * {G}kMaxPartials + blockIdx.x) * "
+                            src.writeline(f"c.flush_column(cols.a{n}, tab, partial + ({n}LL * kPartials + blockIdx.x) * "
                                           f"{G}partial_pitch({self._static_numel('r0_')}));")
                     src.writeline("}")
                 src.writeline("struct Raw {")
@@ -1552,7 +1559,7 @@ class B200Kernel(SIMDKernel):
                     src.writeline("long long blocks = 0;")
                     src.writeline(f"int rc = {launch}, &blocks);")
                     for n, (ptr, ctype) in enumerate(self.columns):
-                        src.writeline(f"if (rc == 0) rc = {G}finish_columns<{ctype}>(b.partial + {n}LL * {G}kMaxPartials * "
+                        src.writeline(f"if (rc == 0) rc = {G}finish_columns<{ctype}>(b.partial + {n}LL * Body::kPartials * "
                                       f"{G}partial_pitch(kCols), blocks, kCols, b.{ptr}, stream);")
                     src.writeline("return rc;")
             else:
@@ -1597,7 +1604,7 @@ class B200Kernel(SIMDKernel):
             # the blocks' partial sums, behind the tensors of the group
             pitch = -(-self._static_numel("r0_") // 4) * 4
             ws = f"ixb_partials_{wrapper.next_kernel_suffix()}"
-            wrapper.writeline(f"{ws} = empty_strided_{device.type}(({len(self.columns) * MAX_PARTIALS * pitch},), (1,), torch.float32)")
+            wrapper.writeline(f"{ws} = empty_strided_{device.type}(({len(self.columns) * self._partials() * pitch},), (1,), torch.float32)")
             call_args.append(ws)
         if device.type == "cuda":
             stream = wrapper.write_get_raw_stream(device.index, V.graph.name)

@@ -1498,7 +1498,6 @@ template <class K> inline int row_resident(K kern, int threads, size_t smem = 0)
 // row of partial sums, and finish_columns adds those.  A kernel of its own reads both operands a second
 // time: 32768 x 4096 bf16, gradient of the input 121 us and of the weight 88,
 // both together 123.
-constexpr int kMaxPartials = 592;   // rows of partial sums of one column sum: blocks of the row kernel at most
 __host__ __device__ constexpr long long partial_pitch(long long cols) { return (cols + 3) / 4 * 4; }
 // 32 columns a block, a warp for every 32nd partial row: there are few of them to go round (eight warps
 // a block took 4 us longer on 1024 columns)
@@ -1653,7 +1652,7 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
     const int resident = row_resident(kern, TEAM * TEAMS, smem);
     if (resident < 1) return (int)cudaErrorInvalidConfiguration;
     long long grid = (long long)sms * resident;
-    if (Body::kColumns > 0 && grid > kMaxPartials) grid = kMaxPartials;
+    if (Body::kColumns > 0 && grid > Body::kPartials) grid = Body::kPartials;
     if constexpr (kPeriod > 0) {      // as many blocks for each offset
       const long long most = grid < kPeriod ? kPeriod : grid / kPeriod * kPeriod;
       grid = (groups + kPeriod - 1) / kPeriod * kPeriod;
@@ -1668,7 +1667,7 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   const int resident = row_resident(kern, TEAM * TEAMS, smem);
   if (resident < 1) return (int)cudaErrorInvalidConfiguration;
   long long grid = (long long)sms * resident;
-  if (Body::kColumns > 0 && grid > kMaxPartials) grid = kMaxPartials;
+  if (Body::kColumns > 0 && grid > Body::kPartials) grid = Body::kPartials;
   if (grid > groups) grid = groups;
   if (blocks != nullptr) *blocks = grid;
   return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);

@@ -125,6 +125,18 @@ def test_long_rows_keep_their_registers(dry_backend, dtype, rows, cols):
     assert not re.search(r"kColumns = [1-9]", code) and "ixb_partials" not in code
 
 
+@needs_nvcc
+@pytest.mark.parametrize("rows,partials", [(413, 416), (4096, 592)])
+def test_partial_sums_are_as_many_as_blocks(dry_backend, rows, partials):
+    """No more rows of partial sums than there are blocks: one for each row, rounded up to whole periods of
+    the offsets from a boundary, or four an SM."""
+    cols = 8003
+    x, dy = (torch.empty(rows, cols, dtype=torch.bfloat16) for _ in range(2))
+    code = _code(_dx_dw, x, torch.empty(cols, dtype=torch.bfloat16), dy, torch.empty(rows, 1))
+    assert "kShiftPeriod = 8;" in code and f"kPartials = {partials};" in code
+    assert re.search(rf"ixb_partials_\d+ = empty_strided_cpu\(\({partials * 8004},\)", code)
+
+
 TOL = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
 
 
@@ -137,7 +149,8 @@ def _close(got, want, dtype):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype,rows,cols", [
     (torch.bfloat16, 2048, 4096), (torch.float32, 1500, 4096), (torch.float16, 5003, 1537), (torch.float32, 1031, 4097),
-    (torch.bfloat16, 1025, 8191), (torch.float16, 20000, 264), (torch.bfloat16, 9000, 520), (torch.float16, 1024, 16384)])
+    (torch.bfloat16, 1025, 8191), (torch.float16, 20000, 264), (torch.bfloat16, 9000, 520), (torch.float16, 1024, 16384),
+    (torch.bfloat16, 131, 8193), (torch.float32, 401, 8192)])
 def test_training_step_of_a_norm(cuda, monkeypatch, dtype, rows, cols):
     """Rows that are no whole number of blocks, several teams a block, odd rows (whose blocks keep to one
     offset), one team of many warps; against 64 bits.  The sum's bound: fp32 partial sums of `rows` terms,
