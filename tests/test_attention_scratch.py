@@ -142,3 +142,27 @@ def test_backward_on_a_full_device(cuda, monkeypatch):
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert ops._score_gradient_limits[0][0] == whole // 2
+
+
+@pytest.mark.gpu
+def test_scratch_is_not_filled_under_deterministic_algorithms(cuda):
+    """Torch then fills what it allocates: the three gradients, which the call returns, and nothing else; the
+    bits are the same."""
+    from torch.profiler import ProfilerActivity, profile
+
+    g = torch.Generator(device=cuda).manual_seed(4)
+    q, k, v, dy = (torch.randn(1, 4, 512, 128, generator=g, device=cuda).bfloat16() for _ in range(4))
+    out, lse = ops.fused_attention(q, k, v, 0.1, causal=True, return_lse=True)
+    want = ops.fused_attention_backward(q, k, v, out, lse, dy, 0.1, causal=True)
+    was = torch.are_deterministic_algorithms_enabled()
+    torch.use_deterministic_algorithms(True)
+    try:
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            got = ops.fused_attention_backward(q, k, v, out, lse, dy, 0.1, causal=True)
+            torch.cuda.synchronize()
+    finally:
+        torch.use_deterministic_algorithms(was)
+    kernels = {e.key: e.count for e in p.key_averages() if e.device_time_total > 0}
+    assert sum(n for name, n in kernels.items() if "fa_bwd" in name) == 3
+    assert sum(n for name, n in kernels.items() if "fa_bwd" not in name) == 3, kernels
+    assert all(torch.equal(a, e) for a, e in zip(got, want))
