@@ -1258,7 +1258,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     float v[1 + NS + NP];
 #pragma unroll
     for (int k = 0; k < 1 + NS + NP; ++k) v[k] = 0.f;
-    const float shift = (m == -INFINITY) ? 0.f : -m * kLog2e;
+    const op::ExpScale ks(m == -INFINITY ? 0.f : m);
     float2 acc[1 + NS][kChains];
 #pragma unroll
     for (int k = 0; k < 1 + NS; ++k)
@@ -1267,7 +1267,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
 #pragma unroll
     for (int p = 0; p < kE / 2; ++p) {
       const float2 x = make_float2(Cast<float>::from(at(val, 2 * p)), Cast<float>::from(at(val, 2 * p + 1)));
-      const float2 t = fma2(x, make_float2(kLog2e, kLog2e), make_float2(shift, shift));
+      const float2 t = fma2(x, make_float2(ks.scale, ks.scale), make_float2(ks.shift, ks.shift));
       float2 ex = make_float2(fast_exp2(t.x), fast_exp2(t.y));
       const bool in0 = inside((2 * p) / Base::kVec, (2 * p) % Base::kVec);
       const bool in1 = inside((2 * p + 1) / Base::kVec, (2 * p + 1) % Base::kVec);
@@ -1414,12 +1414,12 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
         if (inside(i, j)) m = fmaxf(m, Cast<float>::from(at(val, i * Base::kVec + j)));
     if (m == -INFINITY) return;      // nothing but -inf so far
     float s = acc.sum * fast_exp2((acc.max - m) * kLog2e);   // exp2(-inf) == 0 covers the first chunk
-    const float shift = -m * kLog2e;
+    const op::ExpScale ks(m);
 #pragma unroll
     for (int i = 0; i < VPT; ++i)
 #pragma unroll
       for (int j = 0; j < Base::kVec; ++j)
-        if (inside(i, j)) s += fast_exp2(fmaf(Cast<float>::from(at(val, i * Base::kVec + j)), kLog2e, shift));
+        if (inside(i, j)) s += fast_exp2(fmaf(Cast<float>::from(at(val, i * Base::kVec + j)), ks.scale, ks.shift));
     acc.max = m;
     acc.sum = s;
   }

@@ -99,24 +99,34 @@ template <class A> __device__ __forceinline__ typename fres<rank<A>::n>::type ex
     return map1<typename fres<rank<A>::n>::type>([](float x) { return fast_exp2(x * kLog2e); }, a);
   }
 }
+// 2^(a * scale + shift) = exp(a - b) for a row's b.  b * log2 e is past the largest float where |b| is above
+// 2.36e38 (the lowest value of fp32 or bf16 as a mask): there neighbouring floats lie 2e31 apart, so that a - b is
+// 0 or the exponential is 0 or infinite, whatever the scale.
+struct ExpScale {
+  float scale, shift;
+  explicit __device__ __forceinline__ ExpScale(float b) {
+    scale = fabsf(b) > 2e38f ? 1.f : kLog2e;
+    shift = -b * scale;
+  }
+};
 // exp(a - b) where b does not vary along the vector (a row statistic): the subtraction and
 // the pre-scale are one packed fma, 2^(a * log2 e - b * log2 e).  The product b * log2 e
 // is rounded once more than in exp(a - b); the emitter uses this form for groups stored in
 // 16-bit types only.
 template <class A>
 __device__ __forceinline__ typename fres<rank<A>::n>::type exp_sub(const A& a, float b) {
-  const float nb = -b * kLog2e;
+  const ExpScale k(b);
   if constexpr (is_fvec<A>::value) {
     constexpr int N = rank<A>::n;
     vf<N> r;
 #pragma unroll
     for (int p = 0; p < N / 2; ++p) {
-      const float2 t = fma2(pr(a, p), make_float2(kLog2e, kLog2e), make_float2(nb, nb));
+      const float2 t = fma2(pr(a, p), make_float2(k.scale, k.scale), make_float2(k.shift, k.shift));
       set_pr(r, p, make_float2(fast_exp2(t.x), fast_exp2(t.y)));
     }
     return r;
   } else {
-    return map1<typename fres<rank<A>::n>::type>([nb](float x) { return fast_exp2(fmaf(x, kLog2e, nb)); }, a);
+    return map1<typename fres<rank<A>::n>::type>([k](float x) { return fast_exp2(fmaf(x, k.scale, k.shift)); }, a);
   }
 }
 template <class A> __device__ __forceinline__ typename fres<rank<A>::n>::type sigmoid(const A& a) {
