@@ -205,7 +205,9 @@ class GeneratedKernel:
         if rc != 0:
             raise RuntimeError(f"generated kernel failed to launch: cudaError {rc}")
         ms = e0.elapsed_time(e1)
-        gb = sum(a.numel() * a.element_size() for a in args if isinstance(a, torch.Tensor)) / 1e9
+        tensors = [a for a in args if isinstance(a, torch.Tensor)]
+        tensors = tensors[:len(tensors) - self.meta.get("workspaces", 0)]     # (the partial sums of column sums)
+        gb = sum(a.numel() * a.element_size() for a in tensors) / 1e9
         print(f"{self.meta.get('name', self.key)}: {ms:.3f}ms    {gb:.3f}GB    {gb / (ms / 1e3):.2f}GB/s")
 
 

@@ -1574,6 +1574,8 @@ class B200Kernel(SIMDKernel):
         meta = f"family={self.mapping!r}"
         if self.checked_indices:
             meta += ", bounds=True"
+        if self.columns:
+            meta += ", workspaces=1"       # the last tensor of a call: not the group's own
         if self.mapping == "row" and not self._is_dynamic("r0_") and not self.looped:
             cfg = self._row_cfg
             inplace = bool(self.args.inplace_buffers)

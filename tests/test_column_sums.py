@@ -246,3 +246,21 @@ def test_sums_whose_operand_is_overwritten(cuda):
     assert float((s.double() - es)[keep].abs().max() / es[keep].abs().max()) <= 1e-4
     live = torch.arange(rows, device=cuda) != 7
     assert float((d.double() - ed)[live].abs().max() / ed[live].abs().max()) <= 1e-4
+
+
+@pytest.mark.gpu
+def test_bandwidth_print_counts_the_operands(cuda, capsys, monkeypatch):
+    """config.profile_bandwidth: three matrices and three vectors, without the workspace of partial sums."""
+    import inductor_x_b200  # noqa: F401
+
+    rows = cols = 4096
+    x, dy = (torch.randn(rows, cols, device=cuda).bfloat16() for _ in range(2))
+    w, rstd = torch.randn(cols, device=cuda).bfloat16(), torch.rand(rows, 1, device=cuda)
+    torch._dynamo.reset()
+    fn = torch.compile(_dx_dw, dynamic=False)
+    fn(x, w, dy, rstd)
+    capsys.readouterr()
+    monkeypatch.setattr(config, "profile_bandwidth", True)
+    fn(x, w, dy, rstd)
+    lines = re.findall(r"ms\s+([\d.]+)GB", capsys.readouterr().out)
+    assert len(lines) == 1 and abs(float(lines[0]) - (3 * 2 * rows * cols + 2 * cols + 4 * rows + 4 * cols) / 1e9) <= 1e-3
