@@ -83,6 +83,10 @@ class ColumnGroup:
         cols, rows = (_static(v) for v in sums[0].group[1])
         if cols is None or rows is None or rows < 128:
             return None
+        # slow on its own, or few rows to a block of its own (see config; fp32 rows of four over a multiple of
+        # eight belong here as well: 2000 x 2044 17.2 us in two kernels, 12.9 in one, 1500 x 3004 21.0 and 11.8.
+        # bf16 of 4096 columns and less gains nothing below the other threshold, 512 x 6144 10.0 / 8.8,
+        # 800 x 6144 13.0 / 10.6)
         odd = cols % 8 != 0 or cols >= 6144
         if rows * cols < (config.column_sum_elements_odd if odd else config.column_sum_elements):
             return None
@@ -255,7 +259,9 @@ class B200Scheduling(SIMDScheduling):
     # the two groups come close enough after each other the sums are emitted inside the row kernel
     # (gen.cuh, finish_columns), in its turn: the one that comes first waits for the other, or the
     # other is found done.  32768 x 4096 bf16: 121 + 88 us in two kernels, 123 + 4 in one.
-    COLUMN_SUM_WINDOW = 8     # groups between the two at most
+    # How many groups after the first the second may come.  In the backward of encoder and decoder layers it
+    # is the next one; the bound keeps the search short in graphs of thousands.
+    COLUMN_SUM_WINDOW = 8
 
     def codegen_node(self, node):
         if self._done.pop(id(node), None) is not None:
@@ -263,7 +269,7 @@ class B200Scheduling(SIMDScheduling):
         # (combo kernels are emitted past this function)
         if config.merged_column_sums and not inductor_config.combo_kernels and id(node) not in self._put_off:
             sums = ColumnGroup.of(node)
-            partner = self._partner(node, lambda later: sums.fits(later), lambda between: sums) if sums else None
+            partner = self._partner(node, sums.fits, sums) if sums else None
             if partner is not None:
                 self._put_off[id(partner)] = sums
                 return None
@@ -276,7 +282,7 @@ class B200Scheduling(SIMDScheduling):
                 found["sums"] = group
                 return True
 
-            later = self._partner(node, goes_beside, None) if node.is_reduction() else None
+            later = self._partner(node, goes_beside) if node.is_reduction() else None
             if later is not None and not any(found["sums"].is_touched_by(n) for n in self._between(node, later)):
                 self._done[id(later)] = later
                 self._put_off[id(node)] = found["sums"]
@@ -299,7 +305,7 @@ class B200Scheduling(SIMDScheduling):
         to = next(i for i, n in enumerate(order) if n is later)
         return order[at + 1:to]
 
-    def _partner(self, node, wanted, sums):
+    def _partner(self, node, wanted, sums=None):
         """The first group after ``node``, within the window, that is ``wanted`` and is in no pair yet;
         with ``sums`` the search ends at a group that they must not wait for."""
         order = self.scheduler.nodes
@@ -312,7 +318,7 @@ class B200Scheduling(SIMDScheduling):
                 return later
             if inductor_config.graph_partition and not (_is_generated(later) and later.get_device() == node.get_device()):
                 return None      # what follows may belong to another partition of the graph
-            if sums is not None and sums(later).is_touched_by(later):
+            if sums is not None and sums.is_touched_by(later):
                 return None
         return None
 

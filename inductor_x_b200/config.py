@@ -31,11 +31,12 @@ merged_welford = os.environ.get("IXB_MERGED_WELFORD", "0") == "1"
 merged_online_softmax = os.environ.get("IXB_MERGED_ONLINE_SOFTMAX", "1") == "1"
 #: emit a sum over the rows of a matrix (the gradient of a norm's weight) inside the row kernel that
 #: reads the same rows, from ``column_sum_elements`` elements on.  Below that the second reading comes
-#: from L2 and costs no more than the partial sums: backward of a norm, one kernel against two, 4096 x 4096
-#: 21.2 / 29.0 us, 8192 x 1024 13.4 / 15.2, 4096 x 2048 13.7 / 15.5, 2048 x 2048 10.7 / 10.0, 1024 x 4096
-#: 9.7 / 10.1.  Columns that are no whole vectors are read element by element by a kernel of their own, and
+#: from L2 and costs no more than the partial sums: backward of a norm in bf16, two kernels / one, 4096 x 4096
+#: 29.0 / 21.2 us, 8192 x 1024 15.2 / 13.4, 4096 x 2048 15.5 / 13.7, 2048 x 2048 10.0 / 10.7, 1024 x 4096
+#: 10.1 / 9.7.  Columns that are no whole vectors are read element by element by a kernel of their own, and
 #: few long rows leave it too few blocks: those are merged from ``column_sum_elements_odd`` on (2000 x 2047
-#: 13.5 / 42.8, 700 x 5003 16.3 / 24.0, 420 x 7872 9.9 / 18.4)
+#: 42.8 / 13.5, 700 x 5003 24.0 / 16.3, 420 x 7872 18.4 / 9.9), where the row kernel has the registers and the rows
+#: for it (``ColumnGroup._pays``)
 merged_column_sums = os.environ.get("IXB_MERGED_COLUMN_SUMS", "1") == "1"
 column_sum_elements = 1 << 23
 column_sum_elements_odd = 3 << 20

@@ -514,7 +514,6 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   using Base = RowCtx<T, TEAM, TEAMS, VPT, false>;
   static constexpr int kE = VPT * Base::kVec;
   static constexpr bool FULL = !SHIFT && COLS == TEAM * VPT * Base::kVec;
-  static constexpr bool kShift = SHIFT;
   // vector i of every thread lies inside the row
   static __device__ __forceinline__ constexpr bool full(int i) {
     return COLS >= (i + 1) * TEAM * Base::kVec && !(SHIFT && i == 0);
