@@ -25,7 +25,8 @@ def test_masked_rows(cuda, dtype, cols):
     x[32, 3] = lim.max
     x[33, cols // 3:] = float("-inf")
     want = x.double().softmax(-1)
-    for fn in (lambda x: x.softmax(-1), lambda x: torch.log_softmax(x, -1).exp(), lambda x: (x - x.amax(-1, keepdim=True)).float().exp()):
+    forms = (lambda x: x.softmax(-1), lambda x: torch.log_softmax(x, -1).exp(), lambda x: (x - x.amax(-1, keepdim=True)).float().exp())
+    for fn in forms if cols == 4096 else forms[:1]:
         torch._dynamo.reset()
         got = torch.compile(fn, dynamic=False)(x).double()
         if fn(torch.zeros(1, 2))[0, 0] == 1:
