@@ -178,10 +178,11 @@ class ColumnGroup:
             1024 x 24576 159 / 205.  Fewer threads: bf16 1024 x 12288 23.4 / 18.7, 400 x 8192 10.7 / 8.5,
             256 x 12288 9.6 / 10.6
           one sum, ragged: bf16 220 x 16000 21.3 / 16.6, 200 x 16383 31.7 / 27.7, 1024 x 24571 173 / 101,
-            512 x 32767 178 / 162, 150 x 32767 64 / 73, 300 x 50257 146 / 200, 512 x 65535 528 / 540
-          two sums: bf16 400 x 16384 62 / 41, 256 x 16384 28 / 34, 1024 x 32768 339 / 323, 512 x 32767 197 / 226;
-            fp32 1024 x 20000 251 / 198, 512 x 16383 129 / 156
-        (512 x 32767 and 512 x 16383 fill their team, so the words of their rows are shifted one by one.)
+            256 x 32767 65 / 85, 512 x 32767 123 / 131, 2048 x 32767 509 / 463, 300 x 50257 146 / 200,
+            512 x 65535 528 / 540; fp32 256 x 16383 40 / 35, 2048 x 16383 283 / 167
+          two sums: bf16 400 x 16384 62 / 41, 256 x 16384 28 / 34, 1024 x 32768 339 / 323, 512 x 32767 162 / 274,
+            2048 x 32767 785 / 873; fp32 1024 x 20000 251 / 198, 1024 x 16383 174 / 147
+        Where the words of a row are shifted one by one (it fills its team) two sums have no registers.
         With equal thresholds the kernel of its own counts as slow everywhere."""
         full = False
         if self.cols % shape.vec:
@@ -195,7 +196,11 @@ class ColumnGroup:
         elems = shape.elems_per_thread
         if quick:
             return not few and shape.vec == 4 and elems <= 16
-        return elems <= 32 and not (few and elems * len(self.sums) > 16) and not (full and len(self.sums) > 1)
+        if few:
+            return not full and elems * len(self.sums) <= 20
+        if full and len(self.sums) > 1:
+            return False
+        return elems <= 32 or (elems <= 40 and len(self.sums) == 1 and self.rows >= 1024)
 
     def is_touched_by(self, group) -> bool:
         """A group between the two wants the sums, or writes what they are made of."""

@@ -100,11 +100,13 @@ def test_rows_walked_in_chunks_leave_the_sums_to_a_kernel_of_their_own(dry_backe
     (torch.bfloat16, 1024, 12288, 1, True), (torch.bfloat16, 400, 8192, 1, True), (torch.bfloat16, 256, 12288, 1, False),
     # rows of other lengths
     (torch.bfloat16, 220, 16000, 1, True), (torch.bfloat16, 200, 16383, 1, True), (torch.bfloat16, 1024, 24571, 1, True),
-    (torch.bfloat16, 512, 32767, 1, True), (torch.bfloat16, 150, 32767, 1, False), (torch.bfloat16, 300, 50257, 1, False),
+    (torch.bfloat16, 512, 32767, 1, False), (torch.bfloat16, 2048, 32767, 1, True), (torch.bfloat16, 150, 32767, 1, False),
+    (torch.float32, 256, 16383, 1, True), (torch.float32, 256, 32767, 1, False), (torch.bfloat16, 300, 50257, 1, False),
     (torch.bfloat16, 512, 65535, 1, False), (torch.bfloat16, 512, 65529, 1, False),
     # two sums
     (torch.bfloat16, 400, 16384, 2, True), (torch.bfloat16, 256, 16384, 2, False), (torch.bfloat16, 1024, 32768, 2, True),
-    (torch.bfloat16, 512, 32767, 2, False), (torch.float32, 1024, 20000, 2, True), (torch.float32, 512, 16383, 2, False)])
+    (torch.bfloat16, 512, 32767, 2, False), (torch.float32, 1024, 20000, 2, True), (torch.float32, 512, 16383, 2, True),
+    (torch.float32, 512, 32767, 2, False), (torch.bfloat16, 2048, 32767, 2, False)])
 def test_where_one_kernel_is_quicker(dtype, rows, cols, sums, pays):
     from inductor_x_b200.codegen import scheduling, split_tiling
 

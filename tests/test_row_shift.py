@@ -65,15 +65,17 @@ def _shape(code):
     (torch.float16, 511, "scan", (32, 2, 0, 0, 0)), (torch.float16, 511, "pitches", (32, 2, 1, 1, 0)),
     # a row of whole warps whose every place is taken, in the next shape
     (torch.float16, 511, "affine", (32, 3, 2, 2, 8)), (torch.float32, 16379, "affine", (1024, 4, 2, 2, 4)),
-    # ... or, where that would be twice as thick as the row, in its own
-    (torch.float32, 16383, "affine", (1024, 4, 2, 2, 0)), (torch.float32, 32767, "affine", (1024, 8, 2, 2, 0)),
-    (torch.bfloat16, 32767, "affine", (1024, 4, 2, 2, 0)), (torch.bfloat16, 65535, "sum", (1024, 8, 0, 0, 0))])
+    (torch.float32, 16383, "affine", (1024, 5, 2, 2, 4)), (torch.bfloat16, 32767, "affine", (1024, 5, 1, 2, 8)),
+    # ... or, where that is more than a thread may hold or its table has no room, in its own
+    (torch.float32, 32767, "affine", (1024, 8, 2, 2, 0)), (torch.bfloat16, 65535, "sum", (1024, 8, 0, 0, 0)),
+    (torch.bfloat16, 32767, "three", (1024, 4, 2, 3, 0))])
 def test_shape_of_odd_rows(dry_backend, dtype, cols, kind, shape):
     x = torch.empty(40, cols + 9).to(dtype)[:, :cols] if kind == "pitches" else torch.empty(40, cols).to(dtype)
     w, b = (torch.empty(cols).to(dtype) for _ in range(2))
     fn, args = {"sum": (lambda x: x.float().sum(-1), (x,)), "scan": (lambda x: x.cumsum(-1), (x,)),
                 "pitches": (lambda x, w: (x * w).softmax(-1), (x, w)),
-                "affine": (lambda x, w, b: F.layer_norm(x, (cols,), w, b), (x, w, b))}[kind]
+                "affine": (lambda x, w, b: F.layer_norm(x, (cols,), w, b), (x, w, b)),
+                "three": (lambda x, w, b, g: F.layer_norm(x, (cols,), w, b) * g, (x, w, b, w + 1))}[kind]
     assert _shape(_period(fn, *args)[2]) == shape
 
 
