@@ -61,3 +61,27 @@ bool choose_row(int64_t cols, int elsize, int max_vpt, ixb_cfg* cfg);
   IXB_ROW_CASE(BODY, 512, 4, AL_)   \
   IXB_ROW_CASE(BODY, 1024, 4, AL_)  \
   IXB_ROW_CASE(BODY, 1024, 8, AL_)
+
+// The pairs for rows that are worked on in the vectors of memory.  Three vectors a thread beside four:
+// an odd row touches a vector more than its length fills, which takes a length just under a power of two
+// of vectors past it, and half a team idle is what the two and four of the list above would leave.
+#define IXB_ROW_SHIFT_CASE(BODY, TEAM_, VPT_)                                                         \
+  if (cfg.team == (TEAM_) && cfg.vpt == (VPT_))                                                       \
+    return ixb_host::cuda_status(                                                                     \
+        ixb::launch_row_shift<BODY, TEAM_, IXB_ROW_TEAMS(TEAM_), VPT_, IXB_ROW_MIN_CTAS(TEAM_)>(      \
+            p, rows, (int)cols, period, dev->sm_count, cfg.grid, (cudaStream_t)stream));
+#define IXB_ROW_SHIFT_DISPATCH(BODY)                                                                  \
+  IXB_ROW_SHIFT_CASE(BODY, 32, 1)                                                                     \
+  IXB_ROW_SHIFT_CASE(BODY, 32, 2)                                                                     \
+  IXB_ROW_SHIFT_CASE(BODY, 32, 3)                                                                     \
+  IXB_ROW_SHIFT_CASE(BODY, 32, 4)                                                                     \
+  IXB_ROW_SHIFT_CASE(BODY, 64, 3)                                                                     \
+  IXB_ROW_SHIFT_CASE(BODY, 64, 4)                                                                     \
+  IXB_ROW_SHIFT_CASE(BODY, 128, 3)                                                                    \
+  IXB_ROW_SHIFT_CASE(BODY, 128, 4)                                                                    \
+  IXB_ROW_SHIFT_CASE(BODY, 256, 3)                                                                    \
+  IXB_ROW_SHIFT_CASE(BODY, 256, 4)                                                                    \
+  IXB_ROW_SHIFT_CASE(BODY, 512, 3)                                                                    \
+  IXB_ROW_SHIFT_CASE(BODY, 512, 4)                                                                    \
+  IXB_ROW_SHIFT_CASE(BODY, 1024, 3)                                                                   \
+  IXB_ROW_SHIFT_CASE(BODY, 1024, 4)

@@ -165,6 +165,17 @@ template <class U> __device__ __forceinline__ uint4 keep_elements(const uint4& v
   }
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
+// zeros in place of the first n elements of a word
+template <class U> __device__ __forceinline__ uint4 keep_elements_from(const uint4& v, int n) {
+  uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  constexpr int kPerWord = 4 / (int)sizeof(U);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int gone = n - k * kPerWord;
+    w[k] = gone >= kPerWord ? 0u : (kPerWord == 2 && gone == 1 ? w[k] & 0xffff0000u : w[k]);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
 // elements [first, end) of a word
 template <class U> __device__ __forceinline__ void put_elements(U* p, const uint4& v, int first, int end) {
   constexpr int kPer = 16 / (int)sizeof(U);

@@ -61,6 +61,7 @@ template <typename T, int TEAM, int TEAMS, int VPT, bool ALIGNED> struct RowCtx 
       return settle(base, i, words);
     }
   }
+  __device__ __forceinline__ uint4 column(const T* base, int i) const { return load<false>(base, i); }
   // Rows that start off a 16-byte boundary: the two aligned words that cover vector i (only
   // those that hold an element of the row are read) ...
   __device__ __forceinline__ void fetch(const T* base, int i, uint4 (&words)[2]) const {
@@ -212,6 +213,47 @@ template <typename T, int TEAM, int TEAMS, int VPT, bool ALIGNED> struct RowCtx 
   }
 };
 
+// Rows off a 16-byte boundary, worked on in the vectors of memory: vector 0 of lane 0 is the aligned
+// one that holds the row's first element, `off` elements into it, so column vec_col(0) is -off there.
+// What lies before and behind the row reads as zero and is not written.
+template <typename T, int TEAM, int TEAMS, int VPT> struct RowShiftCtx : RowCtx<T, TEAM, TEAMS, VPT, true> {
+  using Base = RowCtx<T, TEAM, TEAMS, VPT, true>;
+  using Base::kVec;
+  int off;
+  __device__ __forceinline__ int vec_col(int i) const { return Base::vec_col(i) - off; }
+  __device__ __forceinline__ bool valid(int i) const { return vec_col(i) < this->cols; }
+  __device__ __forceinline__ bool cut(int i) const { return vec_col(i) < 0 || vec_col(i) + kVec > this->cols; }
+  __device__ __forceinline__ uint4 load(const T* base, int i) const {
+    // (the words at the two ends belong to the neighbouring rows as well, which other blocks may write
+    // in place: no read-only load)
+    return valid(i) ? ldg_word_stream(base + vec_col(i)) : make_uint4(0, 0, 0, 0);
+  }
+  __device__ __forceinline__ uint4 mask(const uint4& v, int i) const {
+    return cut(i) ? keep_elements_from<T>(keep_elements<T>(v, this->cols - vec_col(i)), -vec_col(i)) : v;
+  }
+  // a per-column operand, which starts anywhere
+  __device__ __forceinline__ uint4 column(const T* base, int i) const {
+    if (!valid(i)) return make_uint4(0, 0, 0, 0);
+    float part[kVec];
+    if (cut(i)) {
+#pragma unroll
+      for (int j = 0; j < kVec; ++j)
+        part[j] = (unsigned)(vec_col(i) + j) < (unsigned)this->cols ? Elem<T>::to_f(base[vec_col(i) + j]) : 0.f;
+      return pack<T>(part);
+    }
+    const T* from = base + vec_col(i);
+    const int s = off_boundary(from);
+    const uint4 lo = ldg_shared_word(from - s);
+    return s == 0 ? lo : shift_words<T>(lo, ldg_shared_word(from - s + kVec), s);
+  }
+  __device__ __forceinline__ void store(T* base, int i, const float* vals) const {
+    if (!valid(i)) return;
+    const int c0 = vec_col(i);
+    if (cut(i)) put_elements(base + c0, pack<T>(vals), -c0, this->cols - c0);
+    else stg_stream(base + c0, pack<T>(vals));
+  }
+};
+
 template <class Body, int TEAM, int TEAMS, int VPT, bool ALIGNED, int MIN_CTAS = 1>
 __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     row_kernel(const typename Body::Params p, const long long rows, const int cols) {
@@ -271,6 +313,61 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
         else cur[k][i] = c.load(base, i);
       }
     }
+    const long long rn = r + stride;
+    if (kAhead && rn < rows) fetch(rn);
+    body.row(p, c, r, cur);
+    r = rn;
+  }
+}
+
+// Rows whose length or base moves them off the 16-byte boundaries repeat their offset every `period`
+// rows.  A block keeps to rows of one offset (block b works on rows b % period, + period, ...), so that a
+// word is fetched once and nothing is shifted per row; per-column operands are shifted at start-up.
+// Every row operand has the same offset at a row (the host checks).  Bound: HBM.  RMSNorm against the
+// covering words of row_kernel, which are two loads a vector, shifted per row and requested ahead only
+// where registers allow: see rmsnorm_t.
+template <class Body, int TEAM, int TEAMS, int VPT, int MIN_CTAS>
+__global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
+    row_shift_kernel(const typename Body::Params p, const long long rows, const int cols, const int period) {
+  using T = typename Body::in_t;
+  using Ctx = RowShiftCtx<T, TEAM, TEAMS, VPT>;
+  constexpr int NIN = Body::kRowInputs;
+  __shared__ __align__(16) float exchange[TEAMS * 2 * (TEAM / 32) * 4];
+
+  Ctx c;
+  c.lane = threadIdx.x % TEAM;
+  c.team = threadIdx.x / TEAM;
+  c.cols = cols;
+  c.phase = 0;
+  c.red = exchange + c.team * 2 * (TEAM / 32) * 4;
+  const int cls = (int)(blockIdx.x % (unsigned)period);
+  c.off = off_boundary(Body::row_ptr(p, 0) + cls * (long long)cols);
+
+  pdl_launch_dependents();
+  pdl_wait();
+
+  const long long stride = (long long)(gridDim.x / (unsigned)period) * TEAMS * period;
+  long long r = ((long long)(blockIdx.x / (unsigned)period) * TEAMS + c.team) * period + cls;
+  // (1024 threads have 64 registers each: two operands, or the eight values a vector of 16-bit ones
+  // widens to, leave no room for the next row)
+  constexpr bool kAhead = TEAM < 1024 || (NIN == 1 && sizeof(T) == 4);
+  uint4 nxt[NIN][VPT];
+  auto fetch = [&](long long row) {
+#pragma unroll
+    for (int k = 0; k < NIN; ++k)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) nxt[k][i] = c.load(Body::row_ptr(p, k) + row * (long long)cols, i);
+  };
+  if (kAhead && r < rows) fetch(r);
+  typename Body::template Impl<VPT> body;
+  body.init(p, c, nullptr);
+  while (r < rows) {
+    if (!kAhead) fetch(r);
+    uint4 cur[NIN][VPT];
+#pragma unroll
+    for (int k = 0; k < NIN; ++k)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) cur[k][i] = c.mask(nxt[k][i], i);
     const long long rn = r + stride;
     if (kAhead && rn < rows) fetch(rn);
     body.row(p, c, r, cur);
@@ -438,6 +535,21 @@ cudaError_t launch_row(const typename Body::Params& p, long long rows, int cols,
   if (grid > groups) grid = groups;
   if (grid < 1) return cudaSuccess;
   return launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, stream, p, rows, cols);
+}
+
+// The grid is a whole number of periods: as many blocks of every offset as are resident or needed.
+template <class Body, int TEAM, int TEAMS, int VPT, int MIN_CTAS>
+cudaError_t launch_row_shift(const typename Body::Params& p, long long rows, int cols, int period, int sm_count,
+                             int grid_override, cudaStream_t stream) {
+  auto kern = row_shift_kernel<Body, TEAM, TEAMS, VPT, MIN_CTAS>;
+  static RowLaunchState state;
+  int resident = 0;
+  if (cudaError_t e = row_launch_capacity(state, kern, TEAM * TEAMS, 0, &resident)) return e;
+  const long long groups = ((rows + period - 1) / period + TEAMS - 1) / TEAMS;  // of one offset
+  long long each = (grid_override > 0 ? (long long)grid_override : (long long)sm_count * resident) / period;
+  if (each > groups) each = groups;
+  if (each < 1) each = 1;
+  return launch_pdl(kern, (unsigned)(each * period), TEAM * TEAMS, 0, stream, p, rows, cols, period);
 }
 
 }  // namespace ixb

@@ -354,7 +354,7 @@ template <typename T, bool RESIDUAL> struct RmsNorm {
     __device__ __forceinline__ void init(const Params& p, const Ctx& c, unsigned char*) {
 #pragma unroll
       for (int i = 0; i < VPT; ++i)
-        w_[i] = c.template load<false>(p.w, i);
+        w_[i] = c.column(p.w, i);
     }
     template <class Ctx>
     __device__ __forceinline__ void row(const Params& p, Ctx& c, long long r,
@@ -374,8 +374,7 @@ template <typename T, bool RESIDUAL> struct RmsNorm {
           if (p.h_out != nullptr) c.store(p.h_out + r * (long long)c.cols, i, h[i]);
         }
 #pragma unroll
-        for (int j = 0; j < kVec; ++j)
-          if (c.ok(i, j)) q = fmaf(h[i][j], h[i][j], q);
+        for (int j = 0; j < kVec; ++j) q = fmaf(h[i][j], h[i][j], q);  // (zero outside the row)
       }
       q = c.template reduce<SumOp>(q);
       const float rstd = rsqrtf(q / (float)c.cols + p.eps);
