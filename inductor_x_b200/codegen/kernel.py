@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import contextlib
 import math
+import re
 from typing import Any, Optional
 
 import sympy
@@ -42,6 +43,7 @@ def config_bytes(dtype: torch.dtype) -> int:
     return ixb_config.BYTES_PER_ELEMENT.get(dtype, 8)
 
 G = "ixb::gen::"
+SMALL_EXPR = IxbExprPrinter.small().doprint
 
 REDUCTION_OPS = {
     "sum": "ixb::SumOp", "max": "ixb::MaxOp", "min": "ixb::MinOp", "prod": "ixb::ProdOp",
@@ -51,6 +53,8 @@ REDUCTION_OPS = {
 INT_REDUCTION_OPS = {"sum": "ISum", "prod": "IProd", "max": "IMax", "min": "IMin"}
 
 #: per-column operands hoisted out of the row loop at most (registers + shared memory)
+_LIGHT_OPS = {"to_float", "add", "sub", "mul", "fma", "neg", "abs", "maximum", "minimum", "where", "imod", "idiv", "imod32", "idiv32"}
+_CTYPE_BYTES = {ctype: config_bytes(dtype) for dtype, ctype in CPP_TYPE.items()}
 MAX_CONSTS = 6
 #: streamed operands fetched one row ahead as raw 128-bit vectors
 MAX_STAGED = 2
@@ -129,6 +133,7 @@ class B200Kernel(SIMDKernel):
         self.column_casts: dict = {}  # buffers of column sums -> the buffers of their converted values
         self.column_mode = False     # the node being emitted sums over the rows (see scheduling.py)
         self.checked_indices = 0     # data-dependent indices checked on the device (debug builds)
+        self.indirect = False        # some access goes through a data-dependent index
         self.x_indexing = IndentedBuffer()
         self.r_indexing = IndentedBuffer()
         self.looped = False                      # rows walked in chunks (decided before the range trees exist)
@@ -399,13 +404,20 @@ class B200Kernel(SIMDKernel):
         return rt.symbol() in exp.free_symbols
 
     def _is_indirect(self, index: sympy.Expr) -> bool:
-        return any(str(s).startswith(("tmp", "indirect")) for s in index.free_symbols)
+        found = any(str(s).startswith(("tmp", "indirect")) for s in index.free_symbols)
+        self.indirect |= found
+        return found
 
     def codegen_iteration_ranges_entry(self, entry: IterationRangesEntry) -> None:
         expr = self.rename_indexing(entry.expr)
-        line = f"const auto {entry.name} = {self.sexpr(expr)};"
+        small = not entry.is_reduction and self._small_index() and expr.free_symbols <= {entry.root.symbol()}
+        line = f"const auto {entry.name} = {(SMALL_EXPR if small else self.sexpr)(expr)};"
         # reduced-axis variables live inside the reduction loop of the outer mapping
         (self.r_indexing if entry.is_reduction else self.x_indexing).writeline(line)
+
+    def _small_index(self) -> bool:
+        """Whether the kept index, and what a last tile runs past its end, lies below 2^31."""
+        return not self._is_dynamic("x") and self._numel_hint("x") < 2 ** 31 - 2 ** 20
 
     # ------------------------------------------------------------------ two mappings
     # A reduction group can be laid out in two ways and the choice is only known once the
@@ -1194,7 +1206,7 @@ class B200Kernel(SIMDKernel):
                 lc = self._numel_hint("x") // lb       # the outermost digit: FloorDiv without modulus
                 if self._numel_hint("x") != lb * lc:
                     return None
-            if coef_c != rnumel or pieces[1][0] < coef_c * lc or lb % 16 or lc % 16:
+            if coef_c != rnumel or pieces[1][0] < coef_c * lc or lb < 2 or lc < 2:
                 return None
             if found is not None and found != (lb, lc):
                 return None
@@ -1418,10 +1430,10 @@ class B200Kernel(SIMDKernel):
                 src.writeline("}")
                 # raw vectors of the streamed operands of one row (requested a row ahead)
                 src.writeline("template <class Ctx>")
-                src.writeline("__device__ __forceinline__ void fetch(Ctx& c, const long long xslot, Raw& raw) const {")
+                src.writeline(f"__device__ __forceinline__ void fetch(Ctx& c, const long long {slot}, Raw& raw) const {{")
                 with src.indent():
                     if self.staged:
-                        src.writeline(slot_line)
+                        src.splice(slot_line)
                         src.writeline("const auto r0_index = c.rindex();")
                         src.splice(x_idx)
                         src.splice(r_idx)
@@ -1429,25 +1441,32 @@ class B200Kernel(SIMDKernel):
                             src.writeline(f"c.fetch_row({ptr}, {member});")
                 src.writeline("}")
                 src.writeline("template <bool STAGED, class Ctx>")
-                src.writeline("__device__ __forceinline__ void row(Ctx& c, const Consts& k, const long long xslot, "
+                slot = "xslot"
+                if tiling is not None and self._small_index():
+                    slot = "slot"
+                    slot_line = f"const unsigned xslot = (unsigned)slot;\n{slot_line}"
+                src.writeline(f"__device__ __forceinline__ void row(Ctx& c, const Consts& k, const long long {slot}, "
                               "const Raw& raw, Cols& cols) const {")
                 with src.indent():
-                    src.writeline(slot_line)
+                    src.splice(slot_line)
                     if self.looped:
                         src.splice(x_idx)        # the reduced index is defined inside each chunk loop
                     else:
                         src.writeline("const auto r0_index = c.rindex();")
                         src.writeline("const auto rmask = c.rmask();")
                         src.splice(x_idx)
+                stream = tiling is not None or any(raw != "RawRow" for *_, raw in self.staged) or \
+                    any(v["kind"] == "S" and v["has_r"] for v in self._ph.values())
+                src.writeline(f"static constexpr bool kStream = {'true' if stream else 'false'};   // a block for every few rows of sub-warp teams")
                         src.splice(r_idx)
                     src.splice(row_body)
                 src.writeline("}")
                 # L2 prefetch of the streamed operands of a later row
                 src.writeline("template <class Ctx>")
-                src.writeline("__device__ __forceinline__ void prefetch(Ctx& c, const long long xslot) const {")
+                src.writeline(f"__device__ __forceinline__ void prefetch(Ctx& c, const long long {slot}) const {{")
                 with src.indent():
                     if self._row_prefetch:
-                        src.writeline(slot_line)
+                        src.splice(slot_line)
                         src.writeline("const auto r0_index = c.rindex();")
                         src.splice(x_idx)
                         src.splice(r_idx)
@@ -1475,7 +1494,9 @@ class B200Kernel(SIMDKernel):
                     src.writeline("__device__ __forceinline__ long long first_of_tile(long long slot) const {")
                     with src.indent():
                         src.writeline("// lanes: 4 vectors along the flat index by 8 tiles along the loads' axis")
-                        src.writeline("const long long bv_lo = slot % 4; long long t = slot / 4;")
+                        digit = "unsigned" if self._small_index() else "long long"
+                        src.writeline(f"{digit} t = ({digit})slot;")
+                        src.writeline("const long long bv_lo = t % 4; t /= 4;")
                         src.writeline("const long long c_lo = t % 8; t /= 8;")
                         src.writeline(f"const long long bv_hi = t % {nbv // 4}; t /= {nbv // 4};")
                         src.writeline(f"const long long mid = t % {dc // lb}; t /= {dc // lb};")
@@ -1501,7 +1522,9 @@ class B200Kernel(SIMDKernel):
                         nbv = lb // self.vec
                         tbv = next(t for t in (8, 4, 2, 1) if nbv % t == 0)
                         src.writeline("// lanes along the digit the loads are contiguous in, vectors along the flat index")
-                        src.writeline("const long long c_lo = slot % 32; long long t = slot / 32;")
+                        digit = "unsigned" if self._small_index() else "long long"
+                        src.writeline(f"{digit} t = ({digit})slot;")
+                        src.writeline("const long long c_lo = t % 32; t /= 32;")
                         src.writeline(f"const long long bv_lo = t % {tbv}; t /= {tbv};")
                         src.writeline(f"const long long bv_hi = t % {nbv // tbv}; t /= {nbv // tbv};")
                         src.writeline(f"const long long mid = t % {dc // lb}; t /= {dc // lb};")

@@ -52,6 +52,8 @@ def constant_literal(val, dtype: torch.dtype) -> str:
 class IxbExprPrinter(ExprPrinter):
     """Index expressions as C++ over scalars or ``vi<N>`` (operators + ixb::gen::op calls)."""
 
+    bits = ""    # "32" where every index is known to lie below 2^31
+
     def _print_Integer(self, expr):
         return f"{int(expr)}LL"
 
@@ -60,14 +62,14 @@ class IxbExprPrinter(ExprPrinter):
 
     def _print_FloorDiv(self, expr):
         x, d = expr.args
-        return f"{OP}idiv({self.doprint(x)}, {self.doprint(d)})"
+        return f"{OP}idiv{self.bits}({self.doprint(x)}, {self.doprint(d)})"
 
     def _print_ModularIndexing(self, expr):
         x, d, m = expr.args
         xs = self.doprint(x)
         if d != 1:
-            xs = f"{OP}idiv({xs}, {self.doprint(d)})"
-        return f"{OP}imod({xs}, {self.doprint(m)})"
+            xs = f"{OP}idiv{self.bits}({xs}, {self.doprint(d)})"
+        return f"{OP}imod{self.bits}({xs}, {self.doprint(m)})"
 
     def _print_Min(self, expr):
         out = self.doprint(expr.args[0])
@@ -111,6 +113,13 @@ class IxbExprPrinter(ExprPrinter):
 
     def _print_Identity(self, expr):
         return self.doprint(expr.args[0])
+
+    @classmethod
+    def small(cls):
+        """A printer of digits of an index below 2^31."""
+        p = cls()
+        p.bits = "32"
+        return p
 
     # ---- forms that appear with run-time extents (symbolic sizes) -----------------------
     def _fn(self, name, expr):

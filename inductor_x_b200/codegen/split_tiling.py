@@ -83,7 +83,7 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
     that covers it (measured on the softmax->LayerNorm chain at 4096 bf16 columns: 256
     threads x 2 vectors ran 1.2-2x faster than 128 x 4).  Only rows longer than 1024
     threads x ``target_vpt`` vectors take more per thread, and rows of a few vectors get
-    teams of 8 or 16 lanes so that a warp works on several rows at once.  A row of no
+    teams of 2 to 16 lanes so that a warp works on several rows at once.  A row of no
     power-of-two number of vectors is cut to fit: up to ``MAX_EXACT_VPT`` vectors per thread
     over that team, half or a quarter of it, whichever leaves the fewest vectors idle.
     ``exact=False`` leaves that cut out: the extent is only the first one seen of a run-time
@@ -99,6 +99,14 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
         return None
     vpt = target_vpt
     team = MIN_TEAM
+    if exact and nvec < MIN_TEAM and nvec != 5:
+        # rows of a few vectors: no more lanes than hold one (two of six to eight), since the index
+        # arithmetic of a row is every lane's.  Teams of eight and these: sum of the rows of a permuted
+        # 200 x 452 x 221 x 16 fp32 580 and 217 us, of 2^22 x 16 fp16 87 and 29, softmax of
+        # 300000 x 16 fp32 13.6 and 7.6, maximum of 2^20 x 48 bf16 25.5 and 19.6; five vectors on
+        # four lanes of two 4.7, on eight lanes 3.5 (50000 x 40 fp16)
+        team = 4 if nvec > 2 else 2
+        vpt = 1 if nvec <= 4 else 2
     while team < MAX_TEAM and team * vpt < nvec:
         team *= 2
     while team * vpt < nvec:

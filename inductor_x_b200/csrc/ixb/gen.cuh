@@ -1460,17 +1460,31 @@ __device__ __forceinline__ vf<E> kget(const Ctx& c, const vf<E>& reg) {
 // B_FIRST: inside a tile the output digit runs fastest, so the rows a warp works on at once
 // store one contiguous run (a full 32-byte sector for sixteen 16-bit results); chosen when a
 // row is at least one 128-byte line, i.e. when reading rows that are far apart wastes nothing.
-template <int LB, int LC, int TB, int TC, bool B_FIRST = false>
-__device__ __forceinline__ long long tile_order(long long slot) {
-  static_assert(LB % TB == 0 && LC % TC == 0, "tiles must divide both extents");
-  constexpr long long kPlane = (long long)LB * LC;
-  const long long a = slot / kPlane;
-  const int rem = (int)(slot % kPlane);
-  const int c_lo = B_FIRST ? (rem / TB) % TC : rem % TC;
-  const int b_lo = B_FIRST ? rem % TB : (rem / TC) % TB;
-  const int b_hi = (rem / (TC * TB)) % (LB / TB);
-  const int c_hi = rem / (TC * LB);
-  return a * kPlane + (long long)(c_hi * TC + c_lo) * LB + (b_hi * TB + b_lo);
+// At the ends of the digits the tiles are smaller (a stripe of TC or what is left LC digits is walked tile
+// after tile, the last of them narrower); the divisors are constants in each of the four kinds.
+template <int LB, int TB, int TC, int B, int C, bool B_FIRST>  // a tile of B x C, the first LC digit of its stripe
+__device__ __forceinline__ unsigned in_tile(unsigned b_hi, unsigned in, unsigned c0) {
+  const unsigned c_lo = B_FIRST ? in / B : in % C, b_lo = B_FIRST ? in % B : in / C;
+  return (c0 + c_lo) * LB + b_hi * TB + b_lo;
+}
+template <int LB, int TB, int TC, int C, bool B_FIRST>         // a stripe of C digits
+__device__ __forceinline__ unsigned in_stripe(unsigned rem, unsigned c0) {
+  const unsigned b_hi = rem / (C * TB), in = rem - b_hi * (C * TB);
+  if constexpr (LB % TB != 0) {
+    if (b_hi >= LB / TB) return in_tile<LB, TB, TC, LB % TB, C, B_FIRST>(b_hi, in, c0);
+  }
+  return in_tile<LB, TB, TC, TB, C, B_FIRST>(b_hi, in, c0);
+}
+template <int LB, int LC, int TB, int TC, bool B_FIRST = false, class I>
+__device__ __forceinline__ long long tile_order(I slot) {
+  constexpr I kPlane = (I)LB * LC;
+  const I a = slot / kPlane;
+  const unsigned rem = (unsigned)(slot - a * kPlane);
+  const unsigned c_hi = rem / (TC * LB), in = rem - c_hi * (TC * LB);
+  if constexpr (LC % TC != 0) {
+    if (c_hi >= LC / TC) return (long long)(a * kPlane + in_stripe<LB, TB, TC, LC % TC, B_FIRST>(in, c_hi * TC));
+  }
+  return (long long)(a * kPlane + in_stripe<LB, TB, TC, TC, B_FIRST>(in, c_hi * TC));
 }
 
 // CTAs of a row kernel that fit on one SM, cached per device (the attribute is a property of
@@ -1585,7 +1599,9 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     // places instead of 512 bytes - and DRAM pages are used up while they are open (sum over the
     // last axis of a permuted 64 x 128 x 256 x 64 fp16: 54.6 -> 52.4 us).  Rows in memory order
     // gain nothing from it (43.3 against 44.8 us) and keep the strided batches.
-    const bool blocked = Body::kTiled && rows >= stride * kBatch;
+    // Without per-column operands a block is started for every batch (launch_row_gen): the batches in
+    // flight then follow each other through memory, and so do the rows of a batch.
+    const bool blocked = kStreamRows<Body, TEAM, STAGED> ? rows > stride * (kBatch - 1) : Body::kTiled && rows >= stride * kBatch;
     const long long ustep = blocked ? TEAMS : stride;
     for (long long base = (long long)blockIdx.x * TEAMS * (blocked ? kBatch : 1); base < rows; base += stride * kBatch) {
       if constexpr (STAGED) {
@@ -1634,6 +1650,11 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   if (COLS > 0 && cols != COLS) return (int)cudaErrorInvalidValue;
   // a row longer than the team can hold (a run-time extent beyond the compiled capacity);
   // looped bodies walk any length in chunks
+// Sub-warp teams whose threads load nothing once for all rows get a block for every batch of four rows a
+// team (see stream_grid) where there are more than the resident blocks would see in three batches: the
+// permuted sum of 64 x 128 x 256 x 64 fp16 48.9 -> 45.4 us.
+template <class Body, int TEAM, bool STAGED> constexpr bool kStreamRows = TEAM < 32 && STAGED && Body::kStream && Body::kConsts == 0;
+
   if (cols < 0 || (!Body::kLooped && cols > TEAM * VPT * Elem<T>::kVec)) return (int)cudaErrorInvalidValue;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -1761,6 +1782,7 @@ template <int V, int TX, int TY> struct OuterCtx {
       if (ty % kRowsPerWarp == 0) {
 #pragma unroll
         for (int i = 0; i < V; ++i) part[(warp * TX + tx) * V + i] = r.v[i];
+    if (kStreamRows<Body, TEAM, true> && groups > 3 * (long long)sms * resident) grid = (groups + 3) / 4;
       }
       __syncthreads();
       // only the thread row that stores the tile needs the folded vector (a generated outer
