@@ -1117,6 +1117,14 @@ class B200Kernel(SIMDKernel):
             cs *= 2
         return (tx, cs) if cs > 1 else (self._outer_tx(), 1)
 
+    def _outer_warp(self, tx: int) -> bool:
+        """A warp to a tile instead of a CTA: where the reduced axis has fewer steps than eight for each of
+        the CTA's thread rows, and the tiles are enough for a dozen warps an SM."""
+        if self._is_dynamic("r0_") or self._is_dynamic("x"):
+            return False
+        tiles = self._numel_hint("x") // (tx * self._outer_vec)
+        return self._static_numel("r0_") * tx < 1024 and tiles >= 12 * ixb_config.num_sms
+
     def _transposing_order(self):
         """Constants of the lane order for a pointwise kernel whose stores are contiguous along
         the flat index but whose strided loads are contiguous along another digit C of it (a
@@ -1317,36 +1325,50 @@ class B200Kernel(SIMDKernel):
                         src.writeline("if constexpr (FAST) {")
                         with src.indent():
                             src.writeline("long long rb = c.rbegin();")
-                            src.writeline(f"for (; rb + 7 * c.rstep() < {rnumel}; rb += 8 * c.rstep()) {{")
-                            with src.indent():
+
+                            def batch(n, guarded):
+                                """n reduced steps: their loads, then their arithmetic; `guarded` ones may be
+                                past the end, read the last step instead and are left out of the result"""
+                                step = "rb + u * c.rstep()"
+                                index = f"{step} < {rnumel} ? {step} : {rnumel} - 1" if guarded else step
                                 for name, ctype, _ in loads:
-                                    src.writeline(f"{G}RawVec<{ctype}, kVec> raw_{name}[8];")
+                                    src.writeline(f"{G}RawVec<{ctype}, kVec> raw_{name}[{n}];")
                                 src.writeline("#pragma unroll")
-                                src.writeline("for (int u = 0; u < 8; ++u) {")
+                                src.writeline(f"for (int u = 0; u < {n}; ++u) {{")
                                 with src.indent():
-                                    src.writeline("const long long r0_index = rb + u * c.rstep();")
+                                    src.writeline(f"const long long r0_index = {step};")
+                                    if guarded:
+                                        src.writeline(f"if (r0_index >= {rnumel}) break;")
                                     src.splice(r_idx)
                                     for name, ctype, ptr in loads:
                                         src.writeline(f"raw_{name}[u] = {G}ldraw<{ctype}, kVec>({ptr});")
                                 src.writeline("}")
                                 src.writeline("#pragma unroll")
-                                src.writeline("for (int u = 0; u < 8; ++u) {")
+                                src.writeline(f"for (int u = 0; u < {n}; ++u) {{")
                                 with src.indent():
                                     for name, _, _ in loads:
                                         src.writeline(f"{G}pin(raw_{name}[u]);")
                                 src.writeline("}")
                                 src.writeline("#pragma unroll")
-                                src.writeline("for (int u = 0; u < 8; ++u) {")
+                                src.writeline(f"for (int u = 0; u < {n}; ++u) {{")
                                 with src.indent():
-                                    src.writeline("const long long r0_index = rb + u * c.rstep();")
+                                    src.writeline(f"const long long r0_index = {index};")
                                     src.splice(r_idx)
-                                    for name, ctype, _ in loads:
+                                    for name, ctype, ptr in loads:
                                         src.writeline(f"const auto {name} = {G}widen_raw(raw_{name}[u]);")
                                     src.splice("\n".join(rest))
                                     src.writeline(acc_line)
                                 src.writeline("}")
                             src.writeline("}")
-                            plain_loop("rb")
+                            # What is left.  A warp's tile may be nothing else: four steps at a time, since a
+                            # loop that tests the end at each of them waits for every load by itself.
+                            if self._outer_warp(self._outer_tx()):
+                                src.writeline(f"for (; rb < {rnumel}; rb += 4 * c.rstep()) {{")
+                                with src.indent():
+                                    batch(4, True)
+                                src.writeline("}")
+                            else:
+                                plain_loop("rb")
                         src.writeline("} else {")
                         with src.indent():
                             plain_loop("c.rbegin()")
@@ -1395,6 +1417,10 @@ class B200Kernel(SIMDKernel):
                     for n in range(len(self.columns)):
                         src.writeline(f"{G}vf<kN> a{n};")
                 src.writeline("};")
+
+                            src.writeline(f"for (; rb + 7 * c.rstep() < {rnumel}; rb += 8 * c.rstep()) {{")
+                            with src.indent():
+                                batch(8, False)
                 src.writeline("__device__ __forceinline__ void clear(Cols& cols) const {")
                 with src.indent():
                     for n in range(len(self.columns)):
@@ -1634,6 +1660,8 @@ class B200Kernel(SIMDKernel):
         if device.type == "cuda":
             stream = wrapper.write_get_raw_stream(device.index, V.graph.name)
             wrapper.writeline(f"{name}.run({', '.join(map(str, call_args))}, stream={stream})")
+                if cs == 1 and self._outer_warp(tx):
+                    launch = f"launch_outer_warps_gen<Body, {tx}>"
         else:
             wrapper.writeline(f"{name}.run({', '.join(map(str, call_args))}, stream=None)")
         if self.columns:

@@ -1803,8 +1803,10 @@ template <int V, int TX, int TY> struct OuterCtx {
   }
 };
 
-template <class Body, int TX, int TY, bool ALIGNED>
-__global__ void __launch_bounds__(TX* TY) outer_gen_kernel(const Body body, const long long xnumel) {
+// GROUPS tiles a CTA: more than one where a tile is the work of one warp, whose fold is shuffles alone.
+template <class Body, int TX, int TY, int GROUPS, bool ALIGNED>
+__global__ void __launch_bounds__(TX* TY* GROUPS) outer_gen_kernel(const Body body, const long long xnumel) {
+  static_assert(GROUPS == 1 || TX * TY == 32, "several tiles a CTA: a warp each");
   constexpr int V = Body::kVec;
   __shared__ __align__(16) float part[(TX * TY / 32) * TX * V];
   OuterCtx<V, TX, TY> c;
@@ -1813,10 +1815,10 @@ __global__ void __launch_bounds__(TX* TY) outer_gen_kernel(const Body body, cons
   c.part = part;
   const long long per_cta = (long long)TX * V;
   const long long ntiles = (xnumel + per_cta - 1) / per_cta;
-  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+  for (long long t = (long long)blockIdx.x * GROUPS + threadIdx.x / (TX * TY); t < ntiles; t += (long long)gridDim.x * GROUPS) {
     const long long xbase = t * per_cta + (long long)c.tx * V;
     const long long left = xnumel - xbase;
-    // the choice is uniform per CTA (the fold synchronises the whole CTA)
+    // the choice is uniform per tile (the fold synchronises all that work on it)
     if (ALIGNED && xnumel - t * per_cta >= per_cta) body.template tile<true>(c, xbase, V);
     else body.template tile<false>(c, xbase, left >= V ? V : (left > 0 ? (int)left : 0));
   }
@@ -1907,7 +1909,7 @@ __global__ void __launch_bounds__(TX* TY) outer_split_gen_kernel(const Body body
   __shared__ __align__(8) uint64_t bar;
   OuterSplitCtx<V, TX, TY, CS> c;
   c.tx = threadIdx.x % TX;
-  c.ty = threadIdx.x / TX;
+  c.ty = threadIdx.x / TX % TY;
   c.part = part;
   c.inbox = inbox;
   c.bar = &bar;
@@ -1950,8 +1952,8 @@ template <class Body, int TX = 32>
 int launch_outer_gen(const Body& body, long long xnumel, void* stream, bool aligned = false) {
   if (xnumel <= 0) return 0;
   constexpr int TY = 256 / TX;
-  static const long long cap_a = resident_ctas(outer_gen_kernel<Body, TX, TY, true>, TX * TY);
-  static const long long cap_u = resident_ctas(outer_gen_kernel<Body, TX, TY, false>, TX * TY);
+  static const long long cap_a = resident_ctas(outer_gen_kernel<Body, TX, TY, 1, true>, TX * TY);
+  static const long long cap_u = resident_ctas(outer_gen_kernel<Body, TX, TY, 1, false>, TX * TY);
   const long long per_cta = (long long)TX * Body::kVec;
   long long grid = (xnumel + per_cta - 1) / per_cta;
   // A tile ends with a CTA-wide fold during which the CTA has no loads in flight, so the grid
@@ -1964,10 +1966,25 @@ int launch_outer_gen(const Body& body, long long xnumel, void* stream, bool alig
   }();
   const long long cap = (aligned ? cap_a : cap_u) * waves;
   if (grid > cap) grid = cap;
-  if (aligned) outer_gen_kernel<Body, TX, TY, true><<<(unsigned)grid, TX * TY, 0, (cudaStream_t)stream>>>(body, xnumel);
-  else outer_gen_kernel<Body, TX, TY, false><<<(unsigned)grid, TX * TY, 0, (cudaStream_t)stream>>>(body, xnumel);
+  if (aligned) outer_gen_kernel<Body, TX, TY, 1, true><<<(unsigned)grid, TX * TY, 0, (cudaStream_t)stream>>>(body, xnumel);
+  else outer_gen_kernel<Body, TX, TY, 1, false><<<(unsigned)grid, TX * TY, 0, (cudaStream_t)stream>>>(body, xnumel);
   return (int)cudaGetLastError();
 }
 
 }  // namespace gen
 }  // namespace ixb
+// Short reduced axes: with 256 threads to a tile each would add one or two vectors and then wait for two
+// barriers of the CTA.  A warp a tile has eight times as many steps a thread and folds by shuffles.
+// Bound: HBM.  Maximum over the 26 of 6163 x 26 x 22 x 32 bf16 (memory order): see _outer_warp.
+template <class Body, int TX>
+int launch_outer_warps_gen(const Body& body, long long xnumel, void* stream, bool aligned = false) {
+  if (xnumel <= 0) return 0;
+  constexpr int TY = 32 / TX, GROUPS = 8;
+  const long long tiles = (xnumel + (long long)TX * Body::kVec - 1) / ((long long)TX * Body::kVec);
+  long long grid = (tiles + GROUPS - 1) / GROUPS;
+  if (grid > 0x7fffffffLL) grid = 0x7fffffffLL;
+  if (aligned) outer_gen_kernel<Body, TX, TY, GROUPS, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
+  else outer_gen_kernel<Body, TX, TY, GROUPS, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
+  return (int)cudaGetLastError();
+}
+
