@@ -1158,6 +1158,21 @@ class B200Kernel(SIMDKernel):
             found = (lb, dc, lc)
         return found
 
+    def _moves_bytes(self, body_text: str) -> bool:
+        """Whether a pointwise group is worth a block for every 256 vectors (``stream_grid``): a thread
+        moves 48 bytes or more, whole vectors all of them, and what it computes is next to nothing.  A
+        block that lives for one vector a thread pays its start with what it moves.  Resident grid
+        against a block per 256 vectors: bf16 to fp32 of 8192 x 8192 84 -> 60 us, a * b + c in fp32 127 ->
+        114, a + b in bf16 63.0 -> 57.8, of 2048 x 4096 9.36 -> 8.98; but 32 bytes a thread 43.5 -> 45.0
+        (an inner permute) and 43.3 -> 43.4, silu(a) * b in bf16 28.2 -> 29.3, a rotation with masked loads
+        14.7 -> 15.6."""
+        if f"{G}gather(" in body_text or f"{G}scatter" in body_text or f"{G}atomic" in body_text:
+            return False
+        if not set(re.findall(r"ixb::gen::op::(\w+)", body_text)) <= _LIGHT_OPS:
+            return False
+        moved = re.findall(r"(?:ldvec|stvec)<([\w: ]+), kVec", body_text)
+        return sum(_CTYPE_BYTES.get(t, 0) for t in moved) * self.vec >= 48
+
     def _register_tile(self, order):
         """kC (elements per 128-bit load along C) when every strided load of the group can be
         staged as a register tile under the transposing order ``order``: one storage width, rows
@@ -1336,9 +1351,7 @@ class B200Kernel(SIMDKernel):
                                 src.writeline("#pragma unroll")
                                 src.writeline(f"for (int u = 0; u < {n}; ++u) {{")
                                 with src.indent():
-                                    src.writeline(f"const long long r0_index = {step};")
-                                    if guarded:
-                                        src.writeline(f"if (r0_index >= {rnumel}) break;")
+                                    src.writeline(f"const long long r0_index = {index};")
                                     src.splice(r_idx)
                                     for name, ctype, ptr in loads:
                                         src.writeline(f"raw_{name}[u] = {G}ldraw<{ctype}, kVec>({ptr});")
@@ -1352,13 +1365,19 @@ class B200Kernel(SIMDKernel):
                                 src.writeline("#pragma unroll")
                                 src.writeline(f"for (int u = 0; u < {n}; ++u) {{")
                                 with src.indent():
-                                    src.writeline(f"const long long r0_index = {index};")
+                                    src.writeline(f"const long long r0_index = {step};")
+                                    if guarded:
+                                        src.writeline(f"if (r0_index >= {rnumel}) break;")
                                     src.splice(r_idx)
                                     for name, ctype, ptr in loads:
                                         src.writeline(f"const auto {name} = {G}widen_raw(raw_{name}[u]);")
                                     src.splice("\n".join(rest))
                                     src.writeline(acc_line)
                                 src.writeline("}")
+
+                            src.writeline(f"for (; rb + 7 * c.rstep() < {rnumel}; rb += 8 * c.rstep()) {{")
+                            with src.indent():
+                                batch(8, False)
                             src.writeline("}")
                             # What is left.  A warp's tile may be nothing else: four steps at a time, since a
                             # loop that tests the end at each of them waits for every load by itself.
@@ -1387,6 +1406,10 @@ class B200Kernel(SIMDKernel):
                 slot_line = ("const long long xindex = xslot;" if tiling is None else
                              f"const long long xindex = {G}tile_order<{tiling[0]}, {tiling[1]}, 16, 16, "
                              f"{'true' if b_first else 'false'}>(xslot);")
+                slot = "xslot"
+                if tiling is not None and self._small_index():
+                    slot = "slot"
+                    slot_line = f"const unsigned xslot = (unsigned)slot;\n{slot_line}"
                 row_body = re.sub(r"@B\d+@\n?", "", self._substitute(body_text, False))
                 if shift is not None:
                     row_body = row_body.replace("c.put_row_any(", "c.template put_row_shifted<STAGED>(")
@@ -1397,6 +1420,9 @@ class B200Kernel(SIMDKernel):
                     row_body = row_body.replace(self.consts[old][0], f"{G}kget<{new}, IXB_ROW_KREGS>(c, k.k{new})")
                 src.writeline(f"static constexpr int kN = IXB_ROW_VPT * {cfg.vec};   // elements per thread")
                 src.writeline(f"static constexpr bool kLooped = {'true' if self.looped else 'false'};   // row walked in chunks")
+                stream = tiling is not None or any(raw != "RawRow" for *_, raw in self.staged) or \
+                    any(v["kind"] == "S" and v["has_r"] for v in self._ph.values())
+                src.writeline(f"static constexpr bool kStream = {'true' if stream else 'false'};   // a block for every few rows of sub-warp teams")
                 src.writeline(f"static constexpr bool kTiled = {'true' if tiling is not None else 'false'};   // kept index walked in tiles")
                 pitch, first, period = shift or (0, 0, 0)
                 src.writeline(f"static constexpr int kShiftPeriod = {period};   // rows after which the offset from a "
@@ -1417,10 +1443,6 @@ class B200Kernel(SIMDKernel):
                     for n in range(len(self.columns)):
                         src.writeline(f"{G}vf<kN> a{n};")
                 src.writeline("};")
-
-                            src.writeline(f"for (; rb + 7 * c.rstep() < {rnumel}; rb += 8 * c.rstep()) {{")
-                            with src.indent():
-                                batch(8, False)
                 src.writeline("__device__ __forceinline__ void clear(Cols& cols) const {")
                 with src.indent():
                     for n in range(len(self.columns)):
@@ -1467,10 +1489,6 @@ class B200Kernel(SIMDKernel):
                             src.writeline(f"c.fetch_row({ptr}, {member});")
                 src.writeline("}")
                 src.writeline("template <bool STAGED, class Ctx>")
-                slot = "xslot"
-                if tiling is not None and self._small_index():
-                    slot = "slot"
-                    slot_line = f"const unsigned xslot = (unsigned)slot;\n{slot_line}"
                 src.writeline(f"__device__ __forceinline__ void row(Ctx& c, const Consts& k, const long long {slot}, "
                               "const Raw& raw, Cols& cols) const {")
                 with src.indent():
@@ -1481,9 +1499,6 @@ class B200Kernel(SIMDKernel):
                         src.writeline("const auto r0_index = c.rindex();")
                         src.writeline("const auto rmask = c.rmask();")
                         src.splice(x_idx)
-                stream = tiling is not None or any(raw != "RawRow" for *_, raw in self.staged) or \
-                    any(v["kind"] == "S" and v["has_r"] for v in self._ph.values())
-                src.writeline(f"static constexpr bool kStream = {'true' if stream else 'false'};   // a block for every few rows of sub-warp teams")
                         src.splice(r_idx)
                     src.splice(row_body)
                 src.writeline("}")
@@ -1507,6 +1522,8 @@ class B200Kernel(SIMDKernel):
                 for n, (tag, v) in enumerate(tile_loads.items()):
                     text = v["gather"] if kc is None else f"(STAGED ? {G}take(raw.t{n}, ci) : {v['gather']})"
                     body_text = body_text.replace(tag, text)
+                streams = not self.indirect and (kc is not None or self._moves_bytes(body_text))
+                src.writeline(f"static constexpr bool kStream = {'true' if streams else 'false'};   // a block for every 256 threads' work")
                 if kc is not None:
                     lb, dc, lc = order
                     nbv = lb // self.vec
@@ -1584,6 +1601,8 @@ class B200Kernel(SIMDKernel):
             if outer:
                 tx, cs = self._outer_split()
                 launch = f"launch_outer_gen<Body, {tx}>" if cs == 1 else f"launch_outer_split_gen<Body, {tx}, {cs}>"
+                if cs == 1 and self._outer_warp(tx):
+                    launch = f"launch_outer_warps_gen<Body, {tx}>"
                 src.writeline(f"return {G}{launch}(b, xnumel, stream, "
                               f"{G}pointers_aligned(ptrs, {len([a for a in assigns if 'ptrs[' in a])}));")
             elif self.is_row:
@@ -1660,8 +1679,6 @@ class B200Kernel(SIMDKernel):
         if device.type == "cuda":
             stream = wrapper.write_get_raw_stream(device.index, V.graph.name)
             wrapper.writeline(f"{name}.run({', '.join(map(str, call_args))}, stream={stream})")
-                if cs == 1 and self._outer_warp(tx):
-                    launch = f"launch_outer_warps_gen<Body, {tx}>"
         else:
             wrapper.writeline(f"{name}.run({', '.join(map(str, call_args))}, stream=None)")
         if self.columns:

@@ -395,28 +395,35 @@ __global__ void __launch_bounds__(256) pointwise_tile_gen_kernel(const Body body
     for (int ci = 0; ci < C; ++ci) body.template tile<true, true>(x0 + ci * Body::kStepC, V, raw, ci);
   }
 }
+// Grid of a kernel that moves every byte once and holds nothing from one vector to the next: a block
+// for every 256 vectors, which the hardware starts in order as others end.  Blocks that are resident for the
+// whole launch and stride through the tensor drift apart instead, and the DRAM pages that are open
+// at a time spread over all they have reached: a copy of 512 MB takes 160 us this way and 178 - 186
+// (148 x 8 and x 4 blocks) the other, the transpose of 4096 x 512 x 128 fp16 157 against 199, an inner
+// permute of the same size 170.5 against 175.5.  Rows gathered through an index are in no order anyway and
+// keep the resident grid (23.8 against 26.0 us for 262144 rows of 256 bytes out of 2^20).
+template <class Body> inline long long stream_grid(long long threads, long long resident) {
+  long long grid = (threads + 255) / 256;
+  const long long most = Body::kStream ? 0x7fffffffLL : resident;
+  if (grid > most) grid = most;
+  return grid < 1 ? 1 : grid;
+}
 template <class Body> int launch_pointwise(const Body& body, long long xnumel, void* stream, bool aligned);
 // tiles when every pointer is 16-byte aligned, the plain kernel (per-element gathers) otherwise
 template <class Body> int launch_pointwise_tile(const Body& body, long long xnumel, void* stream, bool aligned) {
   if (xnumel <= 0) return 0;
   if (!aligned) return launch_pointwise(body, xnumel, stream, false);
-  static const long long cap = resident_ctas(pointwise_tile_gen_kernel<Body>, 256);
-  const long long ntiles = xnumel / ((long long)Body::kVec * Body::kTileC);
-  long long grid = (ntiles + 255) / 256;
-  if (grid > cap) grid = cap;
-  if (grid < 1) grid = 1;
+  static const long long cap = Body::kStream ? 0 : resident_ctas(pointwise_tile_gen_kernel<Body>, 256);
+  const long long grid = stream_grid<Body>(xnumel / ((long long)Body::kVec * Body::kTileC), cap);
   pointwise_tile_gen_kernel<Body><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
   return (int)cudaGetLastError();
 }
 
 template <class Body> int launch_pointwise(const Body& body, long long xnumel, void* stream, bool aligned = false) {
   if (xnumel <= 0) return 0;
-  static const long long cap_a = resident_ctas(pointwise_gen_kernel<Body, true>, 256);
-  static const long long cap_u = resident_ctas(pointwise_gen_kernel<Body, false>, 256);
-  const long long ntiles = (xnumel + Body::kVec - 1) / Body::kVec;
-  long long grid = (ntiles + 255) / 256;
-  const long long cap = aligned ? cap_a : cap_u;
-  if (grid > cap) grid = cap;
+  static const long long cap_a = Body::kStream ? 0 : resident_ctas(pointwise_gen_kernel<Body, true>, 256);
+  static const long long cap_u = Body::kStream ? 0 : resident_ctas(pointwise_gen_kernel<Body, false>, 256);
+  const long long grid = stream_grid<Body>((xnumel + Body::kVec - 1) / Body::kVec, aligned ? cap_a : cap_u);
   if (aligned) pointwise_gen_kernel<Body, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
   else pointwise_gen_kernel<Body, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
   return (int)cudaGetLastError();
@@ -1546,6 +1553,11 @@ template <class U> int finish_columns(const float* partial, long long rows, int 
                          (int)rows, cols, out);
 }
 
+// Sub-warp teams whose threads load nothing once for all rows get a block for every batch of four rows a
+// team (see stream_grid) where there are more than the resident blocks would see in three batches: the
+// permuted sum of 64 x 128 x 256 x 64 fp16 48.9 -> 45.4 us.
+template <class Body, int TEAM, bool STAGED> constexpr bool kStreamRows = TEAM < 32 && STAGED && Body::kStream && Body::kConsts == 0;
+
 template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS, int PF, int COLS, bool STAGED>
 __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     row_gen_kernel(const Body body, const long long rows, const int cols) {
@@ -1650,11 +1662,6 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   if (COLS > 0 && cols != COLS) return (int)cudaErrorInvalidValue;
   // a row longer than the team can hold (a run-time extent beyond the compiled capacity);
   // looped bodies walk any length in chunks
-// Sub-warp teams whose threads load nothing once for all rows get a block for every batch of four rows a
-// team (see stream_grid) where there are more than the resident blocks would see in three batches: the
-// permuted sum of 64 x 128 x 256 x 64 fp16 48.9 -> 45.4 us.
-template <class Body, int TEAM, bool STAGED> constexpr bool kStreamRows = TEAM < 32 && STAGED && Body::kStream && Body::kConsts == 0;
-
   if (cols < 0 || (!Body::kLooped && cols > TEAM * VPT * Elem<T>::kVec)) return (int)cudaErrorInvalidValue;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -1680,6 +1687,7 @@ template <class Body, int TEAM, bool STAGED> constexpr bool kStreamRows = TEAM <
     } else if (grid > groups) {
       grid = groups;
     }
+    if (kStreamRows<Body, TEAM, true> && groups > 3 * (long long)sms * resident) grid = (groups + 3) / 4;
     if (blocks != nullptr) *blocks = grid;
     return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
   }
@@ -1782,7 +1790,6 @@ template <int V, int TX, int TY> struct OuterCtx {
       if (ty % kRowsPerWarp == 0) {
 #pragma unroll
         for (int i = 0; i < V; ++i) part[(warp * TX + tx) * V + i] = r.v[i];
-    if (kStreamRows<Body, TEAM, true> && groups > 3 * (long long)sms * resident) grid = (groups + 3) / 4;
       }
       __syncthreads();
       // only the thread row that stores the tile needs the folded vector (a generated outer
@@ -1811,7 +1818,7 @@ __global__ void __launch_bounds__(TX* TY* GROUPS) outer_gen_kernel(const Body bo
   __shared__ __align__(16) float part[(TX * TY / 32) * TX * V];
   OuterCtx<V, TX, TY> c;
   c.tx = threadIdx.x % TX;
-  c.ty = threadIdx.x / TX;
+  c.ty = threadIdx.x / TX % TY;
   c.part = part;
   const long long per_cta = (long long)TX * V;
   const long long ntiles = (xnumel + per_cta - 1) / per_cta;
@@ -1909,7 +1916,7 @@ __global__ void __launch_bounds__(TX* TY) outer_split_gen_kernel(const Body body
   __shared__ __align__(8) uint64_t bar;
   OuterSplitCtx<V, TX, TY, CS> c;
   c.tx = threadIdx.x % TX;
-  c.ty = threadIdx.x / TX % TY;
+  c.ty = threadIdx.x / TX;
   c.part = part;
   c.inbox = inbox;
   c.bar = &bar;
@@ -1948,6 +1955,21 @@ int launch_outer_split_gen(const Body& body, long long xnumel, void* stream, boo
   return (int)cudaLaunchKernelEx(&cfg, outer_split_gen_kernel<Body, TX, TY, CS, false>, body, xnumel);
 }
 
+// Short reduced axes: with 256 threads to a tile each would add one or two vectors and then wait for two
+// barriers of the CTA.  A warp a tile has eight times as many steps a thread and folds by shuffles.
+// Bound: HBM.  Maximum over the 26 of 6163 x 26 x 22 x 32 bf16 (memory order): see _outer_warp.
+template <class Body, int TX>
+int launch_outer_warps_gen(const Body& body, long long xnumel, void* stream, bool aligned = false) {
+  if (xnumel <= 0) return 0;
+  constexpr int TY = 32 / TX, GROUPS = 8;
+  const long long tiles = (xnumel + (long long)TX * Body::kVec - 1) / ((long long)TX * Body::kVec);
+  long long grid = (tiles + GROUPS - 1) / GROUPS;
+  if (grid > 0x7fffffffLL) grid = 0x7fffffffLL;
+  if (aligned) outer_gen_kernel<Body, TX, TY, GROUPS, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
+  else outer_gen_kernel<Body, TX, TY, GROUPS, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
+  return (int)cudaGetLastError();
+}
+
 template <class Body, int TX = 32>
 int launch_outer_gen(const Body& body, long long xnumel, void* stream, bool aligned = false) {
   if (xnumel <= 0) return 0;
@@ -1973,18 +1995,3 @@ int launch_outer_gen(const Body& body, long long xnumel, void* stream, bool alig
 
 }  // namespace gen
 }  // namespace ixb
-// Short reduced axes: with 256 threads to a tile each would add one or two vectors and then wait for two
-// barriers of the CTA.  A warp a tile has eight times as many steps a thread and folds by shuffles.
-// Bound: HBM.  Maximum over the 26 of 6163 x 26 x 22 x 32 bf16 (memory order): see _outer_warp.
-template <class Body, int TX>
-int launch_outer_warps_gen(const Body& body, long long xnumel, void* stream, bool aligned = false) {
-  if (xnumel <= 0) return 0;
-  constexpr int TY = 32 / TX, GROUPS = 8;
-  const long long tiles = (xnumel + (long long)TX * Body::kVec - 1) / ((long long)TX * Body::kVec);
-  long long grid = (tiles + GROUPS - 1) / GROUPS;
-  if (grid > 0x7fffffffLL) grid = 0x7fffffffLL;
-  if (aligned) outer_gen_kernel<Body, TX, TY, GROUPS, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
-  else outer_gen_kernel<Body, TX, TY, GROUPS, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
-  return (int)cudaGetLastError();
-}
-
