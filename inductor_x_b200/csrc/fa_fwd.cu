@@ -44,28 +44,19 @@
 #include <atomic>
 #include "host.h"
 #include "fa_maps.h"
-#include "ixb/tcgen05.cuh"
+#include "ixb/fa_softmax.cuh"
 
 namespace {
 
 using namespace ixb;
 
-constexpr int BM = 128;          // rows of one query tile
-constexpr int NQ = 2;            // query tiles per CTA
-constexpr int BN = 128;          // keys per tile
-constexpr int HD = 128;          // head dimension
+using namespace ixb::fa;
+
 constexpr int kStages = 2;  // (the issuer picks stage descriptors with two-way selects)
-constexpr int kTileBytes = BN * HD * 2;     // one operand tile, 16-bit elements
-constexpr int kHalfBytes = kTileBytes / 2;  // one 64-column TMA box of the tile
-constexpr int kThreads = 128 + NQ * 128;  // a warpgroup for producer and issuer, one per query tile
 // Registers: the block starts with kRegsLaunch a thread (all that 12 warps can have); the first
 // warpgroup gives up what it does not need so that a softmax thread holds its row of 128 scores.
 constexpr int kRegsLaunch = 168, kRegsIssue = 80, kRegsSoftmax = 208;
 static_assert(kRegsIssue + NQ * kRegsSoftmax <= (1 + NQ) * kRegsLaunch, "setmaxnreg draws on the block's own registers");
-constexpr int kSplit = 96;  // keys of P handed to the tensor core ahead of the rest of the tile
-constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kColS = 0, kColO = 256;  // + 128 * tile
-constexpr float kRescaleThreshold = 8.f;    // log2 units
 constexpr size_t kSmemBytes = (size_t)kTileBytes * (NQ + 2 * kStages) + 1024;
 
 struct FaParams {
@@ -79,15 +70,6 @@ struct FaParams {
   int wide;        // the rows of o are multiples of 32 bytes
   int head_group;  // heads whose CTAs are dispatched together (see the CTA order in the kernel)
 };
-
-__device__ __forceinline__ uint32_t pack_pair(float lo, float hi, bool is_bf16) {
-  if (is_bf16) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-  }
-  const __half2 h = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
 
 template <bool IS_BF16>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -353,76 +335,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (p.causal && qi + diag < last) last = qi + diag;
           lim = last - col0;
         }
-        // the row of scores stays in registers: one trip through tensor memory per tile
-        uint32_t raw[BN];
-#pragma unroll
-        for (int c = 0; c < BN / 32; ++c)
-          tc::tmem_ld32(s_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
-        tc::tmem_wait_ld();
-        if (edge) {
-#pragma unroll
-          for (int c = 0; c < BN / 32; ++c) {
-            if (__all_sync(kFull, lim >= c * 32 + 31)) continue;  // (what every row of the warp sees stays)
-#pragma unroll
-            for (int e = c * 32; e < c * 32 + 32; ++e)
-              if (e > lim) raw[e] = 0xff800000u;  // -inf
-          }
-        }
-        // four independent chains: one chain of 64 dependent max3 would cost its latency 64 times
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int e = 0; e < BN; e += 2)
-          mx4[(e >> 1) & 3] = max3(mx4[(e >> 1) & 3], __uint_as_float(raw[e]), __uint_as_float(raw[e + 1]));
-        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        mx *= p.scale_log2;  // scale > 0: scaling commutes with the maximum
-        // lazy rescale: move the reference maximum only when it would grow by > 2^8
-        const bool grow = mx > m_used + kRescaleThreshold;  // also true for the first tile
-        if (__any_sync(kFull, grow)) {
-          const float m_new = grow ? mx : m_used;
-          const float f = !grow ? 1.f : ((m_used == -INFINITY) ? 0.f : fast_exp2(m_used - m_new));
-          l *= f;
-          if (j > 0) {
-            // O may only be touched once O += P(j-1) V(j-1) has completed: it has - S(j),
-            // which this warp has waited for, was committed behind it
-#pragma unroll
-            for (int c = 0; c < HD / 32; ++c) {
-              uint32_t o[32];
-              tc::tmem_ld32(o_addr + c * 32, o);
-              tc::tmem_wait_ld();
-#pragma unroll
-              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-              tc::tmem_st32(o_addr + c * 32, o);
-            }
-            tc::tmem_wait_st();
-          }
-          m_used = m_new;
-        }
-        // ---- P = exp2(s * scale - m_used), written over the scores as 16-bit pairs
-        const float mref = (m_used == -INFINITY) ? 0.f : m_used;
-        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-        const float2 nm2 = make_float2(-mref, -mref);
-        float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // two chains of packed adds
-#pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t pk[16];
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float2 a = fma2(make_float2(__uint_as_float(raw[c * 32 + e]), __uint_as_float(raw[c * 32 + e + 1])), sc2, nm2);
-            const float2 pe = make_float2(fast_exp2(a.x), fast_exp2(a.y));
-            sum2[(e >> 1) & 1] = add2(sum2[(e >> 1) & 1], pe);
-            pk[e / 2] = pack_pair(pe.x, pe.y, IS_BF16);
-          }
-          tc::tmem_st16(s_addr + c * 16, pk);
-          if (c * 32 + 32 == kSplit) {
-            tc::tmem_wait_st();
-            tc::fence_before_sync();
-            tc::mbar_arrive(&p_full[t]);
-          }
-        }
-        tc::tmem_wait_st();
-        tc::fence_before_sync();
-        tc::mbar_arrive(&p_rest[t]);
-        l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+        softmax_tile<IS_BF16>(s_addr, o_addr, edge, lim, j == 0, p.scale_log2, m_used, l, &p_full[t], &p_rest[t]);
         ++seen;
       }
       if (ok && my_n_kv > 0) {
@@ -526,6 +439,8 @@ extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v
   static const int group_env = [] { const char* v = getenv("IXB_FA_HEAD_GROUP"); return v != nullptr ? atoi(v) : 0; }();
   p.head_group = group_env > 0 ? group_env : (causal ? 8 : 1);
   if (!(scale > 0.f)) return IXB_ERR_ARG;  // the row maximum is taken before scaling
+  if (const int cluster = ixb_host::fa_split_size(B, H, Sq, Sk))
+    return ixb_host::fa_split(cluster, is_bf16, mq, mk, mv, o, lse, B, H, Sq, Sk, o_strides, scale, causal, status, (cudaStream_t)stream);
   const dim3 grid((unsigned)(((Sq + BM * NQ - 1) / (BM * NQ)) * (long long)B * H));
   auto kern = is_bf16 ? fa_fwd_kernel<true> : fa_fwd_kernel<false>;
   // the shared-memory opt-in is a property of (kernel, device): set once per device

@@ -43,4 +43,10 @@ inline int make_fa_map(CUtensorMap* map, const void* base, int is_bf16, int B, i
   return r == CUDA_SUCCESS ? IXB_OK : IXB_ERR_ARG;
 }
 
+// fa_split.cu: how many blocks share a query tile's keys where the forward pass is cut that way (0: it is
+// not, fa_fwd.cu), and the launch
+int fa_split_size(int B, int H, int Sq, int Sk);
+int fa_split(int cluster, int is_bf16, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* o, float* lse,
+             int B, int H, int Sq, int Sk, const int64_t* o_strides, float scale, int causal, int32_t* status, cudaStream_t stream);
+
 }  // namespace ixb_host
