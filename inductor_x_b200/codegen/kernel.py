@@ -1135,6 +1135,11 @@ class B200Kernel(SIMDKernel):
         (``inductor_x/codegen/triton.py:856-888, 1303-1332``), done here by the walking order
         alone - the sectors a warp touches on both sides are fully used, without a shared-memory
         tile.  Returns (LB, dC, LC) or None."""
+        found = self._transposing_digits()
+        return None if found is None or found[2] % 32 or found[0] % self.vec else found
+
+    def _transposing_digits(self):
+        """The digits (LB, dC, LC) of the flat index of such a group, whatever their extents."""
         if self.is_row or self._is_dynamic("x") or not getattr(self, "_gather_loads", None):
             return None
         xsym = self._root("x").symbol()
@@ -1151,12 +1156,42 @@ class B200Kernel(SIMDKernel):
             lb, (_, dc, lc) = low[0][2], unit[0]
             if lc is None:
                 lc = xnumel // dc
-            if dc % lb or xnumel % (dc * lc) or lc % 32 or lb % self.vec:
+            if dc % lb or xnumel % (dc * lc):
                 return None
             if found is not None and found != (lb, dc, lc):
                 return None
             found = (lb, dc, lc)
         return found
+
+    def _smem_tile(self):
+        """(LB, dC, LC, vectors of an output row to a block, columns to a block at most, stride of each tile
+        load along the flat index) when the group is transposed by way of shared memory
+        (``pointwise_smem_gen_kernel``), or None.  It takes what register tiles do not, from 32 elements on
+        in both digits (shorter ones leave most of a block without work: 30000 x 16 x 17 fp32 28 us by
+        gathers, 42 so), for one or two operands of 16 or 32 bits; more would leave room for two blocks an SM."""
+        digits, tl = self._transposing_digits(), getattr(self, "_tile_loads", None)
+        if digits is None or self._register_tile(self._transposing_order()) is not None or not 1 <= len(tl) <= 2:
+            return None
+        lb, dc, lc = digits
+        if lb < 32 or lc < 32 or not self._small_index() or self.indirect or self.vec not in (4, 8):
+            return None
+        if not all(v["dtype"] in (torch.float32, torch.float16, torch.bfloat16) for v in tl.values()):
+            return None
+        xsym = self._root("x").symbol()
+        strides = []
+        for v in tl.values():
+            rest, pieces = index_ir._axis_pieces(v["exp"], xsym)
+            low = [c for c, d, m in pieces if d == 1]
+            # what is neither digit is a digit between them or beyond both: one value a block
+            others = [(d, m) for c, d, m in pieces if d != 1 and not (c == 1 and d == dc)]
+            if len(low) != 1 or any(not ((d % lb == 0 and m is not None and dc % (d * m) == 0) or d % (dc * lc) == 0)
+                                    for d, m in others):
+                return None
+            strides.append(low[0])
+        per = 16 // max(config_bytes(v["dtype"]) for v in tl.values())
+        chunks = -(-(lb + self.vec - 1) // self.vec)
+        nk = 16 if len(tl) == 1 and -(-chunks // 16) * 16 <= -(-chunks // 8) * 8 else 8
+        return lb, dc, lc, nk, (16 * per - (per - 1)) // 4 * 4, strides
 
     def _moves_bytes(self, body_text: str) -> bool:
         """Whether a pointwise group is worth a block for every 256 vectors (``stream_grid``): a thread
@@ -1518,9 +1553,10 @@ class B200Kernel(SIMDKernel):
                 src.writeline(f"static constexpr int kVec = {self.vec};")
                 order = self._transposing_order()
                 kc = self._register_tile(order)
+                smem = self._smem_tile()
                 tile_loads = getattr(self, "_tile_loads", {})
                 for n, (tag, v) in enumerate(tile_loads.items()):
-                    text = v["gather"] if kc is None else f"(STAGED ? {G}take(raw.t{n}, ci) : {v['gather']})"
+                    text = v["gather"] if kc is None and smem is None else f"(STAGED ? {G}take(raw.t{n}, ci) : {v['gather']})"
                     body_text = body_text.replace(tag, text)
                 streams = not self.indirect and (kc is not None or self._moves_bytes(body_text))
                 src.writeline(f"static constexpr bool kStream = {'true' if streams else 'false'};   // a block for every 256 threads' work")
@@ -1553,6 +1589,29 @@ class B200Kernel(SIMDKernel):
                         src.splice(x_idx)
                         for n, v in enumerate(tile_loads.values()):
                             src.writeline(f"{G}fetch_tile(raw.t{n}, {v['var']}, {v['idx']});")
+                    src.writeline("}")
+                elif smem is not None:
+                    *_, nk, cols, strides = smem
+                    rows = nk * self.vec + self.vec - 1
+                    src.writeline(f"static constexpr int kTileOps = {len(tile_loads)};")
+                    src.writeline(f"static constexpr int kTileCols = {cols};   // elements of a source row to a block at most")
+                    src.writeline("struct Tile {")
+                    with src.indent():
+                        for n, v in enumerate(tile_loads.values()):
+                            src.writeline(f"{G}TileSmem<{v['ctype']}, kVec, {rows}, {strides[n]}> t{n};")
+                        src.writeline("__device__ __forceinline__ void at(int row, int col) { "
+                                      + " ".join(f"t{n}.row = row; t{n}.col = col;" for n in range(len(tile_loads))) + " }")
+                    src.writeline("};")
+                    src.writeline("template <class Words>")
+                    src.writeline("__device__ __forceinline__ Tile copy_tiles(Words& words, const long long xindex, const int row0, "
+                                  "const int cols) const {")
+                    with src.indent():
+                        src.splice(x_idx)
+                        src.writeline("Tile t;")
+                        for n, v in enumerate(tile_loads.values()):
+                            src.writeline(f"t.t{n} = {G}copy_tile<{v['ctype']}, kVec, {rows}, {strides[n]}>(words[{n}], "
+                                          f"{v['var']} + {G}lane0({v['idx']}) + (long long)row0 * {strides[n]}, -row0, {smem[0]} - row0, cols);")
+                        src.writeline("return t;")
                     src.writeline("}")
                 else:
                     src.writeline("struct Tile {};")
@@ -1632,7 +1691,10 @@ class B200Kernel(SIMDKernel):
                     src.writeline("return rc;")
             else:
                 launcher = "launch_pointwise_tile" if self._register_tile(self._transposing_order()) else "launch_pointwise"
-                src.writeline(f"return {G}{launcher}<Body>(b, xnumel, stream, "
+                targs = "Body"
+                if smem is not None:
+                    launcher, targs = "launch_pointwise_smem", f"Body, {smem[0]}, {smem[1]}LL, {smem[2]}, {smem[3]}"
+                src.writeline(f"return {G}{launcher}<{targs}>(b, xnumel, stream, "
                               f"{G}pointers_aligned(ptrs, {len([a for a in assigns if 'ptrs[' in a])}));")
         src.writeline("}")
         if self.checked_indices:

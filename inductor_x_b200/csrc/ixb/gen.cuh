@@ -408,7 +408,103 @@ template <class Body> inline long long stream_grid(long long threads, long long 
   if (grid > most) grid = most;
   return grid < 1 ? 1 : grid;
 }
+// ---- transposes by way of shared memory ---------------------------------------------------------
+// The same where the extents do not divide into register tiles or rows start off a 16-byte boundary on
+// either side.  A block has NK vectors of up to 120 (60 of 32 bits) output rows; of each of the NK * V + V - 1
+// source rows these may want it copies the aligned words that hold some element of it (16 words a row
+// at most, cp.async), and an output vector is gathered from the V rows.  Output vectors are those of memory:
+// a row's first one begins before the row where the row does not begin on a boundary, so that what
+// is stored is whole 16-byte words but for the ends of a row.  Words are swizzled by the row's vector:
+// the lanes of a warp, eight vectors by four rows of output, read eight rows V apart without a bank conflict
+// (rows off a boundary shift against each other by a word now and then).  Bound: the gathering, a
+// shared load and some ten instructions an element.  Measured: see launch_pointwise_smem.
+constexpr int kTileWords = 16;
+template <class U, int V, int ROWS, int STRIDE> struct TileSmem {
+  const uint4* words = nullptr;  // [ROWS + V][kTileWords], the last V of them never written
+  int row = 0, col = 0;          // of the vector's first element
+  int off = 0;                   // elements between the first word of row 0 and its first element
+};
+template <class U, int V, int ROWS, int STRIDE>
+__device__ __forceinline__ vf<V> take(const TileSmem<U, V, ROWS, STRIDE>& t, int) {
+  constexpr int kPer = 16 / (int)sizeof(U);
+  const unsigned char* from = reinterpret_cast<const unsigned char*>(t.words + t.row * kTileWords);
+  const int off = t.off + t.row * (STRIDE % kPer);
+  vf<V> r;
+#pragma unroll
+  for (int j = 0; j < V; ++j) {  // (elements past the end of a row come from the rows behind the tile, and are masked)
+    const int pos = ((off + j * (STRIDE % kPer)) & (kPer - 1)) + t.col;
+    const int key = (t.row + j) / V & 7;
+    r.v[j] = Mem<U>::ld(reinterpret_cast<const U*>(from + j * (16 * kTileWords) + ((pos * (int)sizeof(U)) ^ (key * 16))));
+  }
+  return r;
+}
+// Source rows of one operand into shared memory: row r of the tile begins at from + (r - first) * STRIDE;
+// rows [lo, hi) of it exist, and `count` elements of each are wanted.
+template <class U, int V, int ROWS, int STRIDE>
+__device__ __forceinline__ TileSmem<U, V, ROWS, STRIDE> copy_tile(uint4* words, const U* from, int lo, int hi, int count) {
+  constexpr int kPer = 16 / (int)sizeof(U);
+  for (int i = threadIdx.x; i < ROWS * kTileWords; i += blockDim.x) {
+    const int r = i / kTileWords, w = i % kTileWords;
+    if (r < lo || r >= hi) continue;
+    const U* row = from + (long long)r * STRIDE;
+    const int off = off_boundary(row);
+    if (w * kPer < off + count)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(words + r * kTileWords + (w ^ ((r / V) & 7)))),
+                   "l"(row - off + w * kPer)
+                   : "memory");
+  }
+  TileSmem<U, V, ROWS, STRIDE> t;
+  t.words = words;
+  t.off = off_boundary(from);
+  return t;
+}
+// LB, DC, LC: digits of the flat index (output rows of LB elements, the loads' axis LC of them DC apart)
+template <class Body, int LB, long long DC, int LC, int NK>
+__global__ void __launch_bounds__(256) pointwise_smem_gen_kernel(const Body body) {
+  constexpr int V = Body::kVec, TX = NK * V, ROWS = TX + V - 1;
+  constexpr int NX = (LB + V - 1 + TX - 1) / TX;
+  constexpr int NC = (LC + Body::kTileCols - 1) / Body::kTileCols, TC = (LC + NC - 1) / NC;
+  __shared__ uint4 words[Body::kTileOps][(ROWS + V) * kTileWords];
+  unsigned b = blockIdx.x;
+  const int c0 = (int)(b % NC) * TC;
+  b /= NC;
+  const int x0 = (int)(b % NX) * TX;
+  b /= NX;
+  const unsigned mid = b % (unsigned)(DC / LB), outer = b / (unsigned)(DC / LB);
+  const long long first = (long long)outer * (DC * LC) + c0 * DC + (long long)mid * LB;  // flat index of (x 0, c0)
+  const int cols = LC - c0 < TC ? LC - c0 : TC;
+  // row r of the tile is element x0 - (V - 1) + r of the output rows
+  typename Body::Tile raw = body.copy_tiles(words, first, x0 - (V - 1), cols);
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int it = threadIdx.x >> 5; it < (cols + 3) / 4 * (NK / 8); it += 8) {
+    const int c = it / (NK / 8) * 4 + (lane >> 3), k = it % (NK / 8) * 8 + (lane & 7);
+    if (c >= cols) continue;
+    const long long row = first + c * DC;
+    int x = x0 + k * V - (int)((unsigned long long)row % V), n = V;
+    if (x < 0) {
+      n += x;
+      x = 0;
+    }
+    if (x + n > LB) n = LB - x;
+    if (n <= 0) continue;
+    raw.at(x - (x0 - (V - 1)), c);
+    if (n == V) body.template tile<true, true>(row + x, V, raw);
+    else body.template tile<false, true>(row + x, n, raw);
+  }
+}
+
 template <class Body> int launch_pointwise(const Body& body, long long xnumel, void* stream, bool aligned);
+template <class Body, int LB, long long DC, int LC, int NK>
+int launch_pointwise_smem(const Body& body, long long xnumel, void* stream, bool aligned) {
+  if (xnumel <= 0) return 0;
+  constexpr int TX = NK * Body::kVec, NX = (LB + Body::kVec - 1 + TX - 1) / TX, NC = (LC + Body::kTileCols - 1) / Body::kTileCols;
+  const long long blocks = xnumel / LB / LC * NX * NC;
+  if (!aligned || blocks > 0x7fffffffLL) return launch_pointwise(body, xnumel, stream, aligned);
+  pointwise_smem_gen_kernel<Body, LB, DC, LC, NK><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(body);
+  return (int)cudaGetLastError();
+}
 // tiles when every pointer is 16-byte aligned, the plain kernel (per-element gathers) otherwise
 template <class Body> int launch_pointwise_tile(const Body& body, long long xnumel, void* stream, bool aligned) {
   if (xnumel <= 0) return 0;

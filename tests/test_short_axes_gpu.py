@@ -26,52 +26,46 @@ def close(got, want, dtype, terms):
     assert float(((got.double() - want).abs() / scale).max()) <= EPS[dtype] * (4 if dtype != torch.float32 else 4 + terms ** 0.5)
 
 
-# extents of the two kept digits: below, at and past one tile of 16, and past several
-@pytest.mark.parametrize("b,c", [(2, 2), (15, 3), (16, 17), (33, 16), (47, 31), (130, 70)])
-@pytest.mark.parametrize("dtype,d", [(torch.float32, 4), (torch.float32, 16), (torch.float16, 24), (torch.bfloat16, 64),
-                                     (torch.float32, 96)])
+# extents of the two kept digits below, at and past one tile of 16, and past several; rows of one vector to 24
+@pytest.mark.parametrize("b,c,dtype,d", [(2, 15, torch.float32, 4), (33, 16, torch.float32, 16), (16, 17, torch.bfloat16, 64),
+                                         (130, 70, torch.float16, 24), (47, 31, torch.float32, 96)])
 def test_rows_in_smaller_tiles(cuda, b, c, dtype, d):
     x = data(cuda, (37, b, c, d), dtype)
     close(compiled(lambda x: x.permute(0, 2, 1, 3).sum(3), x), x.double().permute(0, 2, 1, 3).sum(3), dtype, d)
 
 
-# 1 to 9 vectors of four, whole and ragged; rows for a few blocks, and more than three batches of what is
-# resident (blocks that see one batch)
-@pytest.mark.parametrize("rows", [1, 1003, 300007])
-def test_rows_of_a_few_vectors(cuda, rows):
-    for d in (1, 3, 4, 8, 11, 12, 16, 20, 23, 24, 32, 36):
+# 1, 2 (ragged), 4, 5 and 6 vectors of four; one row, rows for a few blocks, and more than three batches of
+# what is resident (blocks that see one batch)
+@pytest.mark.parametrize("d", [4, 7, 16, 20, 24])
+def test_rows_of_a_few_vectors(cuda, d):
+    for rows in (1, 1003, 300007):
         x = data(cuda, (rows, d), torch.float32)
         close(compiled(lambda x: x.sum(-1), x), x.double().sum(-1), torch.float32, d)
         y = compiled(lambda x: torch.softmax(x, -1), x)
         assert float((y.double() - torch.softmax(x.double(), -1)).abs().max()) <= 1e-6
-        x = x.half()
-        assert torch.equal(compiled(lambda x: x.amax(-1), x), x.amax(-1))
 
 
-# steps of the reduced axis around those of a thread row (32 lanes: 8, 4, 2 and 1 of them) and of a batch,
-# tiles enough for a warp each and a last one that is cut
-@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 32), (torch.float32, 32), (torch.float16, 128), (torch.float32, 100)])
-def test_outer_reductions_with_a_warp_to_a_tile(cuda, dtype, d):
-    for r in (1, 2, 7, 8, 9, 26, 31, 33, 61):
-        x = data(cuda, (2003, r, d), dtype)
-        assert torch.equal(compiled(lambda x: x.amax(1), x), x.amax(1))
+# steps of the reduced axis around those of a warp's thread rows (8, 4, 2 and 1 of them) and of a batch of
+# four, tiles enough for a warp each
+@pytest.mark.parametrize("dtype,r,d", [(torch.bfloat16, 2, 32), (torch.bfloat16, 33, 32), (torch.float16, 26, 128), (torch.float32, 9, 100)])
+def test_outer_reductions_with_a_warp_to_a_tile(cuda, dtype, r, d):
+    x = data(cuda, (4003, r, d), dtype)
+    assert torch.equal(compiled(lambda x: x.amax(1), x), x.amax(1))
+    if r == 33:
         close(compiled(lambda x: x.sum(1), x), x.double().sum(1), dtype, r)
-    i = (x * 1000).to(torch.int32)
-    assert torch.equal(compiled(lambda i: i.sum(1), i), i.sum(1))
-    s = data(cuda, (r,), torch.float32)
-    close(compiled(lambda x, s: (x.float() * s[:, None]).sum(1), x, s), (x.double() * s.double()[:, None]).sum(1), torch.float32, r * 16)
+        i = (x * 1000).to(torch.int32)
+        assert torch.equal(compiled(lambda i: i.sum(1), i), i.sum(1))
 
 
-@pytest.mark.parametrize("n", [1, 7, 255 * 8 + 1, 256 * 8, 3000001])
+@pytest.mark.parametrize("n", [1, 2041, 3000001])
 def test_grids_of_a_block_for_256_vectors(cuda, n):
     a, b = data(cuda, (n,), torch.bfloat16), data(cuda, (n,), torch.bfloat16)
     assert torch.equal(compiled(lambda a, b: a + b, a, b), a + b)
-    assert torch.equal(compiled(lambda a: a.float(), a), a.float())
     if n > 1:   # bases off a boundary
         assert torch.equal(compiled(lambda a, b: a + b, a[1:], b[1:]), a[1:] + b[1:])
 
 
-@pytest.mark.parametrize("dtype,shape", [(torch.float16, (3, 320, 64)), (torch.float32, (5, 128, 96)), (torch.bfloat16, (1, 1024, 2048))])
+@pytest.mark.parametrize("dtype,shape", [(torch.float16, (3, 320, 64)), (torch.float32, (5, 128, 96))])
 def test_register_tiles(cuda, dtype, shape):
     x = data(cuda, shape, dtype)
     assert torch.equal(compiled(lambda x: (x.transpose(1, 2) + 1.0).contiguous(), x), x.transpose(1, 2) + 1.0)
