@@ -506,7 +506,7 @@ class B200Kernel(SIMDKernel):
                     loads.append(exp0)
                     tag = f"@T{len(loads) - 1}@"
                     self.__dict__.setdefault("_tile_loads", {})[tag] = dict(
-                        ctype=ctype, dtype=dtype, var=var, idx=idx, exp=exp0, gather=line)
+                        ctype=ctype, dtype=dtype, var=var, idx=idx, exp=exp0, gather=line, other=other, indirect=())
                     return self.cse.generate(self.compute, tag, dtype=val_dtype)
             if indirect and not masked:
                 # direct part contiguous along the vector: one 128-bit access whenever the
@@ -518,6 +518,12 @@ class B200Kernel(SIMDKernel):
                     al = "FAST" if aligned else "false"
                     line = (f"{G}igather<{ctype}, kVec, {al}>({var}, {idx}, xmask, {other}, nvalid, "
                             f"{', '.join(ind)})")
+                elif exp.free_symbols <= {xsym} | {s for s in exp.free_symbols if str(s) in ind}:
+                    # contiguous inside a row of odd length, perhaps: settled with the whole group (_odd_rows)
+                    table = self.__dict__.setdefault("_row_loads", {})
+                    tag = f"@Q{len(table)}@"
+                    table[tag] = dict(ctype=ctype, dtype=dtype, var=var, idx=idx, exp=exp, gather=line, other=other, indirect=ind)
+                    return self.cse.generate(self.compute, tag, dtype=val_dtype)
             if not indirect and not masked:
                 exp = self._expanded(index)
                 if xsym in exp.free_symbols and index_ir.is_vector_constant(exp, xsym, self.vec):
@@ -1163,6 +1169,51 @@ class B200Kernel(SIMDKernel):
             found = (lb, dc, lc)
         return found
 
+    def _odd_rows(self):
+        """The length LB of the rows that a pointwise group without a better form is walked in: vectors
+        that end with their row (``pointwise_rows_gen_kernel``).  Where LB is no whole number of vectors a
+        vector of the flat index reaches into the next row, so that what is contiguous along a row (a
+        gathered row, a per-column operand) or constant over it (an index, a per-row operand) would be
+        loaded element by element.  None where nothing is gained: rows of less than four vectors, where the ends
+        are most of the work (gather of 500000 x 17 fp16 21.0 us so or so), and of less than sixteen unless
+        what is loaded in runs is as large as the result and not an operand that all rows share (x * w + b,
+        100000 x 37 fp32, 8.2 against 10.3).  Gather of 100000 x 333 bf16 89 -> 32 us, of 50000 x 1023 fp32 136 ->
+        67; permuted 64 x 65 x 66 x 37 fp16 59 -> 17; x * w of 20000 x 3333 bf16 79 -> 55."""
+        loads = [*getattr(self, "_tile_loads", {}).values(), *getattr(self, "_row_loads", {}).values()]
+        if self.is_row or self._is_dynamic("x") or not loads or not self._small_index():
+            return None
+        xsym = self._root("x").symbol()
+        lengths = []
+        for v in loads:
+            split = index_ir._axis_pieces(v["exp"], xsym)
+            if split is not None:
+                lengths += [m for c, d, m in split[1] if d == 1 and m is not None] or \
+                    [min(d for c, d, m in split[1])] * bool(split[1])
+        for lb in sorted(set(lengths), key=lambda n: (-lengths.count(n), n)):
+            if lb % self.vec == 0 or lb < 4 * self.vec or self._numel_hint("x") % lb:
+                continue
+            read = [v for v in loads if self._row_text(v, lb)]
+            if lb < 16 * self.vec:
+                read = [v for v in read if v["indirect"] or (len(index_ir._axis_pieces(v["exp"], xsym)[1]) > 1)]
+            if read:
+                return lb
+        return None
+
+    def _row_text(self, v, lb: int):
+        """How a load reads inside rows of lb elements: one value, a run, or (None) element by element."""
+        split = index_ir._axis_pieces(v["exp"], self._root("x").symbol())
+        if split is None:
+            return None
+        low = [(c, m) for c, d, m in split[1] if d == 1]
+        if any(d % lb for c, d, m in split[1] if d != 1) or (low and low != [(1, lb)]):
+            return None
+        if v["indirect"]:
+            return None if not low else (f"{G}igather_row<{v['ctype']}, kVec>({v['var']}, {v['idx']}, xmask, {v['other']}, nvalid, "
+                                         f"{', '.join(v['indirect'])})")
+        if not low:
+            return f"{G}ld_uniform({v['var']}, {G}lane0({v['idx']}), nvalid > 0, {v['other']})"
+        return f"{G}ldvec<{v['ctype']}, kVec, false>(({v['var']}) + {G}lane0({v['idx']}), nvalid)"
+
     def _smem_tile(self):
         """(LB, dC, LC, vectors of an output row to a block, columns to a block at most, stride of each tile
         load along the flat index) when the group is transposed by way of shared memory
@@ -1555,9 +1606,14 @@ class B200Kernel(SIMDKernel):
                 kc = self._register_tile(order)
                 smem = self._smem_tile()
                 tile_loads = getattr(self, "_tile_loads", {})
+                tiled = kc is not None or smem is not None
+                odd = None if tiled else self._odd_rows()
                 for n, (tag, v) in enumerate(tile_loads.items()):
-                    text = v["gather"] if kc is None and smem is None else f"(STAGED ? {G}take(raw.t{n}, ci) : {v['gather']})"
+                    text = f"(STAGED ? {G}take(raw.t{n}, ci) : {v['gather']})" if tiled else \
+                        (odd and self._row_text(v, odd)) or v["gather"]
                     body_text = body_text.replace(tag, text)
+                for tag, v in getattr(self, "_row_loads", {}).items():
+                    body_text = body_text.replace(tag, (odd and self._row_text(v, odd)) or v["gather"])
                 streams = not self.indirect and (kc is not None or self._moves_bytes(body_text))
                 src.writeline(f"static constexpr bool kStream = {'true' if streams else 'false'};   // a block for every 256 threads' work")
                 if kc is not None:
@@ -1694,6 +1750,8 @@ class B200Kernel(SIMDKernel):
                 targs = "Body"
                 if smem is not None:
                     launcher, targs = "launch_pointwise_smem", f"Body, {smem[0]}, {smem[1]}LL, {smem[2]}, {smem[3]}"
+                elif odd is not None:
+                    launcher, targs = "launch_pointwise_rows", f"Body, {odd}"
                 src.writeline(f"return {G}{launcher}<{targs}>(b, xnumel, stream, "
                               f"{G}pointers_aligned(ptrs, {len([a for a in assigns if 'ptrs[' in a])}));")
         src.writeline("}")

@@ -279,6 +279,15 @@ __device__ __forceinline__ auto igather(const T* p, const I& idx, const M& mask,
   }
 }
 
+// The same for rows off a 16-byte boundary (vectors that end with their row): the run is cut out of the words
+// that cover it, which the lanes beside this one read as well.
+template <class T, int N, class I, class M, class... U>
+__device__ __forceinline__ auto igather_row(const T* p, const I& idx, const M& mask, typename Mem<T>::val other,
+                                            int nvalid, const U&... indirect) {
+  if constexpr (((rank<U>::n == 0) && ...) && rank<I>::n == N) return ldvec<T, N>(p + at(idx, 0), nvalid);
+  else return gather(p, idx, mask, other);
+}
+
 // ---- bounds check of indirect indices (debug builds) ---------------------------------------
 // A module generated with IXB_DEBUG_BOUNDS checks every data-dependent index against the
 // extent it addresses (the reference asserts them on the device,
@@ -340,6 +349,29 @@ __global__ void __launch_bounds__(256) pointwise_gen_kernel(const Body body, con
     else body.template tile<false>(xbase, left >= V ? V : (int)left);
   }
 }
+// ---- rows of odd length ----------------------------------------------------------------------
+// The flat index in rows of LB elements, LB no whole number of vectors: the vectors are those of the flat
+// index, cut at the ends of the rows, so that inside a vector a per-column operand or a gathered row is one run
+// and a per-row operand one value.  Of the two parts of a vector that two rows share each is stored
+// element by element.
+template <class Body, int LB, bool ALIGNED>
+__global__ void __launch_bounds__(256) pointwise_rows_gen_kernel(const Body body, const long long slots) {
+  constexpr int V = Body::kVec, K = (LB + V - 1 + V - 1) / V;  // vectors that a row may touch
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < slots; t += (long long)gridDim.x * blockDim.x) {
+    const unsigned row = (unsigned)t / K, k = (unsigned)t % K;
+    const long long first = (long long)row * LB;
+    int x = (int)k * V - (int)((unsigned)first % V), n = V;
+    if (x < 0) {
+      n += x;
+      x = 0;
+    }
+    if (x + n > LB) n = LB - x;
+    if (n <= 0) continue;
+    if (ALIGNED && n == V) body.template tile<true>(first + x, V);
+    else body.template tile<false>(first + x, n);
+  }
+}
+
 // ---- transposes: a register tile per thread ---------------------------------------------------
 // A pointwise group that stores along the flat index but reads an operand that is contiguous
 // along another digit C of it (a transpose) gives every thread a V x kC micro-tile of that
@@ -496,6 +528,20 @@ __global__ void __launch_bounds__(256) pointwise_smem_gen_kernel(const Body body
 }
 
 template <class Body> int launch_pointwise(const Body& body, long long xnumel, void* stream, bool aligned);
+template <class Body, int LB> int launch_pointwise_rows(const Body& body, long long xnumel, void* stream, bool aligned) {
+  if (xnumel <= 0) return 0;
+  const long long slots = xnumel / LB * ((LB + 2 * (Body::kVec - 1)) / Body::kVec);
+  if (slots > 0x7fffffffLL) return (int)cudaErrorInvalidValue;  // (the generator keeps the index below 2^31, and rows past a vector)
+  static const long long cap_a = Body::kStream ? 0 : resident_ctas(pointwise_rows_gen_kernel<Body, LB, true>, 256);
+  static const long long cap_u = Body::kStream ? 0 : resident_ctas(pointwise_rows_gen_kernel<Body, LB, false>, 256);
+  const long long grid = stream_grid<Body>(slots, aligned ? cap_a : cap_u);
+  if (aligned) pointwise_rows_gen_kernel<Body, LB, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, slots);
+  else pointwise_rows_gen_kernel<Body, LB, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, slots);
+  return (int)cudaGetLastError();
+}
+// Per-element gathers -> by way of shared memory: 200 x 1000 x 1000 fp16 775 -> 122 us (the floor of its bytes),
+// 300 x 701 x 333 fp32 345 -> 88 (86), 500 x 511 x 513 bf16 472 -> 138 (80: rows off a boundary on both sides),
+// 3000 x 100 x 100 fp16 118 -> 39 (18: a fifth of the rows' last vectors are parts), 2000 x 64 x 65 29 -> 10.6 (5).
 template <class Body, int LB, long long DC, int LC, int NK>
 int launch_pointwise_smem(const Body& body, long long xnumel, void* stream, bool aligned) {
   if (xnumel <= 0) return 0;
