@@ -639,6 +639,24 @@ template <int K> __device__ __forceinline__ void warp_sum(float (&v)[K]) {
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(kFull, v[k], o);
 }
+// Two or three sums of a warp: lanes 0, 8 and 16 hold them.  Each step that halves the lanes a value is
+// spread over halves the values as well: six shuffles in place of ten or fifteen.
+__device__ __forceinline__ float warp_sum_split(float a, float b, float c) {
+  const int lane = threadIdx.x & 31;
+  // lanes of the upper half go on with c (and nothing beside it), the others with a and b
+  const bool up = lane & 16;
+  const float other = __shfl_xor_sync(kFull, up ? a : c, 16);
+  const float a1 = (up ? c : a) + other;
+  const float b1 = b + __shfl_xor_sync(kFull, b, 16);   // (of use to the lower half alone)
+  const bool odd = lane & 8;
+  const float send = odd ? a1 : (up ? a1 : b1);
+  const float got = __shfl_xor_sync(kFull, send, 8);
+  float t = (up ? a1 : (odd ? b1 : a1)) + got;
+  t += __shfl_xor_sync(kFull, t, 4);
+  t += __shfl_xor_sync(kFull, t, 2);
+  t += __shfl_xor_sync(kFull, t, 1);
+  return t;
+}
 // NaN-propagating maximum / minimum of a warp in one instruction
 __device__ __forceinline__ float warp_max_nan(float v) {
   float r;
@@ -1016,6 +1034,10 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   // Partial results cross warps through one 16-byte slot per warp; after the team barrier
   // lane l of every warp reads the slot of warp l mod kW and a shuffle tree over kW lanes
   // folds them, so the cost per thread does not grow with the number of warps in the team.
+  // In teams of four warps every thread reads all the slots instead, which saves two rounds of shuffles (and
+  // the three sums of a warp are folded together, warp_sum_split): softmax -> LayerNorm of 16384 x 4096 bf16
+  // 59.2 -> 56.5 us.  Two warps: no difference (20011 x 1537 fp16 46.9, 47.1); 8 and 16: 1 to 3 % slower (rows
+  // of 4096 fp32 44.3, 45.4; 2238 x 7081 fp16 35.2, 36.3).
   __device__ __forceinline__ float* slot_base() { return this->red + this->phase * kW * 4; }
   template <class Op> __device__ __forceinline__ float xreduce(float v) {
     if constexpr (TEAM < 32) {
@@ -1024,38 +1046,22 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       v = warp_all<Op>(v);
       if constexpr (kW > 1) {
         float* slot = slot_base();
-        if ((this->lane & 31) == 0) slot[(this->lane >> 5) * 4] = v;
-        team_barrier(this->team + 1, TEAM);
-        v = slot[(this->lane & (kW - 1)) * 4];
-        v = lane_group_reduce<Op, kW>(v);
+        if constexpr (kW == 4) {
+          if ((this->lane & 31) == 0) slot[this->lane >> 5] = v;
+          team_barrier(this->team + 1, TEAM);
+          const float4 q = *reinterpret_cast<const float4*>(slot);
+          v = Op::combine(Op::combine(q.x, q.z), Op::combine(q.y, q.w));
+        } else {
+          if ((this->lane & 31) == 0) slot[(this->lane >> 5) * 4] = v;
+          team_barrier(this->team + 1, TEAM);
+          v = slot[(this->lane & (kW - 1)) * 4];
+          v = lane_group_reduce<Op, kW>(v);
+        }
         this->phase ^= 1;
       }
       return v;
     }
   }
-  // K sums with one barrier (K <= 4)
-  template <int K> __device__ __forceinline__ void xsum(float (&v)[K]) {
-    static_assert(K <= 4, "a slot holds four floats");
-    if constexpr (TEAM < 32) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) v[k] = lane_group_reduce<SumOp, TEAM>(v[k]);
-    } else {
-      warp_sum<K>(v);
-      if constexpr (kW > 1) {
-        float* slot = slot_base();
-        if ((this->lane & 31) == 0) {
-#pragma unroll
-          for (int k = 0; k < K; ++k) slot[(this->lane >> 5) * 4 + k] = v[k];
-        }
-        team_barrier(this->team + 1, TEAM);
-        const float* mine = slot + (this->lane & (kW - 1)) * 4;
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = lane_group_reduce<SumOp, kW>(mine[k]);
-        this->phase ^= 1;
-      }
-    }
-  }
-
   // ---- inclusive prefix scan along the row (cumsum / cumprod over the stride-1 axis) -----------
   // Row order: vector i of thread t is vector i * TEAM + t of the row.  Per round i every
   // thread scans its own vector, the vector totals are scanned over the team in thread order
@@ -1456,9 +1462,40 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       r = (m == -INFINITY) ? 0.f : fast_exp2((m - mw) * kLog2e);
 #pragma unroll
       for (int k = 0; k < 1 + NS; ++k) v[k] *= r;
-      warp_sum<1 + NS + NP>(v);
       m = mw;
-      if constexpr (kW > 1) {
+      if constexpr (kW == 1) {
+        warp_sum<1 + NS + NP>(v);
+      } else if constexpr (kW == 4) {
+        float* slot = slot_base() + (this->lane >> 5) * 4;
+        if constexpr (1 + NS + NP == 1) {
+          warp_sum<1>(v);
+          if ((this->lane & 31) == 0) *reinterpret_cast<float2*>(slot) = make_float2(mw, v[0]);
+        } else {
+          // lane 8 k holds sum k
+          const float t = warp_sum_split(v[0], v[1], 1 + NS + NP > 2 ? v[NS + NP] : 0.f);
+          if ((this->lane & 7) == 0) slot[((this->lane >> 3) + 1) & 3] = (this->lane & 31) == 24 ? mw : t;
+        }
+        team_barrier(this->team + 1, TEAM);
+        float4 part[kW];
+#pragma unroll
+        for (int w = 0; w < kW; ++w) part[w] = *reinterpret_cast<const float4*>(slot_base() + w * 4);
+        const float mm = max3(fmaxf(part[0].x, part[1].x), part[2].x, part[3].x);
+        const float base = mm == -INFINITY ? 0.f : mm;
+        v[0] = 0.f;
+        if constexpr (NS + NP > 0) v[1] = 0.f;
+        if constexpr (NS + NP > 1) v[2] = 0.f;
+#pragma unroll
+        for (int w = 0; w < kW; ++w) {
+          const float f = fast_exp2((part[w].x - base) * kLog2e);
+          const float pv[3] = {part[w].y, part[w].z, part[w].w};
+#pragma unroll
+          for (int k = 0; k < 1 + NS + NP; ++k) v[k] = k < 1 + NS ? fmaf(pv[k], f, v[k]) : v[k] + pv[k];
+        }
+        r *= fast_exp2((mw - base) * kLog2e);
+        m = mm;
+        this->phase ^= 1;
+      } else {
+        warp_sum<1 + NS + NP>(v);
         float* slot = slot_base();
         if ((this->lane & 31) == 0) {
           float4 s4 = make_float4(mw, v[0], 0.f, 0.f);
