@@ -42,6 +42,7 @@
 // (1000 keys 130, 131, 134 against 129, 4096 causal keys 973 - 1009, 1020 - 1038, 1093 against 985 - 1006:
 // power, not the ex2 unit, is the limit there).
 #include <atomic>
+#include <cmath>
 #include "host.h"
 #include "fa_maps.h"
 #include "ixb/fa_softmax.cuh"
@@ -434,10 +435,15 @@ extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v
   p.wide = ixb_host::rows_aligned32(o, o_strides) ? 1 : 0;
   // Without a mask every query block of a head reads all of its K and V, so the heads go one
   // after the other (group of 1: blockIdx order = head-major, as a 2-D grid would give).
-  // Under a causal mask 8 heads run together (measured at 4096 keys: 1, 8, 16 heads within 1 %
-  // of each other, 64 and more slower - their K and V no longer stay in L2).
+  // Under a causal mask heads run in groups, the long query blocks of all of them first: what a group's
+  // long blocks find of K and V in L2 against the SMs that wait for the last group's long blocks at the end.
+  // One group where the K and V of all heads stay in L2, else equal groups of about 40 MB.  Groups of
+  // 8 heads -> this: 1 x 32 heads of 2048 keys 60 -> 49 us, 2 x 32 87 -> 73, 2 x 16 of 4096 179 -> 145,
+  // 3 x 12 of 5014 295 -> 240, 2 x 8 of 8192 315 -> 272, 4 x 32 of 2048 145 -> 138, 8 x 32 of 4096 995 -> 960.
   static const int group_env = [] { const char* v = getenv("IXB_FA_HEAD_GROUP"); return v != nullptr ? atoi(v) : 0; }();
-  p.head_group = group_env > 0 ? group_env : (causal ? 8 : 1);
+  const double all = (double)B * H, mb = Sk * (2. * HD * 2 / (1 << 20));  // heads, and MB of K and V of each
+  const double groups = all * mb <= 96 ? 1 : ceil(all / (mb < 5 ? floor(40 / mb) : 8));
+  p.head_group = group_env > 0 ? group_env : (causal ? (int)ceil(all / groups) : 1);
   if (!(scale > 0.f)) return IXB_ERR_ARG;  // the row maximum is taken before scaling
   if (const int cluster = ixb_host::fa_split_size(B, H, Sq, Sk))
     return ixb_host::fa_split(cluster, is_bf16, mq, mk, mv, o, lse, B, H, Sq, Sk, o_strides, scale, causal, status, (cudaStream_t)stream);
