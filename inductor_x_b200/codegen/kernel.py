@@ -1327,6 +1327,8 @@ class B200Kernel(SIMDKernel):
             if v.get("online") and not outer:
                 rs, rp = v["riders_s"], v["riders_p"]
                 computed = "" if self.zero_past_end.issuperset(rs) else ", true"
+                if not self.zero_past_end.issuperset(rp):
+                    computed = (computed or ", false") + ", true"
                 v["row"] = (f"c.template online_softmax<{len(rs)}, {len(rp)}{computed}>({v['value']}, "
                             f"{G}refs<kN>({', '.join(rs)}), {G}refs<kN>({', '.join(rp)}))")
             text = text.replace(tag, v["outer"] if outer else v["row"])

@@ -757,11 +757,16 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   __device__ __forceinline__ bool leader() const { return this->lane == 0 && live; }
   // element j of vector i lies inside the row
   __device__ __forceinline__ bool inside(int i, int j) const {
+    // (one test with a constant each, where the length is one: the first vector of a row off a boundary can only
+    // begin before it and the others only end behind it, a row of whole vectors ends with one)
+    if constexpr (SHIFT && COLS >= TEAM * Base::kVec) return full(i) || (i == 0 ? this->vec_col(0) >= -j : this->vec_col(i) < COLS - j);
+    if constexpr (!SHIFT && COLS > 0 && COLS % Base::kVec == 0) return full(i) || this->vec_col(i) < COLS;
     if constexpr (SHIFT) return full(i) || (unsigned)(this->vec_col(i) + j) < (unsigned)ncols();
     return full(i) || this->vec_col(i) + j < ncols();
   }
   // vector i may hold elements that are not the row's
   __device__ __forceinline__ bool cut(int i) const {
+    if constexpr (SHIFT && COLS >= TEAM * Base::kVec) return !full(i) && (i == 0 ? this->vec_col(0) < 0 : this->vec_col(i) > COLS - Base::kVec);
     return !full(i) && ((SHIFT && this->vec_col(i) < 0) || this->vec_col(i) + Base::kVec > ncols());
   }
   __device__ __forceinline__ vi<kE> rindex() const {
@@ -972,6 +977,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       for (int i = 0; i < VPT; ++i) {
         const int c0 = this->vec_col(i);
         if (SHIFT && cut(i)) {
+          if (c0 >= ncols()) continue;
 #pragma unroll
           for (int j = 0; j < Base::kVec; ++j)
             if (inside(i, j)) Mem<U>::st(rowp + c0 + j, val.v[i * Base::kVec + j]);
@@ -1186,8 +1192,9 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
     for (int c = 1; c < kChains; ++c) acc[0] = add2(acc[0], acc[c]);
     return acc[0].x + acc[0].y;
   }
-  template <class A> __device__ __forceinline__ float local_sum(const A& val) const {
-    if constexpr (FULL && op::is_fvec<A>::value) {
+  // ZEROS: what lies past the end of the row is zero in `val`
+  template <bool ZEROS = false, class A> __device__ __forceinline__ float local_sum(const A& val) const {
+    if constexpr ((FULL || (ZEROS && COLS > 0)) && op::is_fvec<A>::value) {
       // kChains independent chains of packed adds: a single chain would serialise on the
       // add latency with only a few warps resident
       float2 acc[kChains];
@@ -1388,7 +1395,8 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
   };
   // COMPUTED: some w is not a plain operand, which is zero past the end of the row, but computed from
   // such zeros, and may be infinite or NaN there; no zero exponential removes that, so it is masked.
-  template <int NS, int NP, bool COMPUTED = false, class A>
+  // PLAIN: the same of the vectors of the plain sums; operands' sums need no test.
+  template <int NS, int NP, bool COMPUTED = false, bool PLAIN = false, class A>
   __device__ __forceinline__ Online<NS, NP> online_softmax(const A& val, const VecRefs<kE, NS>& w,
                                                             const VecRefs<kE, NP>& pl) {
     static_assert(NS + NP <= 2, "a slot holds the maximum, the sum and two riders");
@@ -1445,7 +1453,7 @@ struct GenRowCtx : RowCtx<T, TEAM, TEAMS, VPT, false> {
       v[k] = acc[k][0].x + acc[k][0].y;
     }
 #pragma unroll
-    for (int k = 0; k < NP; ++k) v[1 + NS + k] = local_sum(*pl.p[k]);
+    for (int k = 0; k < NP; ++k) v[1 + NS + k] = local_sum<!PLAIN>(*pl.p[k]);
 
     // warp stage: agree on the warp's maximum, rescale, sum
     float r;
