@@ -12,7 +12,9 @@
 //                        queries), so that P^T and dS^T - written back over S^T and dP^T as
 //                        16-bit values - are the TMEM operands of dV += P^T dO and
 //                        dK += dS^T Q, which stay in TMEM until the tile is finished.  With
-//                        scratch, four warps copy the 16-bit dS^T to memory
+//                        scratch, four warps copy the 16-bit dS^T to memory.  A CTA that has finished
+//                        takes over a pending tile (cluster launch control): its K, V and first Q and dO
+//                        arrive, and its first scores are formed, under the end of the one before
 //   fa_bwd_dq_ds_kernel  one CTA owns two query tiles: dQ += dS K, with dS from memory
 //   fa_bwd_dq_kernel     the same without scratch: S = Q K^T, dP = dO V^T (thread <-> query),
 //                        dS over dP, dQ += dS K - the probabilities are computed once more, seven
@@ -34,7 +36,10 @@
 // tensor core works 2048.  What shortened it: P handed over group by group, Q and dO in rings of
 // their own whose copies are asked for before anything else, the statistics of a tile read ahead into
 // registers (with both operands in shared memory a product takes all 128 bytes a cycle of it, and
-// reads beside it are slow).  Two tiles in flight would need more tensor memory than one SM has.
+// reads beside it are slow).  A tile took 13000 cycles besides its steps while each had a CTA of its own
+// (the launch, tensor memory, the first copies, the results): calls in which tiles are taken over, before and
+// after: 4 x 32 heads of 4096 causal 1590 and 1500 us, 10 x 16 of 1851 525 and 483, 8 x 32 of 1000 326 and 284,
+// 8 x 16 of 1000 without a mask 246 and 226, 8 x 32 of 196 70 and 61.  Two tiles in flight would need more tensor memory than one SM has.
 // Built, measured and dropped: a share of the exponentials on the fma pipe (1049 - 1070 against 1000:
 // the ex2 unit is not the limit, power is); sixteen element-wise warps (the same); dS to memory by way
 // of shared memory and bulk copies (171 against 162 for the 8 heads) or stored by the element-wise
@@ -152,10 +157,10 @@ __global__ void __launch_bounds__(256)
 // --------------------------------------------------------------------- shared pieces
 // CTA order: heads in groups of `head_group` (their operands stay in L2 while the group
 // runs); inside a group tile `slot` of every head before tile `slot + 1` of any.
-__device__ __forceinline__ void cta_order(int n_tiles, int n_bh, int head_group, int* slot, int* bh) {
+__device__ __forceinline__ void cta_order(int index, int n_tiles, int n_bh, int head_group, int* slot, int* bh) {
   const int per_group = n_tiles * head_group;
-  const int group = (int)blockIdx.x / per_group;
-  const int in_group = (int)blockIdx.x - group * per_group;
+  const int group = index / per_group;
+  const int in_group = index - group * per_group;
   const int left = n_bh - group * head_group;
   const int g_heads = left < head_group ? left : head_group;
   *slot = in_group / g_heads;
@@ -216,8 +221,9 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
   unsigned char* q_smem = smem + 2 * kTileBytes;   // kStages tiles
   unsigned char* do_smem = smem + 4 * kTileBytes;  // kStages tiles
 
-  __shared__ __align__(8) uint64_t kv_full, q_full[kStages], q_empty[kStages], do_full[kStages], do_empty[kStages],
-      s_full, dp_full, p_full[NG], ds_full, ds_read, acc_done, drained;
+  __shared__ __align__(16) uint4 next_answer[2];
+  __shared__ __align__(8) uint64_t next_wanted, next_full[2], next_taken[2], kv_full, kv_empty, q_full[kStages], q_empty[kStages],
+      do_full[kStages], do_empty[kStages], s_full, dp_full, p_full[NG], ds_full, ds_read, acc_done, acc_empty, drained;
   // of a query tile: -lse in log2 units (-inf past the end: P = 0) and -delta
   __shared__ __align__(16) float nlse_s[kStages][BM], ndelta_s[kStages][BM];
   __shared__ uint32_t tmem_base_slot;
@@ -228,24 +234,39 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
 
   const int n_kv_tiles = (p.Sk + BN - 1) / BN;
   const int n_q_tiles = (p.Sq + BM - 1) / BM;
-  int kv_tile, bh;
-  cta_order(n_kv_tiles, p.n_bh, p.head_group, &kv_tile, &bh);  // early key tiles see the most queries
   const int hide = hidden_tiles(p.causal, p.Sq, p.Sk, n_kv_tiles);
-  unsigned char* ds_head = p.ds + (long long)bh * p.tiles_per_head * kTileBytes;
   const bool keep_ds = p.ds != nullptr;
-  bh += p.bh0;
-  const int b = bh / p.H, h = bh % p.H;
-  const int kt0 = kv_tile * BN;
   const int diag = p.Sk - p.Sq;  // key j is visible to query i when j <= i + diag
-  int i0 = 0;
-  if (p.causal) {
-    const int first = kt0 - diag;  // first query that sees the first key of the tile
-    i0 = first > 0 ? first / BM : 0;
-  }
-  const int n_it = n_q_tiles > i0 ? n_q_tiles - i0 : 0;
+  // a work item: a key tile of a (batch, head) and the query tiles that see it
+  struct Item {
+    int kt0, i0, n_it, bh, b, h, kv_tile;
+    unsigned char* ds_head;
+  };
+  auto item_of = [&](int index) {
+    Item w;
+    cta_order(index, n_kv_tiles, p.n_bh, p.head_group, &w.kv_tile, &w.bh);  // early key tiles see the most queries
+    w.ds_head = p.ds + (long long)w.bh * p.tiles_per_head * kTileBytes;
+    w.bh += p.bh0;
+    w.b = w.bh / p.H;
+    w.h = w.bh % p.H;
+    w.kt0 = w.kv_tile * BN;
+    w.i0 = 0;
+    if (p.causal) {
+      const int first = w.kt0 - diag;  // first query that sees the first key of the tile
+      w.i0 = first > 0 ? first / BM : 0;
+    }
+    w.n_it = n_q_tiles > w.i0 ? n_q_tiles - w.i0 : 0;  // (a key tile that no query sees is no item of any role's)
+    return w;
+  };
 
   if (threadIdx.x == 0) {
+    mbar_init(&next_wanted, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&next_full[s], 1);
+      mbar_init(&next_taken[s], 2 + kWorkers / 32 + 4);  // producer, issuer, element-wise and storing warps
+    }
     mbar_init(&kv_full, 1);
+    mbar_init(&kv_empty, 1);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&q_full[s], 2);  // the copy and the statistics
       mbar_init(&q_empty[s], 1);
@@ -258,6 +279,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
     mbar_init(&ds_full, kWorkers / 32);
     mbar_init(&ds_read, 4);
     mbar_init(&acc_done, 1);
+    mbar_init(&acc_empty, kWorkers / 32);
     mbar_init(&drained, 1);
     failed = 0;
     mbar_init_fence();
@@ -268,119 +290,162 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
 
-  int q_loads = 0, do_loads = 0;  // producer: query tiles it has asked for
+  // The item after item n of this block: answer n of the scheduler warp.  Taken by a whole warp.
+  auto take_next = [&](int n, bool& ok) {
+    ok = ok && __all_sync(kFull, mbar_wait(&next_full[n & 1], (n >> 1) & 1, &failed));
+    if (!ok) return -1;
+    const int index = __shfl_sync(kFull, tc::next_block(&next_answer[n & 1]), 0);
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&next_taken[n & 1]);
+    return index;
+  };
+
+  int kv_loads = 0, q_loads = 0, do_loads = 0;  // producer: items and query tiles it has asked for
+  int asked = 0;                                // scheduler: the same
   if (warp < 4) tc::regs_dec<kRegsIssue>();
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0 && n_it > 0) {
-      mbar_arrive_expect_tx(&kv_full, 2 * kTileBytes);
-      load_tile(k_smem, &map_k, &kv_full, kt0, h, b);
-      load_tile(v_smem, &map_v, &kv_full, kt0, h, b);
-    }
-    // the statistics of a tile are read a tile ahead, so that nothing waits for that read
-    float lse_r[4], delta_r[4];
-    auto read_stats = [&](int qt0) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int qi = qt0 + e * 32 + lane;
-        const long long at = (long long)bh * p.Sq + qi;
-        lse_r[e] = qi < p.Sq ? p.lse[at] * -kLog2e : -INFINITY;
-        delta_r[e] = qi < p.Sq ? -p.delta[at] : 0.f;
-      }
-    };
-    read_stats(i0 * BM);
     bool ok = true;
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int s = it % kStages, n = it / kStages;
-      const int qt0 = (i0 + it) * BM;
-      if (n > 0) ok = __all_sync(kFull, mbar_wait(&q_empty[s], (n - 1) & 1, &failed));
-      if (!ok) break;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&q_full[s], kTileBytes);
-        load_tile(q_smem + (size_t)s * kTileBytes, &map_q, &q_full[s], qt0, h, b);
+    int step = 0;  // query tiles asked for, over all items
+    for (int n = 0, index = blockIdx.x; index >= 0 && ok; ++n) {
+      const Item w = item_of(index);
+      if (w.n_it > 0) {
+        if (kv_loads > 0) ok = __all_sync(kFull, mbar_wait(&kv_empty, (kv_loads - 1) & 1, &failed));
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&kv_full, 2 * kTileBytes);
+          load_tile(k_smem, &map_k, &kv_full, w.kt0, w.h, w.b);
+          load_tile(v_smem, &map_v, &kv_full, w.kt0, w.h, w.b);
+        }
+        ++kv_loads;
       }
+      // the statistics of a tile are read a tile ahead, so that nothing waits for that read
+      float lse_r[4], delta_r[4];
+      auto read_stats = [&](int qt0) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        nlse_s[s][e * 32 + lane] = lse_r[e];
-        ndelta_s[s][e * 32 + lane] = delta_r[e];
+        for (int e = 0; e < 4; ++e) {
+          const int qi = qt0 + e * 32 + lane;
+          const long long at = (long long)w.bh * p.Sq + qi;
+          lse_r[e] = qi < p.Sq ? p.lse[at] * -kLog2e : -INFINITY;
+          delta_r[e] = qi < p.Sq ? -p.delta[at] : 0.f;
+        }
+      };
+      read_stats(w.i0 * BM);
+      for (int it = 0; it < w.n_it && ok; ++it, ++step) {
+        const int s = step % kStages, u = step / kStages;
+        const int qt0 = (w.i0 + it) * BM;
+        if (u > 0) ok = __all_sync(kFull, mbar_wait(&q_empty[s], (u - 1) & 1, &failed));
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&q_full[s], kTileBytes);
+          load_tile(q_smem + (size_t)s * kTileBytes, &map_q, &q_full[s], qt0, w.h, w.b);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          nlse_s[s][e * 32 + lane] = lse_r[e];
+          ndelta_s[s][e * 32 + lane] = delta_r[e];
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&q_full[s]);
+        q_loads = step + 1;
+        if (it + 1 < w.n_it) read_stats(qt0 + BM);
+        if (u > 0) ok = __all_sync(kFull, mbar_wait(&do_empty[s], (u - 1) & 1, &failed));
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&do_full[s], kTileBytes);
+          load_tile(do_smem + (size_t)s * kTileBytes, &map_do, &do_full[s], qt0, w.h, w.b);
+        }
+        do_loads = step + 1;
       }
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&q_full[s]);
-      q_loads = it + 1;
-      if (it + 1 < n_it) read_stats(qt0 + BM);
-      if (n > 0) ok = __all_sync(kFull, mbar_wait(&do_empty[s], (n - 1) & 1, &failed));
-      if (!ok) break;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&do_full[s], kTileBytes);
-        load_tile(do_smem + (size_t)s * kTileBytes, &map_do, &do_full[s], qt0, h, b);
-      }
-      do_loads = it + 1;
+      if (lane == 0) tc::mbar_arrive(&next_wanted);
+      index = take_next(n, ok);
     }
     if (!ok && lane == 0) failed = 1;
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (n_it > 0) {
-      constexpr uint32_t idesc_kk = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 0);
-      constexpr uint32_t idesc_mn = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 1);
-      const uint64_t k_desc = tc::smem_desc(smem_u32(k_smem), 16, 1024);
-      const uint64_t v_desc = tc::smem_desc(smem_u32(v_smem), 16, 1024);
-      const uint64_t q_desc = tc::smem_desc(smem_u32(q_smem), 16, 1024);
-      const uint64_t do_desc = tc::smem_desc(smem_u32(do_smem), 16, 1024);
-      const uint64_t q_desc_mn = tc::smem_desc(smem_u32(q_smem), kHalfBytes, 1024);
-      const uint64_t do_desc_mn = tc::smem_desc(smem_u32(do_smem), kHalfBytes, 1024);
-      constexpr uint32_t kStep = kTileBytes >> 4;  // one stage further, in descriptor units
-      const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
-      const uint32_t t_s = tmem + kColS, t_dp = tmem + kColDP;
-      const uint32_t t_dv = tmem + kColAcc0, t_dk = tmem + kColAcc1;
-      auto wait = [&](uint64_t* bar, int parity) {
-        const bool up = __all_sync(kFull, mbar_wait(bar, parity, &failed));
-        tc::fence_after_sync();
-        return up;
-      };
-      bool ok = wait(&kv_full, 0) && wait(&q_full[0], 0);
-      if (ok) {
-        issue_ss(t_s, k_desc, q_desc, idesc_kk);  // S^T = K Q^T
+    constexpr uint32_t idesc_kk = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 0);
+    constexpr uint32_t idesc_mn = tc::instr_desc(128, 128, IS_BF16 ? 1 : 0, 0, 1);
+    const uint64_t k_desc = tc::smem_desc(smem_u32(k_smem), 16, 1024);
+    const uint64_t v_desc = tc::smem_desc(smem_u32(v_smem), 16, 1024);
+    const uint64_t q_desc = tc::smem_desc(smem_u32(q_smem), 16, 1024);
+    const uint64_t do_desc = tc::smem_desc(smem_u32(do_smem), 16, 1024);
+    const uint64_t q_desc_mn = tc::smem_desc(smem_u32(q_smem), kHalfBytes, 1024);
+    const uint64_t do_desc_mn = tc::smem_desc(smem_u32(do_smem), kHalfBytes, 1024);
+    constexpr uint32_t kStep = kTileBytes >> 4;  // one stage further, in descriptor units
+    const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
+    const uint32_t t_s = tmem + kColS, t_dp = tmem + kColDP;
+    const uint32_t t_dv = tmem + kColAcc0, t_dk = tmem + kColAcc1;
+    auto wait = [&](uint64_t* bar, int parity) {
+      const bool up = __all_sync(kFull, mbar_wait(bar, parity, &failed));
+      tc::fence_after_sync();
+      return up;
+    };
+    bool ok = true;
+    int step = 0, items = 0;  // query tiles and items worked on so far
+    for (int n = 0, index = blockIdx.x; index >= 0 && ok; ++n) {
+      const Item w = item_of(index);
+      // S^T = K Q^T and dP^T = V dO^T of query tile `at` (over all items); the last of an item free K and V
+      auto scores = [&](int at) {
+        const int s = at & 1;
+        if (!wait(&q_full[s], (at >> 1) & 1)) return false;
+        // (the tensor core runs its MMAs in order: P^T of the tile before has been consumed when this one starts)
+        issue_ss(t_s, k_desc, q_desc + s * kStep, idesc_kk);
         tc::commit_elected(&s_full);
-        ok = wait(&do_full[0], 0);
-      }
-      if (ok) {
-        issue_ss(t_dp, v_desc, do_desc, idesc_kk);  // dP^T = V dO^T
+        return true;
+      };
+      auto score_gradients = [&](int at, bool last) {
+        const int s = at & 1;
+        if (!wait(&do_full[s], (at >> 1) & 1) || (keep_ds && at > 0 && !wait(&ds_read, (at - 1) & 1))) return false;
+        issue_ss(t_dp, v_desc, do_desc + s * kStep, idesc_kk);
         tc::commit_elected(&dp_full);
-      }
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it & 1, s1 = (it + 1) & 1, n1 = (it + 1) >> 1;
-        const bool next = it + 1 < n_it;
-        // dV += P^T dO in two parts: of the two groups, which share the ex2 unit, one is ahead
-        ok = wait(&p_full[0], it & 1);
-        if (!ok) break;
-        issue_ts_group<0>(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, it > 0);
-        ok = wait(&p_full[1], it & 1);
-        if (!ok) break;
-        issue_ts_group<1>(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, true);
-        tc::commit_elected(&do_empty[s]);
-        if (next) {
-          ok = wait(&q_full[s1], n1 & 1);
+        if (last) tc::commit_elected(&kv_empty);
+        return true;
+      };
+      if (w.n_it > 0) {
+        ok = wait(&kv_full, items & 1) && scores(step) && score_gradients(step, w.n_it == 1);
+        for (int it = 0; it < w.n_it && ok; ++it, ++step) {
+          const int s = step & 1;
+          const bool next = it + 1 < w.n_it;
+          // dV += P^T dO in two parts: of the two groups, which share the ex2 unit, one is ahead; the first product
+          // of an item waits until the results of the one before have left the accumulators
+          ok = (it > 0 || items == 0 || wait(&acc_empty, (items - 1) & 1)) && wait(&p_full[0], step & 1);
           if (!ok) break;
-          // the tensor core runs its MMAs in order: P^T has been consumed when this one starts
-          issue_ss(t_s, k_desc, q_desc + s1 * kStep, idesc_kk);
-          tc::commit_elected(&s_full);
-        }
-        ok = wait(&ds_full, it & 1);
-        if (!ok) break;
-        issue_ts(t_dk, t_dp, q_desc_mn + s * kStep, idesc_mn, it > 0);  // dK += dS^T Q
-        tc::commit_elected(&q_empty[s]);
-        if (next) {
-          ok = wait(&do_full[s1], n1 & 1) && (!keep_ds || wait(&ds_read, it & 1));
+          issue_ts_group<0>(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, it > 0);
+          ok = wait(&p_full[1], step & 1);
           if (!ok) break;
-          issue_ss(t_dp, v_desc, do_desc + s1 * kStep, idesc_kk);
-          tc::commit_elected(&dp_full);
+          issue_ts_group<1>(t_dv, t_s, do_desc_mn + s * kStep, idesc_mn, true);
+          tc::commit_elected(&do_empty[s]);
+          if (next) ok = scores(step + 1);
+          ok = ok && wait(&ds_full, step & 1);
+          if (!ok) break;
+          issue_ts(t_dk, t_dp, q_desc_mn + s * kStep, idesc_mn, it > 0);  // dK += dS^T Q
+          tc::commit_elected(&q_empty[s]);
+          if (next) ok = score_gradients(step + 1, it + 2 == w.n_it);
         }
+        if (ok) tc::commit_elected(&acc_done);
+        ++items;
       }
-      if (ok) tc::commit_elected(&acc_done);
-      if (!ok && lane == 0) failed = 1;
+      index = take_next(n, ok);
     }
+    if (!ok && lane == 0) failed = 1;
     __syncwarp();
+  } else if (warp == 2) {
+    // ------------------------------------------------------------------ scheduler
+    // Asked for when the last copies of an item are under way, two steps before its end: soon enough for its K
+    // and V, and not before - a block that asked at the start of a long item would keep a pending one from
+    // those that finish first (2 x 16 heads of 583 causal keys 41.5 us so).
+    bool ok = true;
+    for (int n = 0; ok; ++n) {
+      ok = __all_sync(kFull, mbar_wait(&next_wanted, n & 1, &failed));
+      if (ok && n > 0) ok = __all_sync(kFull, mbar_wait(&next_taken[(n - 1) & 1], ((n - 1) >> 1) & 1, &failed));
+      if (!ok) break;
+      if (lane == 0) tc::request_next_block(&next_answer[n & 1], &next_full[n & 1]);
+      asked = n + 1;
+      ok = __all_sync(kFull, mbar_wait(&next_full[n & 1], (n >> 1) & 1, &failed));
+      if (!ok || __shfl_sync(kFull, tc::next_block(&next_answer[n & 1]), 0) < 0) break;
+    }
+    if (!ok && lane == 0) failed = 1;
   } else if (warp >= 4 + 4 * NG) {
     tc::regs_dec<kRegsStore>();
     // ------------------------------------------------------------------ dS to memory
@@ -390,23 +455,28 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
     const int quad = warp & 3;
     const uint32_t dp_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + kColDP;
     bool ok = true;
-    for (int it = 0; it < n_it && keep_ds; ++it) {
-      ok = __all_sync(kFull, mbar_wait(&ds_full, it & 1, &failed));
-      if (!ok) break;
-      tc::fence_after_sync();
-      uint32_t d[NG][GC / 2];
+    int step = 0;
+    for (int n = 0, index = blockIdx.x; index >= 0 && ok; ++n) {
+      const Item w = item_of(index);
+      for (int it = 0; it < w.n_it && keep_ds; ++it, ++step) {
+        ok = __all_sync(kFull, mbar_wait(&ds_full, step & 1, &failed));
+        if (!ok) break;
+        tc::fence_after_sync();
+        uint32_t d[NG][GC / 2];
 #pragma unroll
-      for (int g = 0; g < NG; ++g) tc::tmem_ld32(dp_addr + GC * g, d[g]);
-      tc::tmem_wait_ld();
-      tc::fence_before_sync();
-      warp_arrive(&ds_read, lane);
-      uint4* dst = reinterpret_cast<uint4*>(ds_head + ds_tile(kv_tile, i0 + it, n_q_tiles, hide) * kTileBytes) +
-                   quad * (BM / 8) * 32 + lane;
+        for (int g = 0; g < NG; ++g) tc::tmem_ld32(dp_addr + GC * g, d[g]);
+        tc::tmem_wait_ld();
+        tc::fence_before_sync();
+        warp_arrive(&ds_read, lane);
+        uint4* dst = reinterpret_cast<uint4*>(w.ds_head + ds_tile(w.kv_tile, w.i0 + it, n_q_tiles, hide) * kTileBytes) +
+                     quad * (BM / 8) * 32 + lane;
 #pragma unroll
-      for (int u = 0; u < BM / 8; ++u) {
-        const uint32_t* w = &d[u * 8 / GC][(u * 4) % (GC / 2)];
-        __stcs(dst + u * 32, make_uint4(w[0], w[1], w[2], w[3]));
+        for (int u = 0; u < BM / 8; ++u) {
+          const uint32_t* v = &d[u * 8 / GC][(u * 4) % (GC / 2)];
+          __stcs(dst + u * 32, make_uint4(v[0], v[1], v[2], v[3]));
+        }
       }
+      index = take_next(n, ok);
     }
     if (!ok) failed = 1;
   } else if (warp >= 4) {
@@ -415,136 +485,144 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
     const int g = (warp - 4) >> 2;  // group: query columns [GC g, GC g + GC) of a tile
     const int quad = warp & 3;
     const int row = quad * 32 + lane;  // key inside the tile
-    const int kj = kt0 + row;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     const uint32_t s_addr = lane_addr + kColS + GC * g;
     const uint32_t dp_addr = lane_addr + kColDP + GC * g;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
+    int step = 0, items = 0;  // query tiles and items so far
 
-    for (int it = 0; it < n_it; ++it) {
-      const int s = it & 1;
-      const int qt0 = (i0 + it) * BM;
-      // the tile's statistics come into registers ahead of its scores: shared memory is busy with
-      // the products' operands, and every read of it is slow
-      float4 stat[GC / 4];
-      bool w = __all_sync(kFull, mbar_wait(&q_full[s], (it >> 1) & 1, &failed));
-      if (w) {
+    for (int n = 0, index = blockIdx.x; index >= 0 && ok; ++n) {
+      const Item w = item_of(index);
+      const int kt0 = w.kt0, kj = kt0 + row;
+      for (int it = 0; it < w.n_it; ++it, ++step) {
+        const int s = step & 1;
+        const int qt0 = (w.i0 + it) * BM;
+        // the tile's statistics come into registers ahead of its scores: shared memory is busy with
+        // the products' operands, and every read of it is slow
+        float4 stat[GC / 4];
+        bool up = __all_sync(kFull, mbar_wait(&q_full[s], (step >> 1) & 1, &failed));
+        if (up) {
 #pragma unroll
-        for (int e = 0; e < GC / 4; ++e) stat[e] = *reinterpret_cast<const float4*>(&nlse_s[s][GC * g + 4 * e]);
-        w = __all_sync(kFull, mbar_wait(&s_full, it & 1, &failed));
-      }
-      if (!w) {
-        ok = false;
-        break;
-      }
-      tc::fence_after_sync();
-      // query column e of this group is visible to key kj when qt0 + GC g + e >= kj - diag; a row
-      // past the last key has no gradients of its own, but its dS would meet zeros of K in dQ
-      // (and need not be finite)
-      const bool edge = (kt0 + BN > p.Sk) || (p.causal && (kt0 + BN - 1 > qt0 + diag));
-      const int lo = !edge ? 0 : kj >= p.Sk ? GC : p.causal ? kj - diag - (qt0 + GC * g) : 0;
-      uint32_t raw[GC];
+          for (int e = 0; e < GC / 4; ++e) stat[e] = *reinterpret_cast<const float4*>(&nlse_s[s][GC * g + 4 * e]);
+          up = __all_sync(kFull, mbar_wait(&s_full, step & 1, &failed));
+        }
+        if (!up) {
+          ok = false;
+          break;
+        }
+        tc::fence_after_sync();
+        // query column e of this group is visible to key kj when qt0 + GC g + e >= kj - diag; a row
+        // past the last key has no gradients of its own, but its dS would meet zeros of K in dQ
+        // (and need not be finite)
+        const bool edge = (kt0 + BN > p.Sk) || (p.causal && (kt0 + BN - 1 > qt0 + diag));
+        const int lo = !edge ? 0 : kj >= p.Sk ? GC : p.causal ? kj - diag - (qt0 + GC * g) : 0;
+        uint32_t raw[GC];
 #pragma unroll
-      for (int c = 0; c < GC / 32; ++c) tc::tmem_ld32(s_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
-      tc::tmem_wait_ld();
-      float2 pr[GC / 2];
+        for (int c = 0; c < GC / 32; ++c) tc::tmem_ld32(s_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
+        tc::tmem_wait_ld();
+        float2 pr[GC / 2];
 #pragma unroll
-      for (int c = 0; c < GC / 32; ++c) {
-        uint32_t pk[16];
+        for (int c = 0; c < GC / 32; ++c) {
+          uint32_t pk[16];
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          const float4 l4 = stat[c * 8 + e / 4];
-          const float2 l2[2] = {make_float2(l4.x, l4.y), make_float2(l4.z, l4.w)};
+          for (int e = 0; e < 32; e += 4) {
+            const float4 l4 = stat[c * 8 + e / 4];
+            const float2 l2[2] = {make_float2(l4.x, l4.y), make_float2(l4.z, l4.w)};
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int at = c * 32 + e + 2 * u;
-            const float2 a = fma2(make_float2(__uint_as_float(raw[at]), __uint_as_float(raw[at + 1])), sc2, l2[u]);
-            float2 x = make_float2(fast_exp2(a.x), fast_exp2(a.y));
-            if (edge) {
-              if (at < lo) x.x = 0.f;
-              if (at + 1 < lo) x.y = 0.f;
+            for (int u = 0; u < 2; ++u) {
+              const int at = c * 32 + e + 2 * u;
+              const float2 a = fma2(make_float2(__uint_as_float(raw[at]), __uint_as_float(raw[at + 1])), sc2, l2[u]);
+              float2 x = make_float2(fast_exp2(a.x), fast_exp2(a.y));
+              if (edge) {
+                if (at < lo) x.x = 0.f;
+                if (at + 1 < lo) x.y = 0.f;
+              }
+              pr[at / 2] = x;
+              pk[e / 2 + u] = pack_pair(x.x, x.y, IS_BF16);
             }
-            pr[at / 2] = x;
-            pk[e / 2 + u] = pack_pair(x.x, x.y, IS_BF16);
+          }
+          // all of this group's S columns are in registers: P^T goes over their first half
+          tc::tmem_st16(s_addr + c * 16, pk);
+        }
+        tc::tmem_wait_st();
+        tc::fence_before_sync();
+        warp_arrive(&p_full[g], lane);
+#pragma unroll
+        for (int e = 0; e < GC / 4; ++e) stat[e] = *reinterpret_cast<const float4*>(&ndelta_s[s][GC * g + 4 * e]);
+
+        if (!__all_sync(kFull, mbar_wait(&dp_full, step & 1, &failed))) {
+          ok = false;
+          break;
+        }
+        tc::fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < GC / 32; ++c) tc::tmem_ld32(dp_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < GC / 32; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            const float4 d4 = stat[c * 8 + e / 4];
+            const float2 d2[2] = {make_float2(d4.x, d4.y), make_float2(d4.z, d4.w)};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int at = c * 32 + e + 2 * u;
+              const float2 x = mul2(pr[at / 2], add2(make_float2(__uint_as_float(raw[at]), __uint_as_float(raw[at + 1])), d2[u]));
+              pk[e / 2 + u] = pack_pair(x.x, x.y, IS_BF16);
+            }
+          }
+          tc::tmem_st16(dp_addr + c * 16, pk);
+        }
+        tc::tmem_wait_st();
+        tc::fence_before_sync();
+        warp_arrive(&ds_full, lane);
+      }
+
+      if (ok && w.n_it > 0) ok = mbar_wait(&acc_done, items & 1, &failed);
+      ok = __all_sync(kFull, ok);
+      if (ok) {
+        tc::fence_after_sync();
+        const bool live = kj < p.Sk;
+        unsigned char* dv_row = reinterpret_cast<unsigned char*>(p.dv.ptr) +
+                                2 * ((long long)w.b * p.dv.sb + (long long)w.h * p.dv.sh + (long long)kj * p.dv.ss) +
+                                2 * GC * g;
+        unsigned char* dk_row = reinterpret_cast<unsigned char*>(p.dk.ptr) +
+                                2 * ((long long)w.b * p.dk.sb + (long long)w.h * p.dk.sh + (long long)kj * p.dk.ss) +
+                                2 * GC * g;
+        if (w.n_it > 0) {
+          store_cols<IS_BF16>(lane_addr + kColAcc0 + GC * g, dv_row, 1.f, live, p.dv.wide);
+          store_cols<IS_BF16>(lane_addr + kColAcc1 + GC * g, dk_row, p.scale, live, p.dk.wide);
+          tc::fence_before_sync();
+          warp_arrive(&acc_empty, lane);
+          ++items;
+        } else if (live) {
+          // no query sees this key tile: the gradients are zero
+          const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+          for (int e = 0; e < GC / 8; ++e) {
+            reinterpret_cast<uint4*>(dv_row)[e] = z;
+            reinterpret_cast<uint4*>(dk_row)[e] = z;
           }
         }
-        // all of this group's S columns are in registers: P^T goes over their first half
-        tc::tmem_st16(s_addr + c * 16, pk);
       }
-      tc::tmem_wait_st();
-      tc::fence_before_sync();
-      warp_arrive(&p_full[g], lane);
-#pragma unroll
-      for (int e = 0; e < GC / 4; ++e) stat[e] = *reinterpret_cast<const float4*>(&ndelta_s[s][GC * g + 4 * e]);
-
-      if (!__all_sync(kFull, mbar_wait(&dp_full, it & 1, &failed))) {
-        ok = false;
-        break;
-      }
-      tc::fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < GC / 32; ++c) tc::tmem_ld32(dp_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
-      tc::tmem_wait_ld();
-#pragma unroll
-      for (int c = 0; c < GC / 32; ++c) {
-        uint32_t pk[16];
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          const float4 d4 = stat[c * 8 + e / 4];
-          const float2 d2[2] = {make_float2(d4.x, d4.y), make_float2(d4.z, d4.w)};
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int at = c * 32 + e + 2 * u;
-            const float2 x = mul2(pr[at / 2], add2(make_float2(__uint_as_float(raw[at]), __uint_as_float(raw[at + 1])), d2[u]));
-            pk[e / 2 + u] = pack_pair(x.x, x.y, IS_BF16);
-          }
-        }
-        tc::tmem_st16(dp_addr + c * 16, pk);
-      }
-      tc::tmem_wait_st();
-      tc::fence_before_sync();
-      warp_arrive(&ds_full, lane);
+      index = take_next(n, ok);
     }
-
-    if (ok && n_it > 0) ok = mbar_wait(&acc_done, 0, &failed);
-    ok = __all_sync(kFull, ok);
-    if (ok) {
-      tc::fence_after_sync();
-      const bool live = kj < p.Sk;
-      unsigned char* dv_row = reinterpret_cast<unsigned char*>(p.dv.ptr) +
-                              2 * ((long long)b * p.dv.sb + (long long)h * p.dv.sh + (long long)kj * p.dv.ss) +
-                              2 * GC * g;
-      unsigned char* dk_row = reinterpret_cast<unsigned char*>(p.dk.ptr) +
-                              2 * ((long long)b * p.dk.sb + (long long)h * p.dk.sh + (long long)kj * p.dk.ss) +
-                              2 * GC * g;
-      if (n_it > 0) {
-        store_cols<IS_BF16>(lane_addr + kColAcc0 + GC * g, dv_row, 1.f, live, p.dv.wide);
-        store_cols<IS_BF16>(lane_addr + kColAcc1 + GC * g, dk_row, p.scale, live, p.dk.wide);
-      } else if (live) {
-        // no query sees this key tile: the gradients are zero
-        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int e = 0; e < GC / 8; ++e) {
-          reinterpret_cast<uint4*>(dv_row)[e] = z;
-          reinterpret_cast<uint4*>(dk_row)[e] = z;
-        }
-      }
-    } else {
-      failed = 1;
-    }
+    if (!ok) failed = 1;
   }
 
   tc::fence_before_sync();
   __syncthreads();
-  if (failed && n_it > 0) {  // (uniform: nobody writes it any more)
+  if (failed) {  // (uniform: nobody writes it any more)
     // a role gave up: what the others have under way has to end before the block does
     if (threadIdx.x == 0) {
-      tc::await_copies<1>(&kv_full, 1);
+      tc::await_copies<1>(&kv_full, kv_loads);
       tc::await_copies<kStages>(q_full, q_loads);
       tc::await_copies<kStages>(do_full, do_loads);
     }
     if (warp == 1) tc::await_products(&drained);
+    if (warp == 2 && lane == 0) tc::await_copies<2>(next_full, asked);
     __syncthreads();
   }
   if (threadIdx.x == 0 && failed && p.status != nullptr) atomicExch(p.status, 1);
@@ -580,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const int n_q_tiles = (p.Sq + BM - 1) / BM;
   int slot, bh;
-  cta_order(n_q_tiles, p.n_bh, p.head_group, &slot, &bh);
+  cta_order((int)blockIdx.x, n_q_tiles, p.n_bh, p.head_group, &slot, &bh);
   const int q_tile = n_q_tiles - 1 - slot;  // late query tiles see the most keys: first
   const int b = bh / p.H, h = bh % p.H;
   const int qt0 = q_tile * BM;
@@ -825,7 +903,7 @@ __global__ void __launch_bounds__(kDsThreads, 1)
   const int n_kv_tiles = (p.Sk + BN - 1) / BN;
   const int n_slots = (n_q_tiles + kQT - 1) / kQT;
   int slot, bh;
-  cta_order(n_slots, p.n_bh, p.head_group, &slot, &bh);
+  cta_order((int)blockIdx.x, n_slots, p.n_bh, p.head_group, &slot, &bh);
   bh = p.n_bh - 1 - bh;  // the last heads first: some of their dS is still in L2
   const int first = (n_slots - 1 - slot) * kQT;  // late query tiles see the most keys: first
   const int tiles = min(kQT, n_q_tiles - first);
