@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* v_smem = smem + kTileBytes * (NQ + kStages);
 
   __shared__ __align__(16) uint4 next_answer[2];
-  __shared__ __align__(8) uint64_t q_full, q_empty, next_full[2], next_taken[2], k_full[kStages], k_empty[kStages], v_full[kStages],
+  __shared__ __align__(8) uint64_t q_full, q_empty, next_wanted, next_full[2], next_taken[2], k_full[kStages], k_empty[kStages], v_full[kStages],
       v_empty[kStages], s_full[NQ], p_full[NQ], p_rest[NQ], pv_done[NQ], drained;
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
     mbar_init(&q_empty, 1);
+    mbar_init(&next_wanted, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&next_full[s], 1);
       mbar_init(&next_taken[s], 2 + NQ * 4);  // producer, issuer and the softmax warps
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc::tma_load_4d(kd, &map_k, &k_full[s], 0, j * BN, w.h, w.b);
             tc::tma_load_4d(kd + kHalfBytes, &map_k, &k_full[s], 64, j * BN, w.h, w.b);
             k_loads = step + j + 1;
+            if (j + 1 == w.n_kv) tc::mbar_arrive(&next_wanted);
             good = u == 0 || mbar_wait(&v_empty[s], (u - 1) & 1, &failed);
             if (!good) break;
             unsigned char* vd = v_smem + (size_t)s * kTileBytes;
@@ -290,10 +292,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
     } else if (warp == 2) {
       // -------------------------------------------------------------------- scheduler
-      // One answer ahead: asked for when every role has taken the one before it.
+      // Asked for when the last K of an item is under way, two steps before its end: soon enough for its Q, and not
+      // before - a block that asked at the start of a long item would keep a pending one from those that
+      // finish first.
       bool ok = true;
       for (int n = 0; ok; ++n) {
-        if (n > 0) ok = __all_sync(kFull, mbar_wait(&next_taken[(n - 1) & 1], ((n - 1) >> 1) & 1, &failed));
+        ok = __all_sync(kFull, mbar_wait(&next_wanted, n & 1, &failed));
+        if (ok && n > 0) ok = __all_sync(kFull, mbar_wait(&next_taken[(n - 1) & 1], ((n - 1) >> 1) & 1, &failed));
         if (!ok) break;
         if (lane == 0) tc::request_next_block(&next_answer[n & 1], &next_full[n & 1]);
         asked = n + 1;
