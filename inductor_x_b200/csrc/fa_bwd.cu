@@ -39,7 +39,8 @@
 // reads beside it are slow).  A tile took 13000 cycles besides its steps while each had a CTA of its own
 // (the launch, tensor memory, the first copies, the results): calls in which tiles are taken over, before and
 // after: 4 x 32 heads of 4096 causal 1590 and 1500 us, 10 x 16 of 1851 525 and 483, 8 x 32 of 1000 326 and 284,
-// 8 x 16 of 1000 without a mask 246 and 226, 8 x 32 of 196 70 and 61.  Two tiles in flight would need more tensor memory than one SM has.
+// 8 x 16 of 1000 without a mask 246 and 226, 8 x 32 of 196 70 and 61.  Two tiles in flight would need more
+// tensor memory than one SM has.
 // Built, measured and dropped: a share of the exponentials on the fma pipe (1049 - 1070 against 1000:
 // the ex2 unit is not the limit, power is); sixteen element-wise warps (the same); dS to memory by way
 // of shared memory and bulk copies (171 against 162 for the 8 heads) or stored by the element-wise
@@ -878,11 +879,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 // One CTA owns two query tiles of a head and walks the key tiles they see: dQ += dS K, with the
 // tiles of dS^T as the first operand (MN-major, no swizzle) and K in MN-major form.  Bound: the 32 KB
 // of dS a product reads; two query tiles share a K tile, which comes from L2.  2.2 GB of dS (4 x 32
-// heads of 4096, causal) in 400 us, 5500 GB/s.  TMEM: 2 x 128 columns.
+// heads of 4096, causal) in 400 us, 5500 GB/s.  Pending items are taken over as in the dK/dV kernel, so that
+// dS keeps coming while the results of an item leave: whole calls 8 x 32 heads of 196 61.0 -> 58.0 us, 12 x 32
+// of 136 causal 73.3 -> 68.2, 8 x 16 of 1000 226 -> 220, 4 x 32 of 4096 causal 1520 -> 1507.
+// TMEM: two sets of 2 x 128 columns, used by the items in turn.
 constexpr int kQT = 2;        // query tiles a CTA
 constexpr int kDsStages = 4;  // tiles of dS^T in flight
-constexpr int kDsThreads = 64 + 128;
-template <bool IS_BF16>
+constexpr int kDsThreads = 64 + 128 + 32;  // producer and issuer, results, scheduler
+// TAKE: there are more items than SMs.  Where there are not, nothing is pending: without the loop over items
+// (TAKE = false) 2 x 8 heads of 2048 causal take 22.7 us in this kernel, with it 23.4.
+template <bool IS_BF16, bool TAKE>
 __global__ void __launch_bounds__(kDsThreads, 1)
     fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap map_k, const BwdParams p) {
   extern __shared__ unsigned char smem_raw[];
@@ -891,8 +897,9 @@ __global__ void __launch_bounds__(kDsThreads, 1)
   unsigned char* k_smem = smem;                    // kStages tiles
   unsigned char* ds_smem = smem + 2 * kTileBytes;  // kDsStages tiles
 
-  __shared__ __align__(8) uint64_t k_full[kStages], k_empty[kStages], ds_full[kDsStages], ds_empty[kDsStages],
-      acc_done, drained;
+  __shared__ __align__(16) uint4 next_answer[2];
+  __shared__ __align__(8) uint64_t next_wanted, next_full[2], next_taken[2], k_full[kStages], k_empty[kStages],
+      ds_full[kDsStages], ds_empty[kDsStages], acc_full[2], acc_empty[2], drained;
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
@@ -902,20 +909,37 @@ __global__ void __launch_bounds__(kDsThreads, 1)
   const int n_q_tiles = (p.Sq + BM - 1) / BM;
   const int n_kv_tiles = (p.Sk + BN - 1) / BN;
   const int n_slots = (n_q_tiles + kQT - 1) / kQT;
-  int slot, bh;
-  cta_order((int)blockIdx.x, n_slots, p.n_bh, p.head_group, &slot, &bh);
-  bh = p.n_bh - 1 - bh;  // the last heads first: some of their dS is still in L2
-  const int first = (n_slots - 1 - slot) * kQT;  // late query tiles see the most keys: first
-  const int tiles = min(kQT, n_q_tiles - first);
   const int hide = hidden_tiles(p.causal, p.Sq, p.Sk, n_kv_tiles);
-  const unsigned char* ds_head = p.ds + (long long)bh * p.tiles_per_head * kTileBytes;
-  bh += p.bh0;
-  const int b = bh / p.H, h = bh % p.H;
-  // key tiles that the first query tile sees, and that either sees
-  const int n_kv0 = p.causal ? min(n_kv_tiles, first + hide + 1) : n_kv_tiles;
-  const int n_kv = p.causal ? min(n_kv_tiles, first + tiles + hide) : n_kv_tiles;
+  struct Item {
+    int first, tiles;  // query tiles
+    int n_kv0, n_kv;   // key tiles that the first query tile sees, and that either sees
+    int b, h;
+    const unsigned char* ds_head;
+  };
+  auto item_of = [&](int index) {
+    Item w;
+    int slot, bh;
+    cta_order(index, n_slots, p.n_bh, p.head_group, &slot, &bh);
+    bh = p.n_bh - 1 - bh;  // the last heads first: some of their dS is still in L2
+    w.first = (n_slots - 1 - slot) * kQT;  // late query tiles see the most keys: first
+    w.tiles = min(kQT, n_q_tiles - w.first);
+    w.ds_head = p.ds + (long long)bh * p.tiles_per_head * kTileBytes;
+    bh += p.bh0;
+    w.b = bh / p.H;
+    w.h = bh % p.H;
+    w.n_kv0 = p.causal ? min(n_kv_tiles, w.first + hide + 1) : n_kv_tiles;
+    w.n_kv = p.causal ? min(n_kv_tiles, w.first + w.tiles + hide) : n_kv_tiles;
+    return w;
+  };
 
   if (threadIdx.x == 0) {
+    mbar_init(&next_wanted, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&next_full[s], 1);
+      mbar_init(&next_taken[s], 2 + 4);  // producer, issuer and the warps of the results
+      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_empty[s], 4);
+    }
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&k_full[s], 1);
       mbar_init(&k_empty[s], 1);
@@ -924,41 +948,60 @@ __global__ void __launch_bounds__(kDsThreads, 1)
       mbar_init(&ds_full[s], 1);
       mbar_init(&ds_empty[s], 1);
     }
-    mbar_init(&acc_done, 1);
     mbar_init(&drained, 1);
     failed = 0;
     mbar_init_fence();
   }
-  if (warp == 1) tc::tmem_alloc(&tmem_base_slot, kQT * 128);
+  if (warp == 1) tc::tmem_alloc(&tmem_base_slot, (TAKE ? 2 : 1) * kQT * 128);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
 
+  // The item after item n of this block: answer n of the scheduler warp.  Taken by a whole warp.
+  auto take_next = [&](int n, bool& ok) {
+    if (!TAKE) return -1;
+    ok = ok && __all_sync(kFull, mbar_wait(&next_full[n & 1], (n >> 1) & 1, &failed));
+    if (!ok) return -1;
+    const int index = __shfl_sync(kFull, tc::next_block(&next_answer[n & 1]), 0);
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&next_taken[n & 1]);
+    return index;
+  };
+
   int k_loads = 0, ds_loads = 0;  // producer: key and dS tiles it has asked for
+  int asked = 0;                  // scheduler: the same
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
-      bool ok = true;
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int s = j % kStages, n = j / kStages;
-        if (n > 0) ok = mbar_wait(&k_empty[s], (n - 1) & 1, &failed);
-        if (!ok) break;
-        mbar_arrive_expect_tx(&k_full[s], kTileBytes);
-        load_tile(k_smem + (size_t)s * kTileBytes, &map_k, &k_full[s], j * BN, h, b);
-        k_loads = j + 1;
-        for (int t = j < n_kv0 ? 0 : 1; t < tiles; ++t) {
-          const int u = ds_loads % kDsStages, m = ds_loads / kDsStages;
-          if (m > 0) ok = mbar_wait(&ds_empty[u], (m - 1) & 1, &failed);
-          if (!ok) break;
-          mbar_arrive_expect_tx(&ds_full[u], kTileBytes);
-          bulk_g2s(ds_smem + (size_t)u * kTileBytes, ds_head + ds_tile(j, first + t, n_q_tiles, hide) * kTileBytes,
-                   kTileBytes, &ds_full[u]);
-          ++ds_loads;
+    bool ok = true;
+    for (int i = 0, index = blockIdx.x; (TAKE ? index >= 0 : i == 0) && ok; ++i) {
+      const Item w = item_of(index);
+      int mine = 1;
+      if (lane == 0) {
+        bool good = true;
+        for (int j = 0; j < w.n_kv && good; ++j) {
+          const int s = k_loads & 1, n = k_loads >> 1;
+          if (n > 0) good = mbar_wait(&k_empty[s], (n - 1) & 1, &failed);
+          if (!good) break;
+          mbar_arrive_expect_tx(&k_full[s], kTileBytes);
+          load_tile(k_smem + (size_t)s * kTileBytes, &map_k, &k_full[s], j * BN, w.h, w.b);
+          ++k_loads;
+          if (TAKE && j + 1 == w.n_kv) tc::mbar_arrive(&next_wanted);
+          const unsigned char* tile = w.ds_head + ds_tile(j, w.first, n_q_tiles, hide) * kTileBytes;
+          for (int t = j < w.n_kv0 ? 0 : 1; t < w.tiles; ++t, ++ds_loads) {
+            const int u = ds_loads & (kDsStages - 1), m = ds_loads / kDsStages;
+            if (m > 0) good = mbar_wait(&ds_empty[u], (m - 1) & 1, &failed);
+            if (!good) break;
+            mbar_arrive_expect_tx(&ds_full[u], kTileBytes);
+            bulk_g2s(ds_smem + u * kTileBytes, tile + t * kTileBytes, kTileBytes, &ds_full[u]);
+          }
         }
+        mine = good ? 1 : 0;
       }
-      if (!ok) failed = 1;
+      ok = __shfl_sync(kFull, mine, 0) != 0;
+      index = take_next(i, ok);
     }
+    if (!ok && lane == 0) failed = 1;
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -969,46 +1012,71 @@ __global__ void __launch_bounds__(kDsThreads, 1)
     constexpr uint32_t kStep = kTileBytes >> 4;
     const uint32_t tmem = __shfl_sync(kFull, tmem_base, 0);
     bool ok = true;
-    int n = 0;  // tiles of dS consumed
-    for (int j = 0; j < n_kv && ok; ++j) {
-      const int s = j % kStages;
-      ok = __all_sync(kFull, mbar_wait(&k_full[s], (j / kStages) & 1, &failed));
-      for (int t = j < n_kv0 ? 0 : 1; t < tiles && ok; ++t, ++n) {
-        const int u = n % kDsStages;
-        ok = __all_sync(kFull, mbar_wait(&ds_full[u], (n / kDsStages) & 1, &failed));
-        if (!ok) break;
-        tc::fence_after_sync();
-        // 16 keys a step: 256 bytes inside 32 keys of a dS tile, 16 rows (2048 bytes) of K
+    int m = 0, n = 0;  // tiles of K and of dS consumed
+    for (int i = 0, index = blockIdx.x; (TAKE ? index >= 0 : i == 0) && ok; ++i) {
+      const Item w = item_of(index);
+      // items use the two sets of accumulators in turn: the results of one leave under the products of the next
+      const uint32_t acc = tmem + (i & 1) * (kQT * 128);
+      if (i > 1) ok = __all_sync(kFull, mbar_wait(&acc_empty[i & 1], ((i >> 1) - 1) & 1, &failed));
+      tc::fence_after_sync();
+      for (int j = 0; j < w.n_kv && ok; ++j, ++m) {
+        const int s = m & 1;
+        ok = __all_sync(kFull, mbar_wait(&k_full[s], (m >> 1) & 1, &failed));
+        for (int t = j < w.n_kv0 ? 0 : 1; t < w.tiles && ok; ++t, ++n) {
+          const int u = n & (kDsStages - 1);
+          ok = __all_sync(kFull, mbar_wait(&ds_full[u], (n / kDsStages) & 1, &failed));
+          if (!ok) break;
+          tc::fence_after_sync();
+          // 16 keys a step: 256 bytes inside 32 keys of a dS tile, 16 rows (2048 bytes) of K
 #pragma unroll
-        for (int kq = 0; kq < 4; ++kq)
-          tc::product_ss_steps<2, 256, 2048>(tmem + 128 * t, ds_desc + u * kStep + kq * (kTileBytes / 4 >> 4),
-                                             k_desc + s * kStep + kq * (2 * 2048 >> 4), idesc, j > 0 || kq > 0 ? 1u : 0u);
-        tc::commit_elected(&ds_empty[u]);
+          for (int kq = 0; kq < 4; ++kq)
+            tc::product_ss_steps<2, 256, 2048>(acc + 128 * t, ds_desc + u * kStep + kq * (kTileBytes / 4 >> 4),
+                                               k_desc + s * kStep + kq * (2 * 2048 >> 4), idesc, j > 0 || kq > 0 ? 1u : 0u);
+          tc::commit_elected(&ds_empty[u]);
+        }
+        if (ok) tc::commit_elected(&k_empty[s]);
       }
-      if (ok) tc::commit_elected(&k_empty[s]);
+      if (ok) tc::commit_elected(&acc_full[i & 1]);
+      index = take_next(i, ok);
     }
-    if (ok) tc::commit_elected(&acc_done);
     if (!ok && lane == 0) failed = 1;
     __syncwarp();
+  } else if (warp == 6) {
+    // ------------------------------------------------------------------ scheduler (as in the dK/dV kernel)
+    bool ok = true;
+    for (int n = 0; ok && TAKE; ++n) {
+      ok = __all_sync(kFull, mbar_wait(&next_wanted, n & 1, &failed));
+      if (ok && n > 0) ok = __all_sync(kFull, mbar_wait(&next_taken[(n - 1) & 1], ((n - 1) >> 1) & 1, &failed));
+      if (!ok) break;
+      if (lane == 0) tc::request_next_block(&next_answer[n & 1], &next_full[n & 1]);
+      asked = n + 1;
+      ok = __all_sync(kFull, mbar_wait(&next_full[n & 1], (n >> 1) & 1, &failed));
+      if (!ok || __shfl_sync(kFull, tc::next_block(&next_answer[n & 1]), 0) < 0) break;
+    }
+    if (!ok && lane == 0) failed = 1;
   } else {
     // ------------------------------------------------------------------ results
     const int quad = warp & 3;
-    bool ok = mbar_wait(&acc_done, 0, &failed);
-    ok = __all_sync(kFull, ok);
-    if (ok) {
+    bool ok = true;
+    for (int i = 0, index = blockIdx.x; (TAKE ? index >= 0 : i == 0) && ok; ++i) {
+      const Item w = item_of(index);
+      ok = __all_sync(kFull, mbar_wait(&acc_full[i & 1], (i >> 1) & 1, &failed));
+      if (!ok) break;
       tc::fence_after_sync();
-      const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-      for (int t = 0; t < tiles; ++t) {
-        const int qi = (first + t) * BM + quad * 32 + lane;
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (i & 1) * (kQT * 128);
+      for (int t = 0; t < w.tiles; ++t) {
+        const int qi = (w.first + t) * BM + quad * 32 + lane;
         unsigned char* dq_row = reinterpret_cast<unsigned char*>(p.dq.ptr) +
-                                2 * ((long long)b * p.dq.sb + (long long)h * p.dq.sh + (long long)qi * p.dq.ss);
+                                2 * ((long long)w.b * p.dq.sb + (long long)w.h * p.dq.sh + (long long)qi * p.dq.ss);
 #pragma unroll
         for (int g = 0; g < NG; ++g)
           store_cols<IS_BF16>(lane_addr + 128 * t + GC * g, dq_row + 2 * GC * g, p.scale, qi < p.Sq, p.dq.wide);
       }
-    } else {
-      failed = 1;
+      tc::fence_before_sync();
+      warp_arrive(&acc_empty[i & 1], lane);
+      index = take_next(i, ok);
     }
+    if (!ok && lane == 0) failed = 1;
   }
 
   tc::fence_before_sync();
@@ -1019,12 +1087,13 @@ __global__ void __launch_bounds__(kDsThreads, 1)
       tc::await_copies<kDsStages>(ds_full, ds_loads);
     }
     if (warp == 1) tc::await_products(&drained);
+    if (warp == 6 && lane == 0) tc::await_copies<2>(next_full, asked);
     __syncthreads();
   }
   if (threadIdx.x == 0 && failed && p.status != nullptr) atomicExch(p.status, 1);
   if (warp == 1) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem_base, kQT * 128);
+    tc::tmem_dealloc(tmem_base, (TAKE ? 2 : 1) * kQT * 128);
   }
 }
 
@@ -1116,13 +1185,15 @@ extern "C" int ixb_fa_bwd_scratch(int dtype, const void* q, const void* k, const
   auto kern_delta = is_bf16 ? fa_bwd_delta_kernel<true> : fa_bwd_delta_kernel<false>;
   auto kern_dkv = is_bf16 ? fa_bwd_dkv_kernel<true> : fa_bwd_dkv_kernel<false>;
   auto kern_dq = is_bf16 ? fa_bwd_dq_kernel<true> : fa_bwd_dq_kernel<false>;
-  auto kern_dq_ds = is_bf16 ? fa_bwd_dq_ds_kernel<true> : fa_bwd_dq_ds_kernel<false>;
-  static std::atomic<bool> configured[3][2][64];
+  auto kern_dq_ds = is_bf16 ? fa_bwd_dq_ds_kernel<true, true> : fa_bwd_dq_ds_kernel<false, true>;
+  auto kern_dq_ds_one = is_bf16 ? fa_bwd_dq_ds_kernel<true, false> : fa_bwd_dq_ds_kernel<false, false>;
+  static std::atomic<bool> configured[4][2][64];
   int devid = 0;
   cudaGetDevice(&devid);
   if (int st = opt_in_smem(kern_dkv, configured[0][is_bf16][devid & 63], kRegsLaunch)) return st;
   if (int st = opt_in_smem(kern_dq, configured[1][is_bf16][devid & 63])) return st;
   if (int st = opt_in_smem(kern_dq_ds, configured[2][is_bf16][devid & 63])) return st;
+  if (int st = opt_in_smem(kern_dq_ds_one, configured[3][is_bf16][devid & 63])) return st;
 
   // The heads go in as many equal launches as the scratch asks for; without room for one head's dS the
   // probabilities are recomputed for dQ.
@@ -1133,6 +1204,9 @@ extern "C" int ixb_fa_bwd_scratch(int dtype, const void* q, const void* k, const
   p.ds = fit > 0 ? static_cast<unsigned char*>(scratch) : nullptr;
   p.tiles_per_head = fit > 0 ? (int)tiles : 0;
 
+  const ixb_devinfo* dev = ixb_host::current_device();
+  if (dev == nullptr) return IXB_ERR_CUDA;
+  const int sms = dev->sm_count;
   cudaStream_t cs = (cudaStream_t)stream;
   const long long rows = n_bh * Sq;
   kern_delta<<<(unsigned)((rows + 15) / 16), 256, 0, cs>>>(
@@ -1142,8 +1216,9 @@ extern "C" int ixb_fa_bwd_scratch(int dtype, const void* q, const void* k, const
     p.bh0 = (int)at;
     p.n_bh = (int)(heads < n_bh - at ? heads : n_bh - at);
     kern_dkv<<<(unsigned)(n_kv_tiles * p.n_bh), kDkvThreads, kSmemBytes, cs>>>(mq, mk, mv, mdo, p);
+    const long long slots = (n_q_tiles + kQT - 1) / kQT * p.n_bh;
     if (fit > 0)
-      kern_dq_ds<<<(unsigned)((n_q_tiles + kQT - 1) / kQT * p.n_bh), kDsThreads, kSmemBytes, cs>>>(mk, p);
+      (slots > sms ? kern_dq_ds : kern_dq_ds_one)<<<(unsigned)slots, kDsThreads, kSmemBytes, cs>>>(mk, p);
     else
       kern_dq<<<(unsigned)(n_q_tiles * p.n_bh), kThreads, kSmemBytes, cs>>>(mq, mk, mv, mdo, p);
   }
