@@ -36,11 +36,18 @@ inline int make_fa_map(CUtensorMap* map, const void* base, int is_bf16, int B, i
   const cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
   const cuuint32_t box[4] = {64, 128, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                        4, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? IXB_OK : IXB_ERR_ARG;
+  auto encode = [&] {
+    return fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+              4, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  if (encode() == CUDA_SUCCESS) return IXB_OK;
+  // A thread that has launched nothing yet (autograd's, where all memory comes out of the allocator's cache) has no
+  // current context, which a call of the driver wants; cudaSetDevice gives it the device's own.
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return IXB_ERR_CUDA;
+  return encode() == CUDA_SUCCESS ? IXB_OK : IXB_ERR_ARG;
 }
 
 // fa_split.cu: how many blocks share a query tile's keys where the forward pass is cut that way (0: it is
