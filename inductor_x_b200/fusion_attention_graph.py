@@ -239,10 +239,14 @@ def _sdpa_setup_context(ctx, inputs, output):
     out, lse = output
     ctx.save_for_backward(query, key, value, out, lse)
     ctx.scale, ctx.is_causal = scale, is_causal
+    # The gradient of the log-sum-exp is not read: no tensor of zeros is made for it (a launch of its own each call).
+    ctx.set_materialize_grads(False)
 
 
 def _sdpa_backward(ctx, d_out, d_lse):
     query, key, value, out, lse = ctx.saved_tensors
+    if d_out is None:  # only the log-sum-exp was used
+        d_out = torch.zeros_like(out)
     dq, dk, dv = torch.ops.b200_graph.b200_sdpa_backward(query, key, value, out, lse, d_out, ctx.scale,
                                                          ctx.is_causal)
     return dq, dk, dv, None, None
