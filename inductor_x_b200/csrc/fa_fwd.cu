@@ -445,9 +445,13 @@ extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v
   // One group where the K and V of all heads stay in L2, else equal groups of about 40 MB.  Groups of
   // 8 heads -> this: 1 x 32 heads of 2048 keys 60 -> 49 us, 2 x 32 87 -> 73, 2 x 16 of 4096 179 -> 145,
   // 3 x 12 of 5014 295 -> 240, 2 x 8 of 8192 315 -> 272, 4 x 32 of 2048 145 -> 138, 8 x 32 of 4096 995 -> 960.
+  // Three query tiles make a block of one tile and a block of two, which sees a key tile less of each: neither is
+  // the long one, and what is left of groups is that both blocks read the same K and V.  Groups of 8 heads and one
+  // group: 4 x 32 heads of 261 16.7 and 17.7 us, of 300 16.9 and 17.8, 16 x 16 of 261 29.2 and 29.9; of two or four
+  // tiles 16.2 and 16.2 (6 x 32 of 200), 19.2 and 17.6 (3 x 32 of 459).
   static const int group_env = [] { const char* v = getenv("IXB_FA_HEAD_GROUP"); return v != nullptr ? atoi(v) : 0; }();
   const double all = (double)B * H, mb = Sk * (2. * HD * 2 / (1 << 20));  // heads, and MB of K and V of each
-  const double groups = all * mb <= 96 ? 1 : ceil(all / (mb < 5 ? floor(40 / mb) : 8));
+  const double groups = (Sq + BM - 1) / BM == 3 ? ceil(all / 8) : all * mb <= 96 ? 1 : ceil(all / (mb < 5 ? floor(40 / mb) : 8));
   p.head_group = group_env > 0 ? group_env : (causal ? (int)ceil(all / groups) : 1);
   if (!(scale > 0.f)) return IXB_ERR_ARG;  // the row maximum is taken before scaling
   if (const int cluster = ixb_host::fa_split_size(B, H, Sq, Sk))
