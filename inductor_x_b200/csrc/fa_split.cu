@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             ls = l_row[lane][r];
           }
         }
-        top[i] = ls > 0.f ? m : -INFINITY;
+        top[i] = m;  // (-inf: the slot saw nothing of the row, or nothing but NaN, which its sum says)
         total[i] = ls;
       }
 #pragma unroll
@@ -333,12 +333,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         float4 v[kRows];
 #pragma unroll
         for (int i = 0; i < kRows; ++i) {
-          const int r = r0 + i * kStep;  // (past the end no slot weighs anything)
-          const float ws = __shfl_sync(kFull, w[i], s);
+          const int r = r0 + i * kStep;
           const float4* piece = &o_smem[(s % NQ * BM + r) * kPieces + (lane ^ (r & 31))];
-          // (a slot that saw nothing of the row wrote nothing, or zeros; uniform)
+          // (a slot without a key tile wrote nothing; every other one counts whatever it weighs, since no weight
+          // makes a NaN or an infinity of it go away)
           v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (ws > 0.f) v[i] = CLUSTER > 1 ? ld_cluster_f32x4(map_to_rank(piece, s / NQ)) : *piece;
+          if (s < n_kv && r < rows) v[i] = CLUSTER > 1 ? ld_cluster_f32x4(map_to_rank(piece, s / NQ)) : *piece;
         }
 #pragma unroll
         for (int i = 0; i < kRows; ++i) {
@@ -353,14 +353,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int i = 0; i < kRows; ++i) {
         const int r = r0 + i * kStep;
         if (r >= rows) break;
-        const float inv = total[i] > 0.f ? 1.f / total[i] : 0.f;
+        const float inv = total[i] == 0.f ? 0.f : 1.f / total[i];  // (a sum may be NaN)
         uint2 out;
         out.x = tc::round_pair<IS_BF16>(acc[i].x * inv, acc[i].y * inv);
         out.y = tc::round_pair<IS_BF16>(acc[i].z * inv, acc[i].w * inv);
         *reinterpret_cast<uint2*>(base + 2 * (long long)(q0 + r) * p.o_stride_s + lane * 8) = out;
         if (lane == 0 && p.lse != nullptr)
           p.lse[((long long)b * p.H + h) * p.Sq + q0 + r] =
-              total[i] > 0.f ? (top[i] + log2f(total[i])) * 0.69314718055994530942f : -INFINITY;
+              total[i] == 0.f ? -INFINITY : (top[i] + log2f(total[i])) * 0.69314718055994530942f;
       }
     }
   }
