@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (live) tc::store_row32<IS_BF16>(orow + c * 64, o, inv, p.wide != 0);
           }
           if (live && p.lse != nullptr) {
-            const float lse = (l > 0.f) ? (m_used + log2f(l)) * 0.69314718055994530942f : -INFINITY;
+            const float lse = l == 0.f ? -INFINITY : (m_used + log2f(l)) * 0.69314718055994530942f;  // (l may be NaN)
             p.lse[((long long)w.b * p.H + w.h) * p.Sq + qi] = lse;
           }
         }

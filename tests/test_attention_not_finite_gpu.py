@@ -37,6 +37,7 @@ def test_not_finite(cuda, b, h, sq, sk, causal):
             finite = torch.isfinite(want)
             assert torch.equal(torch.isfinite(a), finite), what
             assert torch.equal(a[finite], was[finite]), what   # and what is finite is what it was
+        assert bool(got[1][~torch.isfinite(got[1])].isnan().all()), what   # whichever kernel it was
 
     def with_one(t, value, *place):
         t = t.clone()
