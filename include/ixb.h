@@ -231,6 +231,10 @@ int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v, void* o, 
                const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides,
                float scale, int causal, int32_t* status, ixb_stream stream);
 
+/* How ixb_fa_fwd goes about a call of these sizes, for tests and profiles: `heads`, how many heads' blocks are
+ * dispatched together where a block has its query tiles to itself.  The result of a call does not depend on it. */
+int ixb_fa_fwd_plan(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, int32_t* heads);
+
 /* Gradients of ixb_fa_fwd: dq[B,H,Sq,D], dk/dv[B,H,Sk,D] from q, k, v, the forward's
  * output `o` and log-sum-exp `lse` [B,H,Sq] (fp32, contiguous) and the incoming gradient
  * `dout` [B,H,Sq,D]; same dtype, stride and alignment rules as ixb_fa_fwd for all eight

@@ -400,7 +400,39 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// Heads whose blocks are dispatched together.
+// Without a mask every query block of a head reads all of its K and V, so the heads go one
+// after the other (group of 1: blockIdx order = head-major, as a 2-D grid would give).
+// Under a causal mask heads run in groups, the long query blocks of all of them first: what a group's
+// long blocks find of K and V in L2 against the SMs that wait for the last group's long blocks at the end.
+// One group where the K and V of all heads stay in L2, else equal groups of about 40 MB.  Groups of
+// 8 heads -> this: 1 x 32 heads of 2048 keys 60 -> 49 us, 2 x 32 87 -> 73, 2 x 16 of 4096 179 -> 145,
+// 3 x 12 of 5014 295 -> 240, 2 x 8 of 8192 315 -> 272, 4 x 32 of 2048 145 -> 138, 8 x 32 of 4096 the same.
+// Three query tiles make a block of one tile and a block of two, the block of one first.  With as many keys as
+// queries both have three tile products: neither is the long one, and what is left of groups is that both
+// blocks read the same K and V.  Groups of 8 heads and one group: 96 heads of 300 18.6 and 19.7 us, 128 18.7 and 20.3,
+// 192 25.1 and 25.8, 256 31.0 and 31.7; of 384 18.6 and 20.4, 20.6 and 20.6, 26.8 and 26.8, 32.9 and 32.9.  With more
+// keys the block of two has more products (two at three key tiles, n - 3 at n), and which is better goes by how the
+// blocks fall on the SMs at first, by what stays in L2 with more keys: 300 x 384 128 heads 23.0 and 24.1, 144 24.6 and
+// 22.7, 256 37.1 and 35.5; 300 x 500 128 heads 25.7 and 24.7, 160 31.0 and 32.9; 300 x 1000 128 heads 39.0 and 37.0, 320
+// 84.9 and 78.0; 261 x 700 256 heads 61.6 and 53.4.
+int head_group_of(int B, int H, int Sq, int Sk, int causal) {
+  static const int group_env = [] { const char* v = getenv("IXB_FA_HEAD_GROUP"); return v != nullptr ? atoi(v) : 0; }();
+  if (group_env > 0) return group_env;
+  if (!causal) return 1;
+  const double all = (double)B * H, mb = Sk * (2. * HD * 2 / (1 << 20));  // heads, and MB of K and V of each
+  const bool alike = Sq == Sk && ((long long)Sq + BM - 1) / BM == 3;
+  const double groups = alike ? ceil(all / 8) : all * mb <= 96 ? 1 : ceil(all / (mb < 5 ? floor(40 / mb) : 8));
+  return (int)ceil(all / groups);
+}
+
 }  // namespace
+
+extern "C" int ixb_fa_fwd_plan(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, int32_t* heads) {
+  if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0 || heads == nullptr) return IXB_ERR_ARG;
+  *heads = head_group_of(B, H, Sq, Sk, causal);
+  return IXB_OK;
+}
 
 extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v, void* o, float* lse,
                           int32_t B, int32_t H, int32_t Sq, int32_t Sk, int32_t D,
@@ -441,21 +473,7 @@ extern "C" int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v
   p.scale_log2 = scale * 1.4426950408889634f;
   p.causal = causal ? 1 : 0;
   p.wide = ixb_host::rows_aligned32(o, o_strides) ? 1 : 0;
-  // Without a mask every query block of a head reads all of its K and V, so the heads go one
-  // after the other (group of 1: blockIdx order = head-major, as a 2-D grid would give).
-  // Under a causal mask heads run in groups, the long query blocks of all of them first: what a group's
-  // long blocks find of K and V in L2 against the SMs that wait for the last group's long blocks at the end.
-  // One group where the K and V of all heads stay in L2, else equal groups of about 40 MB.  Groups of
-  // 8 heads -> this: 1 x 32 heads of 2048 keys 60 -> 49 us, 2 x 32 87 -> 73, 2 x 16 of 4096 179 -> 145,
-  // 3 x 12 of 5014 295 -> 240, 2 x 8 of 8192 315 -> 272, 4 x 32 of 2048 145 -> 138, 8 x 32 of 4096 995 -> 960.
-  // Three query tiles make a block of one tile and a block of two, which sees a key tile less of each: neither is
-  // the long one, and what is left of groups is that both blocks read the same K and V.  Groups of 8 heads and one
-  // group: 4 x 32 heads of 261 16.7 and 17.7 us, of 300 16.9 and 17.8, 16 x 16 of 261 29.2 and 29.9; of two or four
-  // tiles 16.2 and 16.2 (6 x 32 of 200), 19.2 and 17.6 (3 x 32 of 459).
-  static const int group_env = [] { const char* v = getenv("IXB_FA_HEAD_GROUP"); return v != nullptr ? atoi(v) : 0; }();
-  const double all = (double)B * H, mb = Sk * (2. * HD * 2 / (1 << 20));  // heads, and MB of K and V of each
-  const double groups = (Sq + BM - 1) / BM == 3 ? ceil(all / 8) : all * mb <= 96 ? 1 : ceil(all / (mb < 5 ? floor(40 / mb) : 8));
-  p.head_group = group_env > 0 ? group_env : (causal ? (int)ceil(all / groups) : 1);
+  p.head_group = head_group_of(B, H, Sq, Sk, causal);
   if (!(scale > 0.f)) return IXB_ERR_ARG;  // the row maximum is taken before scaling
   if (const int cluster = ixb_host::fa_split_size(B, H, Sq, Sk))
     return ixb_host::fa_split(cluster, is_bf16, mq, mk, mv, o, lse, B, H, Sq, Sk, o_strides, scale, causal, status, (cudaStream_t)stream);
