@@ -231,9 +231,10 @@ int ixb_fa_fwd(int dtype, const void* q, const void* k, const void* v, void* o, 
                const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides,
                float scale, int causal, int32_t* status, ixb_stream stream);
 
-/* How ixb_fa_fwd goes about a call of these sizes, for tests and profiles: `heads`, how many heads' blocks are
- * dispatched together where a block has its query tiles to itself.  The result of a call does not depend on it. */
-int ixb_fa_fwd_plan(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, int32_t* heads);
+/* How ixb_fa_fwd goes about a call of these sizes on the current device, for tests and profiles: `blocks`, over how
+ * many blocks the keys of a query tile are shared (1, 2, 4 or 8; 0: a block walks all keys of two query tiles, also
+ * without a device), and `heads`, how many heads' blocks are dispatched together in the latter case. */
+int ixb_fa_fwd_plan(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, int32_t* heads, int32_t* blocks);
 
 /* Gradients of ixb_fa_fwd: dq[B,H,Sq,D], dk/dv[B,H,Sk,D] from q, k, v, the forward's
  * output `o` and log-sum-exp `lse` [B,H,Sq] (fp32, contiguous) and the incoming gradient

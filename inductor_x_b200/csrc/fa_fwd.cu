@@ -428,9 +428,10 @@ int head_group_of(int B, int H, int Sq, int Sk, int causal) {
 
 }  // namespace
 
-extern "C" int ixb_fa_fwd_plan(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, int32_t* heads) {
-  if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0 || heads == nullptr) return IXB_ERR_ARG;
+extern "C" int ixb_fa_fwd_plan(int32_t B, int32_t H, int32_t Sq, int32_t Sk, int causal, int32_t* heads, int32_t* blocks) {
+  if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0 || heads == nullptr || blocks == nullptr) return IXB_ERR_ARG;
   *heads = head_group_of(B, H, Sq, Sk, causal);
+  *blocks = ixb_host::fa_split_size(B, H, Sq, Sk);
   return IXB_OK;
 }
 

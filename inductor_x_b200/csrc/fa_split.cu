@@ -373,12 +373,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// The opt-ins of a kernel on the current device, asked for once: a property of (kernel, device).
 template <bool IS_BF16, int CLUSTER>
-int launch_split(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const SplitParams& p, cudaStream_t stream) {
+int configure(int devid) {
   auto kern = fa_split_kernel<IS_BF16, CLUSTER>;
-  static std::atomic<bool> configured[64];  // the opt-in is a property of (kernel, device)
-  int devid = 0;
-  cudaGetDevice(&devid);
+  static std::atomic<bool> configured[64];
   std::atomic<bool>& done = configured[devid & 63];
   if (!done.load(std::memory_order_acquire)) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
@@ -389,19 +388,57 @@ int launch_split(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap
     if (at.numRegs != kRegsLaunch) return IXB_ERR_UNSUPPORTED;
     done.store(true, std::memory_order_release);
   }
+  return IXB_OK;
+}
+
+template <int CLUSTER>
+cudaLaunchConfig_t launch_config(long long blocks, cudaLaunchAttribute* attr, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((long long)((p.Sq + BM - 1) / BM) * p.B * p.H * CLUSTER));
+  cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CLUSTER;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = CLUSTER;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = CLUSTER > 1 ? 1 : 0;
-  return ixb_host::cuda_status(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, p));
+  return cfg;
+}
+
+template <bool IS_BF16, int CLUSTER>
+int launch_split(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const SplitParams& p, cudaStream_t stream) {
+  int devid = 0;
+  cudaGetDevice(&devid);
+  if (int st = configure<IS_BF16, CLUSTER>(devid)) return st;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = launch_config<CLUSTER>((long long)((p.Sq + BM - 1) / BM) * p.B * p.H * CLUSTER, &attr, stream);
+  return ixb_host::cuda_status(cudaLaunchKernelEx(&cfg, fa_split_kernel<IS_BF16, CLUSTER>, mq, mk, mv, p));
+}
+
+// Blocks of clusters of this size that the current device runs at a time (0: none), asked for once.
+template <int CLUSTER>
+int room_for(int devid) {
+  static std::atomic<int> known[64];  // one more than the number
+  std::atomic<int>& room = known[devid & 63];
+  int n = room.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = launch_config<CLUSTER>(CLUSTER, &attr, nullptr);
+    int clusters = 0;
+    if (configure<true, CLUSTER>(devid) != IXB_OK ||
+        cudaOccupancyMaxActiveClusters(&clusters, fa_split_kernel<true, CLUSTER>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    n = 1 + clusters * CLUSTER;
+    room.store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+int room_for(int cluster, int devid, int sms) {
+  return cluster == 1 ? sms : cluster == 2 ? room_for<2>(devid) : cluster == 4 ? room_for<4>(devid) : room_for<8>(devid);
 }
 
 }  // namespace
@@ -414,28 +451,43 @@ namespace ixb_host {
 //                  1.41, and 3.4 more for every further round of items
 //   this one       5 for one row of the tile to 8.5 for all 128 (the merge), 1.6 for each key tile of a
 //                  slot; or what reading K and V takes at 6.2 TB/s
-// in one wave of blocks (148 SMs; clusters of 4 and 8 find room for 132 and 120 blocks), or for Sq <= 128 in
-// several.  Taken where it promises 7 %.  1 x 12 heads 18 x 3086: 40.4 -> 11 - 12 us; 1 x 32, 1 x 8192: 95.7
+// in one wave of blocks (148 SMs; clusters of 2, 4 and 8 find room for 148, 132 and 120 blocks there, room_for), or for
+// Sq <= 128 in several.  Taken where it promises 7 %.  1 x 12 heads 18 x 3086: 40.4 -> 11 - 12 us; 1 x 32, 1 x 8192: 95.7
 // -> 27; 3 x 16, 97 x 1840: 26.6 -> 16; 16 x 12, 1 x 2879: 74 -> 59; causal 1 x 4 of 2000: 30.5 -> 16.8, of 4096:
 // 55.9 -> 34.4; 1 x 12 of 1000 without a mask 19.4 -> 15.5.  Where it is not taken: 2 x 8 of 2048 32.9 against
-// 42.9 (two waves), 4 x 4 of 1288 causal 22.7 against 25.7, 2 x 4 of 128 6.9 against 8.5.
+// 42.9 (two waves), 4 x 4 of 1288 causal 22.7 against 25.7, 2 x 4 of 128 6.9 against 8.5.  A causal mask changes
+// neither time: the last query tile of a call sees every key, and it ends last.
 int fa_split_size(int B, int H, int Sq, int Sk) {
-  static const int forced = [] { const char* v = getenv("IXB_FA_SPLIT"); return v != nullptr ? atoi(v) : -1; }();
+  static const int forced = [] {
+    const char* v = getenv("IXB_FA_SPLIT");
+    const int n = v != nullptr ? atoi(v) : -1;
+    return n == 0 || n == 1 || n == 2 || n == 4 || n == 8 ? n : -1;
+  }();
   if (forced >= 0) return forced;
+  const ixb_devinfo* dev = current_device();
+  int devid = 0;
+  if (dev == nullptr || cudaGetDevice(&devid) != cudaSuccess) return 0;
+  const int sms = dev->sm_count;
   const double heads = (double)B * H;
   const double n_q = (Sq + BM - 1) / BM, n_kv = (Sk + BN - 1) / BN;  // (the last query tile sees every key)
   const bool one = Sq <= BM;
-  const double rounds = ceil(((Sq + 2 * BM - 1) / (2 * BM)) * heads / 148);
+  const double rounds = ceil(((Sq + 2 * BM - 1) / (2 * BM)) * heads / sms);
   if (rounds > 1 && !one) return 0;
   const double plain = one ? 5.3 + rounds * 1.41 * n_kv + (rounds - 1) * 3.4 : 5.5 + 1.6 * n_kv;
   const double read = heads * Sk * 2 * HD * 2 / 6.2e6;
   double best = 0.93 * plain;
   int cluster = 0;
   for (int c = 1; c <= kMaxCluster; c *= 2) {
-    const double waves = ceil(n_q * heads * c / (c == 8 ? 120 : c == 4 ? 132 : 148));
-    if (waves > 1 && !one) break;
-    double t = waves * (5 + 3.5 * (one ? Sq : BM) / BM + 1.6 * ceil(n_kv / (2 * c)));
-    t = t > read ? t : read;
+    auto time = [&](int room) {  // with room for so many blocks at a time
+      const double waves = ceil(n_q * heads * c / room);
+      if (waves > 1 && !one) return (double)INFINITY;
+      const double t = waves * (5 + 3.5 * (one ? Sq : BM) / BM + 1.6 * ceil(n_kv / (2 * c)));
+      return t > read ? t : read;
+    };
+    if (!(time(sms) < best)) continue;  // (and worse with less room)
+    const int room = room_for(c, devid, sms);
+    if (room <= 0) continue;
+    const double t = time(room);
     if (t < best) {
       best = t;
       cluster = c;

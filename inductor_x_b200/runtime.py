@@ -103,7 +103,7 @@ _SIGNATURES = {
     "ixb_fa_fwd": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
                            c_int32, c_int32, c_int32, POINTER(c_int64), POINTER(c_int64),
                            POINTER(c_int64), POINTER(c_int64), c_float, c_int, c_void_p, c_void_p]),
-    "ixb_fa_fwd_plan": (c_int, [c_int32] * 4 + [c_int, POINTER(c_int32)]),
+    "ixb_fa_fwd_plan": (c_int, [c_int32] * 4 + [c_int] + [POINTER(c_int32)] * 2),
     "ixb_fa_bwd": (c_int, [c_int] + [c_void_p] * 10 + [c_int32] * 5 + [POINTER(c_int64)] * 8 +
                    [c_float, c_int, c_void_p, c_void_p]),
     "ixb_fa_bwd_scratch_bytes": (c_size_t, [c_int32] * 4 + [c_int, c_size_t]),

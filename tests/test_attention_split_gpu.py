@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from inductor_x_b200 import ops
+from tests.test_attention_plan import plan
 
 pytestmark = pytest.mark.gpu
 
@@ -34,14 +35,27 @@ def check(b, h, sq, sk, causal, dtype=torch.bfloat16, bsnd=False):
 
 # one head to many (clusters of eight blocks down to one), rows of one tile and its edges, key tiles that the
 # slots share evenly, unevenly, and fewer of them than slots
-@pytest.mark.parametrize("b,h", [(1, 1), (1, 4), (1, 16), (2, 20), (7, 16), (13, 16)])
-@pytest.mark.parametrize("sq,sk", [(1, 129), (1, 2879), (5, 257), (127, 1024), (128, 1153), (64, 2049)])
+FEW_ROWS_HEADS = [(1, 1), (1, 4), (1, 16), (2, 20), (7, 16), (13, 16)]
+FEW_ROWS = [(1, 129), (1, 2879), (5, 257), (127, 1024), (128, 1153), (64, 2049)]
+FEW_HEADS = [(129, 129), (300, 1000), (512, 512), (1000, 1000), (640, 3000)]
+
+
+def test_every_cluster_size_is_among_these(cuda):
+    """On a B200; what is 0 here runs in fa_fwd_kernel."""
+    rows = {plan(b, h, sq, sk)[1] for b, h in FEW_ROWS_HEADS for sq, sk in FEW_ROWS}
+    heads = {plan(1, h, sq, sk)[1] for h in (1, 3, 8) for sq, sk in FEW_HEADS}
+    assert rows == {0, 1, 2, 4, 8} and heads == {0, 2, 4, 8}
+    assert plan(2, 16, 400, 700)[1] == 1     # several query tiles, a block each (test_empty_slots_and_hidden_keys)
+
+
+@pytest.mark.parametrize("b,h", FEW_ROWS_HEADS)
+@pytest.mark.parametrize("sq,sk", FEW_ROWS)
 def test_few_rows(cuda, b, h, sq, sk):
     for causal in (False, True):
         check(b, h, sq, sk, causal)
 
 
-@pytest.mark.parametrize("sq,sk", [(129, 129), (300, 1000), (512, 512), (1000, 1000), (640, 3000)])
+@pytest.mark.parametrize("sq,sk", FEW_HEADS)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_few_heads(cuda, sq, sk, dtype):
     for h, causal in ((1, True), (3, False), (8, True)):
@@ -54,3 +68,4 @@ def test_empty_slots_and_hidden_keys(cuda):
     check(1, 2, 1024, 1024, True)
     check(1, 1, 130, 2000, True)
     check(2, 2, 3, 128 * 17 + 1, True)
+    check(2, 16, 400, 700, True)
