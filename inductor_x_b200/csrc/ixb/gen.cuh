@@ -1804,10 +1804,14 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     const long long ustep = blocked ? TEAMS : stride;
     for (long long base = (long long)blockIdx.x * TEAMS * (blocked ? kBatch : 1); base < rows; base += stride * kBatch) {
       if constexpr (STAGED) {
+        // Rows the batch does not have are not fetched: the last row in their place, as every team of every CTA asked
+        // for it, is one line of L2 that answers one request at a time.  Rows enough for half a batch a CTA,
+        // with that row and without: cumsum of 74898 x 56 bf16 9.3 and 3.5 us, LayerNorm of 131072 x 32 fp32 9.1 and
+        // 6.0, sum of 16384 x 64 fp16 (permuted) 4.1 and 1.7.
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
           const long long r = base + u * ustep + c.team;
-          body.fetch(c, r < rows ? r : rows - 1, raw[u]);
+          if (u == 0 || base + u * ustep < rows) body.fetch(c, r < rows ? r : rows - 1, raw[u]);   // (uniform over the CTA)
         }
       }
 #pragma unroll
