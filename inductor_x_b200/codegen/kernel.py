@@ -1291,13 +1291,23 @@ class B200Kernel(SIMDKernel):
         """(LB, LC) when the kept index of a short-row kernel should be walked in tiles: the
         kept space is [..][LC][LB] with LB fastest (the output's order), every streamed row
         operand has rows adjacent in memory along the LC digit and far apart along LB, and the
-        per-row results are contiguous along LB.  None otherwise."""
+        per-row results are contiguous along LB.  None otherwise.
+
+        Digits of no whole number of tiles have smaller ones at their ends, which cost every lane some arithmetic, so
+        they are walked in plain order unless so much is read, and in rows so long, that DRAM's pages cost more.
+        Plain order and tiles: fp16 of a 30 x 33 plane, rows of 16, 32 MB 12.9 and 18.6 us, of 64, 134 MB 24.0 and 36.5;
+        100 x 1300, rows of 64, 378 MB 62.2 and 60.9, 1.06 GB 175 and 156; 48 x 1000, rows of 48, 295 MB 50 and 60; 1000 x
+        1001, rows of 32, 512 MB 86 and 100.  fp32: 1500 x 2001, rows of 16, 192 MB 38.3 and 34.1; 452 x 221, rows of 16,
+        320 MB 61.8 and 53.7 (maximum), 640 MB 167 and 107; 300 x 333, rows of 32, 256 MB 40.9 and 37.2."""
         if self.looped or self._is_dynamic("x") or self._is_dynamic("r0_"):
             return None
         xr, rr = self._xr_roots()
         rnumel = self._static_numel("r0_")
-        if rnumel * config_bytes(self._narrowest_node_dtype()) > 512:
+        size = config_bytes(self._narrowest_node_dtype())
+        if rnumel * size > 512:
             return None
+        large = rnumel * size >= (64 if size == 4 else 128) and \
+            self._numel_hint("x") * rnumel * size > ixb_config.l2_bytes * (1 if size == 4 else 3)
         loads = [v for v in self._ph.values() if v["kind"] == "L" and v["has_r"] and not v["indirect"]]
         if not loads or any(v["stride"] != 1 for v in loads):
             return None
@@ -1317,7 +1327,7 @@ class B200Kernel(SIMDKernel):
                 lc = self._numel_hint("x") // lb       # the outermost digit: FloorDiv without modulus
                 if self._numel_hint("x") != lb * lc:
                     return None
-            if coef_c != rnumel or pieces[1][0] < coef_c * lc or lb < 2 or lc < 2:
+            if coef_c != rnumel or pieces[1][0] < coef_c * lc or (not large and (lb % 16 or lc % 16)) or lb < 2 or lc < 2:
                 return None
             if found is not None and found != (lb, lc):
                 return None

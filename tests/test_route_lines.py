@@ -1,0 +1,40 @@
+"""Lines between the forms of a generated kernel that their sizes decide: which form a group gets on both sides of each.
+Emitted for CPU tensors that nothing is read from; one module stands in for all of them, nothing is launched."""
+import re
+
+import pytest
+import torch
+
+import inductor_x_b200  # noqa: F401
+from inductor_x_b200.codegen import jit
+
+
+@pytest.fixture
+def source(dry_backend, monkeypatch):
+    from torch._inductor.utils import run_and_get_code
+
+    build, built = jit.compile_source, []
+
+    def one_for_all(src, *args, **kwargs):
+        if not built:
+            built.append(build(src, *args, **kwargs))
+        return built[0]
+
+    monkeypatch.setattr(jit, "compile_source", one_for_all)
+
+    def emitted(fn, *shapes):
+        torch._dynamo.reset()
+        args = [torch.zeros(n, dtype=torch.int64) if dtype == "index" else torch.empty(n, dtype=dtype) for n, dtype in shapes]
+        _, code = run_and_get_code(torch.compile(fn, dynamic=False), *args)
+        return "\n".join(code)
+
+    return emitted
+
+
+F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
+
+
+def test_tiles_with_smaller_ones_at_their_ends(source):
+    for shape, dtype, tiled in (((64, 30, 33, 16), F32, False), ((300, 30, 33, 64), F16, False), ((64, 48, 1000, 48), F16, False),
+                                ((16, 32, 48, 64), F16, True), ((50, 452, 221, 16), F32, True), ((64, 100, 1300, 64), F16, True)):
+        assert ("tile_order<" in source(lambda x: x.permute(0, 2, 1, 3).sum(3), (shape, dtype))) == tiled, shape

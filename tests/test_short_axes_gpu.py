@@ -34,6 +34,13 @@ def test_rows_in_smaller_tiles(cuda, b, c, dtype, d):
     close(compiled(lambda x: x.permute(0, 2, 1, 3).sum(3), x), x.double().permute(0, 2, 1, 3).sum(3), dtype, d)
 
 
+# the same where so much is read that the smaller tiles at the ends are taken
+@pytest.mark.parametrize("shape,dtype", [((200, 33, 70, 96), torch.float32), ((37, 130, 1000, 16), torch.float32), ((100, 47, 700, 64), torch.float16)])
+def test_rows_in_smaller_tiles_of_large_operands(cuda, shape, dtype):
+    x = data(cuda, shape, dtype)
+    assert torch.equal(compiled(lambda x: x.permute(0, 2, 1, 3).amax(3), x), x.permute(0, 2, 1, 3).amax(3))
+
+
 # 1, 2 (ragged), 4, 5 and 6 vectors of four; one row, rows for a few blocks, and more than three batches of
 # what is resident (blocks that see one batch)
 @pytest.mark.parametrize("d", [4, 7, 16, 20, 24])
