@@ -1522,7 +1522,9 @@ class B200Kernel(SIMDKernel):
                 src.writeline(f"static constexpr bool kLooped = {'true' if self.looped else 'false'};   // row walked in chunks")
                 stream = tiling is not None or any(raw != "RawRow" for *_, raw in self.staged) or \
                     any(v["kind"] == "S" and v["has_r"] for v in self._ph.values())
-                src.writeline(f"static constexpr bool kStream = {'true' if stream else 'false'};   // a block for every few rows of sub-warp teams")
+                moved = len(self.staged) + sum(v["kind"] == "S" and v["has_r"] for v in self._ph.values())
+                src.writeline(f"static constexpr int kStream = {moved if stream else 0};   // rows moved for each one worked on, where sub-warp "
+                              "teams may get a block for every few of them")
                 src.writeline(f"static constexpr bool kTiled = {'true' if tiling is not None else 'false'};   // kept index walked in tiles")
                 pitch, first, period = shift or (0, 0, 0)
                 src.writeline(f"static constexpr int kShiftPeriod = {period};   // rows after which the offset from a "

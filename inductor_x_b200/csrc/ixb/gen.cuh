@@ -1741,13 +1741,17 @@ template <class U> int finish_columns(const float* partial, long long rows, int 
 }
 
 // Sub-warp teams whose threads load nothing once for all rows get a block for every batch of four rows a
-// team (see stream_grid) where there are more than the resident blocks would see in three batches: the
-// permuted sum of 64 x 128 x 256 x 64 fp16 48.9 -> 45.4 us.
-template <class Body, int TEAM, bool STAGED> constexpr bool kStreamRows = TEAM < 32 && STAGED && Body::kStream && Body::kConsts == 0;
+// team (see stream_grid) where there are more than the resident blocks would see in three batches and they move
+// more than stays in L2: the permuted sum of 64 x 128 x 256 x 64 fp16 48.9 -> 45.4 us, softmax of 2^24 fp32
+// in rows of 16 24.7 -> 22.0, LayerNorm in rows of 32 24.2 -> 22.0.  Below that nothing drifts apart in DRAM and the
+// blocks' starts are what is left: of 2^22 6.0 -> 6.9, 5.8 -> 6.1, softmax of 65536 x 64 bf16 4.1 -> 4.7.
+template <class Body, int TEAM, bool STAGED> constexpr bool kStreamRows = TEAM < 32 && STAGED && Body::kStream > 0 && Body::kConsts == 0;
+// the L2 of a B200; what a kernel moves beyond it comes from and goes to DRAM
+constexpr long long kL2Bytes = 126ll << 20;
 
 template <class Body, typename T, int TEAM, int TEAMS, int VPT, int MIN_CTAS, int PF, int COLS, bool STAGED>
 __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
-    row_gen_kernel(const Body body, const long long rows, const int cols) {
+    row_gen_kernel(const Body body, const long long rows, const int cols, const bool a_batch_each) {
   // Rows off a 16-byte boundary repeat their offset every kShiftPeriod rows.  Block b works on rows b,
   // b + period, ... only: its offset stays what it is, and the row is worked on in the aligned
   // vectors of memory as if it began there (`off` elements that are masked), per-column operands
@@ -1798,9 +1802,9 @@ __global__ void __launch_bounds__(TEAM* TEAMS, MIN_CTAS)
     // places instead of 512 bytes - and DRAM pages are used up while they are open (sum over the
     // last axis of a permuted 64 x 128 x 256 x 64 fp16: 54.6 -> 52.4 us).  Rows in memory order
     // gain nothing from it (43.3 against 44.8 us) and keep the strided batches.
-    // Without per-column operands a block is started for every batch (launch_row_gen): the batches in
-    // flight then follow each other through memory, and so do the rows of a batch.
-    const bool blocked = kStreamRows<Body, TEAM, STAGED> ? rows > stride * (kBatch - 1) : Body::kTiled && rows >= stride * kBatch;
+    // Where a block is started for every batch (launch_row_gen) the batches in flight follow each other
+    // through memory, and so do the rows of a batch.
+    const bool blocked = a_batch_each || (Body::kTiled && rows >= stride * kBatch);
     const long long ustep = blocked ? TEAMS : stride;
     for (long long base = (long long)blockIdx.x * TEAMS * (blocked ? kBatch : 1); base < rows; base += stride * kBatch) {
       if constexpr (STAGED) {
@@ -1878,9 +1882,14 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
     } else if (grid > groups) {
       grid = groups;
     }
-    if (kStreamRows<Body, TEAM, true> && groups > 3 * (long long)sms * resident) grid = (groups + 3) / 4;
+    bool a_batch_each = false;
+    if (kStreamRows<Body, TEAM, true> && groups > 3 * (long long)sms * resident &&
+        rows * (cols * (long long)sizeof(T) * Body::kStream) > kL2Bytes) {
+      grid = (groups + 3) / 4;
+      a_batch_each = true;
+    }
     if (blocks != nullptr) *blocks = grid;
-    return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
+    return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols, a_batch_each);
   }
   auto kern = row_gen_kernel<Body, T, TEAM, TEAMS, VPT, MIN_CTAS, PF, COLS, false>;
   const int resident = row_resident(kern, TEAM * TEAMS, smem);
@@ -1889,7 +1898,7 @@ int launch_row_gen(const Body& body, long long rows, int cols, void* stream, boo
   if (Body::kColumns > 0 && grid > Body::kPartials) grid = Body::kPartials;
   if (grid > groups) grid = groups;
   if (blocks != nullptr) *blocks = grid;
-  return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols);
+  return (int)launch_pdl(kern, (unsigned)grid, TEAM * TEAMS, smem, (cudaStream_t)stream, body, rows, cols, false);
 }
 
 // ---- outer reduction family -----------------------------------------------------------------

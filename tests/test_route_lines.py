@@ -38,3 +38,9 @@ def test_tiles_with_smaller_ones_at_their_ends(source):
     for shape, dtype, tiled in (((64, 30, 33, 16), F32, False), ((300, 30, 33, 64), F16, False), ((64, 48, 1000, 48), F16, False),
                                 ((16, 32, 48, 64), F16, True), ((50, 452, 221, 16), F32, True), ((64, 100, 1300, 64), F16, True)):
         assert ("tile_order<" in source(lambda x: x.permute(0, 2, 1, 3).sum(3), (shape, dtype))) == tiled, shape
+
+
+def test_rows_that_blocks_are_started_for(source):
+    """How many rows' worth of bytes a row moves, which the launch holds against L2; 0 where blocks are resident."""
+    for fn, moved in ((lambda x: torch.softmax(x, -1), 2), (lambda x: x.sum(-1), 0)):
+        assert f"static constexpr int kStream = {moved};" in source(fn, ((3000, 16), F32))
