@@ -1246,20 +1246,33 @@ class B200Kernel(SIMDKernel):
         nk = 16 if len(tl) == 1 and -(-chunks // 16) * 16 <= -(-chunks // 8) * 8 else 8
         return lb, dc, lc, nk, (16 * per - (per - 1)) // 4 * 4, strides
 
-    def _moves_bytes(self, body_text: str) -> bool:
-        """Whether a pointwise group is worth a block for every 256 vectors (``stream_grid``): a thread
-        moves 48 bytes or more, whole vectors all of them, and what it computes is next to nothing.  A
-        block that lives for one vector a thread pays its start with what it moves.  Resident grid
-        against a block per 256 vectors: bf16 to fp32 of 8192 x 8192 84 -> 60 us, a * b + c in fp32 127 ->
-        114, a + b in bf16 63.0 -> 57.8, of 2048 x 4096 9.36 -> 8.98; but 32 bytes a thread 43.5 -> 45.0
-        (an inner permute) and 43.3 -> 43.4, silu(a) * b in bf16 28.2 -> 29.3, a rotation with masked loads
-        14.7 -> 15.6."""
-        if f"{G}gather(" in body_text or f"{G}scatter" in body_text or f"{G}atomic" in body_text:
-            return False
-        if not set(re.findall(r"ixb::gen::op::(\w+)", body_text)) <= _LIGHT_OPS:
-            return False
-        moved = re.findall(r"(?:ldvec|stvec)<([\w: ]+), kVec", body_text)
-        return sum(_CTYPE_BYTES.get(t, 0) for t in moved) * self.vec >= 48
+    def _stream_threads(self, body_text: str, kc) -> int:
+        """From how many threads' work on a pointwise group is worth a block for every 256 of them (``stream_grid``), or
+        0: never.  A thread moves 48 bytes or more, whole vectors all of them, and what it computes is next to nothing: a
+        block that lives for one vector a thread pays its start with what it moves.  And all of them
+        move more than stays in L2, so that DRAM is what they wait for; what an operation before has left in
+        L2 comes faster than the blocks start.  Resident grid against a block per 256 threads, inputs in L2 /
+        in DRAM: a + b of 2^23 bf16 5.1 and 5.0 / 10.0 and 9.7 us, of 2^24 (100 MB) 12.8 and 14.8 / 17.8 and 17.1, of
+        2^24.5 (142 MB) 23.6 and 22.6 / 25.1 and 23.8, of 2^26 63.8 and 58.5 / 65.6 and 60.0.  32 bytes a thread
+        43.5 and 45.0 (an inner permute) and 43.3 and 43.4, silu(a) * b in bf16 28.2 and 29.3, a rotation with masked loads
+        14.7 and 15.6.
+
+        A result stored in more than one word a thread (16 bits widened to 32) is better off with it at every size:
+        bf16 to fp32 of 2^22 6.6 and 6.2 / 6.9 and 6.3, of 2^24 21.5 and 18.2 / 23.5 and 18.3, of 2^26 84 and 61.
+        Register tiles (``kc``), a thread of which moves several vectors, are from a third of L2 on: fp32 of
+        2^22 (33 MB) 6.3 and 6.8 / 6.8 and 6.9, fp16 of 2^23.5 (47 MB) 9.3 and 8.5, fp32 of 2^24 23.1 and 21.5."""
+        if f"{G}gather(" in body_text and kc is None or f"{G}scatter" in body_text or f"{G}atomic" in body_text:
+            return 0
+        if kc is None and not set(re.findall(r"ixb::gen::op::(\w+)", body_text)) <= _LIGHT_OPS:
+            return 0
+        sizes = {name: [_CTYPE_BYTES.get(t, 0) for t in re.findall(rf"{name}<([\w: ]+), kVec", body_text)] for name in ("ldvec", "stvec")}
+        moved = (sum(sizes["ldvec"]) + sum(sizes["stvec"])) * self.vec
+        if kc is not None:
+            moved = kc * (moved + self.vec * sum(config_bytes(v["dtype"]) for v in self._tile_loads.values()))
+            return ixb_config.l2_bytes // 3 // moved
+        if moved < 48:
+            return 0
+        return 1 if max(sizes["stvec"]) * self.vec > 16 else ixb_config.l2_bytes // moved
 
     def _register_tile(self, order):
         """kC (elements per 128-bit load along C) when every strided load of the group can be
@@ -1630,8 +1643,8 @@ class B200Kernel(SIMDKernel):
                     body_text = body_text.replace(tag, text)
                 for tag, v in getattr(self, "_row_loads", {}).items():
                     body_text = body_text.replace(tag, (odd and self._row_text(v, odd)) or v["gather"])
-                streams = not self.indirect and (kc is not None or self._moves_bytes(body_text))
-                src.writeline(f"static constexpr bool kStream = {'true' if streams else 'false'};   // a block for every 256 threads' work")
+                streams = 0 if self.indirect else self._stream_threads(body_text, kc)
+                src.writeline(f"static constexpr long long kStream = {streams};   // a block for every 256 threads' work from so many on")
                 if kc is not None:
                     lb, dc, lc = order
                     nbv = lb // self.vec

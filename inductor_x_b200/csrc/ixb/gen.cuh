@@ -433,10 +433,11 @@ __global__ void __launch_bounds__(256) pointwise_tile_gen_kernel(const Body body
 // at a time spread over all they have reached: a copy of 512 MB takes 160 us this way and 178 - 186
 // (148 x 8 and x 4 blocks) the other, the transpose of 4096 x 512 x 128 fp16 157 against 199, an inner
 // permute of the same size 170.5 against 175.5.  Rows gathered through an index are in no order anyway and
-// keep the resident grid (23.8 against 26.0 us for 262144 rows of 256 bytes out of 2^20).
+// keep the resident grid (23.8 against 26.0 us for 262144 rows of 256 bytes out of 2^20), and so does what stays in L2
+// (Body::kStream: the threads from which this holds, 0 for never; the generator's _stream_threads says how it is chosen).
 template <class Body> inline long long stream_grid(long long threads, long long resident) {
   long long grid = (threads + 255) / 256;
-  const long long most = Body::kStream ? 0x7fffffffLL : resident;
+  const long long most = Body::kStream > 0 && threads >= Body::kStream ? 0x7fffffffLL : resident;
   if (grid > most) grid = most;
   return grid < 1 ? 1 : grid;
 }
@@ -532,8 +533,8 @@ template <class Body, int LB> int launch_pointwise_rows(const Body& body, long l
   if (xnumel <= 0) return 0;
   const long long slots = xnumel / LB * ((LB + 2 * (Body::kVec - 1)) / Body::kVec);
   if (slots > 0x7fffffffLL) return (int)cudaErrorInvalidValue;  // (the generator keeps the index below 2^31, and rows past a vector)
-  static const long long cap_a = Body::kStream ? 0 : resident_ctas(pointwise_rows_gen_kernel<Body, LB, true>, 256);
-  static const long long cap_u = Body::kStream ? 0 : resident_ctas(pointwise_rows_gen_kernel<Body, LB, false>, 256);
+  static const long long cap_a = resident_ctas(pointwise_rows_gen_kernel<Body, LB, true>, 256);
+  static const long long cap_u = resident_ctas(pointwise_rows_gen_kernel<Body, LB, false>, 256);
   const long long grid = stream_grid<Body>(slots, aligned ? cap_a : cap_u);
   if (aligned) pointwise_rows_gen_kernel<Body, LB, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, slots);
   else pointwise_rows_gen_kernel<Body, LB, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, slots);
@@ -555,7 +556,7 @@ int launch_pointwise_smem(const Body& body, long long xnumel, void* stream, bool
 template <class Body> int launch_pointwise_tile(const Body& body, long long xnumel, void* stream, bool aligned) {
   if (xnumel <= 0) return 0;
   if (!aligned) return launch_pointwise(body, xnumel, stream, false);
-  static const long long cap = Body::kStream ? 0 : resident_ctas(pointwise_tile_gen_kernel<Body>, 256);
+  static const long long cap = resident_ctas(pointwise_tile_gen_kernel<Body>, 256);
   const long long grid = stream_grid<Body>(xnumel / ((long long)Body::kVec * Body::kTileC), cap);
   pointwise_tile_gen_kernel<Body><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
   return (int)cudaGetLastError();
@@ -563,8 +564,8 @@ template <class Body> int launch_pointwise_tile(const Body& body, long long xnum
 
 template <class Body> int launch_pointwise(const Body& body, long long xnumel, void* stream, bool aligned = false) {
   if (xnumel <= 0) return 0;
-  static const long long cap_a = Body::kStream ? 0 : resident_ctas(pointwise_gen_kernel<Body, true>, 256);
-  static const long long cap_u = Body::kStream ? 0 : resident_ctas(pointwise_gen_kernel<Body, false>, 256);
+  static const long long cap_a = resident_ctas(pointwise_gen_kernel<Body, true>, 256);
+  static const long long cap_u = resident_ctas(pointwise_gen_kernel<Body, false>, 256);
   const long long grid = stream_grid<Body>((xnumel + Body::kVec - 1) / Body::kVec, aligned ? cap_a : cap_u);
   if (aligned) pointwise_gen_kernel<Body, true><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);
   else pointwise_gen_kernel<Body, false><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(body, xnumel);

@@ -44,3 +44,14 @@ def test_rows_that_blocks_are_started_for(source):
     """How many rows' worth of bytes a row moves, which the launch holds against L2; 0 where blocks are resident."""
     for fn, moved in ((lambda x: torch.softmax(x, -1), 2), (lambda x: x.sum(-1), 0)):
         assert f"static constexpr int kStream = {moved};" in source(fn, ((3000, 16), F32))
+
+
+def test_threads_that_blocks_are_started_from(source):
+    def threads(fn, *shapes):
+        return int(re.search(r"static constexpr long long kStream = (\d+);", source(fn, *shapes)).group(1))
+
+    n = 1 << 20
+    assert 2 ** 24 / 8 < threads(lambda a, b: a + b, ((n,), BF16), ((n,), BF16)) < 2 ** 24.5 / 8    # 100 and 142 MB
+    assert threads(lambda a: a.float(), ((n,), BF16)) == 1
+    assert threads(lambda a: a * 2, ((n,), BF16)) == threads(lambda a, b: torch.exp(a) * b, ((n,), BF16), ((n,), BF16)) == 0
+    assert 2 ** 22 / 16 < threads(lambda x: (x.transpose(1, 2) + 1).contiguous(), ((8, 64, 64), F32)) < 2 ** 23 / 16
