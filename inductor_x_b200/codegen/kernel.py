@@ -1171,34 +1171,47 @@ class B200Kernel(SIMDKernel):
             found = (lb, dc, lc)
         return found
 
-    def _odd_rows(self):
+    def _odd_rows(self, body_text: str):
         """The length LB of the rows that a pointwise group without a better form is walked in: vectors
         that end with their row (``pointwise_rows_gen_kernel``).  Where LB is no whole number of vectors a
         vector of the flat index reaches into the next row, so that what is contiguous along a row (a
         gathered row, a per-column operand) or constant over it (an index, a per-row operand) would be
-        loaded element by element.  None where nothing is gained: rows of less than four vectors, where the ends
-        are most of the work (gather of 500000 x 17 fp16 21.0 us so or so), and of less than sixteen unless
-        what is loaded in runs is as large as the result and not an operand that all rows share (x * w + b,
-        100000 x 37 fp32, 8.2 against 10.3).  Gather of 100000 x 333 bf16 89 -> 32 us, of 50000 x 1023 fp32 136 ->
-        67; permuted 64 x 65 x 66 x 37 fp16 59 -> 17; x * w of 20000 x 3333 bf16 79 -> 55."""
+        loaded element by element.
+
+        What it gains goes with the vector; what it costs, the parts of vectors at the ends of every row and the
+        warps that hold one, with the rows.  So the line is LB times the vector, by what is read so: rows that
+        are picked or permuted, the part of a longer row, one value a row, a run that all rows share (which L1 has
+        at hand element by element).  Element by element and so, 2^24 elements, us, inputs in L2:
+        gather of rows of 127 bf16 10.4 and 9.7, of 333 10.6 and 8.7, of 1023 10.2 and 7.3; of 191 fp32 10.8 and 11.3, of
+        333 11.6 and 10.7; permuted rows of 65 bf16 21.8 and 20.3, of 333 22.8 and 15.2, of 127 fp32 26.6 and 26.3, of 333
+        26.9 and 24.7; slices of 127 bf16 13.0 and 16.3, of 333 13.0 and 14.0, of 1023 13.1 and 11.3; x * r of 333 bf16
+        11.5 and 11.3, of 1023 11.3 and 9.2; x * w of 1023 bf16 13.3 and 14.1, of 4097 13.0 and 12.3.  fp32 gains
+        nothing from the last three (slices of 2047 23.6 and 25.3, x * r 22.8 and 23.4).  Where there is arithmetic to
+        speak of the vectors that are cut in two do it twice: gelu of gathered rows of 333 bf16 15.9 and 16.2, of 2047
+        15.8 and 13.3, of 1023 fp32 15.7 and 17.5; gelu(x + w) of 4097 bf16 21.1 and 23.3."""
         loads = [*getattr(self, "_tile_loads", {}).values(), *getattr(self, "_row_loads", {}).values()]
         if self.is_row or self._is_dynamic("x") or not loads or not self._small_index():
             return None
+        light = set(re.findall(r"ixb::gen::op::(\w+)", body_text)) <= _LIGHT_OPS | {"lt"}   # (negative indices are wrapped)
         xsym = self._root("x").symbol()
+        pieces = {id(v): split[1] for v in loads if (split := index_ir._axis_pieces(v["exp"], xsym)) is not None}
         lengths = []
-        for v in loads:
-            split = index_ir._axis_pieces(v["exp"], xsym)
-            if split is not None:
-                lengths += [m for c, d, m in split[1] if d == 1 and m is not None] or \
-                    [min(d for c, d, m in split[1])] * bool(split[1])
+        for p in pieces.values():
+            lengths += [m for c, d, m in p if d == 1 and m is not None] or [min(d for c, d, m in p)] * bool(p)
         for lb in sorted(set(lengths), key=lambda n: (-lengths.count(n), n)):
-            if lb % self.vec == 0 or lb < 4 * self.vec or self._numel_hint("x") % lb:
+            if lb % self.vec == 0 or self._numel_hint("x") % lb:
                 continue
-            read = [v for v in loads if self._row_text(v, lb)]
-            if lb < 16 * self.vec:
-                read = [v for v in read if v["indirect"] or (len(index_ir._axis_pieces(v["exp"], xsym)[1]) > 1)]
-            if read:
-                return lb
+            for v in loads:
+                if not self._row_text(v, lb):
+                    continue
+                if not any(d == 1 for c, d, m in pieces[id(v)]):
+                    line = 8000                                       # one value a row
+                else:
+                    line = 1024 if v["indirect"] or len(pieces[id(v)]) > 2 else 4096 if len(pieces[id(v)]) == 2 else 32768
+                if not light:
+                    line = max(line, 16384) if line < 32768 else math.inf
+                if lb * self.vec >= line and (self.vec == 8 or line == 1024):
+                    return lb
         return None
 
     def _row_text(self, v, lb: int):
@@ -1636,7 +1649,7 @@ class B200Kernel(SIMDKernel):
                 smem = self._smem_tile()
                 tile_loads = getattr(self, "_tile_loads", {})
                 tiled = kc is not None or smem is not None
-                odd = None if tiled else self._odd_rows()
+                odd = None if tiled else self._odd_rows(body_text)
                 for n, (tag, v) in enumerate(tile_loads.items()):
                     text = f"(STAGED ? {G}take(raw.t{n}, ci) : {v['gather']})" if tiled else \
                         (odd and self._row_text(v, odd)) or v["gather"]

@@ -367,7 +367,9 @@ __global__ void __launch_bounds__(256) pointwise_rows_gen_kernel(const Body body
     }
     if (x + n > LB) n = LB - x;
     if (n <= 0) continue;
-    if (ALIGNED && n == V) body.template tile<true>(first + x, V);
+    // one form for the whole warp: lanes at an end of a row would have the others wait for a second pass over the body
+    // (gelu(x + w) of 2^24 bf16 in rows of 333 39.5 -> 30.4 us, gather of such rows 9.4 -> 8.7)
+    if (ALIGNED && __all_sync(__activemask(), n == V)) body.template tile<true>(first + x, V);
     else body.template tile<false>(first + x, n);
   }
 }

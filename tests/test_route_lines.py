@@ -55,3 +55,24 @@ def test_threads_that_blocks_are_started_from(source):
     assert threads(lambda a: a.float(), ((n,), BF16)) == 1
     assert threads(lambda a: a * 2, ((n,), BF16)) == threads(lambda a, b: torch.exp(a) * b, ((n,), BF16), ((n,), BF16)) == 0
     assert 2 ** 22 / 16 < threads(lambda x: (x.transpose(1, 2) + 1).contiguous(), ((8, 64, 64), F32)) < 2 ** 23 / 16
+
+
+@pytest.mark.parametrize("dtype,longer,shorter", [(F16, 333, 127), (F32, 333, 127)])
+def test_odd_rows_that_are_picked_or_permuted(source, dtype, longer, shorter):
+    for n, walked in ((longer, True), (shorter, False)):
+        assert ("launch_pointwise_rows" in source(lambda t, i: t[i], ((301, n), dtype), ((77,), "index"))) == walked
+        assert ("launch_pointwise_rows" in source(lambda x: (x.permute(0, 2, 1, 3) * 2).contiguous(), ((2, 5, 6, n), dtype))) == walked
+
+
+def test_odd_rows_that_share_a_run_or_a_value(source):
+    def walked(fn, n, dtype, *others):
+        return "launch_pointwise_rows" in source(fn, ((60, n), dtype), *((shape, dtype) for shape in others))
+
+    for n, dtype, one_a_row, shared, part in ((333, F16, False, False, False), (1023, F16, True, False, True), (4097, F16, True, True, True),
+                                              (4097, F32, False, False, False)):
+        assert walked(lambda x, r: torch.maximum(x, r), n, dtype, (60, 1)) == one_a_row
+        assert walked(lambda x, w: torch.maximum(x, w), n, dtype, (n,)) == shared
+        assert walked(lambda x: x[:, 2:] * 2, n + 2, dtype) == part
+    # arithmetic that a warp with an end in it would do for vectors that are cut
+    for n, dtype in ((65, F32), (333, F16), (4097, F16)):
+        assert not walked(lambda x, w: torch.nn.functional.gelu(x + w), n, dtype, (n,))
