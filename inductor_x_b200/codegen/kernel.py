@@ -1232,16 +1232,17 @@ class B200Kernel(SIMDKernel):
     def _smem_tile(self):
         """(LB, dC, LC, vectors of an output row to a block, columns to a block at most, stride of each tile
         load along the flat index) when the group is transposed by way of shared memory
-        (``pointwise_smem_gen_kernel``), or None.  It takes what register tiles do not, from 32 elements on
-        in both digits (shorter ones leave most of a block without work: 30000 x 16 x 17 fp32 28 us by
-        gathers, 42 so), for one or two operands of 16 or 32 bits; more would leave room for two blocks an SM."""
-        digits, tl = self._transposing_digits(), getattr(self, "_tile_loads", None)
-        if digits is None or self._register_tile(self._transposing_order()) is not None or not 1 <= len(tl) <= 2:
+        (``pointwise_smem_gen_kernel``), or None.  It takes what register tiles do not, where it pays (see
+        ``_smem_pays``), for one or two operands of 16 or 32 bits; more would leave room for two blocks an SM."""
+        digits, tl, order = self._transposing_digits(), getattr(self, "_tile_loads", None), self._transposing_order()
+        if digits is None or self._register_tile(order) is not None or not 1 <= len(tl) <= 2:
             return None
         lb, dc, lc = digits
         if lb < 32 or lc < 32 or not self._small_index() or self.indirect or self.vec not in (4, 8):
             return None
         if not all(v["dtype"] in (torch.float32, torch.float16, torch.bfloat16) for v in tl.values()):
+            return None
+        if not self._smem_pays(lb, lc, order is not None, min(config_bytes(v["dtype"]) for v in tl.values())):
             return None
         xsym = self._root("x").symbol()
         strides = []
@@ -1258,6 +1259,26 @@ class B200Kernel(SIMDKernel):
         chunks = -(-(lb + self.vec - 1) // self.vec)
         nk = 16 if len(tl) == 1 and -(-chunks // 16) * 16 <= -(-chunks // 8) * 8 else 8
         return lb, dc, lc, nk, (16 * per - (per - 1)) // 4 * 4, strides
+
+    @staticmethod
+    def _smem_pays(lb: int, lc: int, ordered: bool, size: int) -> bool:
+        """Whether a transpose goes by way of shared memory: output rows of lb elements of `size` bytes, source rows of lc.
+
+        The other way is a gather an element.  Where the lanes can be `ordered` along the source rows it reads whole
+        sectors, and only long source rows are better off here: gathers and this, 2^23 elements, us, 40 x 64
+        fp16 8.9 and 11.1, x 96 11.0 and 9.1; 128 x 32 fp16 9.8 and 13.6, 96 x 96 11.2 and 8.0; 100 x 160 fp32 from DRAM
+        20.9 and 14.2.  Otherwise a warp's gathers fall on rows lc apart.  If those are whole 16-byte words apart they
+        fall on the same few sets of the caches, and this pays from 6 KB a tile on: 40 x 40 fp16 9.9 and 14.2, 64 x 48
+        10.7 and 10.4, 100 x 40 18.3 and 13.2; 40 x 40 fp32 13.8 and 14.2, 96 x 40 25.5 and 12.6 - with output rows off
+        a boundary, whose ends are parts of vectors, from longer ones on: 33 x 64 fp16 and one more operand 18.5 and 23.2,
+        65 x 128 23.2 and 20.1, 65 x 128 fp32 26.2 and 29.5, 127 x 72 30.8 and 20.6.  If not, L1 serves the
+        gathers until the output rows are long: 65 x 65 fp16 13.8 and 19.1, 129 x 129 13.7 and 17.9, 160 x 201 12.6 and
+        9.6, 200 x 201 14.3 and 8.6; 65 x 65 fp32 15.6 and 30.6, 127 x 127 17.9 and 22.3, 160 x 127 19.4 and 13.4."""
+        if ordered:
+            return lb >= 40 and lc >= 96
+        if lc * size % 16:
+            return lb >= 160
+        return lb * lc * size > 6144 and (lb * size % 16 == 0 or lb >= (64 if size == 2 else 96))
 
     def _stream_threads(self, body_text: str, kc) -> int:
         """From how many threads' work on a pointwise group is worth a block for every 256 of them (``stream_grid``), or

@@ -76,3 +76,11 @@ def test_odd_rows_that_share_a_run_or_a_value(source):
     # arithmetic that a warp with an end in it would do for vectors that are cut
     for n, dtype in ((65, F32), (333, F16), (4097, F16)):
         assert not walked(lambda x, w: torch.nn.functional.gelu(x + w), n, dtype, (n,))
+
+
+@pytest.mark.parametrize("b,c,dtype,shared", [
+    (32, 32, F16, False), (40, 64, F16, False), (40, 96, F16, True), (100, 160, F32, True),      # lanes ordered along the source rows
+    (48, 48, F16, False), (72, 48, F16, True), (48, 40, F32, True), (33, 72, F32, False), (127, 72, F32, True),   # rows whole words apart
+    (33, 33, F32, False), (129, 129, F16, False), (200, 201, F16, True), (160, 127, F32, True)])
+def test_transposes_by_shared_memory(source, b, c, dtype, shared):
+    assert ("launch_pointwise_smem" in source(lambda x: (x.transpose(1, 2) + 1).contiguous(), ((3, b, c), dtype))) == shared
