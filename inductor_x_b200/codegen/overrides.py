@@ -62,14 +62,19 @@ class IxbExprPrinter(ExprPrinter):
 
     def _print_FloorDiv(self, expr):
         x, d = expr.args
-        return f"{OP}idiv{self.bits}({self.doprint(x)}, {self.doprint(d)})"
+        return f"{OP}idiv{self._bits(d)}({self.doprint(x)}, {self.doprint(d)})"
 
     def _print_ModularIndexing(self, expr):
         x, d, m = expr.args
         xs = self.doprint(x)
         if d != 1:
-            xs = f"{OP}idiv{self.bits}({xs}, {self.doprint(d)})"
-        return f"{OP}imod{self.bits}({xs}, {self.doprint(m)})"
+            xs = f"{OP}idiv{self._bits(d)}({xs}, {self.doprint(d)})"
+        return f"{OP}imod{self._bits(m)}({xs}, {self.doprint(m)})"
+
+    def _bits(self, d) -> str:
+        # a power of two is a shift or a mask in 64 bits too, and of signed numbers the compiler sees that a
+        # vector's elements have the same quotient (unsigned ones might wrap): one load instead of four
+        return "" if d.is_Integer and int(d) & (int(d) - 1) == 0 else self.bits
 
     def _print_Min(self, expr):
         out = self.doprint(expr.args[0])

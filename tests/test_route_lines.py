@@ -84,3 +84,8 @@ def test_odd_rows_that_share_a_run_or_a_value(source):
     (33, 33, F32, False), (129, 129, F16, False), (200, 201, F16, True), (160, 127, F32, True)])
 def test_transposes_by_shared_memory(source, b, c, dtype, shared):
     assert ("launch_pointwise_smem" in source(lambda x: (x.transpose(1, 2) + 1).contiguous(), ((3, b, c), dtype))) == shared
+
+
+def test_digits_by_a_power_of_two_keep_64_bits(source):
+    for n, bits in ((4, ""), (8, ""), (12, "32")):
+        assert f"idiv{bits}(xindex, {n}LL)" in source(lambda x, r: x * r, ((999, n), F32), ((999, 1), F32))
