@@ -41,10 +41,13 @@ int softmax_layernorm_t(const void* x, const void* g, const void* gamma, const v
   return IXB_ERR_UNSUPPORTED;
 }
 
+// Vectors of memory that a row may touch, wherever it begins.
+int64_t vectors_touched(int64_t cols, int vec) { return (cols + vec - 1 + vec - 1) / vec; }
+
 // Launch shape of a row worked on in the vectors of memory: the least of the dispatched capacities that
 // holds the vectors it may touch.
 bool choose_shift(int64_t cols, int vec, ixb_cfg* cfg) {
-  const int64_t touched = (cols + vec - 1 + vec - 1) / vec;
+  const int64_t touched = vectors_touched(cols, vec);
   for (int team = 32; team <= 1024; team *= 2)
     for (int vpt = team == 32 ? 1 : 3; vpt <= 4; ++vpt)
       if ((int64_t)team * vpt >= touched) {
@@ -71,11 +74,16 @@ int rmsnorm_t(const void* x, const void* res, const void* w, void* y, void* h_ou
   // ahead, in place of two that are shifted on the spot.  Measured, covering words -> this: fp32 7847 x 2077
   // 58.8 -> 21.0 us, with residual 100 -> 47.8; fp16 1094 x 9460 21.7 -> 10.1; bf16 40000 x 1537 with
   // residual 185 -> 97; 100000 x 67 36.8 -> 25.1; fp32 1094 x 9460, the nearest, 15.7 -> 14.9.
+  // Short rows of 16 bits, so few of them that hardly one is asked for ahead of another, keep the covering words:
+  // the words at their ends, cut element by element, are most of the work.  Covering words and this, fp16:
+  // 250 x 77 2.0 and 2.3 us, 250 x 333 2.1 and 2.4, 1000 x 131 2.3 and 2.4, with residual 2000 x 131 3.1 and 3.5; from
+  // 50000 vectors on, 4000 x 131 3.4 and 3.3, 2000 x 333 3.1 and 3.0, 8000 x 77 4.1 and 3.6.
   const uintptr_t at = reinterpret_cast<uintptr_t>(x) & 15u;
   auto alike = [at](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15u) == at; };
   ixb_cfg shift = {};
   if (!al && at % sizeof(T) == 0 && alike(res) && alike(y) && alike(h_out) && (user == nullptr || user->team <= 0 || user->vpt <= 0) &&
-      choose_shift(cols, Body::kVec, &shift)) {
+      choose_shift(cols, Body::kVec, &shift) &&
+      !(sizeof(T) == 2 && shift.team == 32 && shift.vpt <= (RES ? 1 : 2) && rows * vectors_touched(cols, Body::kVec) < 50000)) {
     shift.grid = cfg.grid;
     cfg = shift;
     int period = Body::kVec;
