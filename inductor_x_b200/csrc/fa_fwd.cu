@@ -416,12 +416,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 // blocks fall on the SMs at first, by what stays in L2 with more keys: 300 x 384 128 heads 23.0 and 24.1, 144 24.6 and
 // 22.7, 256 37.1 and 35.5; 300 x 500 128 heads 25.7 and 24.7, 160 31.0 and 32.9; 300 x 1000 128 heads 39.0 and 37.0, 320
 // 84.9 and 78.0; 261 x 700 256 heads 61.6 and 53.4.
+// Where all blocks run at once no order is the better one for the end, and neighbours read the same K and V in
+// groups of 8: 1 x 32 heads 1024 x 4096 58.1 us (in one group 59.6), 4 x 8 1000 x 3000 45.6 (46.1), 2 x 16 900 x 2000 32.8 (33.0).
 int head_group_of(int B, int H, int Sq, int Sk, int causal) {
   static const int group_env = [] { const char* v = getenv("IXB_FA_HEAD_GROUP"); return v != nullptr ? atoi(v) : 0; }();
   if (group_env > 0) return group_env;
   if (!causal) return 1;
   const double all = (double)B * H, mb = Sk * (2. * HD * 2 / (1 << 20));  // heads, and MB of K and V of each
   const bool alike = Sq == Sk && ((long long)Sq + BM - 1) / BM == 3;
+  const ixb_devinfo* dev = ixb_host::current_device();
+  if (dev != nullptr && ((long long)Sq + BM * NQ - 1) / (BM * NQ) * all <= dev->sm_count) return 8;
   const double groups = alike ? ceil(all / 8) : all * mb <= 96 ? 1 : ceil(all / (mb < 5 ? floor(40 / mb) : 8));
   return (int)ceil(all / groups);
 }

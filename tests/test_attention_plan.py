@@ -49,6 +49,12 @@ def test_forced_sizes(value, blocks):
 
 
 @pytest.mark.gpu
+def test_heads_whose_blocks_all_run_at_once(cuda):
+    assert heads_together(1, 32, 1024, 4096) == heads_together(4, 8, 1000, 3000) == 8
+    assert heads_together(1, 32, 2048, 2048) == 32
+
+
+@pytest.mark.gpu
 def test_clusters_of_every_size_are_taken(cuda):
     blocks = {(h, sq, sk): plan(1, h, sq, sk)[1] for h in (1, 16, 40, 112, 320) for sq, sk in ((1, 2879), (3, 300), (300, 700))}
     assert blocks[1, 1, 2879] == 8 and blocks[16, 1, 2879] == 4 and blocks[40, 1, 2879] == 2 and blocks[112, 1, 2879] == 1
