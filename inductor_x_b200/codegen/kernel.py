@@ -52,9 +52,10 @@ REDUCTION_OPS = {
 
 INT_REDUCTION_OPS = {"sum": "ISum", "prod": "IProd", "max": "IMax", "min": "IMin"}
 
-#: per-column operands hoisted out of the row loop at most (registers + shared memory)
+#: what a body may compute and still do next to nothing but move bytes (``_odd_rows``, ``_stream_threads``)
 _LIGHT_OPS = {"to_float", "add", "sub", "mul", "fma", "neg", "abs", "maximum", "minimum", "where", "imod", "idiv", "imod32", "idiv32"}
 _CTYPE_BYTES = {ctype: config_bytes(dtype) for dtype, ctype in CPP_TYPE.items()}
+#: per-column operands hoisted out of the row loop at most (registers + shared memory)
 MAX_CONSTS = 6
 #: streamed operands fetched one row ahead as raw 128-bit vectors
 MAX_STAGED = 2

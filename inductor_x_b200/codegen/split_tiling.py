@@ -100,11 +100,12 @@ def choose_row_config(rnumel: int, dtype: torch.dtype, rows: Optional[int] = Non
     vpt = target_vpt
     team = MIN_TEAM
     if exact and nvec < MIN_TEAM and nvec != 5:
-        # rows of a few vectors: no more lanes than hold one (two of six to eight), since the index
+        # rows of a few vectors: no more lanes than hold one (two of six and seven), since the index
         # arithmetic of a row is every lane's.  Teams of eight and these: sum of the rows of a permuted
         # 200 x 452 x 221 x 16 fp32 580 and 217 us, of 2^22 x 16 fp16 87 and 29, softmax of
-        # 300000 x 16 fp32 13.6 and 7.6, maximum of 2^20 x 48 bf16 25.5 and 19.6; five vectors on
-        # four lanes of two 4.7, on eight lanes 3.5 (50000 x 40 fp16)
+        # 300000 x 16 fp32 13.6 and 7.6, maximum of 2^20 x 48 bf16 25.5 and 19.6.  Five vectors stay on eight
+        # lanes, since measured the other way round: four lanes of two, of which one has a second vector, 4.7, eight
+        # lanes 3.5 (50000 x 40 fp16)
         team = 4 if nvec > 2 else 2
         vpt = 1 if nvec <= 4 else 2
     while team < MAX_TEAM and team * vpt < nvec:
