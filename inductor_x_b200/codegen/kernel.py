@@ -1209,11 +1209,20 @@ class B200Kernel(SIMDKernel):
                     line = 8000                                       # one value a row
                 else:
                     line = 1024 if v["indirect"] or len(pieces[id(v)]) > 2 else 4096 if len(pieces[id(v)]) == 2 else 32768
-                if not light:
-                    line = max(line, 16384) if line < 32768 else math.inf
-                if lb * self.vec >= line and (self.vec == 8 or line == 1024):
+                if self._row_walk_pays(lb, self.vec, line, light, self._numel_hint("x")):
                     return lb
         return None
+
+    @staticmethod
+    def _row_walk_pays(lb: int, vec: int, line: int, light: bool, numel: int) -> bool:
+        """The rule of ``_odd_rows`` for one load.  A few long rows of 16 bits are walked too: all their vectors are in
+        flight at once and either way takes what a small kernel takes (9 rows of 333 fp16: x with w 1.72 and 1.72 us, slices
+        1.51 and 1.58, x * c 1.63 and 1.75; 40 rows 1.57 and 1.92)."""
+        if light and vec == 8 and lb >= 256 and numel <= 4096:
+            return True
+        if not light:
+            line = max(line, 16384) if line < 32768 else math.inf
+        return lb * vec >= line and (vec == 8 or line == 1024)
 
     def _row_text(self, v, lb: int):
         """How a load reads inside rows of lb elements: one value, a run, or (None) element by element."""
@@ -1243,7 +1252,7 @@ class B200Kernel(SIMDKernel):
             return None
         if not all(v["dtype"] in (torch.float32, torch.float16, torch.bfloat16) for v in tl.values()):
             return None
-        if not self._smem_pays(lb, lc, order is not None, min(config_bytes(v["dtype"]) for v in tl.values())):
+        if not self._smem_pays(lb, lc, order is not None, min(config_bytes(v["dtype"]) for v in tl.values()), self._numel_hint("x")):
             return None
         xsym = self._root("x").symbol()
         strides = []
@@ -1262,8 +1271,9 @@ class B200Kernel(SIMDKernel):
         return lb, dc, lc, nk, (16 * per - (per - 1)) // 4 * 4, strides
 
     @staticmethod
-    def _smem_pays(lb: int, lc: int, ordered: bool, size: int) -> bool:
-        """Whether a transpose goes by way of shared memory: output rows of lb elements of `size` bytes, source rows of lc.
+    def _smem_pays(lb: int, lc: int, ordered: bool, size: int, numel: int) -> bool:
+        """Whether a transpose goes by way of shared memory: output rows of lb elements of `size` bytes, source rows of lc,
+        numel in all.
 
         The other way is a gather an element.  Where the lanes can be `ordered` along the source rows it reads whole
         sectors, and only long source rows are better off here: gathers and this, 2^23 elements, us, 40 x 64
@@ -1274,11 +1284,13 @@ class B200Kernel(SIMDKernel):
         a boundary, whose ends are parts of vectors, from longer ones on: 33 x 64 fp16 and one more operand 18.5 and 23.2,
         65 x 128 23.2 and 20.1, 65 x 128 fp32 26.2 and 29.5, 127 x 72 30.8 and 20.6.  If not, L1 serves the
         gathers until the output rows are long: 65 x 65 fp16 13.8 and 19.1, 129 x 129 13.7 and 17.9, 160 x 201 12.6 and
-        9.6, 200 x 201 14.3 and 8.6; 65 x 65 fp32 15.6 and 30.6, 127 x 127 17.9 and 22.3, 160 x 127 19.4 and 13.4."""
+        9.6, 200 x 201 14.3 and 8.6; 65 x 65 fp32 15.6 and 30.6, 127 x 127 17.9 and 22.3, 160 x 127 19.4 and 13.4.  One or
+        two tiles of 64 elements a row and more stay here: the kernel takes 1.5 us longer (2 x 65 x 59 fp16 1.9 and 3.4), which
+        lies under the host's part of a compiled call, 15 us and more either way."""
         if ordered:
             return lb >= 40 and lc >= 96
         if lc * size % 16:
-            return lb >= 160
+            return lb >= 160 or (lb >= 64 and numel <= 8192)
         return lb * lc * size > 6144 and (lb * size % 16 == 0 or lb >= (64 if size == 2 else 96))
 
     def _stream_threads(self, body_text: str, kc) -> int:
