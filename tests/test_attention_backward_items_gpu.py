@@ -36,3 +36,11 @@ def test_many_items(cuda, B, H, Sq, Sk, causal, dtype):
     for a, want in zip(got, torch.autograd.grad(ref, leaves, dy.double())):
         error = (a.double() - want).flatten(2).norm(dim=-1) / want.flatten(2).norm(dim=-1)
         assert float(error.max()) <= bound
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,causal,dtype", [
+    (5, 32, 136, 136, True, torch.bfloat16), (4, 40, 60, 200, True, torch.float16), (7, 23, 260, 129, False, torch.float16)])
+def test_many_items_without_scratch(cuda, monkeypatch, B, H, Sq, Sk, causal, dtype):
+    """dK/dV blocks that keep no dS and take over items all the same."""
+    monkeypatch.setattr(ops, "SCORE_GRADIENT_BYTES", 0)
+    test_many_items(cuda, B, H, Sq, Sk, causal, dtype)

@@ -25,6 +25,20 @@ def test_roles_wait_for_what_they_started(source, kernel):
         assert "await_copies<2>(next_full, asked)" in body
 
 
+@pytest.mark.parametrize("source,kernel", [("fa_split.cu", "fa_split_kernel"), ("fa_bwd.cu", "fa_bwd_dq_ds_kernel")])
+def test_roles_with_a_barrier_for_each_slot_do_too(source, kernel):
+    with open(os.path.join(CSRC, source)) as f:
+        text = f.read()
+    body = text[re.search(rf"\b{kernel}\(const __grid_constant__", text).end():]
+    body = body[:body.index("\n}\n")]
+    loaded = set(re.findall(r"mbar_arrive_expect_tx\(&(\w+)", body))
+    awaited = set(re.findall(r"await_copies<\w+>\(&?(\w+)(?:\[\w+\])?, ", body))
+    assert loaded and loaded <= awaited
+    assert body.count("await_products(&drained)") == 1 and "mbar_init(&drained, 1)" in body
+    if "request_next_block(" in body:
+        assert "await_copies<2>(next_full, asked)" in body
+
+
 def test_these_waits_are_bounded_and_ignore_the_abort_flag():
     with open(os.path.join(CSRC, "ixb", "tcgen05.cuh")) as f:
         text = f.read()

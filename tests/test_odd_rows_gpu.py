@@ -49,3 +49,25 @@ def test_operands_of_rows(cuda):
     out = buf[33:33 + x.numel()].view(x.shape)   # results off a boundary, in a larger buffer
     compiled(lambda x, w, out: out.copy_(torch.maximum(x, w)), x, w, out)
     assert torch.equal(out, torch.maximum(x, w)) and bool((buf[:33] == 7).all()) and bool((buf[33 + x.numel():] == 7).all())
+
+
+# whole numbers: the sums are exact in any order
+@pytest.mark.parametrize("dtype,cols", [(torch.float32, 333), (torch.bfloat16, 2053)])
+def test_rows_beside_masked_loads_and_atomic_sums(cuda, dtype, cols):
+    from torch._inductor.utils import run_and_get_code
+
+    g = torch.Generator(device=cuda).manual_seed(cols)
+    t, y = (torch.randint(-4, 5, (n, c), generator=g, device=cuda).to(dtype) for n, c in ((61, cols), (77, cols - 3)))
+    i, j = (torch.randint(0, n, (77,), generator=g, device=cuda) for n in (61, 9))
+
+    def padded(t, i, y):
+        return torch.maximum(t[i], torch.nn.functional.pad(y, (3, 0)))
+
+    def summed(t, i, j):
+        return torch.zeros(9, cols, device=t.device, dtype=torch.float32).index_add(0, j, t[i].float())
+
+    for fn, args in ((summed, (t, i, j)), (padded, (t, i, y)))[:1 if cols == 333 else 2]:   # (short rows beside a mask are not)
+        torch._dynamo.reset()
+        got, code = run_and_get_code(torch.compile(fn, dynamic=False), *args)
+        assert torch.equal(got, fn(*args))
+        assert f"launch_pointwise_rows<Body, {cols}>" in "\n".join(code)

@@ -52,6 +52,12 @@ def test_rows_of_a_few_vectors(cuda, d):
         assert float((y.double() - torch.softmax(x.double(), -1)).abs().max()) <= 1e-6
 
 
+# 7 and 8 vectors of four: four lanes of two, and a team of eight
+@pytest.mark.parametrize("d", [28, 32])
+def test_rows_of_seven_and_eight_vectors(cuda, d):
+    test_rows_of_a_few_vectors(cuda, d)
+
+
 # steps of the reduced axis around those of a warp's thread rows (8, 4, 2 and 1 of them) and of a batch of
 # four, tiles enough for a warp each
 @pytest.mark.parametrize("dtype,r,d", [(torch.bfloat16, 2, 32), (torch.bfloat16, 33, 32), (torch.float16, 26, 128), (torch.float32, 9, 100)])
