@@ -89,3 +89,10 @@ def test_transposes_by_shared_memory(source, b, c, dtype, shared):
 def test_digits_by_a_power_of_two_keep_64_bits(source):
     for n, bits in ((4, ""), (8, ""), (12, "32")):
         assert f"idiv{bits}(xindex, {n}LL)" in source(lambda x, r: x * r, ((999, n), F32), ((999, 1), F32))
+
+
+def test_small_calls(source):
+    for shape, shared in (((2, 65, 59), True), ((3, 65, 59), False), ((2, 63, 59), False)):
+        assert ("launch_pointwise_smem" in source(lambda x: (x.transpose(1, 2) + 1).contiguous(), (shape, F16))) == shared, shape
+    for rows, n, dtype, walked in ((9, 333, F16, True), (13, 333, F16, False), (9, 333, F32, False), (9, 255, F16, False)):
+        assert ("launch_pointwise_rows" in source(lambda x, w: torch.maximum(x, w), ((rows, n), dtype), ((n,), dtype))) == walked, (rows, n)
